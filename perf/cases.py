@@ -144,3 +144,15 @@ def tolerance(case):
     # narrowed to TF32 (10 stored mantissa bits, truncated) give 6.9e-4 whatever the contracted extent, the worst
     # single value 2.2e-3.
     return {"rel": 1e-14, "max": 1e-13} if case["f64"] else {"rel": 2.8e-3, "max": 1e-2}
+
+
+def exact(case, seed):
+    """The same contraction by torch.einsum in 64 bits; column-major tensors are row-major ones with their modes reversed."""
+    dtype = torch.float64 if case["f64"] else torch.float32
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    e = _extent(case)
+    a, b, c = (torch.empty(_count(case, t), dtype=dtype, device="cuda").uniform_(-1.0, 1.0, generator=g).double()
+               .reshape([e[m] for m in reversed(case[t])]) for t in "ABC")
+    out = torch.einsum("%s,%s->%s" % (case["A"][::-1], case["B"][::-1], case["C"][::-1]), a, b)
+    return (case["alpha"] * out + case["beta"] * c).reshape(-1)
