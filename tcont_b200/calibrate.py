@@ -69,20 +69,17 @@ def calibrate() -> dict:
     gemm = (("ab", "ka", "kb"), dict(a=8192, b=8192, k=4096))
     table["umma_tf32_tflops"], k = _rate(tc, api, torch, *gemm, F32)
     assert k == "umma_tf32", k
-    table["simt_f32_tflops"], _ = _rate(tc, api, torch, ("ab", "ka", "kb"), dict(a=4096, b=4096, k=1024), F32, env={"TCONT_KERNEL": "simt"})
     gemm64 = (("ab", "ak", "kb"), dict(a=4096, b=4096, k=2048))
     table["dmma_f64_tflops"], k = _rate(tc, api, torch, *gemm64, F64)
     assert k == "dmma_f64_tma", k
-    table["dmma_f64_gather_tflops"], k = _rate(tc, api, torch, *gemm64, F64, env={"TCONT_KERNEL": "gather"})
-    assert k == "dmma_f64", k
-    # one operand whose stride-1 mode leads neither its rows nor the contracted modes: 8-byte gathers
-    table["dmma_f64_gather8_tflops"], k = _rate(tc, api, torch, ("abc", "akc", "kb"), dict(a=2, b=2048, c=2048, k=2048), F64,
-                                                env={"TCONT_KERNEL": "gather"})
-    assert k == "dmma_f64", k
-    table["dmma_f64_gather_narrow_tflops"], k = _rate(tc, api, torch, ("abc", "dca", "bd"), dict(a=312, b=24, c=296, d=312), F64,
-                                                      env={"TCONT_KERNEL": "gather"})
-    assert k == "dmma_f64", k
-    table["simt_f64_tflops"], _ = _rate(tc, api, torch, ("ab", "ak", "bk"), dict(a=4096, b=4096, k=1024), F64, env={"TCONT_KERNEL": "simt"})
+    # gather kernel, per tile shape: rate with every SM busy, and the time one block takes per k tile of 16 on its own
+    for name, scalar, tiles in (("f64", F64, ((64, 64), (128, 32), (32, 32))), ("f32", F32, ((64, 64), (128, 32), (32, 32), (128, 128)))):
+        for t, (bm, bn) in enumerate(tiles):
+            env = {"TCONT_KERNEL": "gather" if scalar == F64 else "simt", "TCONT_GATHER_TILE": str(t), "TCONT_GATHER_CLUSTER": "1"}
+            table[f"gather_{name}_tflops_{t}"], k = _rate(tc, api, torch, ("ab", "ak", "kb"), dict(a=4096, b=4096, k=1024), scalar, env=env)
+            assert k in ("dmma_f64", "simt"), k
+            alone, _ = _rate(tc, api, torch, ("ab", "ak", "kb"), dict(a=bm, b=bn, k=32768), scalar, env=env)
+            table[f"gather_{name}_iter_us_{t}"] = 2.0 * bm * bn * 16 / (alone * 1e6)
     # scattered stores of the TMA-fed kernels: two contractions of the same size with a short contracted
     # extent, one whose tile rows run along C's stride-1 mode and one whose rows do not (every element of C
     # stored on its own); the time of the second per element of C
@@ -91,7 +88,7 @@ def calibrate() -> dict:
     size_c = 30 * 16 * 16 * 24 * 16 * 16
     flops6 = 2.0 * size_c * 24
     for key, scalar in (("scatter_store_ps", F64), ("scatter_store_f32_ps", F32)):
-        # (FP64: the planner itself would send the second one to the CUDA cores, which is what this figure is for)
+        # (FP64: the planner itself would send the second one elsewhere, which is what this figure is for)
         env = {"TCONT_KERNEL": "tma"} if scalar == F64 else None
         _, k1 = _rate(tc, api, torch, ("abcdef", "degb", "gfac"), ext6, scalar, env=env)
         t_scat, k2 = _rate(tc, api, torch, ("abcdef", "dega", "gfbc"), ext6, scalar, env=env)

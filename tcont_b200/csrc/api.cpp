@@ -143,9 +143,7 @@ struct tcontb_run {
     // parts share (borrowed_tA / borrowed_tB: that part's scratch; this run then neither allocates nor transposes).
     const void *borrowed_tA = nullptr, *borrowed_tB = nullptr;
     TransposeParams tpA{}, tpB{};
-    // SIMT tables
-    DeviceBuffer tables;
-    SimtParams simt{};
+    GatherParams gather{};
     // UMMA
     UmmaParams umma{};
     CUtensorMap tmA{}, tmB{};
@@ -313,6 +311,61 @@ tcontb_status encode_map(const UmmaOperand& o, const void* base, int elt, CUtens
     return TCONTB_OK;
 }
 
+// One digit of a mode group as the gather kernel splits it.
+void add_digit(RadixGroup* g, int64_t extent, int64_t x, int64_t y)
+{
+    const int d = g->n++;
+    g->ext[d] = make_fast_div(extent);
+    g->sx[d] = x;
+    g->sy[d] = y;
+}
+
+void fill_gather(const Problem& p, const void* A, const void* B, void* C, const SimtSpec& simt, const GatherSpec& spec, GatherParams* out)
+{
+    GatherParams g{};
+    g.A = A;
+    g.B = B;
+    g.C = C;
+    g.M = spec.rows;
+    g.N = p.Ntot;
+    g.K = p.Ktot;
+    auto mode = [&](int id) -> const Mode& { return p.modes[static_cast<size_t>(id)]; };
+    // rows: C's order, so that stores run along memory; with cut modes their low digits first
+    int cut0 = -1, cut1 = -1;
+    if (spec.t0 > 0) {
+        cut0 = p.M[0];
+        cut1 = p.A[0];
+        const Mode &m0 = mode(cut0), &m1 = mode(cut1);
+        g.m.t0 = static_cast<uint32_t>(spec.t0);
+        g.m.t1 = static_cast<uint32_t>(spec.t1);
+        g.m.lim0 = static_cast<uint32_t>(m0.extent);
+        g.m.lim1 = static_cast<uint32_t>(m1.extent);
+        add_digit(&g.m, spec.t0, m0.sA, m0.sC);
+        add_digit(&g.m, spec.t1, m1.sA, m1.sC);
+        add_digit(&g.m, (m0.extent + spec.t0 - 1) / spec.t0, m0.sA * spec.t0, m0.sC * spec.t0);
+        add_digit(&g.m, (m1.extent + spec.t1 - 1) / spec.t1, m1.sA * spec.t1, m1.sC * spec.t1);
+    }
+    for (int id : p.M)
+        if (id != cut0 && id != cut1) add_digit(&g.m, mode(id).extent, mode(id).sA, mode(id).sC);
+    // columns: stores do not care about their order, gathers do: B's stride-1 mode first where it is one of them
+    const int first_n = !p.B.empty() && mode(p.B[0]).group == GROUP_N ? p.B[0] : -1;
+    if (first_n >= 0) add_digit(&g.n, mode(first_n).extent, mode(first_n).sB, mode(first_n).sC);
+    for (int id : p.N)
+        if (id != first_n) add_digit(&g.n, mode(id).extent, mode(id).sB, mode(id).sC);
+    for (int id : p.K) add_digit(&g.k, mode(id).extent, mode(id).sA, mode(id).sB);
+    for (RadixGroup* r : {&g.m, &g.n, &g.k})
+        if (r->n == 0) add_digit(r, 1, 0, 0);   // no mode of this kind: one element
+    g.m.wide = g.M >= (int64_t(1) << 31) ? 1 : 0;
+    g.n.wide = g.N >= (int64_t(1) << 31) ? 1 : 0;
+    g.k.wide = g.K >= (int64_t(1) << 31) ? 1 : 0;
+    g.a_along_k = simt.a_load_along_k;
+    g.b_along_k = simt.b_load_along_k;
+    g.cluster = spec.cluster;
+    g.flat = spec.flat ? 1 : 0;
+    g.alpha = 1.0;
+    *out = g;
+}
+
 // Device-side set-up shared by the three run constructors; dL/dR/dC must already be set.
 tcontb_status finish_run(tcontb_run* run)
 {
@@ -441,60 +494,8 @@ tcontb_status finish_run(tcontb_run* run)
         if (pl.kernel == KERNEL_UMMA_TF32) TC_CUDA(umma_tf32_configure());
         else TC_CUDA(dmma_tma_configure());
     } else {
-        OffsetTables t;
-        build_offset_tables(p, &t);
-        const size_t n = t.offAm.size() + t.offAk.size() + t.offBn.size() + t.offBk.size() + t.offCm.size() + t.offCn.size();
-        std::vector<int64_t> flat;
-        flat.reserve(n);
-        size_t o[6];
-        const std::vector<int64_t>* src[6] = {&t.offAm, &t.offAk, &t.offBn, &t.offBk, &t.offCm, &t.offCn};
-        for (int i = 0; i < 6; ++i) {
-            o[i] = flat.size();
-            flat.insert(flat.end(), src[i]->begin(), src[i]->end());
-        }
-        TC_CUDA(run->tables.alloc(n * sizeof(int64_t)));
-        TC_CUDA(cudaMemcpy(run->tables.ptr, flat.data(), n * sizeof(int64_t), cudaMemcpyHostToDevice));
-        const int64_t* base = static_cast<const int64_t*>(run->tables.ptr);
-        run->simt.A = kA;
-        run->simt.B = kB;
-        run->simt.C = run->dC;
-        run->simt.M = p.Mtot;
-        run->simt.N = p.Ntot;
-        run->simt.K = p.Ktot;
-        run->simt.offAm = base + o[0];
-        run->simt.offAk = base + o[1];
-        run->simt.offBn = base + o[2];
-        run->simt.offBk = base + o[3];
-        run->simt.offCm = base + o[4];
-        run->simt.offCn = base + o[5];
-        run->simt.a_along_k = pl.simt.a_load_along_k;
-        run->simt.b_along_k = pl.simt.b_load_along_k;
-        if (pl.kernel == KERNEL_DMMA_F64) {
-            TC_CUDA(dmma_configure_all());
-            // 16-byte gathers: rows 2r and 2r+1 of the tile must be neighbours in memory, on a
-            // 16-byte boundary, for every contracted index.
-            auto pairs_ok = [](const std::vector<int64_t>& row, const std::vector<int64_t>& k) {
-                if (row.size() % 2) return false;
-                for (size_t r = 0; r < row.size(); r += 2)
-                    if ((row[r] & 1) || row[r + 1] != row[r] + 1) return false;
-                for (int64_t v : k)
-                    if (v & 1) return false;
-                return true;
-            };
-            // K-major operand: neighbouring k neighbours in memory, every row offset even
-            auto kpairs_ok = [](const std::vector<int64_t>& row, const std::vector<int64_t>& k) {
-                if (k.size() % 2) return false;
-                for (size_t i = 0; i < k.size(); i += 2)
-                    if ((k[i] & 1) || k[i + 1] != k[i] + 1) return false;
-                for (int64_t v : row)
-                    if (v & 1) return false;
-                return true;
-            };
-            if (run->simt.a_along_k == 1 && kpairs_ok(t.offAm, t.offAk) && reinterpret_cast<uintptr_t>(kA) % 16 == 0) run->simt.a_along_k = 3;
-            if (run->simt.b_along_k == 1 && kpairs_ok(t.offBn, t.offBk) && reinterpret_cast<uintptr_t>(kB) % 16 == 0) run->simt.b_along_k = 3;
-            if (run->simt.a_along_k == 0 && pairs_ok(t.offAm, t.offAk) && reinterpret_cast<uintptr_t>(kA) % 16 == 0) run->simt.a_along_k = 2;
-            if (run->simt.b_along_k == 0 && pairs_ok(t.offBn, t.offBk) && reinterpret_cast<uintptr_t>(kB) % 16 == 0) run->simt.b_along_k = 2;
-        }
+        fill_gather(p, kA, kB, run->dC, pl.simt, pl.gather, &run->gather);
+        TC_CUDA(gather_configure());
     }
     const char* st_env = std::getenv("TCONT_STAGE_TIMES");
     run->stage_timing = st_env && std::strcmp(st_env, "1") == 0;
@@ -939,6 +940,9 @@ tcontb_status tcontb_run_upload_inputs(tcontb_run* run, const void* a_host, cons
     return TCONTB_OK;
 }
 
+// The gather kernel applies alpha and beta itself.
+static bool gathers(const Plan& pl) { return pl.kernel == KERNEL_SIMT || pl.kernel == KERNEL_DMMA_F64; }
+
 tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
 {
     if (!run) return fail(TCONTB_INVALID_ARGUMENT, "ExecutionRun is empty");
@@ -946,12 +950,12 @@ tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
     TC_NOT_SHARDED(run, "alpha and beta");
     const bool scaled = alpha != 1.0 || beta != 0.0;
     if (scaled && run->plan.prob.c_strided) return fail(TCONTB_UNSUPPORTED, "alpha and beta are not available when C is a sub-tensor view");
-    if (scaled && !run->splitk.ptr && !run->scaled_ws.ptr) {
+    if (scaled && !run->splitk.ptr && !run->scaled_ws.ptr && !gathers(run->plan)) {
         // allocated here, once, so that launches stay free of allocations
         TC_CUDA(run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt));
     }
     const bool was = run->alpha != 1.0 || run->beta != 0.0;
-    if (!run->splitk.ptr) run->kernels_per_launch += (scaled ? 1 : 0) - (was ? 1 : 0);
+    if (!run->splitk.ptr && !gathers(run->plan)) run->kernels_per_launch += (scaled ? 1 : 0) - (was ? 1 : 0);
     run->alpha = alpha;
     run->beta = beta;
     // the parts of a pipelined host-buffer pass work on ranges of this run's C
@@ -1002,13 +1006,11 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
     const bool t = run->stage_timing;
     // Other scalars than (1, 0): the kernel writes the workspace instead of C (a split-K run does anyway)
     const bool scaled = run->alpha != 1.0 || run->beta != 0.0;
-    const bool redirect = scaled && !run->splitk.ptr;
+    const bool redirect = scaled && !run->splitk.ptr && !gathers(pl);
     UmmaParams umma = run->umma;
-    SimtParams simt = run->simt;
     if (redirect) {
         umma.C = static_cast<float*>(run->scaled_ws.ptr);
         umma.C64 = static_cast<double*>(run->scaled_ws.ptr);
-        simt.C = run->scaled_ws.ptr;
     }
     if (t) TC_CUDA(cudaEventRecord(run->ev[0], run->stream));
     if (pl.tA.needed && !run->borrowed_tA) TC_CUDA(launch_transpose(run->roleA_src(), run->tbufA.ptr, run->tpA, static_cast<int>(run->elt), run->stream));
@@ -1046,10 +1048,13 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
     }
     else if (pl.kernel == KERNEL_DMMA_F64_TMA)
         TC_CUDA(launch_dmma_tma(umma, &run->tmA, &run->tmB, pl.umma.smem_bytes, run->num_sms, run->stream));
-    else if (pl.kernel == KERNEL_DMMA_F64)
-        TC_CUDA(launch_dmma_contract(simt, run->num_sms, run->stream));
-    else
-        TC_CUDA(launch_simt_contract(simt, pl.scalar_type, run->stream));
+    else {
+        GatherParams g = run->gather;
+        g.scaled = scaled ? 1 : 0;
+        g.alpha = run->alpha;
+        g.beta = run->beta;
+        TC_CUDA(launch_gather_contract(g, pl.scalar_type, pl.gather.tile, run->num_sms, run->stream));
+    }
     if (run->splitk.ptr)
         TC_CUDA(launch_splitk_reduce(run->splitk.ptr, run->dC, pl.sizeC, pl.umma.k_splits * (run->tf32x3 ? 3 : 1), pl.sizeC,
                                      static_cast<int>(run->elt), run->stream, run->alpha, run->beta));

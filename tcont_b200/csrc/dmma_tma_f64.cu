@@ -1,7 +1,7 @@
 // dmma_tma_f64.cu -- FP64 direct contraction: TMA-staged operand tiles feeding mma.sync m8n8k4.
 //
 // tcgen05 has no FP64 kind, so the arithmetic is warp-level DMMA (37.0 TFLOP/s measured on B200).
-// What the gather kernel (dmma_f64.cu) spends on address arithmetic is done here by the copy
+// What the gather kernel (gather_contract.cu) spends on address arithmetic is done here by the copy
 // engine: the planner's slab machinery, the same as for the tcgen05 kernel but with 16 doubles per
 // 128-byte row, describes every operand tile as a few multi-mode TMA boxes.
 //

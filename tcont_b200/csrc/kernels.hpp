@@ -21,13 +21,55 @@ struct SimtParams {
     const int64_t* offBk;
     const int64_t* offCm;
     const int64_t* offCn;
-    int a_along_k, b_along_k;  // 0: threads run along the rows, 1: along k, 2 / 3 (FP64 tensor kernel only): along the rows / along k, two at a time
+    int a_along_k, b_along_k;  // 0: threads run along the rows, 1: along k
 };
 cudaError_t launch_simt_contract(const SimtParams& p, int scalar_type, cudaStream_t stream);
 
-// ---- FP64 tensor-core contraction (dmma_f64.cu), same GEMM view ----------------------------
-cudaError_t launch_dmma_contract(const SimtParams& p, int num_sms, cudaStream_t stream);
-cudaError_t dmma_configure_all();  // once per device before the first launch
+// Division by a number known before the launch: n / d = (umulhi(n, mul) + n) >> shr for n < 2^31, with shr = ceil(log2 d)
+// and mul = floor(2^32 (2^shr - d) / d) + 1.  Five instructions where the hardware-less integer division takes thirty.
+struct FastDiv {
+    uint32_t d, mul, shr;
+};
+inline FastDiv make_fast_div(int64_t d)
+{
+    FastDiv f;
+    f.d = static_cast<uint32_t>(d);
+    f.shr = 0;
+    while ((uint64_t(1) << f.shr) < f.d) ++f.shr;
+    f.mul = static_cast<uint32_t>((((uint64_t(1) << f.shr) - f.d) << 32) / f.d + 1);
+    return f;
+}
+
+// ---- any descriptor, gathered operands (gather_contract.cu) -----------------------------------
+// A group of modes (rows, columns or contracted indices) of the GEMM view: flat index -> element offsets in the group's
+// two tensors.  rows: x = A, y = C; columns: x = B, y = C; contracted: x = A, y = B.
+constexpr int kMaxDigits = kMaxModes + 2;
+struct RadixGroup {
+    int n;     // modes (digits), fastest first, at least one
+    int wide;  // flat indices of 2^31 and more: 64-bit division
+    FastDiv ext[kMaxDigits];
+    long long sx[kMaxDigits], sy[kMaxDigits];
+    // Two modes cut in two digits each (rows whose stride-1 mode differs between A and C): digit 0 and t0 x digit 2 are one
+    // index, which must stay below lim0, digit 1 and t1 x digit 3 the other (lim1).  lim0 = 0: no mode is cut.
+    uint32_t t0, t1, lim0, lim1;
+};
+struct GatherParams {
+    const void* A;
+    const void* B;
+    void* C;
+    long long M, N, K;
+    RadixGroup m, n, k;
+    int a_along_k, b_along_k;  // 0: neighbouring threads gather neighbouring rows, 1: neighbouring k
+    int cluster;               // CTAs that share a tile, each a range of k (1: no split)
+    int flat;                  // 1: persistent blocks, one ring of stages across their tiles (cluster 1 only)
+    int scaled;                // 0: C = A B; 1: C = alpha A B + beta C (C read only when beta is not zero)
+    double alpha, beta;
+    long long k_per_cta;       // the rest is filled in by the launcher
+    uint32_t tiles_m, tiles_n;
+    int raster_group;
+};
+cudaError_t gather_configure();  // once per device before the first launch
+cudaError_t launch_gather_contract(const GatherParams& p, int scalar_type, int tile, int num_sms, cudaStream_t stream);
 
 // ---- tensor permutation (transpose.cu) ------------------------------------------------------
 struct TransposeParams {

@@ -407,7 +407,7 @@ bool chunk_kmajor(UmmaOperand* o, int BK, int cta_slabs)
     return true;
 }
 
-void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int bk_request)
+void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int bk_request, bool fuse_rows)
 {
     u->eligible = false;
     const bool f64 = p_in.scalar_type == 1;
@@ -418,13 +418,18 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
     // empty rows, and the table builder splits a row's position back into the two C modes.
     Problem p = p_in;
     int64_t split_inner[2] = {0, 0}, split_outer_cstride[2] = {0, 0};
-    if (f64 && !std::getenv("TCONT_NO_ROW_FUSION")) {
+    if (fuse_rows && !std::getenv("TCONT_NO_ROW_FUSION")) {
         for (int which = 0; which < 2; ++which) {
             std::vector<int>& t = which == 0 ? p.A : p.B;
             std::vector<int>& rows = which == 0 ? p.M : p.N;
-            if (t.size() < 3 || rows.size() < 2 || t[0] != rows[0] || t[1] != rows[1]) continue;
-            const Mode m0 = p.modes[static_cast<size_t>(t[0])], m1 = p.modes[static_cast<size_t>(t[1])];
-            if (slab_padding_f64(m0.extent) <= 1.08) continue;
+            if (t.size() < 3 || rows.size() < 2) continue;
+            const int at = index_of(t, rows[0]);
+            if (at < 0 || at + 1 >= static_cast<int>(t.size()) || t[static_cast<size_t>(at) + 1] != rows[1]) continue;
+            if (f64 && at != 0) continue;
+            const Mode m0 = p.modes[static_cast<size_t>(rows[0])], m1 = p.modes[static_cast<size_t>(rows[1])];
+            if (f64 ? slab_padding_f64(m0.extent) <= 1.08
+                    : at == 0 ? double(ceil_div(m0.extent, 32) * 32) <= 1.08 * double(m0.extent)
+                              : p.modes[static_cast<size_t>(t[0])].group != GROUP_K || m0.extent % 128 == 0) continue;
             if ((which == 0 ? m1.sA : m1.sB) != (which == 0 ? m0.sA : m0.sB) * m0.extent) continue;  // (a view with a gap between them)
             Mode f;
             f.names = m0.names + m1.names;
@@ -437,8 +442,8 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
             p.modes.push_back(f);
             split_inner[which] = m0.extent;
             split_outer_cstride[which] = m1.sC;
-            t[0] = id;
-            t.erase(t.begin() + 1);
+            t[static_cast<size_t>(at)] = id;
+            t.erase(t.begin() + at + 1);
             rows[0] = id;
             rows.erase(rows.begin() + 1);
         }
@@ -710,18 +715,23 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
 // 32-wide chunk on one CTA per tile.  TCONT_UMMA_BK=32 and TCONT_UMMA_PAIR=0 keep the second form.
 void plan_umma(const Problem& p, const CostTable& cost, UmmaSpec* u)
 {
-    const char* bk = std::getenv("TCONT_UMMA_BK");
-    const char* pr = std::getenv("TCONT_UMMA_PAIR");
-    if (p.scalar_type != 1 && !(bk && std::atoi(bk) == 32) && !(pr && pr[0] == '0')) {
-        UmmaSpec v;
-        plan_umma_impl(p, cost, &v, 64);
-        if (v.eligible && v.BK == 64) {
-            *u = v;
-            return;
+    if (p.scalar_type != 1) {
+        const char* bk = std::getenv("TCONT_UMMA_BK");
+        const char* pr = std::getenv("TCONT_UMMA_PAIR");
+        if (!(bk && std::atoi(bk) == 32) && !(pr && pr[0] == '0')) {
+            UmmaSpec v;
+            plan_umma_impl(p, cost, &v, 64, false);
+            if (v.eligible && v.BK == 64) {
+                *u = v;
+                return;
+            }
         }
+        *u = UmmaSpec();
+        plan_umma_impl(p, cost, u, 32, false);
+        return;
     }
     *u = UmmaSpec();
-    plan_umma_impl(p, cost, u, 32);
+    plan_umma_impl(p, cost, u, 32, true);
 }
 
 std::string perm_modes(const Problem& p, const std::vector<int>& ids)
@@ -755,32 +765,97 @@ double wave_efficiency(int64_t tiles, int sms)
     return double(t) / double(ceil_div(t, sms) * sms);
 }
 
-// The gather kernel fetches 16 bytes per load when the stride-1 mode of an operand is the first row
-// mode of its tile (C's order) or the first contracted mode, and has an even extent; else 8 bytes.
-bool gathers_16_bytes(const Problem& p)
+// Tile, cluster and form of the gather kernel: the smallest estimate over its tile shapes and 1, 2, 4, 8 or 16 CTAs per tile.
+// CTAs spread evenly over the SMs; the CTAs an SM holds pass their k tiles together at the rate of a full GPU
+// (throughput), but none faster than one alone (latency), which is what bounds small problems and what a split of k
+// shortens.  Measured on 60 contractions of 2 MFLOP to 280 GFLOP with every tile, cluster and form: the choice is within
+// 11 % of the best one on average.
+GatherSpec plan_gather(const Problem& p, const CostTable& c)
 {
-    auto ok = [&](const std::vector<int>& t, const std::vector<int>& rows) {
-        if (t.empty()) return false;
-        const Mode& m = p.modes[static_cast<size_t>(t[0])];
-        const bool lead = (!rows.empty() && t[0] == rows[0]) || (!p.K.empty() && t[0] == p.K[0]);
-        return lead && m.extent % 2 == 0;
-    };
-    return ok(p.A, p.M) && ok(p.B, p.N);
+    const bool f64 = p.scalar_type == 1;
+    static const int kTile64[3][3] = {{64, 64, 3}, {128, 32, 2}, {32, 32, 4}};   // BM, BN, CTAs per SM
+    static const int kTile32[4][3] = {{64, 64, 4}, {128, 32, 4}, {32, 32, 4}, {128, 128, 2}};
+    const auto* kTile = f64 ? kTile64 : kTile32;
+    const double elt = f64 ? 8.0 : 4.0;
+    GatherSpec best;
+    best.est_us = 1e300;
+    // FP64 sums of this length are off by close to 1e-14 of their norm as one chain of FMAs, and by a fifth of that when cut
+    // into ranges: they stay one chain, so that results do not move by more than 1e-14 with the route.
+    const bool one_chain = f64 && p.Ktot > 49152;
+    const char* force_tile = std::getenv("TCONT_GATHER_TILE");        // tuning switches: 0..3, 1..16
+    const char* force_cluster = std::getenv("TCONT_GATHER_CLUSTER");
+    const char* force_flat = std::getenv("TCONT_GATHER_FLAT");
+    for (int t : {GATHER_BIG, GATHER_SQUARE, GATHER_TALL, GATHER_SMALL}) {   // (of equal estimates the larger tile)
+        if (f64 && t == GATHER_BIG) continue;
+        if (force_tile && std::atoi(force_tile) != t && std::atoi(force_tile) < (f64 ? 3 : 4)) continue;
+        const int64_t bm = kTile[t][0], bn = kTile[t][1];
+        GatherSpec g;
+        g.tile = t;
+        g.rows = p.Mtot;
+        // A's stride-1 mode is a row mode, but not C's: a tile of t0 x t1 indices of the two lets both gathers and stores
+        // run along memory.  Where C is the larger tensor, t0 = 32 keeps whole 128-byte (256-byte) runs of it; else the
+        // least padded shape with 8 elements or more a side.
+        if (p.A[0] != p.M[0] && p.modes[static_cast<size_t>(p.A[0])].group == GROUP_M && p.modes[static_cast<size_t>(p.M[0])].sC == 1) {
+            const int64_t e0 = p.modes[static_cast<size_t>(p.M[0])].extent, e1 = p.modes[static_cast<size_t>(p.A[0])].extent;
+            const int64_t rest = p.Mtot / e0 / e1;
+            const bool c_larger = p.sizeC > p.sizeA;
+            int64_t least = 0;
+            for (int64_t t0 : c_larger ? std::vector<int64_t>{32} : std::vector<int64_t>{8, bm / 8, 16}) {
+                const int64_t t1 = bm / t0, rows = ceil_div(e0, t0) * t0 * ceil_div(e1, t1) * t1 * rest;
+                if (least == 0 || rows < least) {
+                    least = rows;
+                    g.t0 = static_cast<int>(t0);
+                    g.t1 = static_cast<int>(t1);
+                }
+            }
+            g.rows = least;
+            if (double(least) > (c_larger ? 1.1 : 1.5) * double(p.Mtot)) {   // short modes: rows in C's order after all
+                g.t0 = g.t1 = 0;
+                g.rows = p.Mtot;
+            }
+        }
+        const int64_t tiles_m = ceil_div(g.rows, bm), tiles_n = ceil_div(p.Ntot, bn);
+        if (tiles_m > (int64_t(1) << 31) / kMaxGatherCluster / tiles_n) { if (t != GATHER_SQUARE) continue; }
+        const double rate = f64 ? c.gather_f64_tflops[t] : c.gather_f32_tflops[t];
+        const double iter_us = f64 ? c.gather_f64_iter_us[t] : c.gather_f32_iter_us[t];
+        static const double kFixed[4] = {1.3, 1.7, 0.9, 1.7};   // set-up and stores of a tile, in units of gather_fixed_us
+        const double fixed_us = c.gather_fixed_us * kFixed[t];
+        const double sm_iter_us = 2.0 * double(bm) * double(bn) * 16.0 / (rate * 1e6 / c.num_sms);
+        for (int s = 1; s <= kMaxGatherCluster; s *= 2) {
+            if (force_cluster && std::atoi(force_cluster) != s) continue;
+            const int64_t k_tiles = ceil_div(p.Ktot, 16);
+            if (s > 1 && (one_chain || k_tiles < 2 * s || tiles_m * tiles_n * s > 8 * int64_t(c.num_sms))) break;
+            const double iters = double(ceil_div(k_tiles, s));
+            const int64_t per_sm = ceil_div(tiles_m * tiles_n * s, c.num_sms), resident = kTile[t][2];
+            auto round_us = [&](int64_t ctas) { return ctas ? iters * std::max(iter_us, double(ctas) * sm_iter_us) + fixed_us : 0.0; };
+            // Persistent CTAs where a CTA would otherwise be mostly set-up: more than one round of short k loops.  The small
+            // FP64 tile takes that form for up to four k tiles anyway, because it has no k groups to add up at its end.
+            const bool flat = s == 1 && (t == GATHER_SMALL ? one_chain || (f64 && iters <= 4) : per_sm > resident && iters <= 4);
+            double us = flat ? fixed_us + std::max(double(per_sm) * (iters * sm_iter_us + c.gather_tile_us), double(ceil_div(per_sm, resident)) * iters * iter_us)
+                             : double(per_sm / resident) * round_us(resident) + round_us(per_sm % resident);
+            if (s > 1) us += c.gather_reduce_us;
+            us = std::max(us, fixed_us + (double(p.sizeA) + double(p.sizeB) + double(p.sizeC)) * elt / (c.gather_gbs * 1e3));
+            if (g.t0 > 0) us *= 1.6;   // (short runs on both sides: 12 x 12 by 124 FP64, rows cut 4 x 8, 18 us where the rule said 11)
+            if (us < best.est_us) {
+                best = g;
+                best.cluster = s;
+                best.flat = flat;
+                if (force_flat) best.flat = s == 1 && force_flat[0] == '1';
+                best.est_us = us;
+            }
+        }
+    }
+    return best;
 }
 
 double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const CostTable& c)
 {
+    if (kernel == KERNEL_DMMA_F64 || kernel == KERNEL_SIMT) return c.launch_us + plan_gather(p, c).est_us;
     const double elt = p.scalar_type == 1 ? 8.0 : 4.0;
     const double flops = 2.0 * double(p.Mtot) * double(p.Ntot) * double(p.Ktot);
     double c_bytes = double(p.sizeC) * elt;
-    double rate = p.scalar_type == 1 ? c.simt_f64_tflops : c.simt_f32_tflops;
+    double rate = 0;
     double extra_us = 0, scatter_us = 0, extra_floor_us = 0;
-    // tiles are computed whole: the work of an FP64 kernel is that of the extents rounded up to its tile
-    auto padded = [&](int64_t bm, int64_t bn) {
-        return double(ceil_div(p.Mtot, bm) * bm) / double(p.Mtot) * double(ceil_div(p.Ntot, bn) * bn) / double(p.Ntot);
-    };
-    if (kernel == KERNEL_SIMT && p.scalar_type == 1)
-        rate *= wave_efficiency(ceil_div(p.Mtot, 64) * ceil_div(p.Ntot, 64), c.num_sms) / padded(64, 64);
     // TMA-fed kernels: slabs and k chunks are whole, ragged extents are zero-filled and multiplied anyway
     // (extents of 72 in 32-wide slabs and chunks: abcd-aefb-fdce ran at 138 TFLOP/s direct, 415 after a
     // transpose that fuses the ragged modes away)
@@ -788,9 +863,14 @@ double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const Cos
                                double(u.k_iters * u.BK) / double(p.Ktot);
     if ((kernel == KERNEL_DMMA_F64_TMA || kernel == KERNEL_UMMA_TF32) && u.k_splits > 1) {
         // partial tensors written, read back and summed by a second kernel
-        extra_us += c.launch_us + 2.0 * double(u.k_splits) * double(p.sizeC) * elt / (c.hbm_gbs * 1e3);
+        // (set up while the first kernel drains; partial tensors of up to half of L2 are read back from there)
+        const double partials = 2.0 * double(u.k_splits) * double(p.sizeC) * elt;
+        extra_us += 0.5 * c.launch_us + partials / (c.hbm_gbs * 1e3) * (partials < 128e6 ? 0.5 : 1.0);
     }
     if (kernel == KERNEL_DMMA_F64_TMA) {
+        // A 128 x 64 tile keeps the FP64 pipe busy for 1.05 us per k chunk of 16 (128 MMAs a warp) and takes 4.5 us to set up,
+        // fill and drain (M 192, N 384, K 52: 12 tiles in 15 us; M = N = 576, K 256 in four ranges: 21 us)
+        extra_floor_us = 4.5 + double(ceil_div(u.tiles_m * u.tiles_n * u.k_splits, c.num_sms)) * double(u.k_iters_per_split) * (u.BK == 16 ? 1.05 : 0.55) * u.BN / 64.0;
         rate = c.dmma_f64_tflops * wave_efficiency(u.tiles_m * u.tiles_n * u.k_splits, c.num_sms) / tma_padding;
         // Rows of a slab that are not contiguous in C are stored element by element
         // (abcdef-dega-gfbc: 37.7 M elements of C, 1.08 ms against 0.10 ms for its coalesced siblings).
@@ -798,15 +878,6 @@ double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const Cos
         // against 20.2 on the gather kernel, which sees those rows as one flat index)
         if ((u.a.row_elem_cstride != 1 && !u.store_across_slabs) || u.a.slab_mode_ext < 8)
             scatter_us = double(p.sizeC) * double(u.k_splits) * c.scatter_store_ps * 1e-6;
-    }
-    if (kernel == KERNEL_DMMA_F64) {
-        const int64_t bn = p.Ntot <= 48 ? 32 : 64, bm = p.Ntot <= 48 ? 256 : 128;
-        // Measured: 19 to 20 TFLOP/s with 16-byte gathers on both operands (abc-ad-bdc), 13 to 15 with
-        // one operand on 8-byte gathers (abcd-eafb-fdec), 3.5 to 4.4 on the 256 x 32 tiles for narrow N.
-        const double r = p.Ntot <= 48 ? c.dmma_f64_gather_narrow_tflops
-                                      : (gathers_16_bytes(p) ? c.dmma_f64_gather_tflops : c.dmma_f64_gather8_tflops);
-        rate = r *
-               wave_efficiency(ceil_div(p.Mtot, bm) * ceil_div(p.Ntot, bn), c.num_sms) / padded(bm, bn);
     }
     if (kernel == KERNEL_UMMA_TF32) {
         rate = c.umma_tf32_tflops * (1.0 - c.far_row_penalty * u.far_fraction) *
@@ -827,31 +898,26 @@ double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const Cos
     return c.launch_us + std::max({flops / (rate * 1e6), bytes / (c.hbm_gbs * 1e3), scatter_us, extra_floor_us}) + extra_us;
 }
 
-// TF32 goes to the tcgen05 kernel whenever its tiles can be described to TMA.  FP64 takes the
-// cheapest of the TMA-fed tensor-path kernel, the gather tensor-path kernel (needs a tile per SM)
-// and the 64 x 64 CUDA-core tiles, by the cost table.
+// TF32 goes to the tcgen05 kernel whenever its tiles can be described to TMA.  FP64 takes the cheaper of the TMA-fed kernel
+// and the gather kernel, by the cost table; Float32 that TMA cannot describe goes to the gather kernel.  The gather kernel
+// is reported as KERNEL_DMMA_F64 where FP64 work fills the GPU with tiles, as KERNEL_SIMT otherwise.
 int pick_kernel(const Problem& p, const UmmaSpec& u, const CostTable& c)
 {
     if (u.eligible && u.elt == 4) return KERNEL_UMMA_TF32;
     if (p.scalar_type != 1) return KERNEL_SIMT;
     const char* k = std::getenv("TCONT_KERNEL");
     if (k && std::strcmp(k, "simt") == 0) return KERNEL_SIMT;
-    if (k && std::strcmp(k, "tma") == 0 && u.eligible && u.elt == 8) return KERNEL_DMMA_F64_TMA;
-    int best = KERNEL_SIMT;
-    double best_us = contraction_us(p, KERNEL_SIMT, u, c);
-    const int64_t bn = p.Ntot <= 48 ? 32 : 64, bm = p.Ntot <= 48 ? 256 : 128;  // the gather kernel's smallest fitting tile
-    if (k && std::strcmp(k, "gather") == 0 && ceil_div(p.Mtot, bm) * ceil_div(p.Ntot, bn) >= c.num_sms) return KERNEL_DMMA_F64;
-    if (ceil_div(p.Mtot, bm) * ceil_div(p.Ntot, bn) >= c.num_sms) {
-        const double us = contraction_us(p, KERNEL_DMMA_F64, u, c);
-        if (us < best_us) best = KERNEL_DMMA_F64, best_us = us;
-    }
-    if (u.eligible && u.elt == 8) {
-        // The gather kernel's rates come from long contracted extents; on short ones it falls well below
-        // them (8 TFLOP/s at K = 24), so it has to look 30 % better than the TMA-fed kernel to be taken.
-        const double us = contraction_us(p, KERNEL_DMMA_F64_TMA, u, c);
-        if (us < (best == KERNEL_DMMA_F64 ? 1.3 : 1.0) * best_us) best = KERNEL_DMMA_F64_TMA, best_us = us;
-    }
-    return best;
+    const int64_t bn = p.Ntot <= 48 ? 32 : 64, bm = p.Ntot <= 48 ? 256 : 128;
+    const int gather = ceil_div(p.Mtot, bm) * ceil_div(p.Ntot, bn) >= c.num_sms ? KERNEL_DMMA_F64 : KERNEL_SIMT;
+    if (!u.eligible || u.elt != 8 || (k && std::strcmp(k, "gather") == 0)) return gather;
+    if (k && std::strcmp(k, "tma") == 0) return KERNEL_DMMA_F64_TMA;
+    // (a forced split of k is a switch of the TMA-fed kernel; and where its tiles run across slabs the gather kernel would
+    // have to cut its rows in two modes, with runs of 8 elements on both sides)
+    if (std::getenv("TCONT_SPLITK") || u.store_across_slabs) return KERNEL_DMMA_F64_TMA;
+    // The smallest problems are a matter of latency, which both estimates know to a tenth; above 20 us the gather kernel has to
+    // look 30 % better, because its whole-tile rate is 5 to 25 % more than it reaches on uneven tiles and long rows.
+    const double tma_us = contraction_us(p, KERNEL_DMMA_F64_TMA, u, c), gather_us = contraction_us(p, gather, u, c);
+    return tma_us <= (gather_us < 20.0 ? 1.05 : 1.3) * gather_us ? KERNEL_DMMA_F64_TMA : gather;
 }
 
 }  // namespace
@@ -867,19 +933,26 @@ bool read_cost_table_file(const std::string& path, CostTable* table)
     while (f >> key >> v) {
         if (key == "hbm_gbs") c.hbm_gbs = v;
         else if (key == "umma_tf32_tflops") c.umma_tf32_tflops = v;
-        else if (key == "simt_f32_tflops") c.simt_f32_tflops = v;
-        else if (key == "simt_f64_tflops") c.simt_f64_tflops = v;
         else if (key == "launch_us") c.launch_us = v;
         else if (key == "dmma_f64_tflops") c.dmma_f64_tflops = v;
-        else if (key == "dmma_f64_gather_tflops") c.dmma_f64_gather_tflops = v;
-        else if (key == "dmma_f64_gather8_tflops") c.dmma_f64_gather8_tflops = v;
-        else if (key == "dmma_f64_gather_narrow_tflops") c.dmma_f64_gather_narrow_tflops = v;
+        else if (key == "gather_fixed_us") c.gather_fixed_us = v;
+        else if (key == "gather_reduce_us") c.gather_reduce_us = v;
+        else if (key == "gather_tile_us") c.gather_tile_us = v;
+        else if (key == "gather_gbs") c.gather_gbs = v;
         else if (key == "scatter_store_ps") c.scatter_store_ps = v;
         else if (key == "scatter_store_f32_ps") c.scatter_store_f32_ps = v;
         else if (key == "far_row_penalty") c.far_row_penalty = v;
         else if (key == "umma_stage_us") c.umma_stage_us = v;
         else if (key == "umma_store_gbs_per_sm") c.umma_store_gbs_per_sm = v;
         else if (key == "num_sms" && v >= 1) c.num_sms = static_cast<int>(v);
+        else
+            for (int t = 0; t < 4; ++t) {   // gather_f64_tflops_0 ... gather_f32_iter_us_3
+                const std::string i = std::to_string(t);
+                if (t < 3 && key == "gather_f64_tflops_" + i) c.gather_f64_tflops[t] = v;
+                else if (t < 3 && key == "gather_f64_iter_us_" + i) c.gather_f64_iter_us[t] = v;
+                else if (key == "gather_f32_tflops_" + i) c.gather_f32_tflops[t] = v;
+                else if (key == "gather_f32_iter_us_" + i) c.gather_f32_iter_us[t] = v;
+            }
     }
     return true;
 }
@@ -948,8 +1021,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
 
     UmmaSpec direct_umma;
     plan_umma(direct, cost, &direct_umma);
-    const int direct_kernel = pick_kernel(direct, direct_umma, cost);
-    pl.est_direct_us = contraction_us(direct, direct_kernel, direct_umma, cost);
+    int direct_kernel = pick_kernel(direct, direct_umma, cost);
 
     // Transpose-assisted candidate.  A role's transposed layout is
     //     [lead | K modes | remaining row modes in C order]
@@ -1005,7 +1077,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         return k;
     };
     auto starts_with = [](const std::string& s, const std::string& pre) { return s.compare(0, pre.size(), pre) == 0; };
-    std::string roleA_dst = roleA_src, roleB_dst = roleB_src;
+    std::vector<std::pair<std::string, std::string>> candidates{{roleA_src, roleB_src}};
     {
         double best = 1e300;
         for (const std::string& korder : {sorted_by(roleB_src), sorted_by(roleA_src), perm_modes(direct, direct.K)}) {
@@ -1017,8 +1089,8 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
             const double moved = (keepA ? 0.0 : double(direct.sizeA)) + (keepB ? 0.0 : double(direct.sizeB));
             if (moved < best) {
                 best = moved;
-                roleA_dst = keepA ? roleA_src : leadA.first + korder + leadA.second;
-                roleB_dst = keepB ? roleB_src : leadB.first + korder + leadB.second;
+                candidates[0] = {keepA ? roleA_src : leadA.first + korder + leadA.second,
+                                 keepB ? roleB_src : leadB.first + korder + leadB.second};
             }
         }
     }
@@ -1026,21 +1098,74 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     const std::vector<int64_t>& roleA_parent = direct.swapped ? pl.parentB : pl.parentA;
     const std::vector<int64_t>& roleB_parent = direct.swapped ? pl.parentA : pl.parentB;
     const std::vector<int64_t> dense;
-    Problem ttgt;
-    rc = build_problem(pl.modeC, roleA_dst, roleB_dst, pl.ext_mode, pl.ext_val, scalar_type, &ttgt, err, pl.parentC,
-                       roleA_dst == roleA_src ? roleA_parent : dense, roleB_dst == roleB_src ? roleB_parent : dense);
-    if (rc) return rc;
-    UmmaSpec ttgt_umma;
-    plan_umma(ttgt, cost, &ttgt_umma);
-    const int ttgt_kernel = pick_kernel(ttgt, ttgt_umma, cost);
-    TransposeSpec tA, tB;
-    fill_transpose(roleA_src, roleA_dst, pl.ext_mode, pl.ext_val, &tA, roleA_parent);
-    fill_transpose(roleB_src, roleB_dst, pl.ext_mode, pl.ext_val, &tB, roleB_parent);
     const double elt = scalar_type == 1 ? 8.0 : 4.0;
-    double t_us = 0;
-    if (tA.needed) t_us += cost.launch_us + 2.0 * double(tA.elements) * elt / (cost.hbm_gbs * 0.7 * 1e3);
-    if (tB.needed) t_us += cost.launch_us + 2.0 * double(tB.elements) * elt / (cost.hbm_gbs * 0.7 * 1e3);
-    pl.est_ttgt_us = t_us + contraction_us(ttgt, ttgt_kernel, ttgt_umma, cost);
+    Problem ttgt;
+    UmmaSpec ttgt_umma;
+    int ttgt_kernel = KERNEL_SIMT;
+    TransposeSpec tA, tB;
+    pl.est_ttgt_us = 1e300;
+    auto problem_of = [&](const std::pair<std::string, std::string>& layouts, Problem* q) {
+        return build_problem(pl.modeC, layouts.first, layouts.second, pl.ext_mode, pl.ext_val, scalar_type, q, err, pl.parentC,
+                             layouts.first == roleA_src ? roleA_parent : dense, layouts.second == roleB_src ? roleB_parent : dense);
+    };
+    auto transposes_us = [&](const std::pair<std::string, std::string>& layouts, const CostTable& c) {
+        double us = 0;
+        if (layouts.first != roleA_src) us += c.launch_us + 2.0 * double(direct.sizeA) * elt / (c.hbm_gbs * 0.7 * 1e3);
+        if (layouts.second != roleB_src) us += c.launch_us + 2.0 * double(direct.sizeB) * elt / (c.hbm_gbs * 0.7 * 1e3);
+        return us;
+    };
+    // Whether Float32 runs as TF32 or in IEEE single precision is a question of precision, not only of time, and its answer
+    // stays what it was however fast the gather kernel becomes: of the operands as they lie and the first transposed layout,
+    // the cheaper by launches of 6.9 us and CUDA cores at 23.7 TFLOP/s decides, by whether the tcgen05 kernel can stage it.
+    bool tf32 = true;
+    if (scalar_type == 0) {
+        CostTable line = cost;
+        line.launch_us = 6.91584;
+        const double flops = 2.0 * double(direct.Mtot) * double(direct.Ntot) * double(direct.Ktot);
+        const double ieee_us = line.launch_us + std::max(flops / 23.6711e6, (double(direct.sizeA) + double(direct.sizeB) + double(direct.sizeC)) * elt / (line.hbm_gbs * 1e3));
+        auto line_us = [&](const Problem& q, bool* staged) {
+            UmmaSpec u;
+            plan_umma(q, line, &u);
+            *staged = pick_kernel(q, u, line) == KERNEL_UMMA_TF32;
+            if (!*staged) return ieee_us;
+            double us = contraction_us(q, KERNEL_UMMA_TF32, u, line);
+            if (u.k_splits > 1) {   // (a whole launch, and all partials through HBM)
+                const double partials = 2.0 * double(u.k_splits) * double(q.sizeC) * elt;
+                us += 0.5 * line.launch_us + (partials < 128e6 ? 0.5 : 0.0) * partials / (line.hbm_gbs * 1e3);
+            }
+            return us;
+        };
+        Problem q;
+        rc = problem_of(candidates[0], &q);
+        if (rc) return rc;
+        bool direct_staged, moved_staged;
+        const double direct_us = line_us(direct, &direct_staged), moved_us = line_us(q, &moved_staged);
+        const double t_us = transposes_us(candidates[0], line);
+        tf32 = (backend_selection == 0 ? t_us > 0 && t_us + moved_us < direct_us : backend_selection == 2) ? moved_staged : direct_staged;
+        if (!tf32 && direct_kernel == KERNEL_UMMA_TF32) {
+            direct_umma = UmmaSpec();
+            direct_umma.why_not = "runs in IEEE single precision";
+            direct_kernel = KERNEL_SIMT;
+        }
+    }
+    pl.est_direct_us = contraction_us(direct, direct_kernel, direct_umma, cost);
+    for (size_t i = 0; i < (tf32 ? candidates.size() : 1); ++i) {
+        Problem q;
+        rc = problem_of(candidates[i], &q);
+        if (rc) return rc;
+        UmmaSpec u;
+        if (tf32) plan_umma(q, cost, &u);
+        const int kernel = pick_kernel(q, u, cost);
+        const double us = transposes_us(candidates[i], cost) + contraction_us(q, kernel, u, cost);
+        if (us < 0.97 * pl.est_ttgt_us) {   // (an alternative has to be clearly better than the first)
+            pl.est_ttgt_us = us;
+            ttgt = q;
+            ttgt_umma = u;
+            ttgt_kernel = kernel;
+            fill_transpose(roleA_src, candidates[i].first, pl.ext_mode, pl.ext_val, &tA, roleA_parent);
+            fill_transpose(roleB_src, candidates[i].second, pl.ext_mode, pl.ext_val, &tB, roleB_parent);
+        }
+    }
 
     bool use_ttgt;
     if (backend_selection == 1) use_ttgt = false;
@@ -1069,31 +1194,9 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     // flat m (n) index, along k when it is the fastest contracted mode.
     pl.simt.a_load_along_k = first_is(p.A, p.M) ? 0 : (first_is(p.A, p.K) ? 1 : 0);
     pl.simt.b_load_along_k = first_is(p.B, p.N) ? 0 : (first_is(p.B, p.K) ? 1 : 0);
+    pl.gather = plan_gather(p, cost);
     *plan = pl;
     return 0;
-}
-
-void build_offset_tables(const Problem& p, OffsetTables* t)
-{
-    auto fill = [&](const std::vector<int>& grp, int64_t total, int which, std::vector<int64_t>* out) {
-        out->assign(static_cast<size_t>(total), 0);
-        for (int64_t i = 0; i < total; ++i) {
-            int64_t rem = i, off = 0;
-            for (int id : grp) {
-                const Mode& m = p.modes[static_cast<size_t>(id)];
-                const int64_t idx = rem % m.extent;
-                rem /= m.extent;
-                off += idx * (which == 0 ? m.sA : which == 1 ? m.sB : m.sC);
-            }
-            (*out)[static_cast<size_t>(i)] = off;
-        }
-    };
-    fill(p.M, p.Mtot, 0, &t->offAm);
-    fill(p.K, p.Ktot, 0, &t->offAk);
-    fill(p.N, p.Ntot, 1, &t->offBn);
-    fill(p.K, p.Ktot, 1, &t->offBk);
-    fill(p.M, p.Mtot, 2, &t->offCm);
-    fill(p.N, p.Ntot, 2, &t->offCn);
 }
 
 std::string describe_plan(const Plan& pl)
@@ -1123,7 +1226,8 @@ std::string describe_plan(const Plan& pl)
       << ",\"Ktot\":" << p.Ktot << ",\"transpose_a\":" << (pl.tA.needed ? perm(pl.tA) : "null")
       << ",\"transpose_b\":" << (pl.tB.needed ? perm(pl.tB) : "null") << ",\"est_direct_us\":" << pl.est_direct_us
       << ",\"est_ttgt_us\":" << pl.est_ttgt_us << ",\"simt\":{\"a_along_k\":" << pl.simt.a_load_along_k
-      << ",\"b_along_k\":" << pl.simt.b_load_along_k << "}";
+      << ",\"b_along_k\":" << pl.simt.b_load_along_k << "},\"gather\":{\"tile\":" << pl.gather.tile
+      << ",\"cluster\":" << pl.gather.cluster << ",\"flat\":" << (pl.gather.flat ? "true" : "false") << ",\"t0\":" << pl.gather.t0 << ",\"t1\":" << pl.gather.t1 << ",\"est_us\":" << pl.gather.est_us << "}";
     const UmmaSpec& u = pl.umma;
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";

@@ -16,6 +16,8 @@ constexpr int kMaxModes = 16;
 constexpr int kMaxTmaRank = 5;
 
 enum ModeGroup { GROUP_M = 0, GROUP_N = 1, GROUP_K = 2 };
+// KERNEL_SIMT and KERNEL_DMMA_F64 are the gather kernel (gather_contract.cu): the second is FP64 work that fills the GPU
+// with tiles, the first everything else.
 enum KernelKind { KERNEL_SIMT = 0, KERNEL_UMMA_TF32 = 1, KERNEL_DMMA_F64 = 2, KERNEL_DMMA_F64_TMA = 3 };
 
 struct Mode {
@@ -115,18 +117,36 @@ struct SimtSpec {
     int tile = 64;           // BM = BN
 };
 
+// Tiles of the gather kernel (gather_contract.cu).
+enum GatherTile { GATHER_SQUARE = 0, GATHER_TALL = 1, GATHER_SMALL = 2, GATHER_BIG = 3 };
+constexpr int kMaxGatherCluster = 16;
+struct GatherSpec {
+    int tile = GATHER_SQUARE;
+    int cluster = 1;     // CTAs that share an output tile, each contracting a range of k
+    bool flat = false;   // persistent blocks (see GatherParams)
+    // Rows cut in two modes: a tile is t0 indices of C's stride-1 mode times t1 of A's (0: rows in C's order)
+    int t0 = 0, t1 = 0;
+    int64_t rows = 1;    // rows of the GEMM view, cut modes rounded up
+    double est_us = 0;   // without the launch
+};
+
 struct CostTable {
     // Defaults: what `python -m tcont_b200.calibrate` measured on a B200 (the file it writes,
     // tcont_cost_table.NVIDIA_B200.txt beside the library, holds the same figures and is read when the current
     // device has that name; TCONT_COST_TABLE names another "key value" file).
     double hbm_gbs = 6178.9;                // copy through the permutation kernel, read + write
     double umma_tf32_tflops = 674.4;        // tcgen05 kernel, 8192 x 8192 x 4096, CTA pairs with a k chunk of 64
-    double simt_f32_tflops = 23.7;
-    double simt_f64_tflops = 16.4;
     double dmma_f64_tflops = 33.5;          // TMA-fed tensor-path kernel
-    double dmma_f64_gather_tflops = 20.8;   // gather tensor-path kernel, 16-byte gathers
-    double dmma_f64_gather8_tflops = 15.5;  // gather tensor-path kernel, an operand on 8-byte gathers
-    double dmma_f64_gather_narrow_tflops = 6.5;  // gather tensor-path kernel, 256 x 32 tiles (N <= 48)
+    // Gather kernel, per tile shape (64 x 64, 128 x 32, 32 x 32, Float32 128 x 128): what a full GPU does in whole tiles,
+    // and the least time one CTA needs per k tile of 16 when it has an SM to itself.
+    double gather_f64_tflops[3] = {28.0, 18.0, 18.0};
+    double gather_f64_iter_us[3] = {1.55, 1.7, 0.7};
+    double gather_f32_tflops[4] = {32.0, 31.0, 16.0, 42.0};
+    double gather_f32_iter_us[4] = {1.05, 1.25, 0.48, 2.4};
+    double gather_fixed_us = 2.0;           // tables, first gathers and stores of one CTA
+    double gather_tile_us = 0.7;            // the same per tile of a persistent CTA, whose gathers run ahead
+    double gather_reduce_us = 3.0;          // adding up a cluster's partial tiles
+    double gather_gbs = 2200.0;             // tensors read and written once through element-wise gathers and stores
     double scatter_store_ps = 27.6;         // per element of C stored on its own (TMA-fed FP64 kernel)
     double scatter_store_f32_ps = 17.6;     // the same for the tcgen05 kernel's 4-byte elements
     double launch_us = 6.9;                 // one more launch through the library (a contraction too small to matter, in a loop)
@@ -158,6 +178,7 @@ struct Plan {
     TransposeSpec tA, tB;   // transposes feeding role A / role B (src = the caller's tensor of that role)
     int kernel = KERNEL_SIMT;
     SimtSpec simt;
+    GatherSpec gather;
     UmmaSpec umma;
     double est_direct_us = 0, est_ttgt_us = 0;
     double flops = 0;
@@ -177,11 +198,5 @@ std::string describe_plan(const Plan& plan);
 CostTable load_cost_table();
 // Reads "key value" lines into `table` (unknown keys are ignored); false when the file cannot be opened.
 bool read_cost_table_file(const std::string& path, CostTable* table);
-
-// Offset tables of the GEMM view: address(A, m, k) = offAm[m] + offAk[k] and so on.
-struct OffsetTables {
-    std::vector<int64_t> offAm, offAk, offBn, offBk, offCm, offCn;
-};
-void build_offset_tables(const Problem& p, OffsetTables* t);
 
 }  // namespace tcontb
