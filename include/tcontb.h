@@ -109,9 +109,8 @@ tcontb_status tcontb_run_upload_inputs(tcontb_run* run, const void* a_host, cons
 
 /* Beyond the reference, whose backends always overwrite (alpha = 1, beta = 0: cublasGemmEx scalars at
  * backends/ttgt_cutt/src/ttgt_cutt.cpp:742-743, generated kernels store a zeroed accumulator): later
- * launches compute C = alpha * (A*B) + beta * C.  With other values than (1, 0) the contraction
- * writes a workspace of the size of C (allocated by this call, not by the launches) and the
- * partial-sum pass applies the scalars; C is read only when beta is not zero.  Not available on a
+ * launches compute C = alpha * (A*B) + beta * C.  The kernel that writes C applies the scalars (the
+ * partial-sum pass where k is split); C is read only when beta is not zero.  Not available on a
  * run that spans several GPUs. */
 tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta);
 

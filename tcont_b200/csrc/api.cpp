@@ -160,9 +160,8 @@ struct tcontb_run {
     DeviceBuffer pace;  // progress counters of the tcgen05 kernel's pace keeping (see UmmaParams)
     size_t pace_bytes = 0;
     // C = alpha * (A*B) + beta * C (tcontb_run_set_scalars); the reference's semantics are alpha 1, beta 0.
-    // With other values the contraction writes a workspace and the partial-sum pass applies the scalars.
+    // Other values are applied by the kernel that writes C.
     double alpha = 1.0, beta = 0.0;
-    DeviceBuffer scaled_ws;
     // stage timing
     bool stage_timing = false;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -940,9 +939,6 @@ tcontb_status tcontb_run_upload_inputs(tcontb_run* run, const void* a_host, cons
     return TCONTB_OK;
 }
 
-// The gather kernel applies alpha and beta itself.
-static bool gathers(const Plan& pl) { return pl.kernel == KERNEL_SIMT || pl.kernel == KERNEL_DMMA_F64; }
-
 tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
 {
     if (!run) return fail(TCONTB_INVALID_ARGUMENT, "ExecutionRun is empty");
@@ -950,12 +946,6 @@ tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
     TC_NOT_SHARDED(run, "alpha and beta");
     const bool scaled = alpha != 1.0 || beta != 0.0;
     if (scaled && run->plan.prob.c_strided) return fail(TCONTB_UNSUPPORTED, "alpha and beta are not available when C is a sub-tensor view");
-    if (scaled && !run->splitk.ptr && !run->scaled_ws.ptr && !gathers(run->plan)) {
-        // allocated here, once, so that launches stay free of allocations
-        TC_CUDA(run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt));
-    }
-    const bool was = run->alpha != 1.0 || run->beta != 0.0;
-    if (!run->splitk.ptr && !gathers(run->plan)) run->kernels_per_launch += (scaled ? 1 : 0) - (was ? 1 : 0);
     run->alpha = alpha;
     run->beta = beta;
     // the parts of a pipelined host-buffer pass work on ranges of this run's C
@@ -1004,14 +994,12 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
     }
     const Plan& pl = run->plan;
     const bool t = run->stage_timing;
-    // Other scalars than (1, 0): the kernel writes the workspace instead of C (a split-K run does anyway)
+    // Other scalars than (1, 0): the contraction kernel's epilogue applies them, or the partial-sum pass of a split-K run
     const bool scaled = run->alpha != 1.0 || run->beta != 0.0;
-    const bool redirect = scaled && !run->splitk.ptr && !gathers(pl);
     UmmaParams umma = run->umma;
-    if (redirect) {
-        umma.C = static_cast<float*>(run->scaled_ws.ptr);
-        umma.C64 = static_cast<double*>(run->scaled_ws.ptr);
-    }
+    umma.scaled = scaled && !run->splitk.ptr ? 1 : 0;
+    umma.alpha = run->alpha;
+    umma.beta = run->beta;
     if (t) TC_CUDA(cudaEventRecord(run->ev[0], run->stream));
     if (pl.tA.needed && !run->borrowed_tA) TC_CUDA(launch_transpose(run->roleA_src(), run->tbufA.ptr, run->tpA, static_cast<int>(run->elt), run->stream));
     if (t) TC_CUDA(cudaEventRecord(run->ev[1], run->stream));
@@ -1058,9 +1046,6 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
     if (run->splitk.ptr)
         TC_CUDA(launch_splitk_reduce(run->splitk.ptr, run->dC, pl.sizeC, pl.umma.k_splits * (run->tf32x3 ? 3 : 1), pl.sizeC,
                                      static_cast<int>(run->elt), run->stream, run->alpha, run->beta));
-    else if (redirect)
-        TC_CUDA(launch_splitk_reduce(run->scaled_ws.ptr, run->dC, pl.sizeC, 1, pl.sizeC, static_cast<int>(run->elt), run->stream,
-                                     run->alpha, run->beta));
     if (t) {
         TC_CUDA(cudaEventRecord(run->ev[3], run->stream));
         run->ev_valid = true;

@@ -62,6 +62,20 @@ __device__ __forceinline__ void st_global_cs_v4f64(double* p, double a, double b
     asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
 
+// The four elements of C a thread is about to overwrite (C = alpha A B + beta C with beta != 0); 32 bytes when `vec`.
+__device__ __forceinline__ void load_old4(double (&o)[4], const double* dst, bool vec, const double* p0, const double* p1, const double* p2,
+                                          const double* p3)
+{
+    if (vec) {
+        asm volatile("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(dst) : "memory");
+    } else {
+        o[0] = p0 ? __ldcs(p0) : 0.0;
+        o[1] = p1 ? __ldcs(p1) : 0.0;
+        o[2] = p2 ? __ldcs(p2) : 0.0;
+        o[3] = p3 ? __ldcs(p3) : 0.0;
+    }
+}
+
 // Which k a lane feeds into step t of a stage: k = 8 (t / 2) + 2 fk + ((fk ^ (fk >> 1) ^ t) & 1), fk = lane % 4.
 // Any assignment works as long as both operands use the same one.  With this one
 //  * the four rows an MN-major 16-byte load touches per quarter warp differ in k / 2, which after the
@@ -144,7 +158,9 @@ __device__ __forceinline__ void mma_step(double (&acc)[8][NF][2], const double (
     }
 }
 
-template <bool AMN, bool BMN, int NF>
+// SCALED: C = alpha A B + beta C in the epilogue (C read only when beta is not zero); a template parameter because the
+// overwriting kernel has no registers to spare for it.
+template <bool AMN, bool BMN, int NF, bool SCALED>
 __global__ void __launch_bounds__(kThreads64, 1)
 dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                 const __grid_constant__ UmmaParams p)
@@ -300,6 +316,20 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     st_shared_s64(tab + static_cast<uint32_t>(e) * 8u, ok ? off + slab_elem_offset(o, d0, in) : -1);
                 }
                 mbar_arrive(smem_u32(tab_full + slot));
+                if (SCALED && p.beta != 0.0) {
+                    // The tile's old values are wanted about two tiles from now: bring them into L2.  Eight warps cannot keep
+                    // enough reads of C in flight to hide DRAM behind the store phase, which had them wait there.
+                    if (!mbar_wait(smem_u32(tab_full + slot), use & 1u, abort_flag)) break;   // the other builders' entries
+                    const double* C = p.C64;
+                    // one look per four rows (32 bytes), or across slabs per group of eight slabs (64 bytes)
+                    const int step = p.store_across_slabs ? 1 : 4, looks = p.store_across_slabs ? 16 : kBM / 4;
+                    for (int q = bt; q < looks * NF * 16; q += 64) {
+                        const long long r = ld_shared_s64(tab + static_cast<uint32_t>((q % looks) * step) * 8u);
+                        const long long c = ld_shared_s64(tab + static_cast<uint32_t>(kBM + q / looks) * 8u);
+                        if (r >= 0 && c >= 0 && (step == 1 || (q % looks) % 4 == 0 || ((reinterpret_cast<uintptr_t>(C + r + c) & 127u) < 32u)))
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(C + r + c));
+                    }
+                }
             }
         }
     } else {
@@ -400,6 +430,23 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
 #pragma unroll
             for (int j = 0; j < NF; ++j)
                 cn[j] = ld_shared_s64(col_tab + (static_cast<uint32_t>(wn * NF * 8 + 16 * (j >> 1) + (j & 1)) + 2u * fr) * 8u);
+            // alpha and beta on the four elements of every column fragment; all old values are asked for before the first is
+            // used (a round trip to L2 per two fragments cost 2 800 cycles a tile)
+            auto scale_four = [&](long long cm0, long long cm1, long long cm2, long long cm3, bool run4, auto&& at) {
+                double old[NF][4];
+#pragma unroll
+                for (int j = 0; j < NF; ++j) {
+                    const long long c = cn[j];
+                    if (tile_ok && c >= 0 && p.beta != 0.0)
+                        load_old4(old[j], C + cm0 + c, run4 && (reinterpret_cast<uintptr_t>(C + cm0 + c) & 31u) == 0, cm0 >= 0 ? C + cm0 + c : nullptr,
+                                  cm1 >= 0 ? C + cm1 + c : nullptr, cm2 >= 0 ? C + cm2 + c : nullptr, cm3 >= 0 ? C + cm3 + c : nullptr);
+                    else old[j][0] = old[j][1] = old[j][2] = old[j][3] = 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < NF; ++j)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) at(j, q) = p.alpha * at(j, q) + p.beta * old[j][q];
+            };
             if (p.store_across_slabs) {
                 // The warp's 64 rows are four slabs of 16; slab q is index a0 + q of C's stride-1 mode and the rows
                 // of a slab run along another mode.  Row (4 fk + dd) of the four slabs is four neighbouring
@@ -411,6 +458,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     const long long cm0 = ld_shared_s64(row_tab + r * 8u), cm1 = ld_shared_s64(row_tab + (r + 16u) * 8u);
                     const long long cm2 = ld_shared_s64(row_tab + (r + 32u) * 8u), cm3 = ld_shared_s64(row_tab + (r + 48u) * 8u);
                     const bool run4 = cm0 >= 0 && cm1 == cm0 + 1 && cm2 == cm0 + 2 && cm3 == cm0 + 3;
+                    if constexpr (SCALED) scale_four(cm0, cm1, cm2, cm3, run4, [&](int j, int q) -> double& { return acc[2 * q + par][j][h]; });
 #pragma unroll
                     for (int j = 0; j < NF; ++j) {
                         if (tile_ok && cn[j] >= 0) {
@@ -437,6 +485,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 const long long cm0 = ld_shared_s64(row_tab + r * 8u), cm1 = ld_shared_s64(row_tab + r * 8u + 8u);
                 const long long cm2 = ld_shared_s64(row_tab + r * 8u + 16u), cm3 = ld_shared_s64(row_tab + r * 8u + 24u);
                 const bool run4 = cm0 >= 0 && cm1 == cm0 + 1 && cm2 == cm0 + 2 && cm3 == cm0 + 3;
+                if constexpr (SCALED) scale_four(cm0, cm1, cm2, cm3, run4, [&](int j, int q) -> double& { return acc[2 * pr + (q & 1)][j][q >> 1]; });
 #pragma unroll
                 for (int j = 0; j < NF; ++j) {
                     if (tile_ok && cn[j] >= 0) {
@@ -484,8 +533,9 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
 template <bool AMN, bool BMN, int NF>
 cudaError_t launch_variant(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, unsigned grid, cudaStream_t stream)
 {
-    dmma_tma_kernel<AMN, BMN, NF><<<grid, kThreads64, smem_bytes, stream>>>(*static_cast<const CUtensorMap*>(tmapA),
-                                                                             *static_cast<const CUtensorMap*>(tmapB), p);
+    const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
+    auto kernel = p.scaled ? dmma_tma_kernel<AMN, BMN, NF, true> : dmma_tma_kernel<AMN, BMN, NF, false>;
+    kernel<<<grid, kThreads64, smem_bytes, stream>>>(ta, tb, p);
     return cudaGetLastError();
 }
 
@@ -498,14 +548,14 @@ cudaError_t launch_width(const UmmaParams& p, const void* tmapA, const void* tma
     return launch_variant<false, false, NF>(p, tmapA, tmapB, smem_bytes, grid, stream);
 }
 
-template <int NF>
+template <int NF, bool SCALED>
 cudaError_t configure_width()
 {
     const int smem_bytes = kMaxDynamicSmemBytes;  // the same opt-in maximum for every run (the cap is per function and device)
-    cudaError_t e = cudaFuncSetAttribute(dmma_tma_kernel<false, false, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<false, true, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<true, false, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<true, true, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    cudaError_t e = cudaFuncSetAttribute(dmma_tma_kernel<false, false, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<false, true, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<true, false, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<true, true, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     return e;
 }
 
@@ -513,8 +563,11 @@ cudaError_t configure_width()
 
 cudaError_t dmma_tma_configure()
 {
-    const cudaError_t e = configure_width<4>();
-    return e == cudaSuccess ? configure_width<2>() : e;
+    cudaError_t e = configure_width<4, false>();
+    if (e == cudaSuccess) e = configure_width<2, false>();
+    if (e == cudaSuccess) e = configure_width<4, true>();
+    if (e == cudaSuccess) e = configure_width<2, true>();
+    return e;
 }
 
 cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, int num_sms, cudaStream_t stream)

@@ -118,6 +118,8 @@ struct UmmaParams {
     int raster_group;
     float* C;       // tcgen05 TF32 kernel
     double* C64;    // TMA-fed FP64 kernel
+    int scaled;            // 1: the epilogue stores alpha A B + beta C (C read only when beta is not zero); not with k_splits > 1 or owners
+    double alpha, beta;
     int* status;  // device status word: set non-zero when a bounded wait gives up
     long long* prof;  // optional per-CTA cycle counters [grid][8] (TCONT_UMMA_PROF=1), else null
     // Test hooks of the bounded-wait exit (tcgen05 kernel): a shorter wait limit (0 = the default 2 s), and

@@ -146,7 +146,8 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // NP = producer warps (1, or 2 taking turns stage by stage); a template parameter so that the one-producer loop,
 // whose pass per stage is the tightest thing in the pair kernel, carries none of the two-producer bookkeeping
 // (with it as a run-time value the pair kernel lost 8 %).
-template <bool PAIR, int NP>
+// SCALED: C = alpha A B + beta C in the epilogue (C read only when beta is not zero).
+template <bool PAIR, int NP, bool SCALED>
 __global__ void __launch_bounds__(kThreads, 1)
 umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                  const __grid_constant__ UmmaParams p)
@@ -452,6 +453,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
         const int q = warp & 3;
         const int row = q * 32 + lane;
         const int et = threadIdx.x - 64;
+        const float alpha = static_cast<float>(p.alpha), beta = static_cast<float>(p.beta);
         long long iter = 0;
         long long t_tfull = 0, t_epi = clock64();
         for (uint32_t tile = first_unit; tile < total_tiles; tile += unit_step, ++iter) {
@@ -500,6 +502,28 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
                 if (PAIR) mbar_arrive_cluster(tempty_addr);
                 else mbar_arrive(tempty_addr);
             };
+            if (SCALED && p.beta != 0.0) {
+                // The tile's old values are wanted when the accumulator is complete: bring them into L2 meanwhile, a lane per
+                // column, both lines that the warp's 32 rows may touch (4 warps cannot keep enough loads in flight for DRAM).
+                const float* c0 = p.C + row_off;
+                const long long last = __shfl_sync(0xffffffffu, row_ok ? row_off : -1, 31);
+                const long long first = __shfl_sync(0xffffffffu, row_off, 0);
+                const bool on = __shfl_sync(0xffffffffu, row_ok ? 1 : 0, 0) != 0;
+                c0 += first - row_off;
+                for (int c = 0; on && c < (p.BN >> 5); ++c) {
+                    long long off = -1;
+                    if (wide_slabs) {
+                        if (lane < static_cast<int>(ld_shared_u32(cols + static_cast<uint32_t>(c) * 16u + 8u)))
+                            off = ld_shared_s64(cols + static_cast<uint32_t>(c) * 16u) + lane * p.b.row_elem_cstride;
+                    } else {
+                        off = ld_shared_s64(cols + static_cast<uint32_t>(c * 32 + lane) * 8u);
+                    }
+                    if (off >= 0) {
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + off));
+                        if (last >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + (last - first) + off));
+                    }
+                }
+            }
             bool ok = true;
             const long long t0 = p.prof ? clock64() : 0;
             if (lane == 0) ok = mbar_wait(smem_u32(bar_tfull + acc), acc_parity, abort_flag, 0, p.wait_limit_ns);
@@ -520,25 +544,48 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
                         const long long base = ld_shared_s64(cols + static_cast<uint32_t>(c) * 16u);
                         const int nvalid = row_ok ? static_cast<int>(ld_shared_u32(cols + static_cast<uint32_t>(c) * 16u + 8u)) : 0;
                         float* ptr = crow + base;
+                        float old[32];
+                        if constexpr (SCALED) {   // all old values are asked for before the first is used
+                            const float* q_old = ptr;
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) {
+                                old[j] = beta != 0.0f && j < nvalid ? __ldcs(q_old) : 0.0f;
+                                q_old += col_stride;
+                            }
+                        }
+                        if (!SCALED && __all_sync(0xffffffffu, nvalid == 32)) {
+                            // a whole chunk: three instructions a store, no branches (with a test per store one warp per
+                            // scheduler took 26 cycles for each; with one branch per eight stores the low-K
+                            // configuration takes 200 us, like this 178)
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) {
+                                __stcs(ptr, __uint_as_float(v[j]));
+                                ptr += col_stride;
+                            }
+                            return;
+                        }
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
-                            if (j < nvalid) __stcs(ptr, __uint_as_float(v[j]));
+                            float x = __uint_as_float(v[j]);
+                            if constexpr (SCALED) x = alpha * x + beta * old[j];
+                            if (j < nvalid) __stcs(ptr, x);
                             ptr += col_stride;
                         }
                     } else {
-                        // lane j keeps the offset of column 32*c + j; fetch all 32 by shuffle, then store
-                        const long long mine = ld_shared_s64(cols + static_cast<uint32_t>(c * 32 + lane) * 8u);
-                        const int lo = static_cast<int>(mine), hi = static_cast<int>(mine >> 32);
-                        long long co[32];
+                        long long co[32];   // (every lane reads the same word: a broadcast)
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const unsigned ulo = static_cast<unsigned>(__shfl_sync(0xffffffffu, lo, j));
-                            const int shi = __shfl_sync(0xffffffffu, hi, j);
-                            co[j] = (static_cast<long long>(shi) << 32) | ulo;
+                        for (int j = 0; j < 32; ++j) co[j] = ld_shared_s64(cols + static_cast<uint32_t>(c * 32 + j) * 8u);
+                        float old[32];
+                        if constexpr (SCALED) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) old[j] = beta != 0.0f && row_ok && co[j] >= 0 ? __ldcs(crow + co[j]) : 0.0f;
                         }
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (row_ok && co[j] >= 0) __stcs(crow + co[j], __uint_as_float(v[j]));
+                        for (int j = 0; j < 32; ++j) {
+                            float x = __uint_as_float(v[j]);
+                            if constexpr (SCALED) x = alpha * x + beta * old[j];
+                            if (row_ok && co[j] >= 0) __stcs(crow + co[j], x);
+                        }
                     }
                 };
                 uint32_t v0[32], v1[32];
@@ -590,13 +637,19 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
 // the same opt-in maximum, so runs with different stage counts can live side by side.
 cudaError_t umma_tf32_configure()
 {
-    cudaError_t e = cudaFuncSetAttribute(umma_tf32_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(umma_tf32_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(umma_tf32_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(umma_tf32_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes);
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto* kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes);
+    };
+    set(umma_tf32_kernel<false, 1, false>);
+    set(umma_tf32_kernel<false, 2, false>);
+    set(umma_tf32_kernel<true, 1, false>);
+    set(umma_tf32_kernel<true, 2, false>);
+    set(umma_tf32_kernel<false, 1, true>);
+    set(umma_tf32_kernel<false, 2, true>);
+    set(umma_tf32_kernel<true, 1, true>);
+    set(umma_tf32_kernel<true, 2, true>);
+    return e;
 }
 
 cudaError_t launch_umma_tf32(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, int num_sms,
@@ -611,6 +664,8 @@ cudaError_t launch_umma_tf32(const UmmaParams& p, const void* tmapA, const void*
         const long long units = ((p.tiles_m + 1) / 2) * p.tiles_n * p.k_splits;
         if (units <= 0) return cudaErrorInvalidValue;
         const long long clusters = units < num_sms / 2 ? units : num_sms / 2;
+        auto kernel = p.scaled ? (p.producers == 2 ? umma_tf32_kernel<true, 2, true> : umma_tf32_kernel<true, 1, true>)
+                               : (p.producers == 2 ? umma_tf32_kernel<true, 2, false> : umma_tf32_kernel<true, 1, false>);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
         cfg.blockDim = dim3(threads);
@@ -623,14 +678,14 @@ cudaError_t launch_umma_tf32(const UmmaParams& p, const void* tmapA, const void*
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (p.producers == 2) return cudaLaunchKernelEx(&cfg, umma_tf32_kernel<true, 2>, ta, tb, p);
-        return cudaLaunchKernelEx(&cfg, umma_tf32_kernel<true, 1>, ta, tb, p);
+        return cudaLaunchKernelEx(&cfg, kernel, ta, tb, p);
     }
     const long long total = p.tiles_m * p.tiles_n * p.k_splits;
     if (total <= 0) return cudaErrorInvalidValue;
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
-    if (p.producers == 2) umma_tf32_kernel<false, 2><<<grid, threads, smem_bytes, stream>>>(ta, tb, p);
-    else umma_tf32_kernel<false, 1><<<grid, threads, smem_bytes, stream>>>(ta, tb, p);
+    auto kernel = p.scaled ? (p.producers == 2 ? umma_tf32_kernel<false, 2, true> : umma_tf32_kernel<false, 1, true>)
+                           : (p.producers == 2 ? umma_tf32_kernel<false, 2, false> : umma_tf32_kernel<false, 1, false>);
+    kernel<<<grid, threads, smem_bytes, stream>>>(ta, tb, p);
     return cudaGetLastError();
 }
 
