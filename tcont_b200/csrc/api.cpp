@@ -274,15 +274,29 @@ void fill_operand_dev(const UmmaOperand& o, UmmaOperandDev* d)
     d->oob_coord = o.oob_coord;
     for (int i = 0; i < kMaxTmaRank; ++i) {
         d->row_digit_dim[i] = i < o.n_row_digits ? o.row_digit_dim[i] : -1;
-        d->row_digit_ext[i] = i < o.n_row_digits ? static_cast<int>(o.row_digit_ext[i]) : 1;
+        d->row_digit_ext[i] = make_fast_div(i < o.n_row_digits ? o.row_digit_ext[i] : 1);
         d->row_digit_cstride[i] = i < o.n_row_digits ? o.row_digit_cstride[i] : 0;
     }
     d->row_elem_cstride = o.row_elem_cstride;
     d->slab_mode_ext = static_cast<int>(o.slab_mode_ext);
     d->total_slabs = o.total_slabs;
     for (int i = 0; i < 3; ++i) d->k_digit_dim[i] = o.k_digit_dim[i];
+    d->slab_shift = 0;
+    while ((1 << d->slab_shift) < o.slab_w) ++d->slab_shift;
     d->split_inner = static_cast<int>(o.split_inner);
+    d->split_div = make_fast_div(o.split_inner > 0 ? o.split_inner : 1);
     d->split_outer_cstride = o.split_outer_cstride;
+}
+
+// Work units are numbered by whole groups of raster_group tile rows (pair rows for CTA pairs), each swept column by column.
+void fill_raster_divs(const UmmaSpec& u, UmmaParams* p)
+{
+    const int64_t rows = u.pair ? (u.tiles_m + 1) / 2 : u.tiles_m;
+    const int64_t last = rows % u.raster_group;
+    p->div_group = make_fast_div(u.raster_group * u.tiles_n);
+    p->div_rows = make_fast_div(u.raster_group);
+    p->div_last_rows = make_fast_div(last ? last : u.raster_group);
+    p->div_splits = make_fast_div(u.k_splits);
 }
 
 tcontb_status encode_map(const UmmaOperand& o, const void* base, int elt, CUtensorMap* out)
@@ -419,6 +433,7 @@ tcontb_status finish_run(tcontb_run* run)
         run->umma.k_splits = u.k_splits;
         run->umma.k_iters_per_split = static_cast<int>(u.k_iters_per_split);
         run->umma.split_stride = pl.sizeC;
+        fill_raster_divs(u, &run->umma);
         void* out = run->dC;
         const char* x3 = std::getenv("TCONT_TF32X3");
         run->tf32x3 = pl.kernel == KERNEL_UMMA_TF32 && x3 && x3[0] == '1' && !p.strided;

@@ -217,37 +217,21 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmapA)) : "memory");
                 asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmapB)) : "memory");
             }
+            KSteps ks;
+            k_steps(o, ks);
             uint32_t stage = 0, phase = 0;
             uint32_t issued_mask = 0, issued_parity = 0;
             for (uint32_t i = static_cast<uint32_t>(warp); i < my_tiles; i += 2) {
                 const WorkUnit w = decode_unit(blockIdx.x + i * gridDim.x, p, tiles_m, tiles_n);
                 const uint32_t tm = w.tm, tn = w.tn;
-                int base[kMaxTmaRank] = {0, 0, 0, 0, 0};
-                if (active) {
-                    const uint32_t s = (is_a ? tm * SA : tn * SB) + slab;
-                    if (s < static_cast<uint32_t>(o.total_slabs)) {
-                        uint32_t rem = s;
-    #pragma unroll
-                        for (int d = 0; d < kMaxTmaRank; ++d) {
-                            if (d < o.n_row_digits) {
-                                const uint32_t e = static_cast<uint32_t>(o.row_digit_ext[d]);
-                                const int idx = static_cast<int>(rem % e);
-                                rem /= e;
-                                const int v = d == o.chunk_digit ? idx * o.digit0_scale : idx;
-    #pragma unroll
-                                for (int t = 0; t < kMaxTmaRank; ++t)
-                                    if (o.row_digit_dim[d] == t) base[t] = v;
-                            }
-                        }
-                    } else {
-                        // Slab beyond the tensor: start the box past the slab mode's end, TMA fills zeros.
-    #pragma unroll
-                        for (int t = 0; t < kMaxTmaRank; ++t)
-                            if (o.row_digit_dim[o.chunk_digit] == t) base[t] = o.oob_coord;
-                    }
+                int base[kMaxTmaRank];
+                slab_coords(o, (is_a ? tm * SA : tn * SB) + slab, base);
+                int kd0 = 0, kd1 = 0, kd2 = 0;
+                if (w.it0) {   // (a later k range of a split)
+                    kd0 = w.it0 % p.k_digit_ext[0];
+                    kd1 = w.it0 / p.k_digit_ext[0] % p.k_digit_ext[1];
+                    kd2 = w.it0 / (p.k_digit_ext[0] * p.k_digit_ext[1]);
                 }
-                int kd0 = w.it0 % p.k_digit_ext[0], kd1 = (w.it0 / p.k_digit_ext[0]) % p.k_digit_ext[1];
-                int kd2 = w.it0 / (p.k_digit_ext[0] * p.k_digit_ext[1]);
                 for (int it = 0; it < w.n_it; ++it) {
                     const uint32_t ps = first + stage;
                     const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar_empty + ps), phase ^ 1u, abort_flag, 200u));
@@ -256,13 +240,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                         __syncwarp();
                         if (active) {
                             int c[kMaxTmaRank];
-    #pragma unroll
-                            for (int t = 0; t < kMaxTmaRank; ++t) {
-                                c[t] = base[t];
-                                if (o.k_digit_dim[0] == t) c[t] = kd0 * p.BK;
-                                if (o.k_digit_dim[1] == t) c[t] = kd1;
-                                if (o.k_digit_dim[2] == t) c[t] = kd2;
-                            }
+                            k_coords(base, ks, kd0, kd1, kd2, c);
                             tma_load_5d(smem_u32(smem + static_cast<size_t>(ps) * stage_bytes + my_off), tmap,
                                         smem_u32(bar_full + ps), c[0], c[1], c[2], c[3], c[4]);
                         }
@@ -308,7 +286,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     if (!is_row && e - kBM >= NF * 16) continue;
                     const UmmaOperandDev& o = is_row ? p.a : p.b;
                     const int idx = is_row ? e : e - kBM;
-                    const int sl = idx / o.slab_w, in = idx % o.slab_w;
+                    const int sl = idx >> o.slab_shift, in = idx & (o.slab_w - 1);
                     bool ok;
                     int d0 = 0;
                     const long long off = slab_c_offset(o, (is_row ? tm * SA : tn * SB) + sl, &d0, &ok);

@@ -93,13 +93,15 @@ struct UmmaOperandDev {
     int chunk_digit;  // which row digit is the chunk of the slab mode (scaled by digit0_scale, out-of-range past the tensor)
     int k0_scale;  // TMA coordinate of k digit 0 = k iteration * this
     int row_digit_dim[kMaxTmaRank];
-    int row_digit_ext[kMaxTmaRank];
+    FastDiv row_digit_ext[kMaxTmaRank];
     long long row_digit_cstride[kMaxTmaRank];
     long long row_elem_cstride;
     int slab_mode_ext;
     long long total_slabs;
     int k_digit_dim[3];
+    int slab_shift;                 // log2 of slab_w
     int split_inner;                // operand-level row fusion: see UmmaOperand (0 = none)
+    FastDiv split_div;
     long long split_outer_cstride;
 };
 struct UmmaParams {
@@ -116,6 +118,8 @@ struct UmmaParams {
     long long split_stride;
     long long tiles_m, tiles_n;
     int raster_group;
+    // divisors of the raster (filled in by fill_raster_divs): tiles of a whole group of tile rows, rows of a whole group and of the last one, splits
+    FastDiv div_group, div_rows, div_last_rows, div_splits;
     float* C;       // tcgen05 TF32 kernel
     double* C64;    // TMA-fed FP64 kernel
     int scaled;            // 1: the epilogue stores alpha A B + beta C (C read only when beta is not zero); not with k_splits > 1 or owners

@@ -119,17 +119,19 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* tmap, uint
         : "memory");
 }
 
-// Raster order: groups of `g` tile rows are swept column by column, so the CTAs that run
-// together share A and B panels in L2.  Tile and slab counts fit 32 bits (the planner checks).
-__device__ __forceinline__ void decode_tile(uint32_t tile, uint32_t tiles_m, uint32_t tiles_n, uint32_t g, uint32_t* tm, uint32_t* tn)
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) { return (__umulhi(n, f.mul) + n) >> f.shr; }
+
+// Raster order: groups of raster_group tile rows are swept column by column, so the CTAs that run
+// together share A and B panels in L2.  Tile and slab counts fit 31 bits (the planner checks).
+__device__ __forceinline__ void decode_tile(uint32_t tile, const UmmaParams& p, uint32_t tiles_m, uint32_t tiles_n, uint32_t* tm, uint32_t* tn)
 {
-    const uint32_t per_group = g * tiles_n;
-    const uint32_t group = tile / per_group;
+    const uint32_t g = static_cast<uint32_t>(p.raster_group);
+    const uint32_t group = fast_div(tile, p.div_group);
     const uint32_t first_m = group * g;
-    const uint32_t rows = (tiles_m - first_m) < g ? (tiles_m - first_m) : g;
-    const uint32_t local = tile - group * per_group;
-    *tm = first_m + local % rows;
-    *tn = local / rows;
+    const bool whole = tiles_m - first_m >= g;
+    const uint32_t local = tile - group * g * tiles_n;
+    *tn = whole ? fast_div(local, p.div_rows) : fast_div(local, p.div_last_rows);
+    *tm = first_m + local - *tn * (whole ? g : tiles_m - first_m);
 }
 
 // A unit of work: one tile, or with split-K one range of a tile's k iterations.  Units are numbered
@@ -142,10 +144,11 @@ __device__ __forceinline__ WorkUnit decode_unit(uint32_t unit, const UmmaParams&
 {
     WorkUnit w;
     const uint32_t splits = static_cast<uint32_t>(p.k_splits);
-    const uint32_t tile = splits > 1 ? unit / splits : unit;
+    const uint32_t tile = splits > 1 ? fast_div(unit, p.div_splits) : unit;
     w.split = splits > 1 ? unit - tile * splits : 0u;
-    decode_tile(tile, tiles_m, tiles_n, static_cast<uint32_t>(p.raster_group), &w.tm, &w.tn);
-    if (p.tn_rotate) w.tn = (w.tn + static_cast<uint32_t>(p.tn_rotate)) % tiles_n;
+    decode_tile(tile, p, tiles_m, tiles_n, &w.tm, &w.tn);
+    w.tn += static_cast<uint32_t>(p.tn_rotate);   // (below tiles_n)
+    if (w.tn >= tiles_n) w.tn -= tiles_n;
     w.it0 = static_cast<int>(w.split) * p.k_iters_per_split;
     w.n_it = p.k_iters - w.it0 < p.k_iters_per_split ? p.k_iters - w.it0 : p.k_iters_per_split;
     return w;
@@ -161,9 +164,9 @@ __device__ __forceinline__ long long slab_c_offset(const UmmaOperandDev& o, uint
 #pragma unroll
     for (int d = 0; d < kMaxTmaRank; ++d) {
         if (d < o.n_row_digits) {
-            const uint32_t e = static_cast<uint32_t>(o.row_digit_ext[d]);
-            const uint32_t idx = rem % e;
-            rem /= e;
+            const uint32_t q = fast_div(rem, o.row_digit_ext[d]);
+            const uint32_t idx = rem - q * o.row_digit_ext[d].d;
+            rem = q;
             off += static_cast<long long>(idx) * o.row_digit_cstride[d];
             if (d == o.chunk_digit) *digit0 = static_cast<int>(idx);
         }
@@ -178,10 +181,58 @@ __device__ __forceinline__ long long slab_elem_offset(const UmmaOperandDev& o, i
 {
     if (o.split_inner > 0) {
         const int pos = digit0 * o.slab_w + in;
-        return static_cast<long long>(pos % o.split_inner) * o.row_elem_cstride +
-               static_cast<long long>(pos / o.split_inner) * o.split_outer_cstride;
+        const int outer = static_cast<int>(fast_div(static_cast<uint32_t>(pos), o.split_div));
+        return static_cast<long long>(pos - outer * o.split_inner) * o.row_elem_cstride +
+               static_cast<long long>(outer) * o.split_outer_cstride;
     }
     return static_cast<long long>(in) * o.row_elem_cstride;
+}
+
+// TMA coordinates of the box that starts at slab `s` (the k coordinates come on top).
+__device__ __forceinline__ void slab_coords(const UmmaOperandDev& o, uint32_t s, int (&base)[kMaxTmaRank])
+{
+#pragma unroll
+    for (int t = 0; t < kMaxTmaRank; ++t) base[t] = 0;
+    if (s < static_cast<uint32_t>(o.total_slabs)) {
+        uint32_t rem = s;
+#pragma unroll
+        for (int d = 0; d < kMaxTmaRank; ++d) {
+            if (d < o.n_row_digits) {
+                const uint32_t q = fast_div(rem, o.row_digit_ext[d]);
+                const int idx = static_cast<int>(rem - q * o.row_digit_ext[d].d);
+                rem = q;
+                const int v = d == o.chunk_digit ? idx * o.digit0_scale : idx;
+#pragma unroll
+                for (int t = 0; t < kMaxTmaRank; ++t)
+                    if (o.row_digit_dim[d] == t) base[t] = v;
+            }
+        }
+    } else {
+        // Slab beyond the tensor: start the box past the slab mode's end, TMA fills zeros.
+#pragma unroll
+        for (int t = 0; t < kMaxTmaRank; ++t)
+            if (o.row_digit_dim[o.chunk_digit] == t) base[t] = o.oob_coord;
+    }
+}
+
+// What one step of k digit 0, 1, 2 adds to each TMA coordinate of an operand, and the coordinates themselves.
+struct KSteps {
+    int s0[kMaxTmaRank], s1[kMaxTmaRank], s2[kMaxTmaRank];
+};
+__device__ __forceinline__ void k_steps(const UmmaOperandDev& o, KSteps& k)
+{
+#pragma unroll
+    for (int t = 0; t < kMaxTmaRank; ++t) {
+        k.s0[t] = o.k_digit_dim[0] == t ? o.k0_scale : 0;
+        k.s1[t] = o.k_digit_dim[1] == t ? 1 : 0;
+        k.s2[t] = o.k_digit_dim[2] == t ? 1 : 0;
+    }
+}
+// (a tensor dimension carries either a row digit or a k digit, so the two parts never meet in one coordinate)
+__device__ __forceinline__ void k_coords(const int (&base)[kMaxTmaRank], const KSteps& k, int kd0, int kd1, int kd2, int (&c)[kMaxTmaRank])
+{
+#pragma unroll
+    for (int t = 0; t < kMaxTmaRank; ++t) c[t] = base[t] + kd0 * k.s0[t] + kd1 * k.s1[t] + kd2 * k.s2[t];
 }
 
 }  // namespace

@@ -49,6 +49,15 @@ __device__ __forceinline__ unsigned int ld_relaxed(const unsigned int* addr)
     return v;
 }
 
+// One thread of a converged warp.  The compiler knows that a single thread runs behind this predicate and issues tensor
+// copies and MMAs, whose operands are warp-uniform registers, without a loop over the warp's lanes.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+    return leader != 0;
+}
+
 // Address of the same shared-memory location in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank)
 {
@@ -137,6 +146,139 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&v)[32])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Pace keeping: producer of block `blk` waits (bounded) until every producer has started block blk - pace_lead.
+// Returns false when the wait ran out.
+__device__ __forceinline__ bool keep_pace(const UmmaParams& p, int blk, unsigned int peers, long long* waits, long long* clk)
+{
+    red_add_relaxed(p.pace + 1 + blk, 1u);
+    if (blk < p.pace_lead) return true;
+    bool go = true;
+    const long long tp = p.prof ? clock64() : 0;
+    const unsigned int* behind = p.pace + 1 + blk - p.pace_lead;
+    unsigned long long t_start = 0;
+    while (ld_relaxed(behind) + ld_relaxed(p.pace) < peers) {
+        const unsigned long long now = global_timer();
+        if (t_start == 0) { t_start = now; ++*waits; }
+        else if (now - t_start > 50000ull) { go = false; break; }   // 50 us: somebody is not running; stop keeping pace
+    }
+    if (p.prof) *clk += clock64() - tp;
+    return go;
+}
+
+// Give the bulk copies issued into these barriers a bounded time to land before the CTA ends (after a wait gave up).
+__device__ __forceinline__ void drain_copies(uint32_t bar_full, int stages, uint32_t issued_mask, uint32_t issued_parity)
+{
+    for (int s = 0; s < stages; ++s) {
+        if (!(issued_mask & (1u << s))) continue;
+        const unsigned long long t0 = global_timer();
+        while (!mbar_try_wait(bar_full + 8u * static_cast<uint32_t>(s), (issued_parity >> s) & 1u))
+            if (global_timer() - t0 > 100000000ull) break;
+    }
+}
+
+// What both forms of the producer need to know about the CTA.
+struct ProducerEnv {
+    uint32_t smem, a_tile_bytes, stage_bytes, bar_full, bar_empty, abort_flag;
+    uint32_t rank, tiles_m, tiles_n, first_unit, unit_step, total_units;
+};
+
+// Producer whose stage is ONE copy per operand (merged or chunked boxes): a single elected thread waits, announces the
+// stage and issues both copies, with everything it needs in registers.  `pi` = which of NP producers this is.
+template <bool PAIR, int NP>
+__device__ __forceinline__ void produce_two_copies(const UmmaParams& p, const CUtensorMap& tmapA, const CUtensorMap& tmapB, const ProducerEnv& e, int pi)
+{
+    const int SA = p.a.slabs_per_tile, SB = p.b.slabs_per_tile;
+    const bool lead = !PAIR || e.rank == 0;
+    const uint32_t full_cluster = PAIR ? map_to_cta(e.bar_full, 0u) : e.bar_full;
+    const uint32_t tx = PAIR ? 2u * e.stage_bytes : e.stage_bytes;   // in a pair CTA 0 accounts for both CTAs' copies
+    const int stages = p.stages, ext0 = p.k_digit_ext[0], ext1 = p.k_digit_ext[1], skip = p.test_skip_iter;
+    KSteps ka, kb;
+    k_steps(p.a, ka);
+    k_steps(p.b, kb);
+    int stage = 0;
+    uint32_t phase = 0, issued_mask = 0, issued_parity = 0;
+    int cta_iter = 0;
+    const bool pacing = p.pace != nullptr && e.rank == 0 && pi == 0;
+    bool pace_live = pacing, have_slot = false;
+    const unsigned int peers = PAIR ? gridDim.x / 2u : gridDim.x;
+    const int pace_mask = (1 << p.pace_shift) - 1;
+    long long t_empty = 0, pace_waits = 0, pace_clk = 0;
+
+    int base_a_next[kMaxTmaRank], base_b_next[kMaxTmaRank];
+    WorkUnit w_next{};
+    auto look_up = [&](uint32_t unit) {
+        w_next = decode_unit(unit, p, e.tiles_m, e.tiles_n);
+        slab_coords(p.a, (PAIR ? 2u * w_next.tm + e.rank : w_next.tm) * SA, base_a_next);
+        slab_coords(p.b, w_next.tn * SB + (PAIR ? e.rank * (SB / 2) : 0u), base_b_next);
+    };
+    if (e.first_unit < e.total_units) look_up(e.first_unit);
+    for (uint32_t unit = e.first_unit; unit < e.total_units; unit += e.unit_step) {
+        const WorkUnit w = w_next;
+        int base_a[kMaxTmaRank], base_b[kMaxTmaRank];
+#pragma unroll
+        for (int t = 0; t < kMaxTmaRank; ++t) {
+            base_a[t] = base_a_next[t];
+            base_b[t] = base_b_next[t];
+        }
+        int kd0 = 0, kd1 = 0, kd2 = 0;
+        if (w.it0) {   // (a later k range of a split)
+            kd0 = w.it0 % ext0;
+            kd1 = w.it0 / ext0 % ext1;
+            kd2 = w.it0 / (ext0 * ext1);
+        }
+        for (int it = 0; it < w.n_it; ++it, ++cta_iter) {
+            if (NP == 1 || (cta_iter & 1) == pi) {
+                if (pace_live && (cta_iter & pace_mask) == 0) pace_live = keep_pace(p, cta_iter >> p.pace_shift, peers, &pace_waits, &pace_clk);
+                const uint32_t bar = 8u * static_cast<uint32_t>(stage);
+                const long long t0 = p.prof ? clock64() : 0;
+                const bool ok = have_slot || mbar_wait(e.bar_empty + bar, phase ^ 1u, e.abort_flag, 0, p.wait_limit_ns);
+                if (p.prof) t_empty += clock64() - t0;
+                if (ok && cta_iter != skip) {
+                    if (lead) mbar_arrive_expect_tx(e.bar_full + bar, tx);
+                    const uint32_t dst = e.smem + static_cast<uint32_t>(stage) * e.stage_bytes;
+                    int c[kMaxTmaRank];
+                    k_coords(base_a, ka, kd0, kd1, kd2, c);
+                    if (PAIR) tma_load_5d_pair(dst, &tmapA, full_cluster + bar, c[0], c[1], c[2], c[3], c[4]);
+                    else tma_load_5d(dst, &tmapA, full_cluster + bar, c[0], c[1], c[2], c[3], c[4]);
+                    k_coords(base_b, kb, kd0, kd1, kd2, c);
+                    if (PAIR) tma_load_5d_pair(dst + e.a_tile_bytes, &tmapB, full_cluster + bar, c[0], c[1], c[2], c[3], c[4]);
+                    else tma_load_5d(dst + e.a_tile_bytes, &tmapB, full_cluster + bar, c[0], c[1], c[2], c[3], c[4]);
+                    issued_mask |= 1u << stage;
+                    issued_parity = (issued_parity & ~(1u << stage)) | (phase << stage);
+                }
+            }
+            // the next unit's divisions run behind the first copies of this one
+            if (it == 0 && unit + e.unit_step < e.total_units) look_up(unit + e.unit_step);
+            if (++kd0 == ext0) {
+                kd0 = 0;
+                if (++kd1 == ext1) {
+                    kd1 = 0;
+                    ++kd2;
+                }
+            }
+            if (++stage == stages) {
+                stage = 0;
+                phase ^= 1u;
+            }
+            // one look at the stage of this thread's next iteration, so that its latency overlaps the copies just issued
+            if (NP == 1) {
+                have_slot = mbar_test_wait(e.bar_empty + 8u * static_cast<uint32_t>(stage), phase ^ 1u);
+            } else if ((cta_iter & 1) == pi) {
+                const int s2 = stage + 1 == stages ? 0 : stage + 1;
+                const uint32_t ph2 = stage + 1 == stages ? phase ^ 1u : phase;
+                have_slot = mbar_test_wait(e.bar_empty + 8u * static_cast<uint32_t>(s2), ph2 ^ 1u);
+            }
+        }
+    }
+    if (pacing) red_add_relaxed(p.pace, 1u);
+    if (p.prof && pi == 0) {
+        p.prof[blockIdx.x * 8 + 3] = t_empty;
+        p.prof[blockIdx.x * 8 + 6] = pace_clk;
+        p.prof[blockIdx.x * 8 + 7] = pace_waits * 2 + (pacing && !pace_live ? 1 : 0);
+    }
+    if (ld_shared_u32(e.abort_flag) && lead) drain_copies(e.bar_full, stages, issued_mask, issued_parity);
+}
+
 // PAIR = false: one CTA per 128 x BN tile (cta_group::1).
 // PAIR = true : a cluster of two CTAs per 256 x BN tile (cta_group::2).  CTA r of the pair stages its own
 //               128 rows of A and half of the B tile (no multicast; every copy is a plain TMA load into
@@ -210,7 +352,18 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
     const uint32_t first_unit = PAIR ? blockIdx.x / 2u : blockIdx.x;
     const uint32_t unit_step = PAIR ? gridDim.x / 2u : gridDim.x;
 
-    if (warp == 0 || (warp == 6 && NP == 2)) {
+    const bool producer = warp == 0 || (warp == 6 && NP == 2);
+    if (producer && SA == p.a.slabs_per_op && SBL == p.b.slabs_per_op) {
+        // ---------------- TMA producer, one copy per operand and stage ----------------
+        if (elect_one()) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmapA)) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmapB)) : "memory");
+            const ProducerEnv e = {smem_u32(smem), a_tile_bytes, stage_bytes, smem_u32(bar_full), smem_u32(bar_empty), abort_flag,
+                                   rank, tiles_m, tiles_n, first_unit, unit_step, total_tiles};
+            produce_two_copies<PAIR, NP>(p, tmapA, tmapB, e, warp == 0 ? 0 : 1);
+        }
+        __syncwarp();
+    } else if (producer) {
         // ---------------- TMA producer: lane i owns slab i of the stage ----------------
         // With two producers (p.producers == 2, an even number of stages) warp 0 fills the even k iterations of the
         // CTA and warp 6 the odd ones: the wait-announce-copy round trip of one warp may then take two stages' worth
@@ -244,35 +397,14 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
         // that its latency overlaps theirs; `have_slot` says that look found the stage free.
         bool have_slot = false;
 
-        // TMA coordinates of this lane's copy for the rows / columns of a work unit (the k coordinates come on top);
-        // worked out one unit ahead, so that the first copies of a unit do not wait for the divisions
+        // TMA coordinates of this lane's copy for the rows / columns of a work unit, worked out one unit ahead so that
+        // the first copies of a unit do not wait for the divisions
         auto unit_base = [&](const WorkUnit& u, int (&base)[kMaxTmaRank]) {
-#pragma unroll
-            for (int t = 0; t < kMaxTmaRank; ++t) base[t] = 0;
             if (!active) return;
-            const uint32_t s = is_a ? (PAIR ? 2u * u.tm + rank : u.tm) * SA + slab
-                                    : u.tn * SB + (PAIR ? rank * SBL : 0u) + slab;
-            if (s < static_cast<uint32_t>(o.total_slabs)) {
-                uint32_t rem = s;
-#pragma unroll
-                for (int d = 0; d < kMaxTmaRank; ++d) {
-                    if (d < o.n_row_digits) {
-                        const uint32_t e = static_cast<uint32_t>(o.row_digit_ext[d]);
-                        const int idx = static_cast<int>(rem % e);
-                        rem /= e;
-                        const int v = d == o.chunk_digit ? idx * o.digit0_scale : idx;
-#pragma unroll
-                        for (int t = 0; t < kMaxTmaRank; ++t)
-                            if (o.row_digit_dim[d] == t) base[t] = v;
-                    }
-                }
-            } else {
-                // Slab beyond the tensor: start the box past the slab mode's end, TMA fills zeros.
-#pragma unroll
-                for (int t = 0; t < kMaxTmaRank; ++t)
-                    if (o.row_digit_dim[o.chunk_digit] == t) base[t] = o.oob_coord;
-            }
+            slab_coords(o, is_a ? (PAIR ? 2u * u.tm + rank : u.tm) * SA + slab : u.tn * SB + (PAIR ? rank * SBL : 0u) + slab, base);
         };
+        KSteps ks;
+        k_steps(o, ks);
         WorkUnit w_next{};
         int base_next[kMaxTmaRank] = {0, 0, 0, 0, 0};
         if (first_unit < total_tiles) {
@@ -296,22 +428,8 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
             for (int it = 0; it < w.n_it; ++it, ++cta_iter) {
                 const bool mine = np == 1 || (cta_iter & 1) == pi;
                 if (mine && pace_live && (cta_iter & ((1 << p.pace_shift) - 1)) == 0) {
-                    const int blk = cta_iter >> p.pace_shift;
                     int go = 1;
-                    if (lane == 0) {
-                        red_add_relaxed(p.pace + 1 + blk, 1u);
-                        if (blk >= p.pace_lead) {
-                            const long long tp = p.prof ? clock64() : 0;
-                            const unsigned int* behind = p.pace + 1 + blk - p.pace_lead;
-                            unsigned long long t_start = 0;
-                            while (ld_relaxed(behind) + ld_relaxed(p.pace) < pace_peers) {
-                                const unsigned long long now = global_timer();
-                                if (t_start == 0) { t_start = now; ++pace_waits; }
-                                else if (now - t_start > 50000ull) { go = 0; break; }   // 50 us: somebody is not running; stop keeping pace
-                            }
-                            if (p.prof) pace_clk += clock64() - tp;
-                        }
-                    }
+                    if (lane == 0) go = keep_pace(p, cta_iter >> p.pace_shift, pace_peers, &pace_waits, &pace_clk) ? 1 : 0;
                     pace_live = __shfl_sync(0xffffffffu, go, 0) != 0;
                 }
                 const long long t0 = p.prof ? clock64() : 0;
@@ -324,13 +442,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
                     __syncwarp();
                     if (active) {
                         int c[kMaxTmaRank];
-#pragma unroll
-                        for (int t = 0; t < kMaxTmaRank; ++t) {
-                            c[t] = base[t];
-                            if (o.k_digit_dim[0] == t) c[t] = kd0 * o.k0_scale;
-                            if (o.k_digit_dim[1] == t) c[t] = kd1;
-                            if (o.k_digit_dim[2] == t) c[t] = kd2;
-                        }
+                        k_coords(base, ks, kd0, kd1, kd2, c);
                         const uint32_t dst = smem_u32(smem + static_cast<size_t>(stage) * stage_bytes + my_off);
                         if (PAIR) tma_load_5d_pair(dst, tmap, map_to_cta(smem_u32(bar_full + stage), 0u), c[0], c[1], c[2], c[3], c[4]);
                         else tma_load_5d(dst, tmap, smem_u32(bar_full + stage), c[0], c[1], c[2], c[3], c[4]);
@@ -365,18 +477,10 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
             p.prof[blockIdx.x * 8 + 6] = pace_clk;
             p.prof[blockIdx.x * 8 + 7] = pace_waits * 2 + (pacing && !pace_live ? 1 : 0);
         }
-        if (ld_shared_u32(abort_flag) && lane == 0 && rank == 0) {
-            // Give the bulk copies issued into this barrier a bounded time to land before the CTA ends.
-            for (int s = 0; s < p.stages; ++s) {
-                if (!(issued_mask & (1u << s))) continue;
-                const unsigned long long t0 = global_timer();
-                while (!mbar_try_wait(smem_u32(bar_full + s), (issued_parity >> s) & 1u))
-                    if (global_timer() - t0 > 100000000ull) break;
-            }
-        }
+        if (ld_shared_u32(abort_flag) && lane == 0 && rank == 0) drain_copies(smem_u32(bar_full), p.stages, issued_mask, issued_parity);
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(p.a.major) << 15) |
                                    (static_cast<uint32_t>(p.b.major) << 16) | (static_cast<uint32_t>(p.BN >> 3) << 17) |
                                    (static_cast<uint32_t>((PAIR ? 256 : 128) >> 4) << 24);
@@ -390,7 +494,12 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
             // Byte offset of MMA k step kk inside an operand's part of the stage.  MN-major: 1 024 bytes per step
             // (eight k rows of 128 bytes).  K-major: 32 bytes per step inside a 128-byte row of 32 k, and with a
             // k chunk of 64 the second 32 k lie one whole slab image (slab rows x 128 bytes) further on.
-            const uint32_t a_chunk = static_cast<uint32_t>(p.a.slab_w) * 128u, b_chunk = static_cast<uint32_t>(p.b.slab_w) * 128u;
+            const uint32_t a_step = p.a.major ? 1024u : 32u, b_step = p.b.major ? 1024u : 32u;
+            const uint32_t a_off[4] = {0u, a_step, 2u * a_step, 3u * a_step}, b_off[4] = {0u, b_step, 2u * b_step, 3u * b_step};
+            const uint32_t a_half = p.a.major ? 4096u : static_cast<uint32_t>(p.a.slab_w) * 128u;
+            const uint32_t b_half = p.b.major ? 4096u : static_cast<uint32_t>(p.b.slab_w) * 128u;
+            // descriptors without their start address, which is added as address / 16 (shared memory ends below 2^18)
+            const uint64_t a_desc = smem_desc(0u, a_lbo, a_sbo, a_type), b_desc = smem_desc(0u, b_lbo, b_sbo, b_type);
             const int ksteps = p.BK / 8;
             int stage = 0;
             uint32_t phase = 0;
@@ -413,12 +522,11 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
                         tcgen05_fence_after();
                         const uint32_t a_base = smem_u32(smem + static_cast<size_t>(stage) * stage_bytes);
                         const uint32_t b_base = a_base + a_tile_bytes;
-                        for (int kk = 0; kk < ksteps; ++kk) {
-                            const uint32_t ukk = static_cast<uint32_t>(kk);
-                            const uint32_t a_off = p.a.major ? ukk * 1024u : (ukk >> 2) * a_chunk + (ukk & 3u) * 32u;
-                            const uint32_t b_off = p.b.major ? ukk * 1024u : (ukk >> 2) * b_chunk + (ukk & 3u) * 32u;
-                            const uint64_t da = smem_desc(a_base + a_off, a_lbo, a_sbo, a_type);
-                            const uint64_t db = smem_desc(b_base + b_off, b_lbo, b_sbo, b_type);
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk) {
+                            if (kk >= ksteps) break;
+                            const uint64_t da = a_desc + ((a_base + (kk < 4 ? a_off[kk] : a_off[kk - 4] + a_half)) >> 4);
+                            const uint64_t db = b_desc + ((b_base + (kk < 4 ? b_off[kk] : b_off[kk - 4] + b_half)) >> 4);
                             if (PAIR) umma_tf32_pair(tmem_c, da, db, idesc, (it | kk) != 0 ? 1u : 0u);
                             else umma_tf32(tmem_c, da, db, idesc, (it | kk) != 0 ? 1u : 0u);
                         }
@@ -464,7 +572,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
             // this thread's row of C
             bool row_ok;
             int digit0 = 0;
-            const int a_slab = row / p.a.slab_w, a_in = row % p.a.slab_w;
+            const int a_slab = row >> p.a.slab_shift, a_in = row & (p.a.slab_w - 1);
             long long row_off = slab_c_offset(p.a, (PAIR ? 2u * tm + rank : tm) * SA + a_slab, &digit0, &row_ok);
             row_ok = row_ok && (digit0 * p.a.slab_w + a_in < p.a.slab_mode_ext);
             row_off += a_in * p.a.row_elem_cstride;
@@ -478,7 +586,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
                     bool ch_ok;
                     int d0 = 0;
                     const int j = et * 32;
-                    const int b_slab = j / p.b.slab_w, b_in = j % p.b.slab_w;
+                    const int b_slab = j >> p.b.slab_shift, b_in = j & (p.b.slab_w - 1);
                     const long long off = slab_c_offset(p.b, tn * SB + b_slab, &d0, &ch_ok);
                     int nvalid = p.b.slab_mode_ext - (d0 * p.b.slab_w + b_in);
                     nvalid = !ch_ok ? 0 : nvalid > 32 ? 32 : nvalid < 0 ? 0 : nvalid;
@@ -489,7 +597,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
                 for (int j = et; j < p.BN; j += 128) {
                     bool col_ok;
                     int d0 = 0;
-                    const int b_slab = j / p.b.slab_w, b_in = j % p.b.slab_w;
+                    const int b_slab = j >> p.b.slab_shift, b_in = j & (p.b.slab_w - 1);
                     long long off = slab_c_offset(p.b, tn * SB + b_slab, &d0, &col_ok);
                     col_ok = col_ok && (d0 * p.b.slab_w + b_in < p.b.slab_mode_ext);
                     st_shared_s64(cols + static_cast<uint32_t>(j) * 8u, col_ok ? off + b_in * p.b.row_elem_cstride : -1);
