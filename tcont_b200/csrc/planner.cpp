@@ -346,8 +346,9 @@ void merge_slabs(UmmaOperand* o, int BK, int cta_slabs)
     const int W = o->slab_w;  // 32 floats or 16 doubles
     if (o->major != 1 || o->rank > kMaxTmaRank - 1 || o->slab_dim != 0 || o->slab_mode_ext % W || o->slabs_per_op > 1) return;
     const int64_t chunks = o->slab_mode_ext / W;
+    // (with no other row digit a box may run over the last chunk: what lies past it is zero-filled like any slab past the tensor)
     int g = 1;
-    while (g * 2 <= cta_slabs && chunks % (g * 2) == 0 && cta_slabs % (g * 2) == 0) g *= 2;
+    while (g * 2 <= cta_slabs && (chunks % (g * 2) == 0 || o->n_row_digits == 1) && cta_slabs % (g * 2) == 0) g *= 2;
     if (g <= 1) return;
     UmmaOperand n = *o;
     int map[kMaxTmaRank];
@@ -418,6 +419,8 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
     // empty rows, and the table builder splits a row's position back into the two C modes.
     Problem p = p_in;
     int64_t split_inner[2] = {0, 0}, split_outer_cstride[2] = {0, 0};
+    // Float32 does the same: slabs of 32 pad an extent of 72 by a third.  A K-major operand is fused wherever whole
+    // 128-row slabs do not fit its first row mode, because one box of 128 rows then replaces up to 16 small ones.
     if (fuse_rows && !std::getenv("TCONT_NO_ROW_FUSION")) {
         for (int which = 0; which < 2; ++which) {
             std::vector<int>& t = which == 0 ? p.A : p.B;
@@ -713,21 +716,30 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
 // The tcgen05 kernel is planned twice where that can pay: with a k chunk of 64 on CTA pairs, and, where that
 // form does not apply (short or ragged contracted mode, too few tiles, a B tile that does not split), with the
 // 32-wide chunk on one CTA per tile.  TCONT_UMMA_BK=32 and TCONT_UMMA_PAIR=0 keep the second form.
+// Float32: what cannot be staged without operand-level fusion is not staged with it either.  Fusion makes tiles cheaper; it
+// must not take a contraction from IEEE single precision to TF32 (a fused mode can hide a stride TMA does not accept).
 void plan_umma(const Problem& p, const CostTable& cost, UmmaSpec* u)
 {
     if (p.scalar_type != 1) {
+        UmmaSpec plain;
+        plan_umma_impl(p, cost, &plain, 32, false);
+        if (!plain.eligible) {
+            *u = plain;
+            return;
+        }
         const char* bk = std::getenv("TCONT_UMMA_BK");
         const char* pr = std::getenv("TCONT_UMMA_PAIR");
         if (!(bk && std::atoi(bk) == 32) && !(pr && pr[0] == '0')) {
             UmmaSpec v;
-            plan_umma_impl(p, cost, &v, 64, false);
+            plan_umma_impl(p, cost, &v, 64, true);
             if (v.eligible && v.BK == 64) {
                 *u = v;
                 return;
             }
         }
-        *u = UmmaSpec();
-        plan_umma_impl(p, cost, u, 32, false);
+        UmmaSpec v;
+        plan_umma_impl(p, cost, &v, 32, true);
+        *u = v.eligible ? v : plain;
         return;
     }
     *u = UmmaSpec();
@@ -1093,6 +1105,15 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
                                  keepB ? roleB_src : leadB.first + korder + leadB.second};
             }
         }
+    }
+    // Float32, arithmetic-bound: both operands as matrices, A as [rows | K] and B as [K | columns], K in one order, so
+    // that the contracted modes fuse into one and (operand-level fusion in plan_umma) the rows do: no slab and no k chunk
+    // is padded.  abcd-aedf-fbec with extents of 72 computes 1.97 times its flops where the operands lie.
+    if (scalar_type == 0) {
+        std::string rowsA, rowsB;
+        for (char c : pl.modeC) (find_char(roleA_src, c) >= 0 ? rowsA : rowsB).push_back(c);
+        for (const std::string& korder : {sorted_by(roleB_src), sorted_by(roleA_src)})
+            if (!korder.empty() && !rowsB.empty()) candidates.push_back({rowsA + korder, korder + rowsB});
     }
     // (a transposed operand is a dense scratch tensor; one that is used where it lies keeps its parent's strides)
     const std::vector<int64_t>& roleA_parent = direct.swapped ? pl.parentB : pl.parentA;

@@ -575,12 +575,12 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
             const int a_slab = row >> p.a.slab_shift, a_in = row & (p.a.slab_w - 1);
             long long row_off = slab_c_offset(p.a, (PAIR ? 2u * tm + rank : tm) * SA + a_slab, &digit0, &row_ok);
             row_ok = row_ok && (digit0 * p.a.slab_w + a_in < p.a.slab_mode_ext);
-            row_off += a_in * p.a.row_elem_cstride;
+            row_off += slab_elem_offset(p.a, digit0, a_in);
             // Column offsets of this tile.  A 32-column chunk of the accumulator never straddles a
             // B slab when slabs are 32 or more columns wide, so one base offset and a valid-column
             // count per chunk suffice (chunk table); narrower slabs use a per-column table.
             const uint32_t cols = col_off + static_cast<uint32_t>(acc) * 256u * 8u;
-            const bool wide_slabs = p.b.slab_w >= 32;
+            const bool wide_slabs = p.b.slab_w >= 32 && p.b.split_inner == 0;
             if (wide_slabs) {
                 if (et < (p.BN >> 5)) {
                     bool ch_ok;
@@ -600,7 +600,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
                     const int b_slab = j >> p.b.slab_shift, b_in = j & (p.b.slab_w - 1);
                     long long off = slab_c_offset(p.b, tn * SB + b_slab, &d0, &col_ok);
                     col_ok = col_ok && (d0 * p.b.slab_w + b_in < p.b.slab_mode_ext);
-                    st_shared_s64(cols + static_cast<uint32_t>(j) * 8u, col_ok ? off + b_in * p.b.row_elem_cstride : -1);
+                    st_shared_s64(cols + static_cast<uint32_t>(j) * 8u, col_ok ? off + slab_elem_offset(p.b, d0, b_in) : -1);
                 }
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");

@@ -1,4 +1,4 @@
-"""The gather kernel's tiles and forms at the sizes where they can go wrong.
+"""The gather kernel's tiles and forms, and the operand layouts the tcgen05 kernel stages, at the sizes where they can go wrong.
 
 FP64 is held to the reference's criterion, Float32 on the gather kernel to plain IEEE single precision: every output is a
 chain of K fused multiply-adds, each off by at most half a unit in the last place of its partial sum, so that
@@ -9,6 +9,7 @@ import pytest
 
 from cases import to_equation
 from oracle_lib import F32, F64, Contraction
+from test_contraction_gpu import check, run_contraction
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +62,24 @@ def test_gather_kernel_forms(engine, oracle, monkeypatch, name, scalar):
         engine.launch(r)
         np.testing.assert_allclose(engine.copy_output_to_host(r).astype(np.float64), 3.0 * out.astype(np.float64), rtol=4 * unit, atol=0)
     assert seen >= (3 if scalar == F64 else 4)
+
+
+# both operands moved into matrices whose rows are two modes each: 72 = 2.25 slabs, fused 5 184 / 1 296 / ...
+MATRICES = {
+    "72_extents": ("abcd", "aedf", "fbec", dict(a=72, b=40, c=56, d=24, e=40, f=24)),
+    "runs_past_the_end": ("abcd", "aecf", "fbed", dict(a=40, b=72, c=56, d=24, e=40, f=40)),
+    "short_rows": ("abcd", "aecf", "fbed", dict(a=20, b=36, c=44, d=60, e=72, f=40)),
+}
+
+
+@pytest.mark.parametrize("name", list(MATRICES))
+@pytest.mark.parametrize("pair", ["auto", "0"])
+def test_float32_operands_as_matrices(engine, oracle, monkeypatch, name, pair):
+    modes = MATRICES[name]
+    if pair == "0":
+        monkeypatch.setenv("TCONT_UMMA_PAIR", "0")
+    c = Contraction(*modes[:3], modes[3], F32)
+    A, B = oracle.inputs(c, 7, -1.0, 1.0)
+    out, desc = run_contraction(engine, c, A, B, 2)
+    assert desc["kernel"] == "umma_tf32" and desc["backend"] == "ttgt", desc
+    check(oracle, c, A, B, out, desc)

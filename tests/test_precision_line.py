@@ -15,6 +15,7 @@ IEEE = {
     "ragged": (("abcd", "aebf", "fdec", dict(a=61, b=53, c=47, d=59, e=37, f=23)), 0),
 }
 TF32 = {
+    "matrices": (("abcd", "aedf", "fbec", dict(a=72, b=72, c=72, d=72, e=72, f=72)), 0),
     "k_majors_large": (("abcd", "eafb", "fdec", dict(a=72, b=72, c=72, d=72, e=72, f=72)), 0),
 }
 
