@@ -29,6 +29,7 @@
 // call (backends/ttgt_cutt/src/ttgt_cutt.cpp:764-809).
 #include <cuda.h>
 
+#include "chain.cuh"
 #include "kernels.hpp"
 #include "tile_common.cuh"
 
@@ -193,6 +194,8 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    chain_release();
+    chain_wait();
     __syncthreads();
 
     const uint32_t tiles_m = static_cast<uint32_t>(p.tiles_m), tiles_n = static_cast<uint32_t>(p.tiles_n);
@@ -512,9 +515,8 @@ template <bool AMN, bool BMN, int NF>
 cudaError_t launch_variant(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, unsigned grid, cudaStream_t stream)
 {
     const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
-    auto kernel = p.scaled ? dmma_tma_kernel<AMN, BMN, NF, true> : dmma_tma_kernel<AMN, BMN, NF, false>;
-    kernel<<<grid, kThreads64, smem_bytes, stream>>>(ta, tb, p);
-    return cudaGetLastError();
+    return launch_chained(p.scaled ? dmma_tma_kernel<AMN, BMN, NF, true> : dmma_tma_kernel<AMN, BMN, NF, false>, dim3(grid), dim3(kThreads64),
+                          static_cast<size_t>(smem_bytes), stream, 1, ta, tb, p);
 }
 
 template <int NF>

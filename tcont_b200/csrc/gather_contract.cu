@@ -16,6 +16,7 @@
 // (backends/cogent/plan/generators/kernels/kernel_body.py:1253+, kernel_compute.py:127-850).
 #include <cooperative_groups.h>
 
+#include "chain.cuh"
 #include "kernels.hpp"
 
 namespace tcontb {
@@ -270,6 +271,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     } else if (tid < STAGES * BK) {
         fill_k(tid / BK, tid / BK * BK, tid % BK);
     }
+    chain_release();
+    chain_wait();   // (everything above works on the parameters alone)
     __syncthreads();
 
 #pragma unroll
@@ -456,19 +459,8 @@ cudaError_t launch(GatherParams p, int num_sms, cudaStream_t stream)
     p.k_per_cta = (per + Cfg::BK - 1) / Cfg::BK * Cfg::BK;
     const long long tiles = tiles_m * tiles_n, resident = static_cast<long long>(num_sms) * Cfg::MINB;
     const long long grid = p.cluster > 1 ? tiles * p.cluster : !Cfg::FLAT || tiles < resident ? tiles : resident;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(grid));
-    cfg.blockDim = dim3(Cfg::THREADS);
-    cfg.dynamicSmemBytes = Cfg::SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(p.cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = p.cluster > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gather_contract_kernel<Cfg>, p);
+    return launch_chained(gather_contract_kernel<Cfg>, dim3(static_cast<unsigned>(grid)), dim3(Cfg::THREADS), Cfg::SMEM, stream,
+                          static_cast<unsigned>(p.cluster), p);
 }
 
 using F64Square = GatherCfg<double, 64, 64, 2, 2, 1, false, 4, 3>;

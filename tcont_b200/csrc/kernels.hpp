@@ -3,10 +3,33 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <utility>
 
 #include "planner.hpp"
 
 namespace tcontb {
+
+// Every kernel of a run is launched with this: its blocks may be scheduled, and set themselves up, while the kernel in front
+// of it in the stream drains; they wait (chain_wait in chain.cuh) before they touch global memory.
+template <typename... KernelArgs, typename... Args>
+cudaError_t launch_chained(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, unsigned cluster, Args&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 // ---- generic SIMT contraction (simt_contract.cu) -----------------------------------------
 // GEMM view with offset tables: C[offCm[m] + offCn[n]] = sum_k A[offAm[m] + offAk[k]] * B[offBn[n] + offBk[k]].

@@ -149,7 +149,7 @@ struct CostTable {
     double gather_gbs = 2200.0;             // tensors read and written once through element-wise gathers and stores
     double scatter_store_ps = 27.6;         // per element of C stored on its own (TMA-fed FP64 kernel)
     double scatter_store_f32_ps = 17.6;     // the same for the tcgen05 kernel's 4-byte elements
-    double launch_us = 6.9;                 // one more launch through the library (a contraction too small to matter, in a loop)
+    double launch_us = 4.0;                 // one more launch through the library (a contraction too small to matter, in a loop)
     // Fraction of the tcgen05 rate lost per unit of staged bytes whose K rows lie 2 MB or more apart, i.e. every row
     // of a TMA box in another 2 MB page (the calibration probe: the large 4-D configuration with f = 64, A's rows 8 MB
     // apart, half of a pair's bytes; the configuration itself: 18.7 ms where A lies against 14.1 ms through the

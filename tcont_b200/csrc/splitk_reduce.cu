@@ -12,6 +12,7 @@
 // cuBLAS (backends/ttgt_cutt/src/ttgt_cutt.cpp:764-809).
 #include <algorithm>
 
+#include "chain.cuh"
 #include "kernels.hpp"
 
 namespace tcontb {
@@ -22,6 +23,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const T* __restrict_
                                                            int splits, long long stride, bool vector_ok, bool scaled, T alpha,
                                                            T beta)
 {
+    chain_release();
+    chain_wait();
     const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
     long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (vector_ok) {
@@ -64,6 +67,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const T* __restrict_
 __global__ void __launch_bounds__(256) tf32_residual_kernel(const float* __restrict__ x, float* __restrict__ lo, long long elements,
                                                            bool vector_ok)
 {
+    chain_release();
+    chain_wait();
     const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
     long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     auto residual = [](float v) { return v - __uint_as_float(__float_as_uint(v) & 0xffffe000u); };
@@ -90,8 +95,7 @@ cudaError_t launch_tf32_residual(const float* x, float* lo, long long elements, 
     const bool vector_ok = reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(lo) % 16 == 0;
     const long long work = vector_ok ? (elements + 3) / 4 : elements;
     const unsigned grid = static_cast<unsigned>(std::min<long long>((work + 255) / 256, 148ll * 8));
-    tf32_residual_kernel<<<grid, 256, 0, stream>>>(x, lo, elements, vector_ok);
-    return cudaGetLastError();
+    return launch_chained(tf32_residual_kernel, dim3(grid), dim3(256), 0, stream, 1, x, lo, elements, vector_ok);
 }
 
 cudaError_t launch_splitk_reduce(const void* partial, void* C, long long elements, int splits, long long stride, int elt_bytes,
@@ -105,13 +109,10 @@ cudaError_t launch_splitk_reduce(const void* partial, void* C, long long element
     const long long work = vector_ok ? (elements + w - 1) / w : elements;
     const unsigned grid = static_cast<unsigned>(std::min<long long>((work + 255) / 256, 148ll * 8));
     if (elt_bytes == 8)
-        splitk_reduce_kernel<double, double2, 2><<<grid, 256, 0, stream>>>(static_cast<const double*>(partial), static_cast<double*>(C),
-                                                                            elements, splits, stride, vector_ok, scaled, alpha, beta);
-    else
-        splitk_reduce_kernel<float, float4, 4><<<grid, 256, 0, stream>>>(static_cast<const float*>(partial), static_cast<float*>(C),
-                                                                          elements, splits, stride, vector_ok, scaled,
-                                                                          static_cast<float>(alpha), static_cast<float>(beta));
-    return cudaGetLastError();
+        return launch_chained(splitk_reduce_kernel<double, double2, 2>, dim3(grid), dim3(256), 0, stream, 1, static_cast<const double*>(partial),
+                              static_cast<double*>(C), elements, splits, stride, vector_ok, scaled, alpha, beta);
+    return launch_chained(splitk_reduce_kernel<float, float4, 4>, dim3(grid), dim3(256), 0, stream, 1, static_cast<const float*>(partial),
+                          static_cast<float*>(C), elements, splits, stride, vector_ok, scaled, static_cast<float>(alpha), static_cast<float>(beta));
 }
 
 }  // namespace tcontb

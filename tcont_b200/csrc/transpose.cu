@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "chain.cuh"
 #include "kernels.hpp"
 
 namespace tcontb {
@@ -83,6 +84,8 @@ struct VecOf<double> {
 template <typename T, int VEC, typename I>
 __global__ void __launch_bounds__(256) permute_rows_kernel(const T* __restrict__ src, T* __restrict__ dst, TransposeParams p)
 {
+    chain_release();
+    chain_wait();
     constexpr int UNROLL = 4;
     const I vec_per_row = static_cast<I>(p.ext[0] / VEC);
     const I total = static_cast<I>(p.elements / VEC);
@@ -151,6 +154,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 6) permute_tiled_ker
         sbase += idx * p.src_stride[i];
         dbase += idx * p.dst_stride[i];
     }
+    chain_release();
+    chain_wait();
     const int64_t e0 = p.ext[0], e1 = p.ext[g.d0];
     const int64_t s1 = p.src_stride[g.d0];  // source stride of mode d0
     const int64_t d0s = p.dst_stride[0];    // destination stride of source mode 0
@@ -233,11 +238,10 @@ cudaError_t launch_typed(const T* src, T* dst, const TransposeParams& p, cudaStr
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((total + 4 * 256 - 1) / (4 * 256), int64_t(sms) * 16));
         const bool small = p.elements < (int64_t(1) << 31);
-        if (vec && small) permute_rows_kernel<T, VMAX, uint32_t><<<blocks, 256, 0, stream>>>(src, dst, p);
-        else if (vec) permute_rows_kernel<T, VMAX, int64_t><<<blocks, 256, 0, stream>>>(src, dst, p);
-        else if (small) permute_rows_kernel<T, 1, uint32_t><<<blocks, 256, 0, stream>>>(src, dst, p);
-        else permute_rows_kernel<T, 1, int64_t><<<blocks, 256, 0, stream>>>(src, dst, p);
-        return cudaGetLastError();
+        if (vec && small) return launch_chained(permute_rows_kernel<T, VMAX, uint32_t>, dim3(blocks), dim3(256), 0, stream, 1, src, dst, p);
+        if (vec) return launch_chained(permute_rows_kernel<T, VMAX, int64_t>, dim3(blocks), dim3(256), 0, stream, 1, src, dst, p);
+        if (small) return launch_chained(permute_rows_kernel<T, 1, uint32_t>, dim3(blocks), dim3(256), 0, stream, 1, src, dst, p);
+        return launch_chained(permute_rows_kernel<T, 1, int64_t>, dim3(blocks), dim3(256), 0, stream, 1, src, dst, p);
     }
     bool strides_ok = true;
     for (int i = 1; i < p.rank; ++i) strides_ok = strides_ok && p.src_stride[i] % VMAX == 0;
@@ -269,11 +273,10 @@ cudaError_t launch_typed(const T* src, T* dst, const TransposeParams& p, cudaStr
         if (i != d0) blocks *= p.ext[i];
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(g.t1) * static_cast<size_t>(g.t0 + 1) * sizeof(T);   // at most 37 KB
-    if (vec && fixed) permute_tiled_kernel<T, VMAX, true><<<static_cast<unsigned>(blocks), 256, smem, stream>>>(src, dst, p, g);
-    else if (vec) permute_tiled_kernel<T, VMAX, false><<<static_cast<unsigned>(blocks), 256, smem, stream>>>(src, dst, p, g);
-    else if (fixed) permute_tiled_kernel<T, 1, true><<<static_cast<unsigned>(blocks), 256, smem, stream>>>(src, dst, p, g);
-    else permute_tiled_kernel<T, 1, false><<<static_cast<unsigned>(blocks), 256, smem, stream>>>(src, dst, p, g);
-    return cudaGetLastError();
+    if (vec && fixed) return launch_chained(permute_tiled_kernel<T, VMAX, true>, dim3(static_cast<unsigned>(blocks)), dim3(256), smem, stream, 1, src, dst, p, g);
+    if (vec) return launch_chained(permute_tiled_kernel<T, VMAX, false>, dim3(static_cast<unsigned>(blocks)), dim3(256), smem, stream, 1, src, dst, p, g);
+    if (fixed) return launch_chained(permute_tiled_kernel<T, 1, true>, dim3(static_cast<unsigned>(blocks)), dim3(256), smem, stream, 1, src, dst, p, g);
+    return launch_chained(permute_tiled_kernel<T, 1, false>, dim3(static_cast<unsigned>(blocks)), dim3(256), smem, stream, 1, src, dst, p, g);
 }
 
 }  // namespace

@@ -21,6 +21,7 @@
 #include <cuda.h>
 #include <cstdlib>
 
+#include "chain.cuh"
 #include "kernels.hpp"
 #include "tile_common.cuh"
 
@@ -340,6 +341,8 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
         }
     }
     tcgen05_fence_before();
+    chain_release();
+    chain_wait();
     __syncthreads();
     if (PAIR) cluster_sync_all();  // the partner's barriers exist before anything signals them
     tcgen05_fence_after();
@@ -765,6 +768,9 @@ cudaError_t launch_umma_tf32(const UmmaParams& p, const void* tmapA, const void*
 {
     const CUtensorMap& ta = *static_cast<const CUtensorMap*>(tmapA);
     const CUtensorMap& tb = *static_cast<const CUtensorMap*>(tmapB);
+    // One persistent CTA per SM, also when its ring is small: CTAs that are scheduled while the kernel in front still
+    // occupies some SMs would otherwise pair up on the others (low-K configuration behind its transposes: 390 us, not 205)
+    smem_bytes = smem_bytes > kMaxDynamicSmemBytes / 2 + 1024 ? smem_bytes : kMaxDynamicSmemBytes / 2 + 1024;
     // (tuning switch TCONT_UMMA_IDLE_WARP=1: launch the seventh warp although nothing uses it)
     static const bool idle_warp = std::getenv("TCONT_UMMA_IDLE_WARP") != nullptr;
     const unsigned threads = p.producers == 2 || idle_warp ? kThreads : kThreads - 32;
@@ -774,27 +780,14 @@ cudaError_t launch_umma_tf32(const UmmaParams& p, const void* tmapA, const void*
         const long long clusters = units < num_sms / 2 ? units : num_sms / 2;
         auto kernel = p.scaled ? (p.producers == 2 ? umma_tf32_kernel<true, 2, true> : umma_tf32_kernel<true, 1, true>)
                                : (p.producers == 2 ? umma_tf32_kernel<true, 2, false> : umma_tf32_kernel<true, 1, false>);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
-        cfg.blockDim = dim3(threads);
-        cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kernel, ta, tb, p);
+        return launch_chained(kernel, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads), static_cast<size_t>(smem_bytes), stream, 2, ta, tb, p);
     }
     const long long total = p.tiles_m * p.tiles_n * p.k_splits;
     if (total <= 0) return cudaErrorInvalidValue;
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
     auto kernel = p.scaled ? (p.producers == 2 ? umma_tf32_kernel<false, 2, true> : umma_tf32_kernel<false, 1, true>)
                            : (p.producers == 2 ? umma_tf32_kernel<false, 2, false> : umma_tf32_kernel<false, 1, false>);
-    kernel<<<grid, threads, smem_bytes, stream>>>(ta, tb, p);
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(grid), dim3(threads), static_cast<size_t>(smem_bytes), stream, 1, ta, tb, p);
 }
 
 }  // namespace tcontb
