@@ -109,8 +109,10 @@ tcontb_status tcontb_run_upload_inputs(tcontb_run* run, const void* a_host, cons
 
 /* Beyond the reference, whose backends always overwrite (alpha = 1, beta = 0: cublasGemmEx scalars at
  * backends/ttgt_cutt/src/ttgt_cutt.cpp:742-743, generated kernels store a zeroed accumulator): later
- * launches compute C = alpha * (A*B) + beta * C.  The kernel that writes C applies the scalars (the
- * partial-sum pass where k is split); C is read only when beta is not zero.  Not available on a
+ * launches compute C = alpha * (A*B) + beta * C.  The kernel that writes C applies the scalars, or
+ * the partial-sum pass where k is split and for some FP64 runs with a C of up to 64 MB (whose
+ * workspace of the size of C this call allocates); C is read only when beta is not zero.  Not
+ * available on a
  * run that spans several GPUs. */
 tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta);
 

@@ -411,22 +411,25 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
 #pragma unroll
             for (int j = 0; j < NF; ++j)
                 cn[j] = ld_shared_s64(col_tab + (static_cast<uint32_t>(wn * NF * 8 + 16 * (j >> 1) + (j & 1)) + 2u * fr) * 8u);
-            // alpha and beta on the four elements of every column fragment; all old values are asked for before the first is
-            // used (a round trip to L2 per two fragments cost 2 800 cycles a tile)
+            // alpha and beta on the four elements of every column fragment; the old values of two fragments are asked
+            // for before the first is used (four at a time spill: 228 us where two at a time take 220)
             auto scale_four = [&](long long cm0, long long cm1, long long cm2, long long cm3, bool run4, auto&& at) {
-                double old[NF][4];
 #pragma unroll
-                for (int j = 0; j < NF; ++j) {
-                    const long long c = cn[j];
-                    if (tile_ok && c >= 0 && p.beta != 0.0)
-                        load_old4(old[j], C + cm0 + c, run4 && (reinterpret_cast<uintptr_t>(C + cm0 + c) & 31u) == 0, cm0 >= 0 ? C + cm0 + c : nullptr,
-                                  cm1 >= 0 ? C + cm1 + c : nullptr, cm2 >= 0 ? C + cm2 + c : nullptr, cm3 >= 0 ? C + cm3 + c : nullptr);
-                    else old[j][0] = old[j][1] = old[j][2] = old[j][3] = 0.0;
+                for (int j0 = 0; j0 < NF; j0 += 2) {
+                    double old[2][4];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const long long c = cn[j0 + u];
+                        if (tile_ok && c >= 0 && p.beta != 0.0)
+                            load_old4(old[u], C + cm0 + c, run4 && (reinterpret_cast<uintptr_t>(C + cm0 + c) & 31u) == 0, cm0 >= 0 ? C + cm0 + c : nullptr,
+                                      cm1 >= 0 ? C + cm1 + c : nullptr, cm2 >= 0 ? C + cm2 + c : nullptr, cm3 >= 0 ? C + cm3 + c : nullptr);
+                        else old[u][0] = old[u][1] = old[u][2] = old[u][3] = 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) at(j0 + u, q) = p.alpha * at(j0 + u, q) + p.beta * old[u][q];
                 }
-#pragma unroll
-                for (int j = 0; j < NF; ++j)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) at(j, q) = p.alpha * at(j, q) + p.beta * old[j][q];
             };
             if (p.store_across_slabs) {
                 // The warp's 64 rows are four slabs of 16; slab q is index a0 + q of C's stride-1 mode and the rows

@@ -12,6 +12,12 @@
 // of k, and the partial tiles are added through distributed shared memory in ascending rank order (one launch,
 // deterministic).
 //
+// What bounds it: large problems the FP64 pipe or the FP32 pipe (5 184^3: FP64 30.0 TFLOP/s, Float32 40, where the 64 x 64
+// kernel before it had 23.7; 3233 x 2773 x 851 FP64 1 055 -> 640 us), small ones the time a lone block needs per k tile (0.5 us
+// in the 32 x 32 Float32 tile, 1.1 with a fourth of its warps; 0.7 / 1.5 us in the FP64 tiles of 32 / 64) and the way from
+// launch to launch (693 x 47 x 41 Float32 8.2 -> 4.0 us), short contracted extents the stores of C (48825 x 2627 x 7 Float32
+// 332 -> 208 us, 2.5 TB/s of odd-aligned runs).
+//
 // Stands where the reference runs its generated kernels for descriptors of any shape
 // (backends/cogent/plan/generators/kernels/kernel_body.py:1253+, kernel_compute.py:127-850).
 #include <cooperative_groups.h>
