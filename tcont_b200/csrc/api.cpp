@@ -956,7 +956,7 @@ tcontb_status tcontb_run_upload_inputs(tcontb_run* run, const void* a_host, cons
 }
 
 // The TMA-fed FP64 kernel with a C of up to half of L2: its tiles wait for the old values of C, while a workspace written by
-// the kernel and read by the partial-sum pass stays in L2 (C of 38 MB: 40 us in two passes, 43 in one; of 302 MB: 259 and 220).
+// the kernel and read by the partial-sum pass stays in L2 (C of 38 MB: 37 us in two passes, 43 in one; of 302 MB: 259 and 220).
 static bool scales_in_a_second_pass(const tcontb_run* run)
 {
     return run->plan.kernel == KERNEL_DMMA_F64_TMA && !run->splitk.ptr && run->plan.sizeC * static_cast<int64_t>(run->elt) <= (int64_t(64) << 20);
