@@ -111,6 +111,12 @@ struct DeviceBuffer {
         if (ptr) cudaFree(ptr);
     }
     cudaError_t alloc(size_t bytes) { return cudaMalloc(&ptr, bytes ? bytes : 1); }
+    cudaError_t release()
+    {
+        const cudaError_t e = ptr ? cudaFree(ptr) : cudaSuccess;
+        ptr = nullptr;
+        return e;
+    }
 };
 
 // Restores the device that was current when a multi-GPU function started, on every way out of it.
@@ -168,6 +174,7 @@ struct tcontb_run {
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool ev_valid = false;
     int64_t kernels_per_launch = 0;
+    bool half_built = false;  // a second set-up failed: nothing may be launched
     // Several GPUs of one box behind one run (TCONT_NUM_GPUS > 1): the contraction is cut along an
     // external mode, shard g lives on device first_device + g and is an ordinary run of the
     // smaller contraction; this object then only keeps the global host inputs.
@@ -517,6 +524,23 @@ tcontb_status finish_run(tcontb_run* run)
     if (run->stage_timing)
         for (auto& e : run->ev) TC_CUDA(cudaEventCreate(&e));
     return TCONTB_OK;
+}
+
+// The run with another plan of the same contraction (set-up only: no launch of it may be recorded in a graph yet).
+tcontb_status set_up_again(tcontb_run* run, const Plan& plan)
+{
+    for (DeviceBuffer* b : {&run->tbufA, &run->tbufB, &run->status, &run->splitk, &run->loA, &run->loB, &run->prof, &run->pace, &run->scaled_ws})
+        TC_CUDA(b->release());   // (waits for what still uses them)
+    for (auto& e : run->ev) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
+    run->ev_valid = false;
+    run->plan = plan;
+    run->half_built = true;
+    const tcontb_status st = finish_run(run);
+    if (st == TCONTB_OK) run->half_built = false;
+    return st;
 }
 
 tcontb_status alloc_owned(tcontb_run* run)
@@ -1021,6 +1045,7 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         for (size_t g = 1; g < run->shards.size(); ++g) TC_CUDA(cudaStreamWaitEvent(nullptr, run->shard_done[g], 0));
         return TCONTB_OK;
     }
+    if (run->half_built) return fail(TCONTB_RUNTIME_ERROR, "the run's set-up failed");
     const Plan& pl = run->plan;
     const bool t = run->stage_timing;
     // Other scalars than (1, 0): the contraction kernel's epilogue applies them, or the partial-sum pass of a split-K run
@@ -1310,22 +1335,28 @@ tcontb_status tcontb_run_ksplit_enable(tcontb_run* run, int world, int rank)
     TC_NOT_SHARDED(run, "tcontb_run_ksplit_enable");
     if (world < 2 || world > kMaxOwners || rank < 0 || rank >= world) return fail(TCONTB_INVALID_ARGUMENT, "contracted-mode split: need 2..8 ranks and 0 <= rank < ranks");
     if (run->ks.world) return fail(TCONTB_INVALID_ARGUMENT, "contracted-mode split is already enabled on this run");
+    if (run->plan.prob.strided) return fail(TCONTB_UNSUPPORTED, "contracted-mode split is not available on sub-tensor views");
+    std::string why;
+    if (!cuts_into_ranges(run->plan, world, &why)) {
+        // Rows fused across modes, or an operand moved into a matrix, move the edges of the tile columns: staged mode by
+        // mode the ranges may still end where a tile does.
+        const Plan& d = run->plan;
+        bool cut = false;
+        for (int selection = d.backend_selection; !cut && selection <= (d.backend_selection ? d.backend_selection : 2); ++selection) {
+            Plan plain;
+            std::string err, other;
+            if (make_plan(d.modeC.data(), static_cast<int>(d.modeC.size()), d.modeA.data(), static_cast<int>(d.modeA.size()), d.modeB.data(),
+                          static_cast<int>(d.modeB.size()), d.op, d.scalar_type, d.ext_mode.data(), d.ext_val.data(),
+                          static_cast<int>(d.ext_val.size()), selection, device_cost_table(), &plain, &err, nullptr, nullptr, nullptr, false) ||
+                !cuts_into_ranges(plain, world, &other)) continue;
+            cut = true;
+            const tcontb_status st = set_up_again(run, plain);
+            if (st != TCONTB_OK) return st;
+        }
+        if (!cut) return fail(TCONTB_UNSUPPORTED, why);
+    }
+    if (run->tf32x3) return fail(TCONTB_UNSUPPORTED, "contracted-mode split is not available with error-compensated Float32");
     const Plan& pl = run->plan;
-    const Problem& p = pl.prob;
-    const UmmaSpec& u = pl.umma;
-    if (p.strided) return fail(TCONTB_UNSUPPORTED, "contracted-mode split is not available on sub-tensor views");
-    if (pl.kernel != KERNEL_UMMA_TF32 || u.k_splits != 1 || run->tf32x3)
-        return fail(TCONTB_UNSUPPORTED, "contracted-mode split needs the tcgen05 kernel without split-K (Float32 operands TMA can stage; TCONT_SPLITK=1)");
-    // C's slowest mode must be a column mode of the kernel (role B), the most significant digit of the column
-    // slab index, and its ranges must fall on tile-column boundaries: a tile then has exactly one owner.
-    if (p.C.empty() || p.N.empty() || p.C.back() != p.N.back())
-        return fail(TCONTB_UNSUPPORTED, "contracted-mode split: C's slowest mode must belong to the operand that does not hold C's stride-1 mode");
-    const Mode& slow = p.modes[static_cast<size_t>(p.C.back())];
-    const int64_t sb = u.b.slabs_per_tile;
-    const bool single = p.N.size() == 1;
-    if (slow.extent % world || u.b.total_slabs % world || (u.b.total_slabs / world) % sb || u.tiles_n % world || pl.sizeC % world ||
-        (single && (slow.extent / world) % u.b.slab_w))
-        return fail(TCONTB_UNSUPPORTED, "contracted-mode split: the extent of C's slowest mode does not cut into whole tile columns per rank");
     auto& ks = run->ks;
     ks.chunk = pl.sizeC / world;
     if ((static_cast<size_t>(ks.chunk) * run->elt) % 16) return fail(TCONTB_UNSUPPORTED, "contracted-mode split: a rank's range of C is not a multiple of 16 bytes");

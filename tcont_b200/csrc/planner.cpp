@@ -718,7 +718,7 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
 // 32-wide chunk on one CTA per tile.  TCONT_UMMA_BK=32 and TCONT_UMMA_PAIR=0 keep the second form.
 // Float32: what cannot be staged without operand-level fusion is not staged with it either.  Fusion makes tiles cheaper; it
 // must not take a contraction from IEEE single precision to TF32 (a fused mode can hide a stride TMA does not accept).
-void plan_umma(const Problem& p, const CostTable& cost, UmmaSpec* u)
+void plan_umma(const Problem& p, const CostTable& cost, UmmaSpec* u, bool fuse_rows = true)
 {
     if (p.scalar_type != 1) {
         UmmaSpec plain;
@@ -731,14 +731,14 @@ void plan_umma(const Problem& p, const CostTable& cost, UmmaSpec* u)
         const char* pr = std::getenv("TCONT_UMMA_PAIR");
         if (!(bk && std::atoi(bk) == 32) && !(pr && pr[0] == '0')) {
             UmmaSpec v;
-            plan_umma_impl(p, cost, &v, 64, true);
+            plan_umma_impl(p, cost, &v, 64, fuse_rows);
             if (v.eligible && v.BK == 64) {
                 *u = v;
                 return;
             }
         }
         UmmaSpec v;
-        plan_umma_impl(p, cost, &v, 32, true);
+        plan_umma_impl(p, cost, &v, 32, fuse_rows);
         *u = v.eligible ? v : plain;
         return;
     }
@@ -978,7 +978,7 @@ CostTable load_cost_table()
 
 int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* modeB, int nB, char op, int scalar_type,
               const char* ext_mode, const int64_t* ext_val, int n_ext, int backend_selection, const CostTable& cost,
-              Plan* plan, std::string* err, const int64_t* parentC, const int64_t* parentA, const int64_t* parentB)
+              Plan* plan, std::string* err, const int64_t* parentC, const int64_t* parentA, const int64_t* parentB, bool fuse_rows)
 {
     if (!plan || !err) return 1;
     if (nC < 0 || nA < 0 || nB < 0 || n_ext < 0 || nC > kMaxModes || nA > kMaxModes || nB > kMaxModes || n_ext > 64) {
@@ -1032,7 +1032,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     pl.flops = 2.0 * std::sqrt(double(pl.sizeL) * double(pl.sizeR) * double(pl.sizeC));
 
     UmmaSpec direct_umma;
-    plan_umma(direct, cost, &direct_umma);
+    plan_umma(direct, cost, &direct_umma, fuse_rows);
     int direct_kernel = pick_kernel(direct, direct_umma, cost);
 
     // Transpose-assisted candidate.  A role's transposed layout is
@@ -1109,7 +1109,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     // Float32, arithmetic-bound: both operands as matrices, A as [rows | K] and B as [K | columns], K in one order, so
     // that the contracted modes fuse into one and (operand-level fusion in plan_umma) the rows do: no slab and no k chunk
     // is padded.  abcd-aedf-fbec with extents of 72 computes 1.97 times its flops where the operands lie.
-    if (scalar_type == 0) {
+    if (scalar_type == 0 && fuse_rows) {
         std::string rowsA, rowsB;
         for (char c : pl.modeC) (find_char(roleA_src, c) >= 0 ? rowsA : rowsB).push_back(c);
         for (const std::string& korder : {sorted_by(roleB_src), sorted_by(roleA_src)})
@@ -1175,7 +1175,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         rc = problem_of(candidates[i], &q);
         if (rc) return rc;
         UmmaSpec u;
-        if (tf32) plan_umma(q, cost, &u);
+        if (tf32) plan_umma(q, cost, &u, fuse_rows);
         const int kernel = pick_kernel(q, u, cost);
         const double us = transposes_us(candidates[i], cost) + contraction_us(q, kernel, u, cost);
         if (us < 0.97 * pl.est_ttgt_us) {   // (an alternative has to be clearly better than the first)
@@ -1220,6 +1220,28 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     return 0;
 }
 
+bool cuts_into_ranges(const Plan& pl, int ranges, std::string* why)
+{
+    const Problem& p = pl.prob;
+    const UmmaSpec& u = pl.umma;
+    if (pl.kernel != KERNEL_UMMA_TF32 || u.k_splits != 1) {
+        *why = "contracted-mode split needs the tcgen05 kernel without split-K (Float32 operands TMA can stage; TCONT_SPLITK=1)";
+        return false;
+    }
+    if (p.C.empty() || p.N.empty() || p.C.back() != p.N.back()) {
+        *why = "contracted-mode split: C's slowest mode must belong to the operand that does not hold C's stride-1 mode";
+        return false;
+    }
+    *why = "contracted-mode split: the extent of C's slowest mode does not cut into whole tile columns per rank";
+    const Mode& slow = p.modes[static_cast<size_t>(p.C.back())];
+    if (slow.extent % ranges || pl.sizeC % ranges || u.tiles_n % ranges) return false;
+    const int64_t tile_slabs = u.b.slabs_per_tile;
+    // One row digit: the slab mode is all of N (one mode, or two fused ones), so a range ends inside it, and has to end where
+    // a tile does.  More digits: C's slowest mode is the most significant one, and a range is whole indices of it.
+    if (u.b.n_row_digits == 1) return (u.b.slab_mode_ext / ranges) % (u.b.slab_w * tile_slabs) == 0;
+    return u.b.total_slabs % ranges == 0 && (u.b.total_slabs / ranges) % tile_slabs == 0;
+}
+
 std::string describe_plan(const Plan& pl)
 {
     std::ostringstream o;
@@ -1259,7 +1281,12 @@ std::string describe_plan(const Plan& pl)
           << ",\"a_slab_w\":" << u.a.slab_w << ",\"b_slab_w\":" << u.b.slab_w << ",\"a_slabs_per_copy\":" << u.a.slabs_per_op << ",\"b_slabs_per_copy\":" << u.b.slabs_per_op << ",\"a_slabs\":" << u.a.slabs_per_tile
           << ",\"b_slabs\":" << u.b.slabs_per_tile << ",\"smem_bytes\":" << u.smem_bytes
           << ",\"coalesced_store\":" << (u.a.row_elem_cstride == 1 ? "true" : "false")
-          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"producers\":" << u.producers;
+          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"producers\":" << u.producers
+          << ",\"a_fused\":" << u.a.split_inner << ",\"b_fused\":" << u.b.split_inner << ",\"column_ranges\":[";
+        std::string why;
+        for (int r = 2, n = 0; r <= 8; ++r)
+            if (cuts_into_ranges(pl, r, &why)) o << (n++ ? "," : "") << r;
+        o << "]";
     }
     o << "}}";
     return o.str();

@@ -191,7 +191,11 @@ struct Plan {
 int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* modeB, int nB, char op, int scalar_type,
               const char* ext_mode, const int64_t* ext_val, int n_ext, int backend_selection, const CostTable& cost,
               Plan* plan, std::string* err, const int64_t* parentC = nullptr, const int64_t* parentA = nullptr,
-              const int64_t* parentB = nullptr);
+              const int64_t* parentB = nullptr, bool fuse_rows = true);
+
+// Whether C, cut into `ranges` equal contiguous ranges along its slowest mode, is cut along whole tile columns of the
+// tcgen05 kernel (each column of tiles then has exactly one owner); `why` receives the reason if not.
+bool cuts_into_ranges(const Plan& plan, int ranges, std::string* why);
 
 std::string describe_plan(const Plan& plan);
 // Defaults, overridden by the "key value" file TCONT_COST_TABLE names, if any.

@@ -194,3 +194,43 @@ def test_contracted_split_on_cta_pairs(engine, oracle, monkeypatch):
     trunc = oracle.contract(c, A, B, rounding=1)
     scale = oracle.contract(c, np.abs(A), np.abs(B), rounding=1)
     assert float((np.abs(got.astype(np.float64) - trunc) / (scale + 1e-30)).max()) < 2e-5
+
+
+@needs_two
+@pytest.mark.parametrize("ext_c,ext_d", [(40, 12), (36, 28)])
+def test_contracted_split_of_fused_columns(engine, oracle, monkeypatch, ext_c, ext_d):
+    """Two ranks as two runs on one device (their kernels do not wait for one another).  Modes c and d of B are staged as one
+    fused mode whose halves do not end where a tile column does (15 slabs; 31.5 slabs); staged mode by mode, c takes two
+    slabs for each d and they do."""
+    import torch
+    from tcont_b200 import api, sharding
+    monkeypatch.setenv("TCONT_SPLITK", "1")
+    c = Contraction("acbd", "abk", "cdk", dict(a=64, b=8, c=ext_c, d=ext_d, k=128), F32)
+    A, B = oracle.inputs(c, 9, -1.0, 1.0)
+    eq = to_equation(engine, c, 1)
+    runs, outs = [], []
+    for r in range(2):
+        local, sl = sharding.shard_contracted(eq, "k", 2, r)
+        dA = torch.from_numpy(sharding.take_slice(A, eq.modeA, eq.extent, "k", sl)).cuda()
+        dB = torch.from_numpy(sharding.take_slice(B, eq.modeB, eq.extent, "k", sl)).cuda()
+        dC = torch.full((c.size(c.modeC) // 2,), float("nan"), dtype=torch.float32, device="cuda")
+        plan = engine.plan(local)
+        assert plan.describe()["umma"]["b_fused"] == ext_c and 2 not in plan.describe()["umma"]["column_ranges"]
+        run = api.prepare_on_device(plan, dA.data_ptr(), dB.data_ptr(), dC.data_ptr(), keep=(dA, dB, dC))
+        run.ksplit_enable(2, r)
+        runs.append(run)
+        outs.append(dC)
+    runs[0].ksplit_attach(1, runs[1])
+    runs[1].ksplit_attach(0, runs[0])
+    for _ in range(2):
+        for run in runs:
+            engine.launch(run)
+        torch.cuda.synchronize()              # the barrier among the ranks
+        for run in runs:
+            run.ksplit_reduce()
+        torch.cuda.synchronize()
+    got = torch.cat(outs).cpu().numpy()
+    trunc = oracle.contract(c, A, B, rounding=1)
+    scale = oracle.contract(c, np.abs(A), np.abs(B), rounding=1)
+    assert float((np.abs(got.astype(np.float64) - trunc) / (scale + 1e-30)).max()) < 2e-5
+    assert all(r.device_status() == 0 for r in runs)
