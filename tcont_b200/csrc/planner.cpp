@@ -1237,8 +1237,10 @@ bool cuts_into_ranges(const Plan& pl, int ranges, std::string* why)
     if (slow.extent % ranges || pl.sizeC % ranges || u.tiles_n % ranges) return false;
     const int64_t tile_slabs = u.b.slabs_per_tile;
     // One row digit: the slab mode is all of N (one mode, or two fused ones), so a range ends inside it, and has to end where
-    // a tile does.  More digits: C's slowest mode is the most significant one, and a range is whole indices of it.
+    // a tile does.  More digits: C's slowest mode is the most significant one, and a range is whole indices of it -- unless it
+    // is the slab mode (B's stride-1 mode), whose chunks are the least significant digit.
     if (u.b.n_row_digits == 1) return (u.b.slab_mode_ext / ranges) % (u.b.slab_w * tile_slabs) == 0;
+    if (u.b.major == 1 && p.B[0] == p.C.back()) return false;
     return u.b.total_slabs % ranges == 0 && (u.b.total_slabs / ranges) % tile_slabs == 0;
 }
 

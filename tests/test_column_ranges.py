@@ -61,15 +61,23 @@ def test_fused_columns_that_end_inside_a_slab_are_not_cut(engine, monkeypatch):
     check(d)
 
 
-def test_tile_columns_of_fused_modes_have_one_owner(engine, monkeypatch):
+def test_slowest_mode_that_is_the_slab_mode_is_not_cut(engine, monkeypatch):
+    monkeypatch.setenv("TCONT_SPLITK", "1")
+    # B's stride-1 mode d is C's slowest: its chunks are the fastest digit of the column slabs, the ranges would be c's
+    d = describe(engine, Contraction("acd", "ak", "dkc", dict(a=64, c=16, d=64, k=64), F32), 1)
+    assert d["kernel"] == "umma_tf32" and d["umma"]["b_major"] == "MN" and d["umma"]["column_ranges"] == []
+
+
+def test_every_tile_column_has_one_owner(engine, monkeypatch):
     monkeypatch.setenv("TCONT_SPLITK", "1")
     rng = np.random.default_rng(11)
     pool = (2, 4, 6, 8, 12, 16, 20, 24, 32, 36, 40, 64, 72, 96)
-    fused = 0
+    cut = fused = 0
     for _ in range(1500):
         c = random_contraction(rng, F32, max_out=3_000_000, max_macs=10**9, pool=pool)
         d = describe(engine, c)
-        if d["kernel"] == "umma_tf32" and d["umma"]["b_fused"] and d["umma"]["column_ranges"]:
-            fused += 1
+        if d["kernel"] == "umma_tf32" and d["umma"]["column_ranges"]:
+            cut += 1
+            fused += d["umma"]["b_fused"] > 0
             check(d)
-    assert fused > 10
+    assert cut > 100 and fused > 10
