@@ -789,12 +789,13 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c)
     static const int kTile32[4][3] = {{64, 64, 4}, {128, 32, 4}, {32, 32, 4}, {128, 128, 2}};
     const auto* kTile = f64 ? kTile64 : kTile32;
     const double elt = f64 ? 8.0 : 4.0;
-    GatherSpec best;
+    GatherSpec best;   // (what runs when no candidate below qualifies: a forced cluster this contraction cannot have, an unusable rate)
+    best.rows = p.Mtot;
     best.est_us = 1e300;
     // FP64 sums of this length are off by close to 1e-14 of their norm as one chain of FMAs, and by a fifth of that when cut
     // into ranges: they stay one chain, so that results do not move by more than 1e-14 with the route.
     const bool one_chain = f64 && p.Ktot > 49152;
-    const char* force_tile = std::getenv("TCONT_GATHER_TILE");        // tuning switches: 0..3, 1..16
+    const char* force_tile = std::getenv("TCONT_GATHER_TILE");        // tuning switches: 0..3, 1..16 (1 where that many are impossible)
     const char* force_cluster = std::getenv("TCONT_GATHER_CLUSTER");
     const char* force_flat = std::getenv("TCONT_GATHER_FLAT");
     for (int t : {GATHER_BIG, GATHER_SQUARE, GATHER_TALL, GATHER_SMALL}) {   // (of equal estimates the larger tile)
@@ -1272,7 +1273,7 @@ std::string describe_plan(const Plan& pl)
       << ",\"transpose_b\":" << (pl.tB.needed ? perm(pl.tB) : "null") << ",\"est_direct_us\":" << pl.est_direct_us
       << ",\"est_ttgt_us\":" << pl.est_ttgt_us << ",\"simt\":{\"a_along_k\":" << pl.simt.a_load_along_k
       << ",\"b_along_k\":" << pl.simt.b_load_along_k << "},\"gather\":{\"tile\":" << pl.gather.tile
-      << ",\"cluster\":" << pl.gather.cluster << ",\"flat\":" << (pl.gather.flat ? "true" : "false") << ",\"t0\":" << pl.gather.t0 << ",\"t1\":" << pl.gather.t1 << ",\"est_us\":" << pl.gather.est_us << "}";
+      << ",\"cluster\":" << pl.gather.cluster << ",\"flat\":" << (pl.gather.flat ? "true" : "false") << ",\"t0\":" << pl.gather.t0 << ",\"t1\":" << pl.gather.t1 << ",\"rows\":" << pl.gather.rows << ",\"est_us\":" << pl.gather.est_us << "}";
     const UmmaSpec& u = pl.umma;
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";

@@ -42,7 +42,7 @@ def test_gather_kernel_forms(engine, oracle, monkeypatch, name, scalar):
     unit = 2.0 ** (-24 if scalar == F32 else -53)
     monkeypatch.setenv("TCONT_KERNEL", "gather" if scalar == F64 else "simt")
     forms = [(t, s, f) for t in range(3 if scalar == F64 else 4) for s, f in ((1, 0), (1, 1), (2, 0), (8, 0), (16, 0))]
-    seen = 0
+    seen = set()
     for tile, cluster, flat in forms:
         monkeypatch.setenv("TCONT_GATHER_TILE", str(tile))
         monkeypatch.setenv("TCONT_GATHER_CLUSTER", str(cluster))
@@ -50,9 +50,13 @@ def test_gather_kernel_forms(engine, oracle, monkeypatch, name, scalar):
         p = engine.plan(to_equation(engine, c, 1))
         d = p.describe()
         assert d["kernel"] in ("simt", "dmma_f64")
-        if (d["gather"]["tile"], d["gather"]["cluster"], d["gather"]["flat"]) != (tile, cluster, bool(flat)):
-            continue   # (a cluster longer than the contracted extent)
-        seen += 1
+        form = (d["gather"]["tile"], d["gather"]["cluster"], d["gather"]["flat"])
+        if cluster == 1 or cluster <= k // 32:     # (at least two k tiles of 16 for every CTA of a cluster)
+            assert form == (tile, cluster, bool(flat)), form
+        form += (d["gather"]["t0"], d["gather"]["rows"])
+        if form in seen:
+            continue   # (a cluster longer than the contracted extent: one CTA per tile instead)
+        seen.add(form)
         r = engine.prepare(p, A, B)
         engine.launch(r)
         out = engine.copy_output_to_host(r)
@@ -61,7 +65,6 @@ def test_gather_kernel_forms(engine, oracle, monkeypatch, name, scalar):
         r.set_scalars(2.0, 1.0)                    # 2 A B + A B: exact multiples up to one rounding
         engine.launch(r)
         np.testing.assert_allclose(engine.copy_output_to_host(r).astype(np.float64), 3.0 * out.astype(np.float64), rtol=4 * unit, atol=0)
-    assert seen >= (3 if scalar == F64 else 4)
 
 
 # both operands moved into matrices whose rows are two modes each: 72 = 2.25 slabs, fused 5 184 / 1 296 / ...

@@ -2,7 +2,7 @@
 import pytest
 
 from cases import CONFIGS, fixture_contraction, golden_fixtures, to_equation
-from oracle_lib import Contraction
+from oracle_lib import F32, F64, Contraction
 
 
 def describe(engine, c, selection=0):
@@ -258,3 +258,22 @@ def test_tcgen05_kernel_forms(engine, monkeypatch):
     assert low_k["pair"] is False and low_k["producers"] == 1
     monkeypatch.setenv("TCONT_UMMA_PRODUCERS", "1")
     assert describe(engine, c22, 1)["umma"]["producers"] == 1
+
+
+@pytest.mark.parametrize("scalar", [F32, F64])
+@pytest.mark.parametrize("cluster", ["16", "3"])
+def test_gather_plan_without_a_candidate_covers_all_rows(engine, monkeypatch, scalar, cluster):
+    """A forced cluster that the contracted extent is too short for (or that does not exist) falls back to one CTA per tile."""
+    monkeypatch.setenv("TCONT_KERNEL", "gather" if scalar == F64 else "simt")
+    monkeypatch.setenv("TCONT_GATHER_CLUSTER", cluster)
+    g = describe(engine, Contraction("ab", "ak", "kb", dict(a=65, b=33, k=17), scalar), 1)["gather"]
+    assert g["cluster"] == 1 and g["rows"] >= 65
+
+
+def test_gather_plan_with_unusable_rates_covers_all_rows(engine, monkeypatch, tmp_path):
+    table = tmp_path / "table.txt"
+    table.write_text("".join(f"gather_f64_tflops_{t} 0\n" for t in range(3)))
+    monkeypatch.setenv("TCONT_COST_TABLE", str(table))
+    monkeypatch.setenv("TCONT_KERNEL", "gather")
+    g = describe(engine, Contraction("ab", "ak", "kb", dict(a=65, b=33, k=17), F64), 1)["gather"]
+    assert g["cluster"] == 1 and g["rows"] >= 65
