@@ -1137,8 +1137,9 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         return us;
     };
     // Whether Float32 runs as TF32 or in IEEE single precision is a question of precision, not only of time, and its answer
-    // stays what it was however fast the gather kernel becomes: of the operands as they lie and the first transposed layout,
-    // the cheaper by launches of 6.9 us and CUDA cores at 23.7 TFLOP/s decides, by whether the tcgen05 kernel can stage it.
+    // does not follow the kernels' speed: of the operands as they lie and the first transposed layout, the cheaper by launches
+    // of 6.9 us, the tcgen05 kernel with every mode staged on its own, and CUDA cores at 23.7 TFLOP/s decides, by whether the
+    // tcgen05 kernel can stage it.
     bool tf32 = true;
     if (scalar_type == 0) {
         CostTable line = cost;
@@ -1147,7 +1148,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         const double ieee_us = line.launch_us + std::max(flops / 23.6711e6, (double(direct.sizeA) + double(direct.sizeB) + double(direct.sizeC)) * elt / (line.hbm_gbs * 1e3));
         auto line_us = [&](const Problem& q, bool* staged) {
             UmmaSpec u;
-            plan_umma(q, line, &u);
+            plan_umma(q, line, &u, false);
             *staged = pick_kernel(q, u, line) == KERNEL_UMMA_TF32;
             if (!*staged) return ieee_us;
             double us = contraction_us(q, KERNEL_UMMA_TF32, u, line);
