@@ -947,6 +947,8 @@ bool read_cost_table_file(const std::string& path, CostTable* table)
         if (key == "hbm_gbs") c.hbm_gbs = v;
         else if (key == "umma_tf32_tflops") c.umma_tf32_tflops = v;
         else if (key == "launch_us") c.launch_us = v;
+        else if (key == "simt_f32_tflops") c.line_f32_tflops = v;
+        else if (key == "line_launch_us") c.line_launch_us = v;
         else if (key == "dmma_f64_tflops") c.dmma_f64_tflops = v;
         else if (key == "gather_fixed_us") c.gather_fixed_us = v;
         else if (key == "gather_reduce_us") c.gather_reduce_us = v;
@@ -1137,15 +1139,15 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         return us;
     };
     // Whether Float32 runs as TF32 or in IEEE single precision is a question of precision, not only of time, and its answer
-    // does not follow the kernels' speed: of the operands as they lie and the first transposed layout, the cheaper by launches
-    // of 6.9 us, the tcgen05 kernel with every mode staged on its own, and CUDA cores at 23.7 TFLOP/s decides, by whether the
-    // tcgen05 kernel can stage it.
+    // does not follow the kernels' speed: of the operands as they lie and the first transposed layout, the cheaper decides, by
+    // whether the tcgen05 kernel can stage it.  Cheaper by launches of 6.9 us, CUDA cores at 23.7 TFLOP/s (line_launch_us and
+    // line_f32_tflops of the cost table) and the tcgen05 kernel with every mode staged on its own.
     bool tf32 = true;
     if (scalar_type == 0) {
         CostTable line = cost;
-        line.launch_us = 6.91584;
+        line.launch_us = cost.line_launch_us;
         const double flops = 2.0 * double(direct.Mtot) * double(direct.Ntot) * double(direct.Ktot);
-        const double ieee_us = line.launch_us + std::max(flops / 23.6711e6, (double(direct.sizeA) + double(direct.sizeB) + double(direct.sizeC)) * elt / (line.hbm_gbs * 1e3));
+        const double ieee_us = line.launch_us + std::max(flops / (line.line_f32_tflops * 1e6), (double(direct.sizeA) + double(direct.sizeB) + double(direct.sizeC)) * elt / (line.hbm_gbs * 1e3));
         auto line_us = [&](const Problem& q, bool* staged) {
             UmmaSpec u;
             plan_umma(q, line, &u, false);

@@ -160,6 +160,10 @@ struct CostTable {
     double umma_stage_us = 0.45;
     // What one SM's epilogue stores per second (GB/s): a 128 x 256 fp32 tile takes 3.7 us to leave (cfg4).
     double umma_store_gbs_per_sm = 35.5;
+    // The line between IEEE single precision and TF32 (see make_plan): which Float32 contractions give up precision for time
+    // is decided by these two, not by how fast the kernels are now.
+    double line_f32_tflops = 23.7;          // table key simt_f32_tflops
+    double line_launch_us = 6.9;
     int num_sms = 148;  // SMs of the device the plan is made for (api.cpp fills it in from the current device)
 };
 

@@ -50,3 +50,14 @@ def test_no_contraction_moves_to_tf32(engine, monkeypatch):
         assert before == "1" or not now, (C, A, B, ext)
         tf32 += now
     assert tf32 > 0.9 * was.count("1")     # (and the tensor cores are still used)
+
+
+def test_cost_table_sets_the_line(engine, monkeypatch, tmp_path):
+    (modes, selection) = IEEE["two_k_majors"]
+    table = tmp_path / "table.txt"
+    table.write_text("simt_f32_tflops 1\n")      # slow CUDA cores: one transpose and the tensor cores are worth it
+    monkeypatch.setenv("TCONT_COST_TABLE", str(table))
+    c = Contraction(*modes[:3], modes[3], F32)
+    assert engine.plan(to_equation(engine, c, selection)).describe()["kernel"] == "umma_tf32"
+    table.write_text("simt_f32_tflops 1\nline_launch_us 1000\n")   # (and two launches more are not)
+    assert engine.plan(to_equation(engine, c, selection)).describe()["kernel"] == "simt"
