@@ -166,8 +166,9 @@ struct tcontb_run {
     DeviceBuffer pace;  // progress counters of the tcgen05 kernel's pace keeping (see UmmaParams)
     size_t pace_bytes = 0;
     // C = alpha * (A*B) + beta * C (tcontb_run_set_scalars); the reference's semantics are alpha 1, beta 0.
-    // Other values are applied by the kernel that writes C (but see scales_in_a_second_pass).
+    // Other values are applied by the kernel that writes C, or by the partial-sum pass (scale_pass).
     double alpha = 1.0, beta = 0.0;
+    bool scale_pass = false;
     DeviceBuffer scaled_ws;
     // stage timing
     bool stage_timing = false;
@@ -463,6 +464,12 @@ tcontb_status finish_run(tcontb_run* run)
             TC_CUDA(run->loB.alloc(static_cast<size_t>(run->kernB_elements) * run->elt));
             run->kernels_per_launch += 4;  // two residual passes, two more contractions
         }
+        // The TMA-fed FP64 kernel with a C of up to half of L2 applies alpha and beta in a second pass: its tiles wait for the old
+        // values of C, while a workspace written by the kernel and read by the partial-sum pass stays in L2 (C of 38 MB: 37 us
+        // in two passes, 43 in one; of 302 MB: 259 and 220).  TCONT_SCALE_PASSES=1|2 overrides the rule.
+        run->scale_pass = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1 && pl.sizeC * static_cast<int64_t>(run->elt) <= (int64_t(64) << 20);
+        if (const char* sp = std::getenv("TCONT_SCALE_PASSES"))
+            run->scale_pass = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1 && sp[0] != '1';
         run->umma.C = static_cast<float*>(out);
         run->umma.C64 = static_cast<double*>(out);
         run->umma.status = static_cast<int*>(run->status.ptr);
@@ -979,13 +986,6 @@ tcontb_status tcontb_run_upload_inputs(tcontb_run* run, const void* a_host, cons
     return TCONTB_OK;
 }
 
-// The TMA-fed FP64 kernel with a C of up to half of L2: its tiles wait for the old values of C, while a workspace written by
-// the kernel and read by the partial-sum pass stays in L2 (C of 38 MB: 37 us in two passes, 43 in one; of 302 MB: 259 and 220).
-static bool scales_in_a_second_pass(const tcontb_run* run)
-{
-    return run->plan.kernel == KERNEL_DMMA_F64_TMA && !run->splitk.ptr && run->plan.sizeC * static_cast<int64_t>(run->elt) <= (int64_t(64) << 20);
-}
-
 tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
 {
     if (!run) return fail(TCONTB_INVALID_ARGUMENT, "ExecutionRun is empty");
@@ -993,7 +993,7 @@ tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
     TC_NOT_SHARDED(run, "alpha and beta");
     const bool scaled = alpha != 1.0 || beta != 0.0;
     if (scaled && run->plan.prob.c_strided) return fail(TCONTB_UNSUPPORTED, "alpha and beta are not available when C is a sub-tensor view");
-    if (scales_in_a_second_pass(run)) {
+    if (run->scale_pass) {
         // allocated here, once, so that launches stay free of allocations
         if (scaled && !run->scaled_ws.ptr) TC_CUDA(run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt));
         const bool was = run->alpha != 1.0 || run->beta != 0.0;
@@ -1051,7 +1051,7 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
     // Other scalars than (1, 0): the contraction kernel's epilogue applies them, or the partial-sum pass of a split-K run
     const bool scaled = run->alpha != 1.0 || run->beta != 0.0;
     UmmaParams umma = run->umma;
-    const bool redirect = scaled && scales_in_a_second_pass(run);
+    const bool redirect = scaled && run->scale_pass;
     if (redirect) umma.C64 = static_cast<double*>(run->scaled_ws.ptr);
     umma.scaled = scaled && !run->splitk.ptr && !redirect ? 1 : 0;
     umma.alpha = run->alpha;
