@@ -11,6 +11,19 @@ namespace tcontb {
 
 // Every kernel of a run is launched with this: its blocks may be scheduled, and set themselves up, while the kernel in front
 // of it in the stream drains; they wait (chain_wait in chain.cuh) before they touch global memory.
+//
+// Blocks that are scheduled while the kernel in front still holds some SMs fill the free ones to the brim, and a grid that
+// does not fill the GPU then runs on half of it.  spread_smem is the dynamic shared memory with which an SM holds no more
+// blocks of such a grid than an even share (228 KB an SM, 1 KB of it reserved per block).
+constexpr int kSmemPerSm = 228 * 1024;
+constexpr int kMaxSpreadSmem = kSmemPerSm / 2 - 1024 + 128;   // one block per SM
+inline int spread_smem(long long blocks, int num_sms, int resident, int smem)
+{
+    const long long per_sm = (blocks + num_sms - 1) / num_sms;
+    if (per_sm >= resident) return smem;
+    const int least = (kSmemPerSm / static_cast<int>(per_sm + 1) - 1024 + 128) / 128 * 128;
+    return smem > least ? smem : least;
+}
 template <typename... KernelArgs, typename... Args>
 cudaError_t launch_chained(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, unsigned cluster, Args&&... args)
 {
@@ -87,7 +100,8 @@ struct GatherParams {
     int flat;                  // 1: persistent blocks, one ring of stages across their tiles (cluster 1 only)
     int scaled;                // 0: C = A B; 1: C = alpha A B + beta C (C read only when beta is not zero)
     double alpha, beta;
-    long long k_per_cta;       // the rest is filled in by the launcher
+    int release_late;          // the rest is filled in by the launcher: when the next kernel's blocks may be scheduled
+    long long k_per_cta;
     uint32_t tiles_m, tiles_n;
     int raster_group;
 };
