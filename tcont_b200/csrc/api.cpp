@@ -522,6 +522,7 @@ tcontb_status finish_run(tcontb_run* run)
         if (u.smem_bytes > kMaxDynamicSmemBytes) return fail(TCONTB_RUNTIME_ERROR, "plan asks for more shared memory than a block can have");
         if (pl.kernel == KERNEL_UMMA_TF32) TC_CUDA(umma_tf32_configure());
         else TC_CUDA(dmma_tma_configure());
+        TC_CUDA(splitk_reduce_configure());
     } else {
         fill_gather(p, kA, kB, run->dC, pl.simt, pl.gather, &run->gather);
         TC_CUDA(gather_configure());

@@ -198,6 +198,7 @@ cudaError_t dmma_tma_configure();
 
 // ---- split-K: C[e] = sum over s of partial[s * stride + e], s ascending (splitk_reduce.cu) ----
 // With alpha != 1 or beta != 0: C[e] = alpha * sum + beta * C[e] (C is read only when beta != 0).
+cudaError_t splitk_reduce_configure();  // once per device before the first launch
 cudaError_t launch_splitk_reduce(const void* partial, void* C, long long elements, int splits, long long stride, int elt_bytes,
                                  cudaStream_t stream, double alpha = 1.0, double beta = 0.0);
 

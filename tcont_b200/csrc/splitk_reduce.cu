@@ -98,6 +98,11 @@ cudaError_t launch_tf32_residual(const float* x, float* lo, long long elements, 
     return launch_chained(tf32_residual_kernel, dim3(grid), dim3(256), 0, stream, 1, x, lo, elements, vector_ok);
 }
 
+cudaError_t splitk_reduce_configure()
+{
+    return cudaFuncSetAttribute(splitk_reduce_kernel<double, double2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSpreadSmem);
+}
+
 cudaError_t launch_splitk_reduce(const void* partial, void* C, long long elements, int splits, long long stride, int elt_bytes,
                                  cudaStream_t stream, double alpha, double beta)
 {
@@ -108,8 +113,12 @@ cudaError_t launch_splitk_reduce(const void* partial, void* C, long long element
                            (stride * elt_bytes) % 16 == 0;
     const long long work = vector_ok ? (elements + w - 1) / w : elements;
     const unsigned grid = static_cast<unsigned>(std::min<long long>((work + 255) / 256, 148ll * 8));
+    // FP64: a block of the kernel in front holds all registers of its SM, so this kernel's blocks come to the SMs one block of
+    // that kernel after the other leaves, and a small grid would end up on the first few (192 x 128 x 10368 in 36 ranges, 48
+    // blocks here: 55 us in all with 8 blocks an SM, 48 with one; 52 before launches were chained).  Behind the tcgen05 kernel
+    // they find room on every SM from the start.
     if (elt_bytes == 8)
-        return launch_chained(splitk_reduce_kernel<double, double2, 2>, dim3(grid), dim3(256), 0, stream, 1, static_cast<const double*>(partial),
+        return launch_chained(splitk_reduce_kernel<double, double2, 2>, dim3(grid), dim3(256), spread_smem(grid, 148, 8, 0), stream, 1, static_cast<const double*>(partial),
                               static_cast<double*>(C), elements, splits, stride, vector_ok, scaled, alpha, beta);
     return launch_chained(splitk_reduce_kernel<float, float4, 4>, dim3(grid), dim3(256), 0, stream, 1, static_cast<const float*>(partial),
                           static_cast<float*>(C), elements, splits, stride, vector_ok, scaled, static_cast<float>(alpha), static_cast<float>(beta));
