@@ -847,7 +847,9 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c)
             double us = flat ? fixed_us + std::max(double(per_sm) * (iters * sm_iter_us + c.gather_tile_us), double(ceil_div(per_sm, resident)) * iters * iter_us)
                              : double(per_sm / resident) * round_us(resident) + round_us(per_sm % resident);
             if (s > 1) us += c.gather_reduce_us;
-            us = std::max(us, fixed_us + (double(p.sizeA) + double(p.sizeB) + double(p.sizeC)) * elt / (c.gather_gbs * 1e3));
+            // tensors of up to half of L2 move at twice the rate (6912 x 240 x 4 FP64, 13 MB: 5.9 us)
+            const double bytes = (double(p.sizeA) + double(p.sizeB) + double(p.sizeC)) * elt;
+            us = std::max(us, fixed_us + bytes / ((bytes <= 64e6 ? 2.0 : 1.0) * c.gather_gbs * 1e3));
             if (g.t0 > 0) us *= 1.6;   // (short runs on both sides: 12 x 12 by 124 FP64, rows cut 4 x 8, 18 us where the rule said 11)
             if (us < best.est_us) {
                 best = g;
@@ -924,13 +926,14 @@ int pick_kernel(const Problem& p, const UmmaSpec& u, const CostTable& c)
     const int gather = ceil_div(p.Mtot, bm) * ceil_div(p.Ntot, bn) >= c.num_sms ? KERNEL_DMMA_F64 : KERNEL_SIMT;
     if (!u.eligible || u.elt != 8 || (k && std::strcmp(k, "gather") == 0)) return gather;
     if (k && std::strcmp(k, "tma") == 0) return KERNEL_DMMA_F64_TMA;
-    // (a forced split of k is a switch of the TMA-fed kernel; and where its tiles run across slabs the gather kernel would
-    // have to cut its rows in two modes, with runs of 8 elements on both sides)
-    if (std::getenv("TCONT_SPLITK") || u.store_across_slabs) return KERNEL_DMMA_F64_TMA;
+    if (std::getenv("TCONT_SPLITK")) return KERNEL_DMMA_F64_TMA;   // (a forced split of k is a switch of the TMA-fed kernel)
     // The smallest problems are a matter of latency, which both estimates know to a tenth; above 20 us the gather kernel has to
-    // look 30 % better, because its whole-tile rate is 5 to 25 % more than it reaches on uneven tiles and long rows.
+    // look 30 % better, because its whole-tile rate is 5 to 25 % more than it reaches on uneven tiles and long rows.  Where the
+    // TMA-fed kernel's tiles run across slabs, A's stride-1 mode is not C's, and its gathers or C's stores are short runs:
+    // there already above 10 us (1024 x 2048 x 40, estimated at 18 and 20 us, takes 22.5 and 15.8; 4096 x 128 x 8, at 8 and 9,
+    // 3.8 and 7.3).
     const double tma_us = contraction_us(p, KERNEL_DMMA_F64_TMA, u, c), gather_us = contraction_us(p, gather, u, c);
-    return tma_us <= (gather_us < 20.0 ? 1.05 : 1.3) * gather_us ? KERNEL_DMMA_F64_TMA : gather;
+    return tma_us <= (gather_us < (u.store_across_slabs ? 10.0 : 20.0) ? 1.05 : 1.3) * gather_us ? KERNEL_DMMA_F64_TMA : gather;
 }
 
 }  // namespace

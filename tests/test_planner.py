@@ -277,3 +277,12 @@ def test_gather_plan_with_unusable_rates_covers_all_rows(engine, monkeypatch, tm
     monkeypatch.setenv("TCONT_KERNEL", "gather")
     g = describe(engine, Contraction("ab", "ak", "kb", dict(a=65, b=33, k=17), F64), 1)["gather"]
     assert g["cluster"] == 1 and g["rows"] >= 65
+
+
+@pytest.mark.parametrize("modes,ext", [
+    (("abcde", "efba", "cfd"), dict(a=16, b=16, c=8, d=16, e=16, f=8)),     # rows that the TMA-fed kernel would take across slabs
+    (("abcde", "efba", "cfd"), dict(a=16, b=24, c=12, d=20, e=18, f=4)),
+])
+def test_small_fp64_is_gathered(engine, modes, ext):
+    d = describe(engine, Contraction(*modes, ext, F64))
+    assert d["kernel"] in ("simt", "dmma_f64") and d["backend"] == "direct"
