@@ -957,6 +957,7 @@ bool read_cost_table_file(const std::string& path, CostTable* table)
         else if (key == "gather_reduce_us") c.gather_reduce_us = v;
         else if (key == "gather_tile_us") c.gather_tile_us = v;
         else if (key == "gather_gbs") c.gather_gbs = v;
+        else if (key == "permute_tile_ns") c.permute_tile_ns = v;
         else if (key == "scatter_store_ps") c.scatter_store_ps = v;
         else if (key == "scatter_store_f32_ps") c.scatter_store_f32_ps = v;
         else if (key == "far_row_penalty") c.far_row_penalty = v;
@@ -1135,11 +1136,24 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         return build_problem(pl.modeC, layouts.first, layouts.second, pl.ext_mode, pl.ext_val, scalar_type, q, err, pl.parentC,
                              layouts.first == roleA_src ? roleA_parent : dense, layouts.second == roleB_src ? roleB_parent : dense);
     };
-    auto transposes_us = [&](const std::pair<std::string, std::string>& layouts, const CostTable& c) {
-        double us = 0;
-        if (layouts.first != roleA_src) us += c.launch_us + 2.0 * double(direct.sizeA) * elt / (c.hbm_gbs * 0.7 * 1e3);
-        if (layouts.second != roleB_src) us += c.launch_us + 2.0 * double(direct.sizeB) * elt / (c.hbm_gbs * 0.7 * 1e3);
-        return us;
+    // `tiles`: also by the tiles of the permutation kernel, 64 x 64 at most along the stride-1 modes of source and destination.
+    // Short ones on both sides make many small tiles: 15 x 15 of 50 MB take 171 us, not the 23 of the bandwidth.
+    auto transpose_us = [&](const std::string& src, const std::string& dst, int64_t elements, const CostTable& c, bool tiles) {
+        if (src == dst) return 0.0;
+        auto run = [&](const std::string& of, const std::string& in) {   // extent of the first modes that stay together
+            int64_t e = ext_of(of[0]);
+            for (size_t i = 1; i < of.size() && find_char(in, of[i]) == find_char(in, of[i - 1]) + 1; ++i) e *= ext_of(of[i]);
+            return e;
+        };
+        double us = 2.0 * double(elements) * elt / (c.hbm_gbs * 0.7 * 1e3);
+        if (tiles && src[0] != dst[0]) {
+            const int64_t e0 = run(src, dst), e1 = run(dst, src);
+            us = std::max(us, double(elements) / double(e0) / double(e1) * double(ceil_div(e0, 64) * ceil_div(e1, 64)) * c.permute_tile_ns * 1e-3);
+        }
+        return c.launch_us + us;
+    };
+    auto transposes_us = [&](const std::pair<std::string, std::string>& layouts, const CostTable& c, bool tiles) {
+        return transpose_us(roleA_src, layouts.first, direct.sizeA, c, tiles) + transpose_us(roleB_src, layouts.second, direct.sizeB, c, tiles);
     };
     // Whether Float32 runs as TF32 or in IEEE single precision is a question of precision, not only of time, and its answer
     // does not follow the kernels' speed: of the operands as they lie and the first transposed layout, the cheaper decides, by
@@ -1168,7 +1182,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         if (rc) return rc;
         bool direct_staged, moved_staged;
         const double direct_us = line_us(direct, &direct_staged), moved_us = line_us(q, &moved_staged);
-        const double t_us = transposes_us(candidates[0], line);
+        const double t_us = transposes_us(candidates[0], line, false);
         tf32 = (backend_selection == 0 ? t_us > 0 && t_us + moved_us < direct_us : backend_selection == 2) ? moved_staged : direct_staged;
         if (!tf32 && direct_kernel == KERNEL_UMMA_TF32) {
             direct_umma = UmmaSpec();
@@ -1184,7 +1198,9 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         UmmaSpec u;
         if (tf32) plan_umma(q, cost, &u, fuse_rows);
         const int kernel = pick_kernel(q, u, cost);
-        const double us = transposes_us(candidates[i], cost) + contraction_us(q, kernel, u, cost);
+        // (the TMA-fed kernels gain much more by another layout than the gather kernel does, so for them the tiles do not decide)
+        const bool gathers = kernel == KERNEL_SIMT || kernel == KERNEL_DMMA_F64;
+        const double us = transposes_us(candidates[i], cost, gathers) + contraction_us(q, kernel, u, cost);
         if (us < 0.97 * pl.est_ttgt_us) {   // (an alternative has to be clearly better than the first)
             pl.est_ttgt_us = us;
             ttgt = q;

@@ -286,3 +286,17 @@ def test_gather_plan_with_unusable_rates_covers_all_rows(engine, monkeypatch, tm
 def test_small_fp64_is_gathered(engine, modes, ext):
     d = describe(engine, Contraction(*modes, ext, F64))
     assert d["kernel"] in ("simt", "dmma_f64") and d["backend"] == "direct"
+
+
+# 15 x 19 tiles of a permutation: moving the tensor takes longer than contracting it where it lies
+@pytest.mark.parametrize("modes,ext,scalar", [
+    (("abcde", "efbad", "cf"), dict(a=19, b=13, c=29, d=15, e=15, f=223), F32),
+    (("abcde", "efcad", "bf"), dict(a=13, b=9, c=13, d=13, e=8, f=161), F32),
+    (("abcde", "efbad", "cf"), dict(a=15, b=13, c=9, d=17, e=19, f=61), F64),
+])
+def test_short_permutation_tiles_count(engine, modes, ext, scalar):
+    assert describe(engine, Contraction(*modes, ext, scalar))["backend"] == "direct"
+
+
+def test_long_permutation_tiles_still_pay(engine):
+    assert describe(engine, Contraction("abcde", "efba", "cfd", dict(a=31, b=47, c=43, d=43, e=53, f=7), F32))["backend"] == "ttgt"
