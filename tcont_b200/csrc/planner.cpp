@@ -782,7 +782,7 @@ double wave_efficiency(int64_t tiles, int sms)
 // (throughput), but none faster than one alone (latency), which is what bounds small problems and what a split of k
 // shortens.  Measured on 60 contractions of 2 MFLOP to 280 GFLOP with every tile, cluster and form: the choice is within
 // 11 % of the best one on average.
-GatherSpec plan_gather(const Problem& p, const CostTable& c)
+GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors = true)
 {
     const bool f64 = p.scalar_type == 1;
     static const int kTile64[3][3] = {{64, 64, 3}, {128, 32, 2}, {32, 32, 4}};   // BM, BN, CTAs per SM
@@ -795,6 +795,14 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c)
     // FP64 sums of this length are off by close to 1e-14 of their norm as one chain of FMAs, and by a fifth of that when cut
     // into ranges: they stay one chain, so that results do not move by more than 1e-14 with the route.
     const bool one_chain = f64 && p.Ktot > 49152;
+    // An operand whose stride-1 mode is contracted, but not the first of the contracted modes (those are in the other operand's
+    // order): every element of it is fetched as a 32-byte sector of its own, by every tile that needs it.  168 x 192 x 4096
+    // FP64, 36 tiles of 32 x 32 in 16 ranges of k: 62 us, 38 of them for 151 MB of such sectors.  Counted where the TMA-fed
+    // kernel behind a permutation is the alternative; the gather kernel behind one is not reliably faster (the same
+    // contractions: 0.5 to 1.3 times the time).
+    auto scattered = [&](const std::vector<int>& t) { return f64 && count_sectors && p.modes[static_cast<size_t>(t[0])].group == GROUP_K && t[0] != p.K[0] ? int64_t(1) : int64_t(0); };
+    const int64_t scattered_a = scattered(p.A), scattered_b = scattered(p.B);
+    double sector_us = 0;
     const char* force_tile = std::getenv("TCONT_GATHER_TILE");        // tuning switches: 0..3, 1..16 (1 where that many are impossible)
     const char* force_cluster = std::getenv("TCONT_GATHER_CLUSTER");
     const char* force_flat = std::getenv("TCONT_GATHER_FLAT");
@@ -857,15 +865,17 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c)
                 best.flat = flat;
                 if (force_flat) best.flat = s == 1 && force_flat[0] == '1';
                 best.est_us = us;
+                sector_us = double(scattered_a * g.rows * tiles_n + scattered_b * p.Ntot * tiles_m) * double(p.Ktot) * 32.0 / (c.gather_sector_gbs * 1e3);
             }
         }
     }
+    best.est_us += sector_us;   // (the choice of a tile is as good without it: its rates have it in part)
     return best;
 }
 
-double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const CostTable& c)
+double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const CostTable& c, bool count_sectors = true)
 {
-    if (kernel == KERNEL_DMMA_F64 || kernel == KERNEL_SIMT) return c.launch_us + plan_gather(p, c).est_us;
+    if (kernel == KERNEL_DMMA_F64 || kernel == KERNEL_SIMT) return c.launch_us + plan_gather(p, c, count_sectors).est_us;
     const double elt = p.scalar_type == 1 ? 8.0 : 4.0;
     const double flops = 2.0 * double(p.Mtot) * double(p.Ntot) * double(p.Ktot);
     double c_bytes = double(p.sizeC) * elt;
@@ -957,6 +967,7 @@ bool read_cost_table_file(const std::string& path, CostTable* table)
         else if (key == "gather_reduce_us") c.gather_reduce_us = v;
         else if (key == "gather_tile_us") c.gather_tile_us = v;
         else if (key == "gather_gbs") c.gather_gbs = v;
+        else if (key == "gather_sector_gbs") c.gather_sector_gbs = v;
         else if (key == "permute_tile_ns") c.permute_tile_ns = v;
         else if (key == "scatter_store_ps") c.scatter_store_ps = v;
         else if (key == "scatter_store_f32_ps") c.scatter_store_f32_ps = v;
@@ -1200,7 +1211,10 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         const int kernel = pick_kernel(q, u, cost);
         // (the TMA-fed kernels gain much more by another layout than the gather kernel does, so for them the tiles do not decide)
         const bool gathers = kernel == KERNEL_SIMT || kernel == KERNEL_DMMA_F64;
-        const double us = transposes_us(candidates[i], cost, gathers) + contraction_us(q, kernel, u, cost);
+        double us = transposes_us(candidates[i], cost, gathers) + contraction_us(q, kernel, u, cost);
+        // Partial sums behind the FP64 kernel: a thread adds its partials up one after the other, 0.12 us each (96 x 64 x 2992
+        // in 41 ranges: 20.8 us without that, 24.6 measured).  Where the operands lie the kernels' estimates are compared as they were fitted.
+        if (kernel == KERNEL_DMMA_F64_TMA && u.k_splits > 1) us += 0.12 * u.k_splits;
         if (us < 0.97 * pl.est_ttgt_us) {   // (an alternative has to be clearly better than the first)
             pl.est_ttgt_us = us;
             ttgt = q;
@@ -1211,6 +1225,8 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         }
     }
 
+    if (ttgt_kernel != KERNEL_UMMA_TF32 && ttgt_kernel != KERNEL_DMMA_F64_TMA)
+        pl.est_direct_us = contraction_us(direct, direct_kernel, direct_umma, cost, false);
     bool use_ttgt;
     if (backend_selection == 1) use_ttgt = false;
     else if (backend_selection == 2) use_ttgt = true;

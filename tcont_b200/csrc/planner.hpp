@@ -147,6 +147,7 @@ struct CostTable {
     double gather_tile_us = 0.7;            // the same per tile of a persistent CTA, whose gathers run ahead
     double gather_reduce_us = 3.0;          // adding up a cluster's partial tiles
     double gather_gbs = 2200.0;             // tensors read and written once through element-wise gathers and stores
+    double gather_sector_gbs = 4000.0;      // 32-byte sectors fetched from L2 for one element each
     double permute_tile_ns = 3.3;           // permutation kernel, per tile with every SM busy (tiles of 100 to 600 elements: 2.9 to 4.5)
     double scatter_store_ps = 27.6;         // per element of C stored on its own (TMA-fed FP64 kernel)
     double scatter_store_f32_ps = 17.6;     // the same for the tcgen05 kernel's 4-byte elements

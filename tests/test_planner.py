@@ -300,3 +300,13 @@ def test_short_permutation_tiles_count(engine, modes, ext, scalar):
 
 def test_long_permutation_tiles_still_pay(engine):
     assert describe(engine, Contraction("abcde", "efba", "cfd", dict(a=31, b=47, c=43, d=43, e=53, f=7), F32))["backend"] == "ttgt"
+
+
+@pytest.mark.parametrize("modes,ext", [
+    (("ab", "cad", "dcb"), dict(a=168, b=192, c=64, d=64)),
+    (("abcd", "eafb", "fdec"), dict(a=24, b=24, c=16, d=32, e=24, f=24)),
+])
+def test_sectors_fetched_for_one_element_count(engine, modes, ext):
+    """Operands that are K-major on different modes: a transpose and the TMA-fed kernel instead of scattered gathers."""
+    d = describe(engine, Contraction(*modes, ext, F64))
+    assert (d["backend"], d["kernel"]) == ("ttgt", "dmma_f64_tma")
