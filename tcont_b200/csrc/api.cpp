@@ -486,14 +486,15 @@ tcontb_status finish_run(tcontb_run* run)
                 run->umma.prof = static_cast<long long*>(run->prof.ptr);
             }
         }
+        const int64_t units = (u.pair ? (u.tiles_m + 1) / 2 : u.tiles_m) * u.tiles_n * u.k_splits;
+        const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(units, u.pair ? run->num_sms / 2 : run->num_sms));
+        run->umma.release_late = units >= 16 * ctas && u.k_iters_per_split <= 4 ? 1 : 0;
         run->umma.pace = nullptr;
         if (pl.kernel == KERNEL_UMMA_TF32) {
             // Pace keeping pays where the CTAs walk long panels that do not fit into L2 together: a full grid with
             // several work units each, 32 or more k iterations per unit, operands of 64 MB or more (the large 4-D
             // configuration: 28 -> 21 GB read from DRAM per launch, 2 to 4 % less time; on another GPU 47 GB without).
             // TCONT_UMMA_PACE=0/1 overrides the rule; lead and block size: TCONT_UMMA_PACE_LEAD / _SHIFT.
-            const int64_t units = (u.pair ? (u.tiles_m + 1) / 2 : u.tiles_m) * u.tiles_n * u.k_splits;
-            const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(units, u.pair ? run->num_sms / 2 : run->num_sms));
             const int64_t a_elems = pl.tA.needed ? pl.tA.elements : (p.swapped ? pl.sizeR : pl.sizeL);
             const int64_t b_elems = pl.tB.needed ? pl.tB.elements : (p.swapped ? pl.sizeL : pl.sizeR);
             bool pace = units >= 2 * ctas && u.k_iters_per_split >= 32 && (a_elems + b_elems) * static_cast<int64_t>(run->elt) >= (64ll << 20);

@@ -341,7 +341,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
         }
     }
     tcgen05_fence_before();
-    chain_release();
+    if (!p.release_late) chain_release();
     chain_wait();
     __syncthreads();
     if (PAIR) cluster_sync_all();  // the partner's barriers exist before anything signals them
@@ -364,6 +364,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
             const ProducerEnv e = {smem_u32(smem), a_tile_bytes, stage_bytes, smem_u32(bar_full), smem_u32(bar_empty), abort_flag,
                                    rank, tiles_m, tiles_n, first_unit, unit_step, total_tiles};
             produce_two_copies<PAIR, NP>(p, tmapA, tmapB, e, warp == 0 ? 0 : 1);
+            if (p.release_late) chain_release();
         }
         __syncwarp();
     } else if (producer) {
@@ -480,6 +481,7 @@ umma_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
             p.prof[blockIdx.x * 8 + 6] = pace_clk;
             p.prof[blockIdx.x * 8 + 7] = pace_waits * 2 + (pacing && !pace_live ? 1 : 0);
         }
+        if (p.release_late) chain_release();
         if (ld_shared_u32(abort_flag) && lane == 0 && rank == 0) drain_copies(smem_u32(bar_full), p.stages, issued_mask, issued_parity);
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
