@@ -119,6 +119,8 @@ struct DeviceBuffer {
     }
 };
 
+constexpr int64_t kScalePassInL2 = int64_t(64) << 20;  // bytes of C: half of L2
+
 // Restores the device that was current when a multi-GPU function started, on every way out of it.
 struct DeviceGuard {
     int device;
@@ -466,10 +468,12 @@ tcontb_status finish_run(tcontb_run* run)
         }
         // The TMA-fed FP64 kernel with a C of up to half of L2 applies alpha and beta in a second pass: its tiles wait for the old
         // values of C, while a workspace written by the kernel and read by the partial-sum pass stays in L2 (C of 38 MB: 37 us
-        // in two passes, 43 in one; of 302 MB: 259 and 220).  TCONT_SCALE_PASSES=1|2 overrides the rule.
-        run->scale_pass = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1 && pl.sizeC * static_cast<int64_t>(run->elt) <= (int64_t(64) << 20);
-        if (const char* sp = std::getenv("TCONT_SCALE_PASSES"))
-            run->scale_pass = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1 && sp[0] != '1';
+        // in two passes, 43 in one; of 302 MB: 259 and 220).  Tiles across slabs read and write C in pieces of 64 bytes; with k
+        // chunks of 16 and few of them they take two passes whatever the size (C of 132 MB, K 48: 140 us in two, 168 in one; of 755 MB, K 16:
+        // 596 and 672; with chunks of 8, 453 MB, K 8: 334 and 308; 20 chunks of 16, 73 MB: 274 and 264).  TCONT_SCALE_PASSES=1|2 overrides the rule.
+        const bool unsplit = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1;
+        run->scale_pass = unsplit && (pl.sizeC * static_cast<int64_t>(run->elt) <= kScalePassInL2 || (u.store_across_slabs && u.BK == 16 && u.k_iters <= 6));
+        if (const char* sp = std::getenv("TCONT_SCALE_PASSES")) run->scale_pass = unsplit && sp[0] != '1';
         run->umma.C = static_cast<float*>(out);
         run->umma.C64 = static_cast<double*>(out);
         run->umma.status = static_cast<int*>(run->status.ptr);
@@ -1105,8 +1109,9 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         TC_CUDA(launch_splitk_reduce(run->splitk.ptr, run->dC, pl.sizeC, pl.umma.k_splits * (run->tf32x3 ? 3 : 1), pl.sizeC,
                                      static_cast<int>(run->elt), run->stream, run->alpha, run->beta));
     else if (redirect)
-        TC_CUDA(launch_splitk_reduce(run->scaled_ws.ptr, run->dC, pl.sizeC, 1, pl.sizeC, static_cast<int>(run->elt), run->stream,
-                                     run->alpha, run->beta));
+        TC_CUDA(pl.sizeC * static_cast<int64_t>(run->elt) > kScalePassInL2
+                    ? launch_scale_pass(static_cast<const double*>(run->scaled_ws.ptr), static_cast<double*>(run->dC), pl.sizeC, run->stream, run->alpha, run->beta)
+                    : launch_splitk_reduce(run->scaled_ws.ptr, run->dC, pl.sizeC, 1, pl.sizeC, static_cast<int>(run->elt), run->stream, run->alpha, run->beta));
     if (t) {
         TC_CUDA(cudaEventRecord(run->ev[3], run->stream));
         run->ev_valid = true;

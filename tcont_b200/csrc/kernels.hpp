@@ -206,6 +206,8 @@ cudaError_t dmma_tma_configure();
 cudaError_t splitk_reduce_configure();  // once per device before the first launch
 cudaError_t launch_splitk_reduce(const void* partial, void* C, long long elements, int splits, long long stride, int elt_bytes,
                                  cudaStream_t stream, double alpha = 1.0, double beta = 0.0);
+// One partial, tensors beyond L2: scheduled when the kernel in front has ended (see the .cu file).
+cudaError_t launch_scale_pass(const double* product, double* C, long long elements, cudaStream_t stream, double alpha, double beta);
 
 // ---- error-compensated Float32 (splitk_reduce.cu): lo = x - truncate_to_tf32(x), exact in fp32 ----
 cudaError_t launch_tf32_residual(const float* x, float* lo, long long elements, cudaStream_t stream);

@@ -107,3 +107,20 @@ def test_float32(engine, oracle, monkeypatch, name):
         want = alpha * product + beta * C0.astype(np.float64)
         bound = 2e-5 * abs(alpha) * scale + 4 * 2.0**-24 * (np.abs(alpha * product) + np.abs(beta * C0.astype(np.float64)))
         assert (np.abs(out - want) <= bound).all(), (alpha, beta)
+
+
+def test_fp64_beyond_l2(engine, oracle, monkeypatch):
+    """A C of more than 64 MB: rows across slabs with a k chunk of 16 take a second pass over C, and can be kept from it."""
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    c = Contraction("abcd", "dbea", "ec", dict(a=40, b=16, c=56, d=250, e=16), F64)
+    A, B = oracle.inputs(c, 23, -1.0, 1.0)
+    C0 = np.random.default_rng(5).uniform(-4.0, 4.0, c.size("abcd"))
+    assert C0.nbytes > 64 << 20
+    product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
+    for passes in (None, "1"):
+        if passes:
+            monkeypatch.setenv("TCONT_SCALE_PASSES", passes)
+        desc, got = scaled_run(engine, c, A, B, C0, [(0.3, -0.7)])
+        assert desc["umma"]["store_across_slabs"] and desc["umma"]["BK"] == 16
+        bound = 20 * 2.0**-53 * (0.3 * scale + abs(0.7 * C0))
+        assert (np.abs(got[0] - (0.3 * product - 0.7 * C0)) <= bound).all()
