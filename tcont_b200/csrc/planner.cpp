@@ -858,6 +858,12 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors 
             // tensors of up to half of L2 move at twice the rate (6912 x 240 x 4 FP64, 13 MB: 5.9 us)
             const double bytes = (double(p.sizeA) + double(p.sizeB) + double(p.sizeC)) * elt;
             us = std::max(us, fixed_us + bytes / ((bytes <= 64e6 ? 2.0 : 1.0) * c.gather_gbs * 1e3));
+            // Rows in C's order although A's stride-1 mode is another row mode: every element of A comes in a sector of its own, which
+            // the rates stand for once; 128 x 32 tiles on 33 to 64 columns fetch A twice (31185 x 35 x 311 FP64: 217 us, where
+            // 64 x 64 tiles with rows cut 8 x 8 take 130; 2480625 x 35 x 87 Float32: 7884, 128 x 128 tiles 4155).  (An A in L2 can be: 9367 x
+            // 33 x 63 Float32 takes 10 us in them, 14 in others.)
+            if (t == GATHER_TALL && tiles_n == 2 && double(p.sizeA) * elt > 32e6 && g.t0 == 0 && p.A[0] != p.M[0] && p.modes[static_cast<size_t>(p.A[0])].group == GROUP_M)
+                us += double(g.rows) * double(p.Ktot) * 32.0 / (c.gather_sector_gbs * 1e3);
             if (g.t0 > 0) us *= 1.6;   // (short runs on both sides: 12 x 12 by 124 FP64, rows cut 4 x 8, 18 us where the rule said 11)
             if (us < best.est_us) {
                 best = g;

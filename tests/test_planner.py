@@ -310,3 +310,13 @@ def test_sectors_fetched_for_one_element_count(engine, modes, ext):
     """Operands that are K-major on different modes: a transpose and the TMA-fed kernel instead of scattered gathers."""
     d = describe(engine, Contraction(*modes, ext, F64))
     assert (d["backend"], d["kernel"]) == ("ttgt", "dmma_f64_tma")
+
+
+@pytest.mark.parametrize("modes,ext", [
+    (("abcd", "deca", "be"), dict(a=35, b=35, c=27, d=33, e=311)),
+    (("abcde", "ecbfa", "fd"), dict(a=23, b=21, c=19, d=42, e=21, f=91)),
+])
+def test_scattered_rows_are_not_fetched_twice(engine, modes, ext):
+    """33 to 64 columns: not in 32-column tiles where every element of A comes in a sector of its own."""
+    d = describe(engine, Contraction(*modes, ext, F64), 1)
+    assert d["kernel"] in ("simt", "dmma_f64") and (d["gather"]["t0"] > 0 or d["gather"]["tile"] != 1)
