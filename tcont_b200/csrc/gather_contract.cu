@@ -23,12 +23,12 @@
 #include <cooperative_groups.h>
 
 #include "chain.cuh"
+#include "fast_div.cuh"
 #include "kernels.hpp"
 
 namespace tcontb {
 namespace {
 
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) { return (__umulhi(n, f.mul) + n) >> f.shr; }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 template <int BYTES>
@@ -491,7 +491,6 @@ using F32SquareFlat = GatherCfg<float, 64, 64, 1, 4, 1, true, 4, 4>;
 using F32Tall = GatherCfg<float, 128, 32, 2, 2, 1, false, 4, 4>;
 using F32TallFlat = GatherCfg<float, 128, 32, 2, 2, 1, true, 4, 3>;
 using F32Small = GatherCfg<float, 32, 32, 1, 2, 4, false, 4, 4>;
-using F32SmallFlat = GatherCfg<float, 32, 32, 1, 2, 1, true, 4, 7>;
 
 }  // namespace
 
@@ -515,7 +514,6 @@ cudaError_t gather_configure()
     set(gather_contract_kernel<F32Tall>, F32Tall::SMEM);
     set(gather_contract_kernel<F32TallFlat>, F32TallFlat::SMEM);
     set(gather_contract_kernel<F32Small>, F32Small::SMEM);
-    set(gather_contract_kernel<F32SmallFlat>, F32SmallFlat::SMEM);
     return e;
 }
 
@@ -530,7 +528,7 @@ cudaError_t launch_gather_contract(const GatherParams& p, int scalar_type, int t
         if (tile == GATHER_BIG) return p.flat ? launch<F32BigFlat>(p, num_sms, stream) : launch<F32Big>(p, num_sms, stream);
         if (tile == GATHER_SQUARE) return p.flat ? launch<F32SquareFlat>(p, num_sms, stream) : launch<F32Square>(p, num_sms, stream);
         if (tile == GATHER_TALL) return p.flat ? launch<F32TallFlat>(p, num_sms, stream) : launch<F32Tall>(p, num_sms, stream);
-        if (tile == GATHER_SMALL) return p.flat ? launch<F32SmallFlat>(p, num_sms, stream) : launch<F32Small>(p, num_sms, stream);
+        if (tile == GATHER_SMALL && !p.flat) return launch<F32Small>(p, num_sms, stream);
     }
     return cudaErrorInvalidValue;
 }

@@ -61,8 +61,9 @@ struct SimtParams {
 };
 cudaError_t launch_simt_contract(const SimtParams& p, int scalar_type, cudaStream_t stream);
 
-// Division by a number known before the launch: n / d = (umulhi(n, mul) + n) >> shr for n < 2^31, with shr = ceil(log2 d)
-// and mul = floor(2^32 (2^shr - d) / d) + 1.  Five instructions where the hardware-less integer division takes thirty.
+// Division by a number known before the launch, by multiplication (Granlund and Montgomery, 1994): n / d = (umulhi(n, mul) + n)
+// >> shr for n < 2^31, with shr = ceil(log2 d) and mul = floor(2^32 (2^shr - d) / d) + 1.  Five instructions where the
+// hardware-less integer division takes thirty.
 struct FastDiv {
     uint32_t d, mul, shr;
 };

@@ -869,7 +869,7 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors 
                 best = g;
                 best.cluster = s;
                 best.flat = flat;
-                if (force_flat) best.flat = s == 1 && force_flat[0] == '1';
+                if (force_flat) best.flat = s == 1 && force_flat[0] == '1' && (f64 || t != GATHER_SMALL);   // (the small Float32 tile has no such form)
                 best.est_us = us;
                 sector_us = double(scattered_a * g.rows * tiles_n + scattered_b * p.Ntot * tiles_m) * double(p.Ktot) * 32.0 / (c.gather_sector_gbs * 1e3);
             }

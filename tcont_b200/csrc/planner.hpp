@@ -131,9 +131,12 @@ struct GatherSpec {
 };
 
 struct CostTable {
-    // Defaults: what `python -m tcont_b200.calibrate` measured on a B200 (the file it writes,
-    // tcont_cost_table.NVIDIA_B200.txt beside the library, holds the same figures and is read when the current
-    // device has that name; TCONT_COST_TABLE names another "key value" file).
+    // tcont_cost_table.NVIDIA_B200.txt beside the library is read over these when the current device has that name;
+    // TCONT_COST_TABLE names another "key value" file.  The rates of the TMA-fed kernels, HBM, scattered stores and far rows
+    // are what `python -m tcont_b200.calibrate` measured on a B200.  The gather kernel's figures, launch_us and the tile and
+    // sector costs are fitted: to every tile, cluster and form of 60 contractions of 2 MFLOP to 280 GFLOP, the last two to 234
+    // drawn ones.  calibrate measures the gather kernel's rates and launch_us too, alone and on one pattern (28 to 31 and 5.9
+    // where the fit has 28 to 32 and 4.0): a table it writes is close to this one, not equal, and gives other routes in ties.
     double hbm_gbs = 6178.9;                // copy through the permutation kernel, read + write
     double umma_tf32_tflops = 674.4;        // tcgen05 kernel, 8192 x 8192 x 4096, CTA pairs with a k chunk of 64
     double dmma_f64_tflops = 33.5;          // TMA-fed tensor-path kernel

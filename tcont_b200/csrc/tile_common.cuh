@@ -6,6 +6,7 @@
 
 #include <cstdint>
 
+#include "fast_div.cuh"
 #include "kernels.hpp"
 
 namespace tcontb {
@@ -118,8 +119,6 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* tmap, uint
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
         : "memory");
 }
-
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) { return (__umulhi(n, f.mul) + n) >> f.shr; }
 
 // Raster order: groups of raster_group tile rows are swept column by column, so the CTAs that run
 // together share A and B panels in L2.  Tile and slab counts fit 31 bits (the planner checks).

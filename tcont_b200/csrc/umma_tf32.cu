@@ -3,9 +3,10 @@
 // One persistent CTA per SM, three roles:
 //   warp 0      TMA producer.  An operand tile is a run of "slabs"; each slab is one 2-D box of a
 //               5-D tensor map laid over the operand's own (strided, multi-mode) layout, written
-//               with a 128-byte swizzle so that it is already a UMMA canonical tile.  Lane i owns
+//               with a 128-byte swizzle so that it is already a UMMA canonical tile.  Where one copy
+//               covers an operand's part of a stage, one elected thread issues both; else lane i owns
 //               slab i and issues its own cp.async.bulk.tensor per K step (no cluster multicast).
-//   warp 1      allocates tensor memory, and its lane 0 issues tcgen05.mma kind::tf32
+//   warp 1      allocates tensor memory, and an elected thread issues tcgen05.mma kind::tf32
 //               (M = 128, N = BN, K = 8 per instruction) into one of two TMEM accumulators.
 //   warps 2-5   epilogue: tcgen05.ld the accumulator (lane = row), scatter it to C's final,
 //               permuted position; with C's stride-1 mode on the slab rows a warp writes 128
