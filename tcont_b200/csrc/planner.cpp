@@ -793,7 +793,8 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors 
     best.rows = p.Mtot;
     best.est_us = 1e300;
     // FP64 sums of this length are off by close to 1e-14 of their norm as one chain of FMAs, and by a fifth of that when cut
-    // into ranges: they stay one chain, so that results do not move by more than 1e-14 with the route.
+    // into ranges.  They stay one chain here only so that results recorded with it do not move by that much; where tiles are
+    // few it costs 15 times the time, and the TMA-fed kernel does cut them.
     const bool one_chain = f64 && p.Ktot > 49152;
     // An operand whose stride-1 mode is contracted, but not the first of the contracted modes (those are in the other operand's
     // order): every element of it is fetched as a 32-byte sector of its own, by every tile that needs it.  168 x 192 x 4096
