@@ -492,7 +492,7 @@ tcontb_status finish_run(tcontb_run* run)
         }
         const int64_t units = (u.pair ? (u.tiles_m + 1) / 2 : u.tiles_m) * u.tiles_n * u.k_splits;
         const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(units, u.pair ? run->num_sms / 2 : run->num_sms));
-        run->umma.release_late = units >= 16 * ctas && u.k_iters_per_split <= 4 ? 1 : 0;
+        run->umma.release_late = pl.kernel == KERNEL_UMMA_TF32 && units >= 16 * ctas && u.k_iters_per_split <= 4 ? 1 : 0;
         run->umma.pace = nullptr;
         if (pl.kernel == KERNEL_UMMA_TF32) {
             // Pace keeping pays where the CTAs walk long panels that do not fit into L2 together: a full grid with

@@ -194,7 +194,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (!p.release_late) chain_release();
+    chain_release();
     chain_wait();
     __syncthreads();
 
@@ -263,7 +263,6 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     }
                 }
             }
-            if (p.release_late) chain_release();
             if (ld_shared_u32(abort_flag) && lane == 0) {
                 // Give the bulk copies issued into these barriers a bounded time to land before the block ends.
                 for (int s = 0; s < p.stages; ++s) {

@@ -175,10 +175,11 @@ struct UmmaParams {
     // owner_base[o][i].  owners = 0 or 1: everything goes to C.  `tn_rotate` shifts the order in which a GPU
     // visits the tile columns, so that the GPUs of a job write to different owners at any one time.
     int store_across_slabs;  // FP64 kernel: see UmmaSpec
-    // 1: the next kernel's blocks may be scheduled when this one's copies are issued, 0: at once.  Late where every block
-    // stores many tiles of few k iterations: 806400 x 112 x 48 Float32 behind its permutation, 43 tiles a block: let in at once
-    // 200 us, late 184, not chained 187; 81920 x 1152 x 16 FP64, 78 tiles: 244, 234, 230; 230656 x 480 x 32: 339, 320, 320.
-    // Short kernels and long k loops lose by it (8192 x 768 x 16 FP64, 5 tiles: 19.5, late 20.5; 3540 x 3249 x 520: 461, 471).
+    // tcgen05 kernel.  1: the next kernel's blocks may be scheduled when this one's copies are issued, 0: at once.  Late where
+    // every block stores many tiles of few k iterations: 806400 x 112 x 48 behind its permutation, 43 tiles a block: let in at
+    // once 200 us, late 184, not chained 187.  Short kernels lose by it (4096 x 3072 x 32, 3 tiles: 16.9, late 17.3).  The FP64
+    // kernel always releases at once: a choice in front of its main loop costs that loop 1.4 % (5184^3: 9518 and 9643 us),
+    // which is more than output-bound kernels gain (81920 x 1152 x 16: 244, late 234).
     int release_late;
     // tcgen05 kernel, pace keeping: the CTAs (pairs) of a launch walk their panels along k at about the same
     // pace, so that a panel one of them fetched is still in L2 when the others of its tile row or column ask for
