@@ -443,6 +443,7 @@ tcontb_status finish_run(tcontb_run* run)
         run->umma.raster_group = u.raster_group;
         run->umma.k_splits = u.k_splits;
         run->umma.k_iters_per_split = static_cast<int>(u.k_iters_per_split);
+        run->umma.full_chunks = static_cast<int>(u.full_chunks);
         run->umma.split_stride = pl.sizeC;
         fill_raster_divs(u, &run->umma);
         void* out = run->dC;

@@ -148,6 +148,7 @@ struct UmmaParams {
     int pair;  // 1: two-CTA clusters, 256 x BN tiles (cta_group::2); 0: one CTA per 128 x BN tile
     int producers;  // tcgen05 kernel: 2 = two producer warps taking turns stage by stage (needs an even number of stages)
     int k_digit_ext[3];
+    int full_chunks;  // FP64 kernel: chunks of the chunked mode (k digit 0) below this one hold more than eight k (k chunk of 8: none)
     int k_iters;
     // Split-K: every tile is computed k_splits times over consecutive ranges of k_iters_per_split
     // iterations; split s writes its partial tile at C + s * split_stride (a workspace laid out like

@@ -529,6 +529,12 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
         u->k_digit_ext[i] = i == 0 ? ceil_div(e, BK) : e;
         u->k_iters *= u->k_digit_ext[i];
     }
+    u->k_computed = double(u->k_iters) * BK;
+    if (f64 && BK == 16) {   // the FP64 kernel leaves out the second half of a last chunk of eight k or fewer
+        const bool half = kc_ext % 16 >= 1 && kc_ext % 16 <= 8;
+        u->full_chunks = u->k_digit_ext[0] - (half ? 1 : 0);
+        if (half) u->k_computed *= 1.0 - 0.5 / double(u->k_digit_ext[0]);
+    }
     if (!stage_operand(p, p.A, p.M, true, kc, BK, &u->a, &u->why_not)) return;
     if (!stage_operand(p, p.B, p.N, false, kc, BK, &u->b, &u->why_not)) return;
 
@@ -892,7 +898,7 @@ double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const Cos
     // (extents of 72 in 32-wide slabs and chunks: abcd-aefb-fdce ran at 138 TFLOP/s direct, 415 after a
     // transpose that fuses the ragged modes away)
     const double tma_padding = double(u.tiles_m * u.BM) / double(p.Mtot) * double(u.tiles_n * u.BN) / double(p.Ntot) *
-                               double(u.k_iters * u.BK) / double(p.Ktot);
+                               u.k_computed / double(p.Ktot);
     if ((kernel == KERNEL_DMMA_F64_TMA || kernel == KERNEL_UMMA_TF32) && u.k_splits > 1) {
         // partial tensors written, read back and summed by a second kernel
         // (set up while the first kernel drains; partial tensors of up to half of L2 are read back from there)

@@ -98,6 +98,8 @@ struct UmmaSpec {
     int n_k_digits = 1;
     int64_t k_digit_ext[3] = {1, 1, 1};  // digit 0 = chunks of the chunked K mode
     int64_t k_iters = 1, tiles_m = 1, tiles_n = 1;
+    int64_t full_chunks = 0;             // FP64 kernel: the chunks of digit 0 that hold more than eight k
+    double k_computed = 1;               // contracted indices a tile multiplies, zero-filled ones included
     int k_splits = 1;               // ranges of the k iterations computed as separate work units (split-K)
     int64_t k_iters_per_split = 1;
     double far_fraction = 0;  // share of a stage's bytes whose K rows are 64 KB or more apart in memory
