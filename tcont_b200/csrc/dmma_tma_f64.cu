@@ -85,83 +85,80 @@ __device__ __forceinline__ void load_old4(double (&o)[4], const double* dst, boo
 //    2 fr + par with fr two apart in the swizzle) take different halves of it.
 __device__ __forceinline__ uint32_t step_k(uint32_t t, uint32_t fk) { return 8u * (t >> 1) + 2u * fk + ((fk ^ (fk >> 1) ^ t) & 1u); }
 
-// Where a thread finds its fragments of one operand for one k:
+// Where a thread finds its fragments of one operand, as byte offsets from the start of the stage:
 //   MN-major (rows of the stage are k, 16 consecutive m per 128-byte row, slabs of 16 m one slab apart;
 //   or 8 m per 64-byte row, two slabs per 16 m):
-//     one 16-byte load at  q0 + pair * pitch  holds fragments 2 pair and 2 pair + 1
+//     one 16-byte load at  step + pair * PITCH  holds fragments 2 pair and 2 pair + 1
 //   K-major (rows of the stage are m, BK consecutive k per row: 128 bytes, or 64 with a k chunk of 8):
-//     fragment i at  (i odd ? q1 : q0) + (i / 2) * pitch,  pitch = 16 rows
+//     fragment i at  step + (i odd ? odd : 0) + (i / 2) * PITCH,  PITCH = 16 rows
 // The 16-byte chunk index inside a row is XORed with (row % 8) (128-byte rows, 128-byte swizzle) or
-// with (row / 2) % 4 (64-byte rows, 64-byte swizzle).
-struct FragAddr {
-    uint32_t q0, q1;
+// with (row / 2) % 4 (64-byte rows, 64-byte swizzle).  In all of them 16 m are BK * 128 bytes apart, step 1 differs from step 0
+// and steps 2, 3 from 0, 1 by a thread's own constant: worked out once per block, because between two MMAs of a warp every
+// instruction is time in which it feeds the pipe nothing (5184^3: 8 670 us with the offsets worked out per step and two ways
+// through a stage, 8 246 now; 98 % of the pipe's cycles).
+template <int BK>
+struct FragOffsets {
+    static constexpr uint32_t PITCH = BK * 128u;
+    uint32_t step0, step1, later, odd;
+
+    // `slabs8`: MN-major rows of 64 bytes (slabs of 8); the thread's slab, fr / 4, is already part of thread_base
+    template <bool MN>
+    __device__ __forceinline__ void set(uint32_t thread_base, uint32_t fr, uint32_t fk, bool slabs8)
+    {
+        auto offset = [&](uint32_t t) {
+            const uint32_t k = step_k(t, fk);
+            if (MN) return slabs8 ? thread_base + k * 64u + (((fr & 3u) ^ ((k >> 1) & 3u)) << 4) : thread_base + k * 128u + ((fr ^ (k & 7u)) << 4);
+            const uint32_t kk = (k & 1u) * 8u, kc = k >> 1;
+            return thread_base + kk + (BK == 8 ? (kc ^ (fr & 3u)) << 4 : (kc ^ ((2u * fr) & 7u)) << 4);   // (rows 2 fr and 2 fr + 1 share (row / 2) % 4)
+        };
+        step0 = offset(0);
+        step1 = offset(1);
+        later = offset(2) - step0;
+        odd = MN ? 0u : BK == 8 ? 64u : (fk & 1u) ? 112u : 144u;   // the next row, its chunk index with bit 0 flipped
+    }
 };
 
-// `rows64`: K-major rows of 64 bytes (k chunk of 8); `slabs8`: MN-major rows of 64 bytes (slabs of 8)
-template <bool MN>
-__device__ __forceinline__ FragAddr frag_addr(uint32_t thread_base, uint32_t k, uint32_t fr, bool rows64, bool slabs8)
+template <bool MN, int N, int BK>
+__device__ __forceinline__ void load_frag(double (&f)[N], int i, uint32_t q, uint32_t odd)
 {
-    FragAddr f;
     if (MN) {
-        // (with slabs of 8 the thread's slab, fr / 4, is already part of thread_base)
-        f.q0 = slabs8 ? thread_base + k * 64u + (((fr & 3u) ^ ((k >> 1) & 3u)) << 4) : thread_base + k * 128u + ((fr ^ (k & 7u)) << 4);
-        f.q1 = 0;
+        if ((i & 1) == 0) ld_shared_v2f64(q + static_cast<uint32_t>(i >> 1) * FragOffsets<BK>::PITCH, f[i], f[i + 1]);
     } else {
-        const uint32_t kk = (k & 1u) * 8u, kc = k >> 1;
-        if (rows64) {
-            f.q0 = thread_base + kk + ((kc ^ (fr & 3u)) << 4);  // rows 2 fr and 2 fr + 1 share (row / 2) % 4
-            f.q1 = f.q0 + 64u;
-        } else {
-            f.q0 = thread_base + kk + ((kc ^ ((2u * fr) & 7u)) << 4);
-            f.q1 = thread_base + 128u + kk + ((kc ^ ((2u * fr + 1u) & 7u)) << 4);
-        }
+        f[i] = ld_shared_f64(q + ((i & 1) ? odd : 0u) + static_cast<uint32_t>(i >> 1) * FragOffsets<BK>::PITCH);
     }
-    return f;
 }
 
-// load `n` fragments (n = 8 for A, 4 for B), all at once
-template <bool MN, int N>
-__device__ __forceinline__ void load_all(double (&f)[N], const FragAddr& q, uint32_t pitch)
+// load `n` fragments (n = 8 for A, 4 or 2 for B), all at once
+template <bool MN, int N, int BK>
+__device__ __forceinline__ void load_all(double (&f)[N], uint32_t q, uint32_t odd)
 {
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        if (MN) {
-            if ((i & 1) == 0) ld_shared_v2f64(q.q0 + static_cast<uint32_t>(i >> 1) * pitch, f[i], f[i + 1]);
-        } else {
-            f[i] = ld_shared_f64(((i & 1) ? q.q1 : q.q0) + static_cast<uint32_t>(i >> 1) * pitch);
-        }
-    }
+    for (int i = 0; i < N; ++i) load_frag<MN, N, BK>(f, i, q, odd);
 }
 
-// One k4 step of a warp: 8 NF MMAs on the current fragments (NF = 4 or 2 column fragments); with PF the fragment loads of the next
+// One k4 step of a warp: 8 NF MMAs on the current fragments (NF = 4 or 2 column fragments); the fragment loads of the next
 // step are issued between them, where the FP64 tensor pipe leaves issue slots free.
 // acc[i][j][h]: row m = 16 (i / 2) + 4 (lane % 4) + 2 h + (i % 2), column n = 16 (j / 2) + 2 (lane / 4) + (j % 2).
-template <bool PF, bool AMN, bool BMN, int NF>
+template <bool AMN, bool BMN, int NF, int BK>
 __device__ __forceinline__ void mma_step(double (&acc)[8][NF][2], const double (&ac)[8], const double (&bc)[NF], double (&an)[8],
-                                         double (&bn)[NF], const FragAddr& qa, const FragAddr& qb, uint32_t a_pitch, uint32_t b_pitch)
+                                         double (&bn)[NF], uint32_t qa, uint32_t a_odd, uint32_t qb, uint32_t b_odd)
 {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
 #pragma unroll
         for (int j = 0; j < NF; ++j) dmma_m8n8k4(acc[i][j], bc[j], ac[i]);
-        if (PF) {
-            if (AMN) {
-                if ((i & 1) == 0) ld_shared_v2f64(qa.q0 + static_cast<uint32_t>(i >> 1) * a_pitch, an[i], an[i + 1]);
-            } else {
-                an[i] = ld_shared_f64(((i & 1) ? qa.q1 : qa.q0) + static_cast<uint32_t>(i >> 1) * a_pitch);
-            }
-            if (BMN) {
-                if ((i == 1 || i == 3) && i < NF) ld_shared_v2f64(qb.q0 + static_cast<uint32_t>(i >> 1) * b_pitch, bn[i - 1], bn[i]);
-            } else {
-                if (i < NF) bn[i] = ld_shared_f64(((i & 1) ? qb.q1 : qb.q0) + static_cast<uint32_t>(i >> 1) * b_pitch);
-            }
+        load_frag<AMN, 8, BK>(an, i, qa, a_odd);
+        if (BMN) {
+            if ((i == 1 || i == 3) && i < NF) load_frag<true, NF, BK>(bn, i - 1, qb, b_odd);
+        } else {
+            if (i < NF) load_frag<false, NF, BK>(bn, i, qb, b_odd);
         }
     }
 }
 
 // SCALED: C = alpha A B + beta C in the epilogue (C read only when beta is not zero); a template parameter because the
 // overwriting kernel has no registers to spare for it.
-template <bool AMN, bool BMN, int NF, bool SCALED>
+template <bool AMN, bool BMN, int NF, int BK, bool SCALED>
 __global__ void __launch_bounds__(kThreads64, 1)
 dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                 const __grid_constant__ UmmaParams p)
@@ -319,16 +316,13 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
         const int cw = warp & 3, grp = (warp >> 2) - 1, wm = cw & 1, wn = cw >> 1;
         const uint32_t fr = static_cast<uint32_t>(lane >> 2), fk = static_cast<uint32_t>(lane & 3);
         const uint32_t first = static_cast<uint32_t>(grp) * ring;
-        // pitch between fragment pairs: one 16-wide slab (MN-major) or 16 rows (K-major)
-        const bool rows64 = p.BK == 8;
-        const uint32_t k_row = rows64 ? 64u : 128u;
         const bool a8 = AMN && p.a.slab_w == 8, b8 = BMN && p.b.slab_w == 8;  // 16 m = two slabs of 8
-        const uint32_t a_pitch = AMN ? static_cast<uint32_t>(p.a.slab_bytes) * (a8 ? 2u : 1u) : 16u * k_row;
-        const uint32_t b_pitch = BMN ? static_cast<uint32_t>(p.b.slab_bytes) * (b8 ? 2u : 1u) : 16u * k_row;
-        const uint32_t a_thread = AMN ? static_cast<uint32_t>(wm * 4) * a_pitch + (a8 ? (fr >> 2) * static_cast<uint32_t>(p.a.slab_bytes) : 0u)
-                                      : (static_cast<uint32_t>(wm * 64) + 2u * fr) * k_row;
-        const uint32_t b_thread = a_tile_bytes + (BMN ? static_cast<uint32_t>(wn * (NF / 2)) * b_pitch + (b8 ? (fr >> 2) * static_cast<uint32_t>(p.b.slab_bytes) : 0u)
-                                                      : (static_cast<uint32_t>(wn * NF * 8) + 2u * fr) * k_row);
+        constexpr uint32_t PITCH = FragOffsets<BK>::PITCH;
+        FragOffsets<BK> fa, fb;
+        fa.template set<AMN>(AMN ? static_cast<uint32_t>(wm * 4) * PITCH + (a8 ? (fr >> 2) * static_cast<uint32_t>(p.a.slab_bytes) : 0u)
+                                 : (static_cast<uint32_t>(wm * 64) + 2u * fr) * (BK * 8u), fr, fk, a8);
+        fb.template set<BMN>(a_tile_bytes + (BMN ? static_cast<uint32_t>(wn * (NF / 2)) * PITCH + (b8 ? (fr >> 2) * static_cast<uint32_t>(p.b.slab_bytes) : 0u)
+                                                 : (static_cast<uint32_t>(wn * NF * 8) + 2u * fr) * (BK * 8u)), fr, fk, b8);
 
         double acc[8][NF][2];
 #pragma unroll
@@ -347,60 +341,47 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
 
             const WorkUnit w = decode_unit(blockIdx.x + i * gridDim.x, p, tiles_m, tiles_n);
             double* __restrict__ C = p.C64 + static_cast<long long>(w.split) * p.split_stride;
-            bool tile_ok = true;
-            // fa0/fb0 may already hold the first fragments of the stage about to be worked on: the last step
-            // of a stage fetches them when the next stage has landed by then, instead of ending with a
-            // step without loads and starting the next stage with loads nothing overlaps
-            bool have_first = false;
+            bool tile_ok;
+            // One path through a stage, with few instructions that are not between two MMAs: the last step of a stage fetches the
+            // first fragments of the next one, whose barrier is looked at a step earlier (behind the last stage of a tile the
+            // fragments are fetched from that stage again and not used).  A wait that gave up leaves wrong fragments, and
+            // tile_ok says so.
             double fa0[8], fb0[NF], fa1[8], fb1[NF];
-            int chunk = w.it0 ? w.it0 % p.k_digit_ext[0] : 0;   // chunk of the chunked mode
-            for (int it = 0; it < w.n_it; ++it) {
-                if (i == 0 && my_tiles > 1 && it == w.n_it / 2) asm volatile("bar.arrive 1, 256;" ::: "memory");
-                const uint32_t ps = first + stage;
-                bool ok = true;
-                if (!have_first) {
-                    const long long tw = prof ? clock64() : 0;
-                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar_full + ps), phase, abort_flag));
-                    if (prof) t_full += clock64() - tw;
+            uint32_t chunk = static_cast<uint32_t>(w.it0 ? w.it0 % p.k_digit_ext[0] : 0);   // chunk of the chunked mode
+            {
+                const long long tw = prof ? clock64() : 0;
+                tile_ok = mbar_wait(smem_u32(bar_full + first + stage), phase, abort_flag);
+                tile_ok = __all_sync(0xffffffffu, tile_ok);
+                if (prof) t_full += clock64() - tw;
+            }
+            uint32_t sb = smem_u32(smem) + (first + stage) * stage_bytes;
+            load_all<AMN, 8, BK>(fa0, sb + fa.step0, fa.odd);
+            load_all<BMN, NF, BK>(fb0, sb + fb.step0, fb.odd);
+            for (int left = w.n_it; left > 0; --left) {
+                if (i == 0 && my_tiles > 1 && left == w.n_it - w.n_it / 2) asm volatile("bar.arrive 1, 256;" ::: "memory");
+                const uint32_t bar_done = smem_u32(bar_empty + first + stage);
+                if (++stage == ring) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
-                tile_ok = tile_ok && ok;
-                const uint32_t next_stage = stage + 1 == ring ? 0u : stage + 1u, next_phase = stage + 1 == ring ? phase ^ 1u : phase;
-                bool next_first = false;
-                if (ok) {
-                    const uint32_t sb = smem_u32(smem) + ps * stage_bytes;
-                    FragAddr qa, qb;
-                    if (!have_first) {
-                        qa = frag_addr<AMN>(sb + a_thread, step_k(0, fk), fr, rows64, a8), qb = frag_addr<BMN>(sb + b_thread, step_k(0, fk), fr, rows64, b8);
-                        load_all<AMN, 8>(fa0, qa, a_pitch);
-                        load_all<BMN, NF>(fb0, qb, b_pitch);
-                    }
-                    qa = frag_addr<AMN>(sb + a_thread, step_k(1, fk), fr, rows64, a8), qb = frag_addr<BMN>(sb + b_thread, step_k(1, fk), fr, rows64, b8);
-                    mma_step<true, AMN, BMN, NF>(acc, fa0, fb0, fa1, fb1, qa, qb, a_pitch, b_pitch);
-                    // (the last chunk of a mode that is 1 to 8 past a multiple of 16 holds zeros in its second half: 5184^3 with
-                    // contracted modes of 72 computed a tenth of its k for nothing, 9 520 us)
-                    if (chunk < p.full_chunks) {
-                        qa = frag_addr<AMN>(sb + a_thread, step_k(2, fk), fr, rows64, a8), qb = frag_addr<BMN>(sb + b_thread, step_k(2, fk), fr, rows64, b8);
-                        mma_step<true, AMN, BMN, NF>(acc, fa1, fb1, fa0, fb0, qa, qb, a_pitch, b_pitch);
-                        qa = frag_addr<AMN>(sb + a_thread, step_k(3, fk), fr, rows64, a8), qb = frag_addr<BMN>(sb + b_thread, step_k(3, fk), fr, rows64, b8);
-                        mma_step<true, AMN, BMN, NF>(acc, fa0, fb0, fa1, fb1, qa, qb, a_pitch, b_pitch);
-                    }
-                    // last step: one look at the next stage's barrier; if its data is there, fetch from it
-                    if (it + 1 < w.n_it)
-                        next_first = __all_sync(0xffffffffu, mbar_test_wait(smem_u32(bar_full + first + next_stage), next_phase));
-                    if (next_first) {
-                        const uint32_t nb = smem_u32(smem) + (first + next_stage) * stage_bytes;
-                        qa = frag_addr<AMN>(nb + a_thread, step_k(0, fk), fr, rows64, a8), qb = frag_addr<BMN>(nb + b_thread, step_k(0, fk), fr, rows64, b8);
-                        mma_step<true, AMN, BMN, NF>(acc, fa1, fb1, fa0, fb0, qa, qb, a_pitch, b_pitch);
-                    } else {
-                        mma_step<false, AMN, BMN, NF>(acc, fa1, fb1, fa0, fb0, qa, qb, a_pitch, b_pitch);
-                    }
+                uint32_t later_a = 0, later_b = 0;
+                // (the last chunk of a mode that is 1 to 8 past a multiple of 16 holds zeros in its second half: 5184^3 with
+                // contracted modes of 72 computed a tenth of its k for nothing, 9 520 us)
+                if (BK == 16 && chunk < static_cast<uint32_t>(p.full_chunks)) {
+                    mma_step<AMN, BMN, NF, BK>(acc, fa0, fb0, fa1, fb1, sb + fa.step1, fa.odd, sb + fb.step1, fb.odd);
+                    later_a = fa.later;
+                    later_b = fb.later;
+                    mma_step<AMN, BMN, NF, BK>(acc, fa1, fb1, fa0, fb0, sb + fa.step0 + later_a, fa.odd, sb + fb.step0 + later_b, fb.odd);
                 }
-                have_first = next_first;
+                const uint32_t bar_next = smem_u32(bar_full + first + stage);
+                const bool more = left > 1, landed = !more || mbar_test_wait(bar_next, phase);
+                mma_step<AMN, BMN, NF, BK>(acc, fa0, fb0, fa1, fb1, sb + fa.step1 + later_a, fa.odd, sb + fb.step1 + later_b, fb.odd);
+                if (!__all_sync(0xffffffffu, landed)) tile_ok = __all_sync(0xffffffffu, mbar_wait(bar_next, phase, abort_flag)) && tile_ok;
+                if (more) sb = smem_u32(smem) + (first + stage) * stage_bytes;
+                mma_step<AMN, BMN, NF, BK>(acc, fa1, fb1, fa0, fb0, sb + fa.step0, fa.odd, sb + fb.step0, fb.odd);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(bar_empty + ps));  // this warp is done reading the stage
-                stage = next_stage;
-                phase = next_phase;
-                if (++chunk == p.k_digit_ext[0]) chunk = 0;
+                if (lane == 0) mbar_arrive(bar_done);  // this warp is done reading the stage
+                if (++chunk == static_cast<uint32_t>(p.k_digit_ext[0])) chunk = 0;
             }
             if (prof) { const long long t1 = clock64(); t_main += t1 - t0; t0 = t1; }
 
@@ -518,51 +499,46 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     if (threadIdx.x == 0 && ld_shared_u32(abort_flag)) atomicMax(p.status, 1);
 }
 
-template <bool AMN, bool BMN, int NF>
-cudaError_t launch_variant(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, unsigned grid, cudaStream_t stream)
+// The kernel's forms, one function per (majors, columns, k chunk, scaled); `use` is called with the one that matches.
+template <bool AMN, bool BMN, int NF, int BK, typename Use>
+cudaError_t with_scaled(bool scaled, Use&& use)
 {
-    const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
-    return launch_chained(p.scaled ? dmma_tma_kernel<AMN, BMN, NF, true> : dmma_tma_kernel<AMN, BMN, NF, false>, dim3(grid), dim3(kThreads64),
-                          static_cast<size_t>(smem_bytes), stream, 1, ta, tb, p);
+    return scaled ? use(dmma_tma_kernel<AMN, BMN, NF, BK, true>) : use(dmma_tma_kernel<AMN, BMN, NF, BK, false>);
 }
-
-template <int NF>
-cudaError_t launch_width(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, unsigned grid, cudaStream_t stream)
+template <int NF, int BK, typename Use>
+cudaError_t with_majors(bool amn, bool bmn, bool scaled, Use&& use)
 {
-    if (p.a.major && p.b.major) return launch_variant<true, true, NF>(p, tmapA, tmapB, smem_bytes, grid, stream);
-    if (p.a.major) return launch_variant<true, false, NF>(p, tmapA, tmapB, smem_bytes, grid, stream);
-    if (p.b.major) return launch_variant<false, true, NF>(p, tmapA, tmapB, smem_bytes, grid, stream);
-    return launch_variant<false, false, NF>(p, tmapA, tmapB, smem_bytes, grid, stream);
+    if (amn) return bmn ? with_scaled<true, true, NF, BK>(scaled, use) : with_scaled<true, false, NF, BK>(scaled, use);
+    return bmn ? with_scaled<false, true, NF, BK>(scaled, use) : with_scaled<false, false, NF, BK>(scaled, use);
 }
-
-template <int NF, bool SCALED>
-cudaError_t configure_width()
+template <typename Use>
+cudaError_t with_kernel(int bn, int bk, bool amn, bool bmn, bool scaled, Use&& use)
 {
-    const int smem_bytes = kMaxDynamicSmemBytes;  // the same opt-in maximum for every run (the cap is per function and device)
-    cudaError_t e = cudaFuncSetAttribute(dmma_tma_kernel<false, false, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<false, true, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<true, false, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(dmma_tma_kernel<true, true, NF, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    return e;
+    if (bk == 16) return bn == 64 ? with_majors<4, 16>(amn, bmn, scaled, use) : with_majors<2, 16>(amn, bmn, scaled, use);
+    return bn == 64 ? with_majors<4, 8>(amn, bmn, scaled, use) : with_majors<2, 8>(amn, bmn, scaled, use);
 }
 
 }  // namespace
 
+// The dynamic shared-memory cap is per function and device: every run sets the same opt-in maximum.
 cudaError_t dmma_tma_configure()
 {
-    cudaError_t e = configure_width<4, false>();
-    if (e == cudaSuccess) e = configure_width<2, false>();
-    if (e == cudaSuccess) e = configure_width<4, true>();
-    if (e == cudaSuccess) e = configure_width<2, true>();
+    cudaError_t e = cudaSuccess;
+    for (int form = 0; form < 32 && e == cudaSuccess; ++form)
+        e = with_kernel(form & 1 ? 64 : 32, form & 2 ? 16 : 8, form & 4, form & 8, form & 16,
+                        [](auto* kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes); });
     return e;
 }
 
 cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, int num_sms, cudaStream_t stream)
 {
     const long long total = p.tiles_m * p.tiles_n * p.k_splits;
-    if (total <= 0 || p.k_splits < 1 || p.stages < 2 || (p.stages & 1) || (p.BN != 64 && p.BN != 32)) return cudaErrorInvalidValue;
+    if (total <= 0 || p.k_splits < 1 || p.stages < 2 || (p.stages & 1) || (p.BN != 64 && p.BN != 32) || (p.BK != 16 && p.BK != 8)) return cudaErrorInvalidValue;
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
-    return p.BN == 64 ? launch_width<4>(p, tmapA, tmapB, smem_bytes, grid, stream) : launch_width<2>(p, tmapA, tmapB, smem_bytes, grid, stream);
+    const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
+    return with_kernel(p.BN, p.BK, p.a.major != 0, p.b.major != 0, p.scaled != 0, [&](auto* kernel) {
+        return launch_chained(kernel, dim3(grid), dim3(kThreads64), static_cast<size_t>(smem_bytes), stream, 1, ta, tb, p);
+    });
 }
 
 }  // namespace tcontb
