@@ -435,6 +435,7 @@ tcontb_status finish_run(tcontb_run* run)
         run->umma.pair = u.pair ? 1 : 0;
         run->umma.producers = u.producers;
         run->umma.store_across_slabs = u.store_across_slabs ? 1 : 0;
+        run->umma.pieces32 = u.pieces32 ? 1 : 0;
         run->umma.n_k_digits = u.n_k_digits;
         for (int i = 0; i < 3; ++i) run->umma.k_digit_ext[i] = static_cast<int>(u.k_digit_ext[i]);
         run->umma.k_iters = static_cast<int>(u.k_iters);
@@ -467,13 +468,13 @@ tcontb_status finish_run(tcontb_run* run)
             TC_CUDA(run->loB.alloc(static_cast<size_t>(run->kernB_elements) * run->elt));
             run->kernels_per_launch += 4;  // two residual passes, two more contractions
         }
-        // The TMA-fed FP64 kernel with a C of up to half of L2 applies alpha and beta in a second pass: its tiles wait for the old
-        // values of C, while a workspace written by the kernel and read by the partial-sum pass stays in L2 (C of 38 MB: 37 us
-        // in two passes, 43 in one; of 302 MB: 259 and 220).  Tiles across slabs read and write C in pieces of 64 bytes; with k
-        // chunks of 16 and few of them they take two passes whatever the size (C of 132 MB, K 48: 140 us in two, 168 in one; of 755 MB, K 16:
-        // 596 and 672; with chunks of 8, 453 MB, K 8: 334 and 308; 20 chunks of 16, 73 MB: 274 and 264).  TCONT_SCALE_PASSES=1|2 overrides the rule.
+        // Tiles across slabs read the old values of C in pieces of 32 bytes: with a C of up to half of L2, or few k chunks, and k
+        // chunks of 16, the TMA-fed FP64 kernel writes a workspace instead, and a second pass applies alpha and beta (C of 72 MB,
+        // K 72: 107 us in two passes, 171 in one; 131 MB, K 48: 143 and 177; 755 MB, K 16: 699 and 738; 231 MB, K 312: 689 and 670;
+        // with chunks of 8, 302 MB, K 24: 242 and 168).  With rows along C one pass is faster (4.7 M elements, K 48: 24 us, 35 in
+        // two; 16.8 M, K 16: 66 and 96).  TCONT_SCALE_PASSES=1|2 overrides the rule.
         const bool unsplit = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1;
-        run->scale_pass = unsplit && (pl.sizeC * static_cast<int64_t>(run->elt) <= kScalePassInL2 || (u.store_across_slabs && u.BK == 16 && u.k_iters <= 6));
+        run->scale_pass = unsplit && u.store_across_slabs && u.BK == 16 && (pl.sizeC * static_cast<int64_t>(run->elt) <= kScalePassInL2 || u.k_iters <= 6);
         if (const char* sp = std::getenv("TCONT_SCALE_PASSES")) run->scale_pass = unsplit && sp[0] != '1';
         run->umma.C = static_cast<float*>(out);
         run->umma.C64 = static_cast<double*>(out);

@@ -63,18 +63,9 @@ __device__ __forceinline__ void st_global_cs_v4f64(double* p, double a, double b
     asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
 
-// The four elements of C a thread is about to overwrite (C = alpha A B + beta C with beta != 0); 32 bytes when `vec`.
-__device__ __forceinline__ void load_old4(double (&o)[4], const double* dst, bool vec, const double* p0, const double* p1, const double* p2,
-                                          const double* p3)
+__device__ __forceinline__ void ld_global_cs_v4f64(double (&o)[4], const double* p)
 {
-    if (vec) {
-        asm volatile("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(dst) : "memory");
-    } else {
-        o[0] = p0 ? __ldcs(p0) : 0.0;
-        o[1] = p1 ? __ldcs(p1) : 0.0;
-        o[2] = p2 ? __ldcs(p2) : 0.0;
-        o[3] = p3 ? __ldcs(p3) : 0.0;
-    }
+    asm volatile("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(p) : "memory");
 }
 
 // Which k a lane feeds into step t of a stage: k = 8 (t / 2) + 2 fk + ((fk ^ (fk >> 1) ^ t) & 1), fk = lane % 4.
@@ -176,6 +167,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     const uint32_t abort_flag = smem_u32(bar_empty + 8);
     uint64_t* tab_full = bar_empty + 10;   // [group][buffer]
     uint64_t* tab_empty = tab_full + 4;    // [group][buffer]
+    const uint32_t ragged = smem_u32(tab_empty + 4);   // [group][buffer]: 1 + number of the last tile with rows or columns beyond C
     const uint32_t tabs = smem_u32(aux + 256);  // [group][buffer]: long long [128] row offsets, [64] column offsets (-1 = beyond C)
 
     if (threadIdx.x == 0) {
@@ -187,6 +179,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             mbar_init(smem_u32(tab_full + s), 64);  // every builder thread
             mbar_init(smem_u32(tab_empty + s), 4);  // one arrival per consumer warp
         }
+        for (uint32_t t = 0; t < 4; ++t) st_shared_u32(ragged + t * 4u, 0u);
         st_shared_u32(abort_flag, 0u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -291,6 +284,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     int d0 = 0;
                     const long long off = slab_c_offset(o, (is_row ? tm * SA : tn * SB) + sl, &d0, &ok);
                     ok = ok && (d0 * o.slab_w + in < o.slab_mode_ext);
+                    if (!ok) st_shared_u32(ragged + slot * 4u, i + 1u);
                     st_shared_s64(tab + static_cast<uint32_t>(e) * 8u, ok ? off + slab_elem_offset(o, d0, in) : -1);
                 }
                 mbar_arrive(smem_u32(tab_full + slot));
@@ -391,96 +385,83 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             const uint32_t row_tab = tabs + slot * kTabBytes, col_tab = row_tab + kBM * 8u;
             if (prof) { const long long t1 = clock64(); t_tab += t1 - t0; t0 = t1; }
 
-            // store: four consecutive rows per (fragment pair, column fragment), 32 bytes when aligned
-            long long cn[NF];
+            // Store.  Four elements of C a thread holds for each of 4 x NF (u, column fragment) lie next to each other:
+            //   rows along C    : rows 16 u + 4 fk + q, element q in acc[2 u + (q & 1)][j][q >> 1]
+            //   rows across slabs: the warp's 64 rows are four slabs of 16, slab q is index a0 + q of C's stride-1 mode; row
+            //                      4 fk + u of the four slabs, element q in acc[2 q + (u & 1)][j][u >> 1]
+            long long cn[NF], cm[4];
 #pragma unroll
             for (int j = 0; j < NF; ++j)
                 cn[j] = ld_shared_s64(col_tab + (static_cast<uint32_t>(wn * NF * 8 + 16 * (j >> 1) + (j & 1)) + 2u * fr) * 8u);
-            // alpha and beta on the four elements of every column fragment; the old values of two fragments are asked
-            // for before the first is used (four at a time spill: 228 us where two at a time take 220)
-            auto scale_four = [&](long long cm0, long long cm1, long long cm2, long long cm3, bool run4, auto&& at) {
+            const uint32_t row_u = p.store_across_slabs ? 8u : 128u, row_q = p.store_across_slabs ? 128u : 8u;   // table bytes from u to u + 1, q to q + 1
+            const uint32_t rows = row_tab + (static_cast<uint32_t>(wm * 64) + 4u * fk) * 8u;
 #pragma unroll
-                for (int j0 = 0; j0 < NF; j0 += 2) {
-                    double old[2][4];
+            for (int u = 0; u < 4; ++u) cm[u] = ld_shared_s64(rows + static_cast<uint32_t>(u) * row_u);
+            const bool whole = p.pieces32 && tile_ok && (reinterpret_cast<uintptr_t>(C) & 31u) == 0 && ld_shared_u32(ragged + slot * 4u) != i + 1u;
+            auto store_tile = [&](auto&& at) {
+                if (whole) {
+                    // Straight-line: a warp alone on its scheduler takes 5 to 20 cycles for every instruction and branch between
+                    // two stores (with alignment and bounds tested per store 4 200 cycles a tile, whatever the pieces' layout;
+                    // tested per tile here 2 900, by the table builders 1 700).  9216 x 4096 x 24, C of 302 MB: accumulating 206 -> 168
+                    // us, with rows along C 223 -> 146; overwriting 110 -> 90.
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const long long c = cn[j0 + u];
-                        if (tile_ok && c >= 0 && p.beta != 0.0)
-                            load_old4(old[u], C + cm0 + c, run4 && (reinterpret_cast<uintptr_t>(C + cm0 + c) & 31u) == 0, cm0 >= 0 ? C + cm0 + c : nullptr,
-                                      cm1 >= 0 ? C + cm1 + c : nullptr, cm2 >= 0 ? C + cm2 + c : nullptr, cm3 >= 0 ? C + cm3 + c : nullptr);
-                        else old[u][0] = old[u][1] = old[u][2] = old[u][3] = 0.0;
+                    for (int u = 0; u < 4; ++u) {
+                        if constexpr (SCALED) {   // the old values of all column fragments are asked for before the first is used
+                            double old[NF][4];
+#pragma unroll
+                            for (int j = 0; j < NF; ++j) {
+                                if (p.beta != 0.0) ld_global_cs_v4f64(old[j], C + cm[u] + cn[j]);
+                                else old[j][0] = old[j][1] = old[j][2] = old[j][3] = 0.0;
+                            }
+#pragma unroll
+                            for (int j = 0; j < NF; ++j)
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) at(u, j, q) = p.alpha * at(u, j, q) + p.beta * old[j][q];
+                        }
+#pragma unroll
+                        for (int j = 0; j < NF; ++j) st_global_cs_v4f64(C + cm[u] + cn[j], at(u, j, 0), at(u, j, 1), at(u, j, 2), at(u, j, 3));
                     }
+                } else if (tile_ok) {
+                    // ragged or odd-aligned pieces: 32 bytes where they can be, 16 where two elements are neighbours, else one by one
 #pragma unroll
-                    for (int u = 0; u < 2; ++u)
+                    for (int u = 0; u < 4; ++u) {
+                        long long r[4];
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) at(j0 + u, q) = p.alpha * at(j0 + u, q) + p.beta * old[u][q];
+                        for (int q = 0; q < 4; ++q) r[q] = ld_shared_s64(rows + static_cast<uint32_t>(u) * row_u + static_cast<uint32_t>(q) * row_q);
+                        const bool run4 = r[0] >= 0 && r[1] == r[0] + 1 && r[2] == r[0] + 2 && r[3] == r[0] + 3;
+#pragma unroll
+                        for (int j = 0; j < NF; ++j) {
+                            if (cn[j] < 0) continue;
+                            double x[4];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                x[q] = at(u, j, q);
+                                if constexpr (SCALED) x[q] = p.alpha * x[q] + (p.beta != 0.0 && r[q] >= 0 ? p.beta * __ldcs(C + r[q] + cn[j]) : 0.0);
+                            }
+                            if (run4 && (reinterpret_cast<uintptr_t>(C + r[0] + cn[j]) & 31u) == 0) {
+                                st_global_cs_v4f64(C + r[0] + cn[j], x[0], x[1], x[2], x[3]);
+                                continue;
+                            }
+#pragma unroll
+                            for (int q = 0; q < 4; q += 2) {
+                                double* d = C + r[q] + cn[j];
+                                if (r[q] >= 0 && r[q + 1] == r[q] + 1 && (reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
+                                    __stcs(reinterpret_cast<double2*>(d), make_double2(x[q], x[q + 1]));
+                                } else {
+                                    if (r[q] >= 0) __stcs(d, x[q]);
+                                    if (r[q + 1] >= 0) __stcs(C + r[q + 1] + cn[j], x[q + 1]);
+                                }
+                            }
+                        }
+                    }
                 }
             };
-            if (p.store_across_slabs) {
-                // The warp's 64 rows are four slabs of 16; slab q is index a0 + q of C's stride-1 mode and the rows
-                // of a slab run along another mode.  Row (4 fk + dd) of the four slabs is four neighbouring
-                // elements of C: acc[2 q + (dd & 1)][j][dd >> 1], q = 0..3.
+            if (p.store_across_slabs) store_tile([&](int u, int j, int q) -> double& { return acc[2 * q + (u & 1)][j][u >> 1]; });
+            else store_tile([&](int u, int j, int q) -> double& { return acc[2 * u + (q & 1)][j][q >> 1]; });
 #pragma unroll
-                for (int dd = 0; dd < 4; ++dd) {
-                    const int par = dd & 1, h = dd >> 1;
-                    const uint32_t r = static_cast<uint32_t>(wm * 64) + 4u * fk + static_cast<uint32_t>(dd);
-                    const long long cm0 = ld_shared_s64(row_tab + r * 8u), cm1 = ld_shared_s64(row_tab + (r + 16u) * 8u);
-                    const long long cm2 = ld_shared_s64(row_tab + (r + 32u) * 8u), cm3 = ld_shared_s64(row_tab + (r + 48u) * 8u);
-                    const bool run4 = cm0 >= 0 && cm1 == cm0 + 1 && cm2 == cm0 + 2 && cm3 == cm0 + 3;
-                    if constexpr (SCALED) scale_four(cm0, cm1, cm2, cm3, run4, [&](int j, int q) -> double& { return acc[2 * q + par][j][h]; });
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-                    for (int j = 0; j < NF; ++j) {
-                        if (tile_ok && cn[j] >= 0) {
-                            double* dst = C + cm0 + cn[j];
-                            if (run4 && (reinterpret_cast<uintptr_t>(dst) & 31u) == 0) {
-                                st_global_cs_v4f64(dst, acc[par][j][h], acc[2 + par][j][h], acc[4 + par][j][h], acc[6 + par][j][h]);
-                            } else {
-                                if (cm0 >= 0) __stcs(dst, acc[par][j][h]);
-                                if (cm1 >= 0) __stcs(C + cm1 + cn[j], acc[2 + par][j][h]);
-                                if (cm2 >= 0) __stcs(C + cm2 + cn[j], acc[4 + par][j][h]);
-                                if (cm3 >= 0) __stcs(C + cm3 + cn[j], acc[6 + par][j][h]);
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < NF; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-            } else
-#pragma unroll
-            for (int pr = 0; pr < 4; ++pr) {
-                const uint32_t r = static_cast<uint32_t>(wm * 64 + 16 * pr) + 4u * fk;
-                const long long cm0 = ld_shared_s64(row_tab + r * 8u), cm1 = ld_shared_s64(row_tab + r * 8u + 8u);
-                const long long cm2 = ld_shared_s64(row_tab + r * 8u + 16u), cm3 = ld_shared_s64(row_tab + r * 8u + 24u);
-                const bool run4 = cm0 >= 0 && cm1 == cm0 + 1 && cm2 == cm0 + 2 && cm3 == cm0 + 3;
-                if constexpr (SCALED) scale_four(cm0, cm1, cm2, cm3, run4, [&](int j, int q) -> double& { return acc[2 * pr + (q & 1)][j][q >> 1]; });
-#pragma unroll
-                for (int j = 0; j < NF; ++j) {
-                    if (tile_ok && cn[j] >= 0) {
-                        double* dst = C + cm0 + cn[j];
-                        if (run4 && (reinterpret_cast<uintptr_t>(dst) & 31u) == 0) {
-                            st_global_cs_v4f64(dst, acc[2 * pr][j][0], acc[2 * pr + 1][j][0], acc[2 * pr][j][1], acc[2 * pr + 1][j][1]);
-                        } else {
-                            // ragged or odd-aligned runs: 16 bytes where two rows are neighbours, else one by one
-                            if (cm0 >= 0 && cm1 == cm0 + 1 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-                                __stcs(reinterpret_cast<double2*>(dst), make_double2(acc[2 * pr][j][0], acc[2 * pr + 1][j][0]));
-                            } else {
-                                if (cm0 >= 0) __stcs(dst, acc[2 * pr][j][0]);
-                                if (cm1 >= 0) __stcs(C + cm1 + cn[j], acc[2 * pr + 1][j][0]);
-                            }
-                            double* dst2 = C + cm2 + cn[j];
-                            if (cm2 >= 0 && cm3 == cm2 + 1 && (reinterpret_cast<uintptr_t>(dst2) & 15u) == 0) {
-                                __stcs(reinterpret_cast<double2*>(dst2), make_double2(acc[2 * pr][j][1], acc[2 * pr + 1][j][1]));
-                            } else {
-                                if (cm2 >= 0) __stcs(dst2, acc[2 * pr][j][1]);
-                                if (cm3 >= 0) __stcs(C + cm3 + cn[j], acc[2 * pr + 1][j][1]);
-                            }
-                        }
-                    }
-                    acc[2 * pr][j][0] = acc[2 * pr][j][1] = acc[2 * pr + 1][j][0] = acc[2 * pr + 1][j][1] = 0.0;
-                }
-            }
+                for (int j = 0; j < NF; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(tab_empty + slot));  // this warp is done with the tables
             if (prof) t_store += clock64() - t0;

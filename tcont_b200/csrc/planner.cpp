@@ -716,6 +716,17 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
             o.row_digit_cstride[0] = 0;
         }
     }
+    if (f64) {
+        auto fours = [](const UmmaOperand& o, int from_digit) {
+            bool ok = o.split_inner == 0 || o.split_outer_cstride % 4 == 0;
+            for (int d = from_digit; d < o.n_row_digits; ++d) ok = ok && o.row_digit_cstride[d] % 4 == 0;
+            return ok;
+        };
+        // (across slabs the first digit is C's stride-1 mode, in whole eights, and the elements of a slab lie along another mode)
+        const bool rows = u->store_across_slabs ? fours(u->a, 1) && u->a.row_elem_cstride % 4 == 0
+                                                : fours(u->a, 0) && u->a.row_elem_cstride == 1 && u->a.split_inner % 4 == 0;
+        u->pieces32 = rows && fours(u->b, 0) && u->b.row_elem_cstride % 4 == 0;
+    }
     u->eligible = true;
 }
 

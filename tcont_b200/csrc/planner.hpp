@@ -109,6 +109,9 @@ struct UmmaSpec {
     // FP64 kernel: the slabs of an A tile are consecutive indices of C's stride-1 mode (which is not A's stride-1
     // mode); a thread stores the same row of four neighbouring slabs as one 32-byte piece
     bool store_across_slabs = false;
+    // FP64 kernel: the four elements of C a thread stores at a time are neighbours and, where C itself is, on a multiple of 32
+    // bytes, unless some of them lie beyond C
+    bool pieces32 = false;
     int smem_bytes = 0;
     int elt = 4;  // element bytes: 4 = tcgen05 TF32 kernel, 8 = TMA-fed FP64 tensor-path kernel
 };

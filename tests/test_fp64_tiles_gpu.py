@@ -37,3 +37,47 @@ def test_last_chunk_of_eight_or_fewer(engine, oracle, monkeypatch, chunked, layo
     u = desc["umma"]
     assert desc["kernel"] == "dmma_f64_tma"
     hold(oracle, c, A, B, out, chunked * other, u["k_splits"])
+
+
+# the epilogue's straight-line form (whole tiles, everything on multiples of 32 bytes) and the other one, tile by tile: ragged
+# last tiles, columns on odd multiples of 16 bytes (a = 130), C itself on one, fused rows, tiles across slabs, several tiles a group
+STORES = {
+    "whole": ("ab", "ak", "kb", dict(a=512, b=320, k=24), 0),
+    "last_tiles_ragged": ("ab", "ka", "bk", dict(a=1028, b=1060, k=16), 0),
+    "odd_columns": ("ab", "ak", "kb", dict(a=130, b=640, k=24), 0),
+    "odd_c": ("ab", "ak", "kb", dict(a=512, b=320, k=24), 2),
+    "fused_rows": ("acb", "abk", "kc", dict(a=12, b=60, c=128, k=24), 0),
+    "fused_rows_odd": ("acb", "abk", "kc", dict(a=6, b=50, c=128, k=24), 0),
+    "across_slabs": ("abcd", "dbea", "ec", dict(a=24, b=9, c=64, d=48, e=24), 0),
+    "across_slabs_ragged": ("abcd", "dbea", "ec", dict(a=24, b=9, c=60, d=54, e=40), 0),
+}
+
+
+@pytest.mark.parametrize("name", list(STORES))
+@pytest.mark.parametrize("beta", [0.0, -0.7])
+def test_stores(engine, oracle, monkeypatch, name, beta):
+    import torch
+    from tcont_b200 import api
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    monkeypatch.setenv("TCONT_SPLITK", "1")
+    monkeypatch.setenv("TCONT_SCALE_PASSES", "1")
+    C, A_, B_, ext, shift = STORES[name]
+    c = Contraction(C, A_, B_, ext, F64)
+    A, B = oracle.inputs(c, 31, -1.0, 1.0)
+    n = c.size(C)
+    C0 = np.random.default_rng(7).uniform(-4.0, 4.0, n)
+    guarded = torch.full((n + 16,), 7.0, dtype=torch.float64, device="cuda")
+    dC = guarded[shift:shift + n]
+    dC.copy_(torch.from_numpy(C0))
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    plan = engine.plan(to_equation(engine, c, 1))
+    run = api.prepare_on_device(plan, dA.data_ptr(), dB.data_ptr(), dC.data_ptr(), keep=(dA, dB, guarded))
+    run.set_scalars(1.0, beta)
+    engine.launch(run)
+    torch.cuda.synchronize()
+    assert plan.describe()["kernel"] == "dmma_f64_tma" and run.device_status() == 0
+    outside = torch.cat([guarded[:shift], guarded[shift + n:]])
+    assert bool((outside == 7.0).all())
+    exact, scale = oracle.contract(c, A, B) + beta * C0, oracle.contract(c, np.abs(A), np.abs(B)) + abs(beta * C0)
+    k = ext.get("k", ext.get("e"))
+    assert (np.abs(dC.cpu().numpy() - exact) <= (k + 4) * 2.0**-53 * scale).all()
