@@ -155,6 +155,9 @@ struct tcontb_run {
     // UMMA
     UmmaParams umma{};
     CUtensorMap tmA{}, tmB{};
+    // tiles across two stride-1 modes: C, and the workspace that alpha and beta are applied from
+    AcrossParams across{};
+    CUtensorMap tmC{}, tmWs{};
     DeviceBuffer status;
     DeviceBuffer splitk;  // partial tensors of a split-K contraction, k_splits copies of C (three times that with tf32x3)
     // Error-compensated Float32 (TCONT_TF32X3=1, tcgen05 kernel only): the part of each operand that
@@ -335,6 +338,64 @@ tcontb_status encode_map(const UmmaOperand& o, const void* base, int elt, CUtens
     return TCONTB_OK;
 }
 
+// A tensor map of the across_tf32 kernel.
+tcontb_status encode_across_map(const AcrossSpec::Map& m, void* base, CUtensorMapSwizzle swizzle, CUtensorMap* out)
+{
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return fail(TCONTB_RUNTIME_ERROR, "cuTensorMapEncodeTiled is not available from the CUDA driver");
+    cuuint64_t dims[kMaxTmaRank], strides[kMaxTmaRank - 1];
+    cuuint32_t box[kMaxTmaRank], estr[kMaxTmaRank];
+    for (int d = 0; d < kMaxTmaRank; ++d) {
+        dims[d] = static_cast<cuuint64_t>(m.ext[d]);
+        box[d] = static_cast<cuuint32_t>(m.box[d]);
+        estr[d] = 1;
+        if (d > 0) strides[d - 1] = static_cast<cuuint64_t>(m.stride[d]) * 4u;
+    }
+    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, kMaxTmaRank, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(TCONTB_RUNTIME_ERROR, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
+    return TCONTB_OK;
+}
+
+tcontb_status finish_across(tcontb_run* run, const void* A, const void* B)
+{
+    const AcrossSpec& s = run->plan.across;
+    AcrossParams& p = run->across;
+    p = AcrossParams{};
+    p.rows_first = s.rows_first ? 1 : 0;
+    p.inner = make_fast_div(s.rows_first ? s.tiles_m : s.tiles_n);
+    p.n_chunks = make_fast_div(s.n_chunks);
+    p.p0 = make_fast_div(s.p0);
+    p.y_chunks = make_fast_div(s.y_chunks);
+    p.x_chunks = make_fast_div(s.x_chunks);
+    p.o0 = make_fast_div(s.o0);
+    p.o1 = make_fast_div(s.o1);
+    p.row_others = s.row_others;
+    p.column_others = s.column_others;
+    p.k_ext = static_cast<int>(s.k_ext);
+    p.k1_ext = static_cast<int>(s.k1);
+    p.units = static_cast<uint32_t>(s.tiles_m * s.tiles_n);
+    p.BN = s.BN;
+    p.BK = s.BK;
+    p.stages = s.stages;
+    p.k_iters = static_cast<int>(s.k_iters);
+    p.b_major = s.b_major;
+    p.n_ext = static_cast<int>(s.n_ext);
+    p.x_ext = static_cast<int>(s.x_ext);
+    p.release_late = p.units >= 16u * static_cast<uint32_t>(run->num_sms) && s.k_iters <= 4 ? 1 : 0;
+    p.status = static_cast<int*>(run->status.ptr);
+    tcontb_status st = encode_across_map(s.a, const_cast<void*>(A), CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, &run->tmA);
+    if (st == TCONTB_OK) st = encode_across_map(s.b, const_cast<void*>(B), s.b_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, &run->tmB);
+    if (st == TCONTB_OK) st = encode_across_map(s.c, run->dC, CU_TENSOR_MAP_SWIZZLE_64B, &run->tmC);
+    if (st != TCONTB_OK) return st;
+    // alpha and beta: the kernel writes a workspace, a second pass applies them (C of 226 MB: 258 us, 413 with the copy of A)
+    run->scale_pass = true;
+    if (across_tf32_smem(s.stages, s.BN, s.BK) > kMaxDynamicSmemBytes) return fail(TCONTB_RUNTIME_ERROR, "plan asks for more shared memory than a block can have");
+    TC_CUDA(across_tf32_configure());
+    TC_CUDA(splitk_reduce_configure());
+    return TCONTB_OK;
+}
+
 // One digit of a mode group as the gather kernel splits it.
 void add_digit(RadixGroup* g, int64_t extent, int64_t x, int64_t y)
 {
@@ -390,6 +451,16 @@ void fill_gather(const Problem& p, const void* A, const void* B, void* C, const 
     *out = g;
 }
 
+// The same contraction planned again without tiles across two stride-1 modes.
+bool plan_without_across(const Plan& d, Plan* out)
+{
+    std::string err;
+    auto parent = [](const std::vector<int64_t>& v) { return v.empty() ? nullptr : v.data(); };
+    return make_plan(d.modeC.data(), static_cast<int>(d.modeC.size()), d.modeA.data(), static_cast<int>(d.modeA.size()), d.modeB.data(),
+                     static_cast<int>(d.modeB.size()), d.op, d.scalar_type, d.ext_mode.data(), d.ext_val.data(), static_cast<int>(d.ext_val.size()),
+                     d.backend_selection, device_cost_table(), out, &err, parent(d.parentC), parent(d.parentA), parent(d.parentB), true, false) == 0;
+}
+
 // Device-side set-up shared by the three run constructors; dL/dR/dC must already be set.
 tcontb_status finish_run(tcontb_run* run)
 {
@@ -397,6 +468,16 @@ tcontb_status finish_run(tcontb_run* run)
     const Problem& p = pl.prob;
     TC_CUDA(cudaGetDevice(&run->device));
     TC_CUDA(cudaDeviceGetAttribute(&run->num_sms, cudaDevAttrMultiProcessorCount, run->device));
+    if (pl.across.on) {
+        // What that kernel does not do: a C that bulk stores cannot address (the parts of a pass may start anywhere in one), and
+        // error compensation, when it is asked for after planning.
+        const char* x3 = std::getenv("TCONT_TF32X3");
+        if (reinterpret_cast<uintptr_t>(run->dC) % 16 || (x3 && x3[0] == '1')) {
+            Plan plain;
+            if (!plan_without_across(pl, &plain)) return fail(TCONTB_RUNTIME_ERROR, "no other plan for this contraction");
+            run->plan = plain;
+        }
+    }
     int major = 0;
     TC_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, run->device));
     if (major != 10) return fail(TCONTB_RUNTIME_ERROR, "this library holds sm_100a kernels only; the current device is not a B200-class GPU");
@@ -425,7 +506,11 @@ tcontb_status finish_run(tcontb_run* run)
     TC_CUDA(run->status.alloc(sizeof(int)));
     TC_CUDA(cudaMemset(run->status.ptr, 0, sizeof(int)));
 
-    if (pl.kernel == KERNEL_UMMA_TF32 || pl.kernel == KERNEL_DMMA_F64_TMA) {
+    run->scale_pass = run->tf32x3 = false;
+    if (pl.across.on) {
+        const tcontb_status st = finish_across(run, kA, kB);
+        if (st != TCONTB_OK) return st;
+    } else if (pl.kernel == KERNEL_UMMA_TF32 || pl.kernel == KERNEL_DMMA_F64_TMA) {
         const UmmaSpec& u = pl.umma;
         fill_operand_dev(u.a, &run->umma.a);
         fill_operand_dev(u.b, &run->umma.b);
@@ -1003,7 +1088,16 @@ tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
     if (scaled && run->plan.prob.c_strided) return fail(TCONTB_UNSUPPORTED, "alpha and beta are not available when C is a sub-tensor view");
     if (run->scale_pass) {
         // allocated here, once, so that launches stay free of allocations
-        if (scaled && !run->scaled_ws.ptr) TC_CUDA(run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt));
+        if (scaled && !run->scaled_ws.ptr) {
+            TC_CUDA(run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt));
+            if (run->plan.across.on) {
+                const tcontb_status st = encode_across_map(run->plan.across.c, run->scaled_ws.ptr, CU_TENSOR_MAP_SWIZZLE_64B, &run->tmWs);
+                if (st != TCONTB_OK) {
+                    TC_CUDA(run->scaled_ws.release());
+                    return st;
+                }
+            }
+        }
         const bool was = run->alpha != 1.0 || run->beta != 0.0;
         run->kernels_per_launch += (scaled ? 1 : 0) - (was ? 1 : 0);
     }
@@ -1069,7 +1163,9 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
     if (t) TC_CUDA(cudaEventRecord(run->ev[1], run->stream));
     if (pl.tB.needed && !run->borrowed_tB) TC_CUDA(launch_transpose(run->roleB_src(), run->tbufB.ptr, run->tpB, static_cast<int>(run->elt), run->stream));
     if (t) TC_CUDA(cudaEventRecord(run->ev[2], run->stream));
-    if (pl.kernel == KERNEL_UMMA_TF32 && run->tf32x3) {
+    if (pl.across.on) {
+        TC_CUDA(launch_across_tf32(run->across, &run->tmA, &run->tmB, redirect ? &run->tmWs : &run->tmC, run->num_sms, run->stream));
+    } else if (pl.kernel == KERNEL_UMMA_TF32 && run->tf32x3) {
         TC_CUDA(launch_tf32_residual(static_cast<const float*>(run->kernA), static_cast<float*>(run->loA.ptr), run->kernA_elements, run->stream));
         TC_CUDA(launch_tf32_residual(static_cast<const float*>(run->kernB), static_cast<float*>(run->loB.ptr), run->kernB_elements, run->stream));
         const CUtensorMap* maps[3][2] = {{&run->tmA, &run->tmB}, {&run->tmA, &run->tmBlo}, {&run->tmAlo, &run->tmB}};
@@ -1111,7 +1207,7 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         TC_CUDA(launch_splitk_reduce(run->splitk.ptr, run->dC, pl.sizeC, pl.umma.k_splits * (run->tf32x3 ? 3 : 1), pl.sizeC,
                                      static_cast<int>(run->elt), run->stream, run->alpha, run->beta));
     else if (redirect)
-        TC_CUDA(pl.sizeC * static_cast<int64_t>(run->elt) > kScalePassInL2
+        TC_CUDA(run->elt == 8 && pl.sizeC * static_cast<int64_t>(run->elt) > kScalePassInL2
                     ? launch_scale_pass(static_cast<const double*>(run->scaled_ws.ptr), static_cast<double*>(run->dC), pl.sizeC, run->stream, run->alpha, run->beta)
                     : launch_splitk_reduce(run->scaled_ws.ptr, run->dC, pl.sizeC, 1, pl.sizeC, static_cast<int>(run->elt), run->stream, run->alpha, run->beta));
     if (t) {
@@ -1346,6 +1442,12 @@ tcontb_status tcontb_run_ksplit_enable(tcontb_run* run, int world, int rank)
     if (run->ks.world) return fail(TCONTB_INVALID_ARGUMENT, "contracted-mode split is already enabled on this run");
     if (run->plan.prob.strided) return fail(TCONTB_UNSUPPORTED, "contracted-mode split is not available on sub-tensor views");
     std::string why;
+    if (run->plan.across.on) {
+        Plan plain;
+        if (!plan_without_across(run->plan, &plain)) return fail(TCONTB_RUNTIME_ERROR, "no other plan for this contraction");
+        const tcontb_status st = set_up_again(run, plain);
+        if (st != TCONTB_OK) return st;
+    }
     if (!cuts_into_ranges(run->plan, world, &why)) {
         // Rows fused across modes, or an operand moved into a matrix, move the edges of the tile columns: staged mode by
         // mode the ranges may still end where a tile does.

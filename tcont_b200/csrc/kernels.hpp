@@ -200,6 +200,26 @@ cudaError_t launch_umma_tf32(const UmmaParams& p, const void* tmapA, const void*
 constexpr int kMaxDynamicSmemBytes = 227 * 1024;
 cudaError_t umma_tf32_configure();
 
+// ---- TF32 with tiles across A's and C's stride-1 modes (across_tf32.cu) ------------------------
+struct AcrossParams {
+    // A unit's index: rows (chunks of y, chunks of x, other row modes o0, o1) and columns (chunks of n, other column modes p0, p1) of
+    // tiles.  rows_first: the rows run faster, and x slowest among them; else the columns do, and x follows y.  `inner` = how many
+    // of the faster kind there are.
+    int rows_first;
+    FastDiv inner, n_chunks, p0, y_chunks, x_chunks, o0, o1;
+    int row_others, column_others;   // how many of the other modes there are
+    int k_ext, k1_ext;               // extents of the chunked contracted mode and of the next one
+    uint32_t units;
+    int BN, BK, stages, k_iters;
+    int b_major;            // 1: B's stride-1 mode is the column mode, 0: the chunked contracted mode
+    int n_ext, x_ext;       // extents of the column mode and of A's stride-1 mode
+    int release_late;       // see UmmaParams
+    int* status;
+};
+cudaError_t across_tf32_configure();  // once per device before the first launch
+int across_tf32_smem(int stages, int BN, int BK);
+cudaError_t launch_across_tf32(const AcrossParams& p, const void* tmapA, const void* tmapB, const void* tmapC, int num_sms, cudaStream_t stream);
+
 // ---- TMA-fed FP64 tensor-path contraction (dmma_tma_f64.cu), same parameter block ------------
 cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, int num_sms,
                             cudaStream_t stream);

@@ -947,6 +947,100 @@ double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const Cos
     return c.launch_us + std::max({flops / (rate * 1e6), bytes / (c.hbm_gbs * 1e3), scatter_us, extra_floor_us}) + extra_us;
 }
 
+// Float32 where A's stride-1 mode x is a row mode but not C's, y (across_tf32.cu).  Everything a tensor map needs is checked
+// here, so that a plan that has it can run.
+AcrossSpec plan_across(const Problem& p, const CostTable& c)
+{
+    AcrossSpec s;
+    if (p.scalar_type != 0 || p.M.size() < 2 || p.N.empty() || p.K.empty() || p.K.size() > 3) return s;
+    if (p.A.size() > kMaxTmaRank || p.B.size() > kMaxTmaRank || p.C.size() > kMaxTmaRank || p.B.size() < 2) return s;
+    auto mode = [&](int id) -> const Mode& { return p.modes[static_cast<size_t>(id)]; };
+    const int x = p.A[0], y = p.M[0];
+    if (mode(x).group != GROUP_M || x == y || mode(y).sC != 1 || mode(x).sA != 1) return s;
+    const bool b_kmajor = mode(p.B[0]).group == GROUP_K;
+    int kc = p.K[0], n = p.B[0];
+    if (b_kmajor) {
+        kc = p.B[0];
+        n = p.N[0];
+        for (int id : p.N)
+            if (mode(id).extent > mode(n).extent) n = id;
+    } else {
+        for (int id : p.K)   // rows of a box are one stride of this mode apart
+            if (mode(id).sA < mode(kc).sA) kc = id;
+    }
+    const int64_t kc_ext = mode(kc).extent, n_ext = mode(n).extent;
+    s.b_major = b_kmajor ? 0 : 1;
+    s.BK = b_kmajor ? 32 : kc_ext <= 8 ? 8 : kc_ext <= 16 ? 16 : 32;
+    if (!b_kmajor && kc_ext % 24 == 0 && double(ceil_div(kc_ext, 32) * 32) > 1.15 * double(kc_ext)) s.BK = 24;
+    s.BN = n_ext <= 32 ? 32 : 64;
+    s.n_ext = n_ext;
+    s.x_ext = mode(x).extent;
+    std::vector<int> rows, columns, ks;   // the other modes
+    for (int id : p.M)
+        if (id != x && id != y) rows.push_back(id);
+    for (int id : p.N)
+        if (id != n) columns.push_back(id);
+    for (int id : p.K)
+        if (id != kc) ks.push_back(id);
+    auto fill = [&](AcrossSpec::Map& m, std::vector<int> order, const std::vector<int>& first, const std::vector<int>& second, int which) {
+        order.insert(order.end(), first.begin(), first.end());
+        order.insert(order.end(), second.begin(), second.end());
+        int64_t span = 1;
+        for (size_t d = 0; d < order.size(); ++d) {
+            const Mode& q = mode(order[d]);
+            m.ext[d] = q.extent;
+            m.stride[d] = which == 0 ? q.sA : which == 1 ? q.sB : q.sC;
+            if (d == 0 ? m.stride[0] != 1 : m.stride[d] % 4 != 0) return false;   // (16 bytes)
+            span += (q.extent - 1) * m.stride[d];
+        }
+        for (size_t d = order.size(); d < kMaxTmaRank; ++d) m.stride[d] = (span + 3) / 4 * 4;
+        return span < (int64_t(1) << 37);
+    };
+    if (!fill(s.a, {x, kc, y}, rows, ks, 0) || !fill(s.b, b_kmajor ? std::vector<int>{kc, n} : std::vector<int>{n, kc}, columns, ks, 1) ||
+        !fill(s.c, {y, x, n}, rows, columns, 2)) return s;
+    s.a.box[0] = 32; s.a.box[1] = s.BK; s.a.box[2] = 16;
+    s.b.box[0] = 32; s.b.box[1] = b_kmajor ? s.BN : s.BK;
+    s.c.box[0] = 16; s.c.box[1] = 16; s.c.box[2] = 8;
+    s.row_others = static_cast<int>(rows.size());
+    s.column_others = static_cast<int>(columns.size());
+    if (!rows.empty()) s.o0 = mode(rows[0]).extent;
+    if (rows.size() > 1) s.o1 = mode(rows[1]).extent;
+    if (!columns.empty()) s.p0 = mode(columns[0]).extent;
+    if (!ks.empty()) s.k1 = mode(ks[0]).extent;
+    s.k_ext = kc_ext;
+    s.y_chunks = ceil_div(mode(y).extent, 16);
+    s.x_chunks = ceil_div(s.x_ext, 32);
+    s.n_chunks = ceil_div(n_ext, s.BN);
+    s.tiles_m = s.y_chunks * s.x_chunks;
+    for (int id : rows) s.tiles_m *= mode(id).extent;
+    s.tiles_n = s.n_chunks;
+    for (int id : columns) s.tiles_n *= mode(id).extent;
+    s.k_iters = ceil_div(kc_ext, s.BK);
+    for (int id : ks) s.k_iters *= mode(id).extent;
+    if (s.tiles_m >= (int64_t(1) << 30) / s.tiles_n || s.k_iters >= (int64_t(1) << 24)) return s;
+    // Rows first, so that tiles that run together cover whole rows of C (C[a,b,c,d,e] of 251 MB from A of 1.3: 79 -> 43 us), and x
+    // last among them, because its 32 rows lie far apart in C and the fewer of them are written at a time the better (C of 1.0 GB:
+    // 339 us with x behind y, 210 behind all; of 453 MB: 208 and 118).  Unless A is too large to be read from L2 again by the other
+    // columns' tiles later, and is read in its own order (A of 107 MB, two tile columns: 78 us rows first, 68 columns first; of 162
+    // MB, four: 180 and 123; of 33 MB, four: 36.4 and 36.1; of 1.4 GB, one: 411 us with x last, 313 behind y).
+    // TCONT_ACROSS_ROWS_FIRST=0|1 overrides the rule.
+    s.rows_first = p.sizeA * 4 <= (int64_t(64) << 20);
+    if (const char* e = std::getenv("TCONT_ACROSS_ROWS_FIRST")) s.rows_first = e[0] == '1';
+    // two stages at least beside the staged pieces of C
+    const int stage_bytes = 16 * 128 * s.BK + s.BN * s.BK * 4;
+    s.stages = std::min(8, (227 * 1024 - 2 * 1024 - 64 * 1024) / stage_bytes);
+    // A CTA passes a stage no faster than an SM takes it in, and a piece of 8 columns no faster than it is staged and stored.
+    const double pieces = std::ceil(std::min<double>(double(n_ext), s.BN) / 8.0);
+    const double tile_us = std::max(double(s.k_iters) * double(stage_bytes) / 110e3, c.across_piece_us * pieces) + c.across_tile_us;
+    // Rows of y that are no multiple of 32 bytes end inside a sector, which is then read first (C of 188 MB with y = 28: 91 us, y = 32
+    // 33); a C in L2 does not mind.
+    const double c_bytes = 4.0 * double(p.sizeC), torn = mode(y).extent % 8 != 0 && c_bytes > 64e6 ? 3.0 : 1.0;
+    const double bytes = 4.0 * (double(p.sizeA) + double(p.sizeB)) + torn * c_bytes;
+    s.est_us = c.launch_us + std::max(double(ceil_div(s.tiles_m * s.tiles_n, c.num_sms)) * tile_us, bytes / (c.across_gbs * 1e3));
+    s.on = true;
+    return s;
+}
+
 // TF32 goes to the tcgen05 kernel whenever its tiles can be described to TMA.  FP64 takes the cheaper of the TMA-fed kernel
 // and the gather kernel, by the cost table; Float32 that TMA cannot describe goes to the gather kernel.  The gather kernel
 // is reported as KERNEL_DMMA_F64 where FP64 work fills the GPU with tiles, as KERNEL_SIMT otherwise.
@@ -996,6 +1090,9 @@ bool read_cost_table_file(const std::string& path, CostTable* table)
         else if (key == "scatter_store_ps") c.scatter_store_ps = v;
         else if (key == "scatter_store_f32_ps") c.scatter_store_f32_ps = v;
         else if (key == "far_row_penalty") c.far_row_penalty = v;
+        else if (key == "across_piece_us") c.across_piece_us = v;
+        else if (key == "across_tile_us") c.across_tile_us = v;
+        else if (key == "across_gbs") c.across_gbs = v;
         else if (key == "umma_stage_us") c.umma_stage_us = v;
         else if (key == "umma_store_gbs_per_sm") c.umma_store_gbs_per_sm = v;
         else if (key == "num_sms" && v >= 1) c.num_sms = static_cast<int>(v);
@@ -1020,7 +1117,7 @@ CostTable load_cost_table()
 
 int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* modeB, int nB, char op, int scalar_type,
               const char* ext_mode, const int64_t* ext_val, int n_ext, int backend_selection, const CostTable& cost,
-              Plan* plan, std::string* err, const int64_t* parentC, const int64_t* parentA, const int64_t* parentB, bool fuse_rows)
+              Plan* plan, std::string* err, const int64_t* parentC, const int64_t* parentA, const int64_t* parentB, bool fuse_rows, bool across)
 {
     if (!plan || !err) return 1;
     if (nC < 0 || nA < 0 || nB < 0 || n_ext < 0 || nC > kMaxModes || nA > kMaxModes || nB > kMaxModes || n_ext > 64) {
@@ -1251,12 +1348,21 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
 
     if (ttgt_kernel != KERNEL_UMMA_TF32 && ttgt_kernel != KERNEL_DMMA_F64_TMA)
         pl.est_direct_us = contraction_us(direct, direct_kernel, direct_umma, cost, false);
+    // (the error-compensated mode and a contracted-mode split keep the other form)
+    const char* x3 = std::getenv("TCONT_TF32X3");
+    if (across && fuse_rows && tf32 && direct_kernel == KERNEL_UMMA_TF32 && backend_selection != 2 && !(x3 && x3[0] == '1') && !std::getenv("TCONT_NO_ROWS_ACROSS_SLABS")) {
+        pl.across = plan_across(direct, cost);
+        const char* force = std::getenv("TCONT_ACROSS");   // tuning switch: 1 wherever it can run
+        if (pl.across.on && (pl.across.est_us < 0.97 * pl.est_direct_us || (force && force[0] == '1'))) pl.est_direct_us = pl.across.est_us;
+        else pl.across.on = false;
+    }
     bool use_ttgt;
     if (backend_selection == 1) use_ttgt = false;
     else if (backend_selection == 2) use_ttgt = true;
     else use_ttgt = (tA.needed || tB.needed) && pl.est_ttgt_us < pl.est_direct_us;
 
     if (use_ttgt) {
+        pl.across.on = false;
         pl.backend = 1;
         pl.prob = ttgt;
         pl.prob.swapped = direct.swapped;  // roles still map to the caller's operands as in `direct`
@@ -1287,6 +1393,10 @@ bool cuts_into_ranges(const Plan& pl, int ranges, std::string* why)
 {
     const Problem& p = pl.prob;
     const UmmaSpec& u = pl.umma;
+    if (pl.across.on) {
+        *why = "contracted-mode split: tiles across two stride-1 modes have no columns of their own per rank";
+        return false;
+    }
     if (pl.kernel != KERNEL_UMMA_TF32 || u.k_splits != 1) {
         *why = "contracted-mode split needs the tcgen05 kernel without split-K (Float32 operands TMA can stage; TCONT_SPLITK=1)";
         return false;
@@ -1337,6 +1447,9 @@ std::string describe_plan(const Plan& pl)
       << ",\"b_along_k\":" << pl.simt.b_load_along_k << "},\"gather\":{\"tile\":" << pl.gather.tile
       << ",\"cluster\":" << pl.gather.cluster << ",\"flat\":" << (pl.gather.flat ? "true" : "false") << ",\"t0\":" << pl.gather.t0 << ",\"t1\":" << pl.gather.t1 << ",\"rows\":" << pl.gather.rows << ",\"est_us\":" << pl.gather.est_us << "}";
     const UmmaSpec& u = pl.umma;
+    if (pl.across.on)
+        o << ",\"across\":{\"BN\":" << pl.across.BN << ",\"BK\":" << pl.across.BK << ",\"stages\":" << pl.across.stages << ",\"tiles_m\":" << pl.across.tiles_m
+          << ",\"tiles_n\":" << pl.across.tiles_n << ",\"k_iters\":" << pl.across.k_iters << ",\"b_major\":\"" << (pl.across.b_major ? "MN" : "K") << "\"}";
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";
     else {

@@ -116,6 +116,26 @@ struct UmmaSpec {
     int elt = 4;  // element bytes: 4 = tcgen05 TF32 kernel, 8 = TMA-fed FP64 tensor-path kernel
 };
 
+// Float32 tiles across A's and C's stride-1 modes (across_tf32.cu): 16 indices of C's stride-1 mode y times 32 of A's, x, times
+// BN of one mode n of B.
+struct AcrossSpec {
+    struct Map {
+        int64_t ext[kMaxTmaRank] = {1, 1, 1, 1, 1}, stride[kMaxTmaRank] = {0, 0, 0, 0, 0};   // elements
+        int box[kMaxTmaRank] = {1, 1, 1, 1, 1};
+    };
+    bool on = false;
+    // a: x, chunked contracted mode, y, other row modes, other contracted ones; b: its stride-1 mode and the other of (n, chunked
+    // contracted mode), other column modes, other contracted ones; c: y, x, n, other row modes, other column modes
+    Map a, b, c;
+    int row_others = 0, column_others = 0;
+    int64_t o0 = 1, o1 = 1, p0 = 1, k1 = 1;   // extents of the first of each kind
+    int64_t k_ext = 1, y_chunks = 1, x_chunks = 1, n_chunks = 1;
+    int BN = 32, BK = 32, stages = 2, b_major = 1;
+    bool rows_first = false;   // order of the tiles (see AcrossParams)
+    int64_t tiles_m = 1, tiles_n = 1, k_iters = 1, n_ext = 1, x_ext = 1;
+    double est_us = 0;
+};
+
 struct SimtSpec {
     int a_load_along_k = 0;  // 0: threads run along m when loading A (m contiguous), 1: along k
     int b_load_along_k = 0;
@@ -170,6 +190,12 @@ struct CostTable {
     double umma_stage_us = 0.45;
     // What one SM's epilogue stores per second (GB/s): a 128 x 256 fp32 tile takes 3.7 us to leave (cfg4).
     double umma_store_gbs_per_sm = 35.5;
+    // Tiles across two stride-1 modes (across_tf32.cu): a piece of 512 rows x 8 columns leaves a CTA in this, a tile of 512 rows
+    // takes the other beside; tensors move at this rate.  Fitted to 90 drawn contractions: the choice is the faster one of the two
+    // forms for 79 of them, within 8 % for 4.
+    double across_piece_us = 0.29;
+    double across_tile_us = 0.05;
+    double across_gbs = 4900.0;
     // The line between IEEE single precision and TF32 (see make_plan): which Float32 contractions give up precision for time
     // is decided by these two, not by how fast the kernels are now.
     double line_f32_tflops = 23.7;          // table key simt_f32_tflops
@@ -194,6 +220,7 @@ struct Plan {
     SimtSpec simt;
     GatherSpec gather;
     UmmaSpec umma;
+    AcrossSpec across;      // KERNEL_UMMA_TF32: this form of it runs when `on`
     double est_direct_us = 0, est_ttgt_us = 0;
     double flops = 0;
     int64_t sizeL = 1, sizeR = 1, sizeC = 1;  // caller's left, right, output element counts
@@ -205,7 +232,7 @@ struct Plan {
 int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* modeB, int nB, char op, int scalar_type,
               const char* ext_mode, const int64_t* ext_val, int n_ext, int backend_selection, const CostTable& cost,
               Plan* plan, std::string* err, const int64_t* parentC = nullptr, const int64_t* parentA = nullptr,
-              const int64_t* parentB = nullptr, bool fuse_rows = true);
+              const int64_t* parentB = nullptr, bool fuse_rows = true, bool across = true);
 
 // Whether C, cut into `ranges` equal contiguous ranges along its slowest mode, is cut along whole tile columns of the
 // tcgen05 kernel (each column of tiles then has exactly one owner); `why` receives the reason if not.

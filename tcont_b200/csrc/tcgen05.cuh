@@ -1,0 +1,78 @@
+// tcgen05.cuh -- what the tensor-core kernels (umma_tf32.cu, across_tf32.cu) share: single-CTA MMAs, descriptors, commits, loads
+// from tensor memory.
+#pragma once
+#include <cstdint>
+
+#include "tile_common.cuh"
+
+namespace tcontb {
+namespace {
+
+// One thread of a converged warp.  The compiler knows that a single thread runs behind this predicate and issues tensor
+// copies and MMAs, whose operands are warp-uniform registers, without a loop over the warp's lanes.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+    return leader != 0;
+}
+
+__device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+__device__ __forceinline__ void umma_commit(uint32_t bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void umma_tf32(uint32_t tmem_c, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_c), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
+
+// Shared-memory matrix descriptor, descriptor version 1 (Blackwell).
+//   bits  0-13 start address >> 4      bits 16-29 leading byte offset >> 4
+//   bits 32-45 stride byte offset >> 4 bits 46-47 version      bits 61-63 layout type
+// Layout types used here: 2 = 128-byte swizzle in 16-byte units (K-major operands);
+// 1 = 128-byte swizzle in 32-byte units, the only layout the tensor core accepts for an MN-major
+// operand of a 32-bit type (TMA writes it with CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B).
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout_type)
+{
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((addr >> 4) & 0x3fffu);
+    d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3fffu) << 16;
+    d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3fffu) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(layout_type) << 61;
+    return d;
+}
+
+// 32 lanes x 8 columns
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+
+// Give the bulk copies issued into these barriers a bounded time to land before the CTA ends (after a wait gave up).
+__device__ __forceinline__ void drain_copies(uint32_t bar_full, int stages, uint32_t issued_mask, uint32_t issued_parity)
+{
+    for (int s = 0; s < stages; ++s) {
+        if (!(issued_mask & (1u << s))) continue;
+        const unsigned long long t0 = global_timer();
+        while (!mbar_try_wait(bar_full + 8u * static_cast<uint32_t>(s), (issued_parity >> s) & 1u))
+            if (global_timer() - t0 > 100000000ull) break;
+    }
+}
+
+}  // namespace
+}  // namespace tcontb
