@@ -451,14 +451,28 @@ void fill_gather(const Problem& p, const void* A, const void* B, void* C, const 
     *out = g;
 }
 
-// The same contraction planned again without tiles across two stride-1 modes.
-bool plan_without_across(const Plan& d, Plan* out)
+// The same contraction planned again without tiles across two stride-1 modes, on the caller's choice of route or another.
+bool plan_without_across(const Plan& d, Plan* out, int selection = -1)
 {
     std::string err;
     auto parent = [](const std::vector<int64_t>& v) { return v.empty() ? nullptr : v.data(); };
     return make_plan(d.modeC.data(), static_cast<int>(d.modeC.size()), d.modeA.data(), static_cast<int>(d.modeA.size()), d.modeB.data(),
                      static_cast<int>(d.modeB.size()), d.op, d.scalar_type, d.ext_mode.data(), d.ext_val.data(), static_cast<int>(d.ext_val.size()),
-                     d.backend_selection, device_cost_table(), out, &err, parent(d.parentC), parent(d.parentA), parent(d.parentB), true, false) == 0;
+                     selection < 0 ? d.backend_selection : selection, device_cost_table(), out, &err, parent(d.parentC), parent(d.parentA), parent(d.parentB), true, false) == 0;
+}
+
+tcontb_status finish_run(tcontb_run* run);
+
+// The run without scratch copies of its operands.
+tcontb_status finish_where_they_lie(tcontb_run* run)
+{
+    cudaGetLastError();
+    TC_CUDA(run->tbufA.release());
+    TC_CUDA(run->tbufB.release());
+    Plan plain;
+    if (!plan_without_across(run->plan, &plain, 1)) return fail(TCONTB_RUNTIME_ERROR, "no other plan for this contraction");
+    run->plan = plain;
+    return finish_run(run);
 }
 
 // Device-side set-up shared by the three run constructors; dL/dR/dC must already be set.
@@ -482,24 +496,33 @@ tcontb_status finish_run(tcontb_run* run)
     TC_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, run->device));
     if (major != 10) return fail(TCONTB_RUNTIME_ERROR, "this library holds sm_100a kernels only; the current device is not a B200-class GPU");
 
+    // Scratch copies: where there is no room for them and the caller left the route open, the operands are used where they lie.
+    if (pl.tA.needed && !run->borrowed_tA) {
+        const cudaError_t e = run->tbufA.alloc(static_cast<size_t>(pl.tA.dst_elements) * run->elt);
+        if (e == cudaErrorMemoryAllocation && pl.backend_selection == 0) return finish_where_they_lie(run);
+        TC_CUDA(e);
+    }
+    if (pl.tB.needed && !run->borrowed_tB) {
+        const cudaError_t e = run->tbufB.alloc(static_cast<size_t>(pl.tB.dst_elements) * run->elt);
+        if (e == cudaErrorMemoryAllocation && pl.backend_selection == 0) return finish_where_they_lie(run);
+        TC_CUDA(e);
+    }
     const void* kA = run->roleA_src();
     const void* kB = run->roleB_src();
     run->kernels_per_launch = 1;
     if (pl.tA.needed && run->borrowed_tA) {
         kA = run->borrowed_tA;
     } else if (pl.tA.needed) {
-        if (!make_transpose_params(pl.tA.rank, pl.tA.src_extent, pl.tA.perm, &run->tpA, pl.tA.strided_src ? pl.tA.src_stride : nullptr))
+        if (!make_transpose_params(pl.tA.rank, pl.tA.src_extent, pl.tA.perm, &run->tpA, pl.tA.strided_src ? pl.tA.src_stride : nullptr, pl.tA.dst_extent))
             return fail(TCONTB_RUNTIME_ERROR, "bad transpose plan for A");
-        TC_CUDA(run->tbufA.alloc(static_cast<size_t>(pl.tA.elements) * run->elt));
         kA = run->tbufA.ptr;
         run->kernels_per_launch++;
     }
     if (pl.tB.needed && run->borrowed_tB) {
         kB = run->borrowed_tB;
     } else if (pl.tB.needed) {
-        if (!make_transpose_params(pl.tB.rank, pl.tB.src_extent, pl.tB.perm, &run->tpB, pl.tB.strided_src ? pl.tB.src_stride : nullptr))
+        if (!make_transpose_params(pl.tB.rank, pl.tB.src_extent, pl.tB.perm, &run->tpB, pl.tB.strided_src ? pl.tB.src_stride : nullptr, pl.tB.dst_extent))
             return fail(TCONTB_RUNTIME_ERROR, "bad transpose plan for B");
-        TC_CUDA(run->tbufB.alloc(static_cast<size_t>(pl.tB.elements) * run->elt));
         kB = run->tbufB.ptr;
         run->kernels_per_launch++;
     }
@@ -1089,7 +1112,15 @@ tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
     if (run->scale_pass) {
         // allocated here, once, so that launches stay free of allocations
         if (scaled && !run->scaled_ws.ptr) {
-            TC_CUDA(run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt));
+            const cudaError_t e = run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt);
+            if (e == cudaErrorMemoryAllocation && run->plan.across.on) {   // no room for it: the form whose epilogue applies them
+                cudaGetLastError();
+                Plan plain;
+                if (!plan_without_across(run->plan, &plain)) return fail(TCONTB_RUNTIME_ERROR, "no other plan for this contraction");
+                const tcontb_status st = set_up_again(run, plain);
+                return st == TCONTB_OK ? tcontb_run_set_scalars(run, alpha, beta) : st;
+            }
+            TC_CUDA(e);
             if (run->plan.across.on) {
                 const tcontb_status st = encode_across_map(run->plan.across.c, run->scaled_ws.ptr, CU_TENSOR_MAP_SWIZZLE_64B, &run->tmWs);
                 if (st != TCONTB_OK) {

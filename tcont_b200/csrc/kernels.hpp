@@ -119,7 +119,9 @@ struct TransposeParams {
 };
 // Builds merged params for dst mode i = src mode perm[i]; returns false for a bad permutation.
 // `src_stride` (optional): element strides of the source modes when the source is a view into a larger tensor.
-bool make_transpose_params(int rank, const int64_t* src_extent, const int* perm, TransposeParams* out, const int64_t* src_stride = nullptr);
+// `dst_extent` (optional): extents of the destination modes, padding included.
+bool make_transpose_params(int rank, const int64_t* src_extent, const int* perm, TransposeParams* out, const int64_t* src_stride = nullptr,
+                           const int64_t* dst_extent = nullptr);
 cudaError_t launch_transpose(const void* src, void* dst, const TransposeParams& p, int elem_bytes, cudaStream_t stream);
 
 // ---- TF32 tcgen05 contraction (umma_tf32.cu) -------------------------------------------------

@@ -771,17 +771,19 @@ std::string perm_modes(const Problem& p, const std::vector<int>& ids)
 }
 
 void fill_transpose(const std::string& src, const std::string& dst, const std::string& ext_mode,
-                    const std::vector<int64_t>& ext_val, TransposeSpec* t, const std::vector<int64_t>& src_parent = {})
+                    const std::vector<int64_t>& ext_val, TransposeSpec* t, const std::vector<int64_t>& src_parent = {}, const std::vector<int64_t>& padded = {})
 {
-    t->needed = src != dst;
+    t->needed = src != dst || !padded.empty();
     t->rank = static_cast<int>(src.size());
-    t->elements = 1;
+    t->elements = t->dst_elements = 1;
     t->strided_src = !src_parent.empty();
     int64_t st = 1;
     for (size_t i = 0; i < src.size(); ++i) {
         t->src_extent[i] = ext_val[static_cast<size_t>(find_char(ext_mode, src[i]))];
         t->elements *= t->src_extent[i];
         t->perm[i] = find_char(src, dst[i]);
+        t->dst_extent[i] = padded.empty() ? ext_val[static_cast<size_t>(find_char(ext_mode, dst[i]))] : padded[i];
+        t->dst_elements *= t->dst_extent[i];
         t->src_stride[i] = st;   // the source may be a view: strides from its parent's extents
         st *= src_parent.empty() ? t->src_extent[i] : src_parent[i];
     }
@@ -1254,6 +1256,39 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         for (const std::string& korder : {sorted_by(roleB_src), sorted_by(roleA_src)})
             if (!korder.empty() && !rowsB.empty()) candidates.push_back({rowsA + korder, korder + rowsB});
     }
+    // FP64 operands TMA cannot describe where they lie, because some stride is no multiple of 16 bytes: both as such matrices, the
+    // last mode of the run that starts each padded where that makes every stride behind it even (61 x 53 rows of A: 61 x 54).
+    // 3233 x 2773 x 851: 640 us on the gather kernel, 514 behind the two padded copies; 1297 x 1633 x 7859 3 444 and 1 230.  (Sums of more than 49 152 products stay
+    // one chain of FMAs on the gather kernel, see plan_gather.)
+    std::vector<int64_t> paddedA, paddedB;   // of the last candidate; empty = dense
+    size_t padded_candidate = 0;
+    const char* padded_env = std::getenv("TCONT_PADDED_COPIES");   // tuning switch: 0 never, 1 wherever they can be staged
+    const bool padded_forced = padded_env && padded_env[0] == '1';
+    if (scalar_type == 1 && !direct.strided && !direct_umma.eligible && direct.Ktot <= 49152 && direct.M.size() > 0 && direct.N.size() > 0 && !(padded_env && padded_env[0] == '0')) {
+        std::string rowsA, rowsB;
+        for (char c : pl.modeC) (find_char(roleA_src, c) >= 0 ? rowsA : rowsB).push_back(c);
+        const std::string korder = sorted_by(roleB_src);
+        // (rows that lie next to one another in C become one mode, and so do all contracted ones)
+        size_t run = 1;
+        while (run < rowsA.size() && find_char(pl.modeC, rowsA[run]) == find_char(pl.modeC, rowsA[run - 1]) + 1) ++run;
+        auto pad = [&](const std::string& layout, size_t first_run) {
+            std::vector<int64_t> v;
+            int64_t product = 1;
+            for (size_t i = 0; i < layout.size(); ++i) {
+                v.push_back(ext_of(layout[i]));
+                if (i < first_run) product *= v.back();
+            }
+            if (product % 2 == 0) return std::vector<int64_t>();
+            ++v[first_run - 1];   // (all extents of the run are odd)
+            return v;
+        };
+        if (!korder.empty()) {
+            padded_candidate = candidates.size();
+            candidates.push_back({rowsA + korder, korder + rowsB});
+            paddedA = pad(candidates.back().first, run);
+            paddedB = pad(candidates.back().second, korder.size());
+        }
+    }
     // (a transposed operand is a dense scratch tensor; one that is used where it lies keeps its parent's strides)
     const std::vector<int64_t>& roleA_parent = direct.swapped ? pl.parentB : pl.parentA;
     const std::vector<int64_t>& roleB_parent = direct.swapped ? pl.parentA : pl.parentB;
@@ -1264,14 +1299,22 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     int ttgt_kernel = KERNEL_SIMT;
     TransposeSpec tA, tB;
     pl.est_ttgt_us = 1e300;
-    auto problem_of = [&](const std::pair<std::string, std::string>& layouts, Problem* q) {
-        return build_problem(pl.modeC, layouts.first, layouts.second, pl.ext_mode, pl.ext_val, scalar_type, q, err, pl.parentC,
-                             layouts.first == roleA_src ? roleA_parent : dense, layouts.second == roleB_src ? roleB_parent : dense);
+    auto padded = [&](size_t candidate, bool is_a) -> const std::vector<int64_t>& {
+        return candidate > 0 && candidate == padded_candidate ? (is_a ? paddedA : paddedB) : dense;
+    };
+    auto problem_of = [&](size_t candidate, Problem* q) {
+        const auto& layouts = candidates[candidate];
+        const std::vector<int64_t> &padA = padded(candidate, true), &padB = padded(candidate, false);
+        const int rc_build = build_problem(pl.modeC, layouts.first, layouts.second, pl.ext_mode, pl.ext_val, scalar_type, q, err, pl.parentC,
+                                           !padA.empty() ? padA : layouts.first == roleA_src ? roleA_parent : dense,
+                                           !padB.empty() ? padB : layouts.second == roleB_src ? roleB_parent : dense);
+        q->strided = direct.strided;   // (padding is not a view)
+        return rc_build;
     };
     // `tiles`: also by the tiles of the permutation kernel, 64 x 64 at most along the stride-1 modes of source and destination.
     // Short ones on both sides make many small tiles: 15 x 15 of 50 MB take 171 us, not the 23 of the bandwidth.
-    auto transpose_us = [&](const std::string& src, const std::string& dst, int64_t elements, const CostTable& c, bool tiles) {
-        if (src == dst) return 0.0;
+    auto transpose_us = [&](const std::string& src, const std::string& dst, int64_t elements, const CostTable& c, bool tiles, bool padded_copy) {
+        if (src == dst && !padded_copy) return 0.0;
         auto run = [&](const std::string& of, const std::string& in) {   // extent of the first modes that stay together
             int64_t e = ext_of(of[0]);
             for (size_t i = 1; i < of.size() && find_char(in, of[i]) == find_char(in, of[i - 1]) + 1; ++i) e *= ext_of(of[i]);
@@ -1284,8 +1327,10 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         }
         return c.launch_us + us;
     };
-    auto transposes_us = [&](const std::pair<std::string, std::string>& layouts, const CostTable& c, bool tiles) {
-        return transpose_us(roleA_src, layouts.first, direct.sizeA, c, tiles) + transpose_us(roleB_src, layouts.second, direct.sizeB, c, tiles);
+    auto transposes_us = [&](size_t candidate, const CostTable& c, bool tiles) {
+        const auto& layouts = candidates[candidate];
+        return transpose_us(roleA_src, layouts.first, direct.sizeA, c, tiles, !padded(candidate, true).empty()) +
+               transpose_us(roleB_src, layouts.second, direct.sizeB, c, tiles, !padded(candidate, false).empty());
     };
     // Whether Float32 runs as TF32 or in IEEE single precision is a question of precision, not only of time, and its answer
     // does not follow the kernels' speed: of the operands as they lie and the first transposed layout, the cheaper decides, by
@@ -1310,11 +1355,11 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
             return us;
         };
         Problem q;
-        rc = problem_of(candidates[0], &q);
+        rc = problem_of(0, &q);
         if (rc) return rc;
         bool direct_staged, moved_staged;
         const double direct_us = line_us(direct, &direct_staged), moved_us = line_us(q, &moved_staged);
-        const double t_us = transposes_us(candidates[0], line, false);
+        const double t_us = transposes_us(0, line, false);
         tf32 = (backend_selection == 0 ? t_us > 0 && t_us + moved_us < direct_us : backend_selection == 2) ? moved_staged : direct_staged;
         if (!tf32 && direct_kernel == KERNEL_UMMA_TF32) {
             direct_umma = UmmaSpec();
@@ -1324,15 +1369,22 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     }
     pl.est_direct_us = contraction_us(direct, direct_kernel, direct_umma, cost);
     for (size_t i = 0; i < (tf32 ? candidates.size() : 1); ++i) {
+        // (short contractions gain nothing by padded copies that the estimates could tell: 88 000 x 13 x 39 36 us, 38 behind them, 987 x
+        // 1820 x 234 63 and 59)
+        if (i > 0 && i == padded_candidate && pl.est_direct_us < 60.0 && !padded_forced) continue;
         Problem q;
-        rc = problem_of(candidates[i], &q);
+        rc = problem_of(i, &q);
         if (rc) return rc;
         UmmaSpec u;
         if (tf32) plan_umma(q, cost, &u, fuse_rows);
         const int kernel = pick_kernel(q, u, cost);
         // (the TMA-fed kernels gain much more by another layout than the gather kernel does, so for them the tiles do not decide)
         const bool gathers = kernel == KERNEL_SIMT || kernel == KERNEL_DMMA_F64;
-        double us = transposes_us(candidates[i], cost, gathers) + contraction_us(q, kernel, u, cost);
+        double us = transposes_us(i, cost, gathers || (i > 0 && i == padded_candidate)) + contraction_us(q, kernel, u, cost);
+        // (stores come on top of the arithmetic where they are not all of 32 aligned bytes: 10469 x 9025 x 63, odd, 798 us with 360 of
+        // arithmetic, 580 on the gather kernel; 82431 x 2205 x 7 818 and 546)
+        if (i > 0 && i == padded_candidate && kernel == KERNEL_DMMA_F64_TMA) us += double(q.sizeC) * double(u.k_splits) * (u.pieces32 ? 0.8e-6 : 4.6e-6);
+        if (padded_forced && i > 0 && i == padded_candidate && kernel == KERNEL_DMMA_F64_TMA) us = 0;
         // Partial sums behind the FP64 kernel: a thread adds its partials up one after the other, 0.12 us each (96 x 64 x 2992
         // in 41 ranges: 20.8 us without that, 24.6 measured).  Where the operands lie the kernels' estimates are compared as they were fitted.
         if (kernel == KERNEL_DMMA_F64_TMA && u.k_splits > 1) us += 0.12 * u.k_splits;
@@ -1341,8 +1393,8 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
             ttgt = q;
             ttgt_umma = u;
             ttgt_kernel = kernel;
-            fill_transpose(roleA_src, candidates[i].first, pl.ext_mode, pl.ext_val, &tA, roleA_parent);
-            fill_transpose(roleB_src, candidates[i].second, pl.ext_mode, pl.ext_val, &tB, roleB_parent);
+            fill_transpose(roleA_src, candidates[i].first, pl.ext_mode, pl.ext_val, &tA, roleA_parent, padded(i, true));
+            fill_transpose(roleB_src, candidates[i].second, pl.ext_mode, pl.ext_val, &tB, roleB_parent, padded(i, false));
         }
     }
 

@@ -51,6 +51,8 @@ struct TransposeSpec {
     int64_t src_extent[kMaxModes] = {0};
     int perm[kMaxModes] = {0};
     int64_t elements = 0;
+    int64_t dst_extent[kMaxModes] = {0};   // extents of the destination modes, padding included
+    int64_t dst_elements = 0;
     bool strided_src = false;              // the source is a view: src_stride holds its element strides
     int64_t src_stride[kMaxModes] = {0};
 };

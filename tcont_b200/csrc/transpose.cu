@@ -15,7 +15,7 @@
 
 namespace tcontb {
 
-bool make_transpose_params(int rank, const int64_t* src_extent, const int* perm, TransposeParams* out, const int64_t* src_stride)
+bool make_transpose_params(int rank, const int64_t* src_extent, const int* perm, TransposeParams* out, const int64_t* src_stride, const int64_t* dst_extent)
 {
     if (rank < 1 || rank > kMaxModes) return false;
     bool seen[kMaxModes] = {false};
@@ -27,7 +27,7 @@ bool make_transpose_params(int rank, const int64_t* src_extent, const int* perm,
     int64_t s = 1;
     for (int i = 0; i < rank; ++i) {
         dst_stride_of_src[perm[i]] = s;
-        s *= src_extent[perm[i]];
+        s *= dst_extent ? dst_extent[i] : src_extent[perm[i]];   // (a destination mode may be padded)
     }
     // Merge source modes j, j+1 that are also neighbours (same order) in the destination.
     int pos_in_dst[kMaxModes];
@@ -38,7 +38,8 @@ bool make_transpose_params(int rank, const int64_t* src_extent, const int* perm,
     int64_t st = 1, dense = 1;
     for (int j = 0; j < rank; ++j) {
         const int64_t sj = src_stride ? src_stride[j] : dense;
-        if (n > 0 && pos_in_dst[j] == pos_in_dst[j - 1] + 1 && sj == out->src_stride[n - 1] * out->ext[n - 1]) {
+        if (n > 0 && pos_in_dst[j] == pos_in_dst[j - 1] + 1 && sj == out->src_stride[n - 1] * out->ext[n - 1] &&
+            dst_stride_of_src[j] == out->dst_stride[n - 1] * out->ext[n - 1]) {
             out->ext[n - 1] *= src_extent[j];
         } else {
             out->ext[n] = src_extent[j];
@@ -231,7 +232,7 @@ cudaError_t launch_typed(const T* src, T* dst, const TransposeParams& p, cudaStr
         if (p.dst_stride[i] == 1) d0 = i;
     if (d0 == 0) {
         bool strides_ok = true;   // (a view's rows must start on 16-byte boundaries for the vector loads)
-        for (int i = 1; i < p.rank; ++i) strides_ok = strides_ok && p.src_stride[i] % VMAX == 0;
+        for (int i = 1; i < p.rank; ++i) strides_ok = strides_ok && p.src_stride[i] % VMAX == 0 && p.dst_stride[i] % VMAX == 0;
         const bool vec = aligned && strides_ok && p.ext[0] % VMAX == 0;
         const int64_t total = p.elements / (vec ? VMAX : 1);
         int dev = 0, sms = 148;
@@ -244,7 +245,7 @@ cudaError_t launch_typed(const T* src, T* dst, const TransposeParams& p, cudaStr
         return launch_chained(permute_rows_kernel<T, 1, int64_t>, dim3(blocks), dim3(256), 0, stream, 1, src, dst, p);
     }
     bool strides_ok = true;
-    for (int i = 1; i < p.rank; ++i) strides_ok = strides_ok && p.src_stride[i] % VMAX == 0;
+    for (int i = 0; i < p.rank; ++i) strides_ok = strides_ok && (i == 0 || p.src_stride[i] % VMAX == 0) && (i == d0 || p.dst_stride[i] % VMAX == 0);
     const bool vec = aligned && strides_ok && p.ext[0] % VMAX == 0 && p.ext[d0] % VMAX == 0;
     // whole tiles of (nearly) equal size along both modes, a multiple of the vector width
     constexpr int kTileMax = sizeof(T) == 4 ? 96 : TILE;

@@ -81,3 +81,31 @@ def test_stores(engine, oracle, monkeypatch, name, beta):
     exact, scale = oracle.contract(c, A, B) + beta * C0, oracle.contract(c, np.abs(A), np.abs(B)) + abs(beta * C0)
     k = ext.get("k", ext.get("e"))
     assert (np.abs(dC.cpu().numpy() - exact) <= (k + 4) * 2.0**-53 * scale).all()
+
+
+# odd strides: both operands copied to matrices whose strides are even, rows in one run or several, contracted modes in A's order,
+# in B's or in neither's, an operand that already lies in the right order, one that needs no padding
+PADDED = {
+    "four_d": ("abcd", "aebf", "fdec", dict(a=61, b=5, c=7, d=9, e=13, f=23)),
+    "rows_apart": ("abcd", "aecf", "bfde", dict(a=19, b=7, c=11, d=13, e=9, f=15)),
+    "in_order": ("ab", "ak", "kb", dict(a=131, b=67, k=35)),
+    "even_rows": ("abc", "adc", "db", dict(a=38, b=45, c=7, d=21)),
+    "even_k": ("abcd", "eafd", "fbec", dict(a=21, b=13, c=9, d=15, e=6, f=11)),
+    "swapped": ("abc", "db", "adc", dict(a=33, b=27, c=5, d=41)),
+    "long_k": ("ab", "ac", "cb", dict(a=45, b=33, c=1001)),
+}
+
+
+@pytest.mark.parametrize("name", list(PADDED))
+def test_padded_copies(engine, oracle, monkeypatch, name):
+    monkeypatch.setenv("TCONT_PADDED_COPIES", "1")
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    C, A_, B_, ext = PADDED[name]
+    c = Contraction(C, A_, B_, ext, F64)
+    A, B = oracle.inputs(c, 43, -1.0, 1.0)
+    out, desc = run_contraction(engine, c, A, B, 2, launches=2)
+    assert desc["kernel"] == "dmma_f64_tma" and desc["backend"] == "ttgt" and not desc["views"], desc
+    k = 1
+    for m, e in ext.items():
+        k *= 1 if m in C else e
+    hold(oracle, c, A, B, out, k, desc["umma"]["k_splits"])
