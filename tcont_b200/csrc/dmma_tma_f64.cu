@@ -68,13 +68,9 @@ __device__ __forceinline__ void ld_global_cs_v4f64(double (&o)[4], const double*
     asm volatile("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(p) : "memory");
 }
 
-// Which k a lane feeds into step t of a stage: k = 8 (t / 2) + 2 fk + ((fk ^ (fk >> 1) ^ t) & 1), fk = lane % 4.
-// Any assignment works as long as both operands use the same one.  With this one
-//  * the four rows an MN-major 16-byte load touches per quarter warp differ in k / 2, which after the
-//    XOR swizzle puts the quarter's eight 16-byte chunks into eight different bank groups;
-//  * the two lanes of a half warp that meet in the same 16-byte chunk of a K-major operand (rows
-//    2 fr + par with fr two apart in the swizzle) take different halves of it.
-__device__ __forceinline__ uint32_t step_k(uint32_t t, uint32_t fk) { return 8u * (t >> 1) + 2u * fk + ((fk ^ (fk >> 1) ^ t) & 1u); }
+// Which k a lane feeds into step t of a stage: k = 4 t + fk, fk = lane % 4, so that an unsplit sum is one chain of FMAs in
+// ascending order of k, the same bits as the gather kernel's.
+__device__ __forceinline__ uint32_t step_k(uint32_t t, uint32_t fk) { return 4u * t + fk; }
 
 // Where a thread finds its fragments of one operand, as byte offsets from the start of the stage:
 //   MN-major (rows of the stage are k, 16 consecutive m per 128-byte row, slabs of 16 m one slab apart;
@@ -105,7 +101,7 @@ struct FragOffsets {
         step0 = offset(0);
         step1 = offset(1);
         later = offset(2) - step0;
-        odd = MN ? 0u : BK == 8 ? 64u : (fk & 1u) ? 112u : 144u;   // the next row, its chunk index with bit 0 flipped
+        odd = MN ? 0u : BK == 8 ? 64u : (fk & 2u) ? 112u : 144u;   // the next row, its chunk index with bit 0 flipped
     }
 };
 
