@@ -544,6 +544,7 @@ tcontb_status finish_run(tcontb_run* run)
         run->umma.producers = u.producers;
         run->umma.store_across_slabs = u.store_across_slabs ? 1 : 0;
         run->umma.pieces32 = u.pieces32 ? 1 : 0;
+        run->umma.slim = u.slim ? 1 : 0;
         run->umma.n_k_digits = u.n_k_digits;
         for (int i = 0; i < 3; ++i) run->umma.k_digit_ext[i] = static_cast<int>(u.k_digit_ext[i]);
         run->umma.k_iters = static_cast<int>(u.k_iters);

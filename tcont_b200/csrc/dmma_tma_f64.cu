@@ -87,6 +87,7 @@ template <int BK>
 struct FragOffsets {
     static constexpr uint32_t PITCH = BK * 128u;
     uint32_t step0, step1, later, odd;
+    uint32_t single;   // K-major, from row 2 fr to row 2 (fr % 4) + fr / 4: a fragment that is not one of a pair
 
     // `slabs8`: MN-major rows of 64 bytes (slabs of 8); the thread's slab, fr / 4, is already part of thread_base
     template <bool MN>
@@ -102,6 +103,7 @@ struct FragOffsets {
         step1 = offset(1);
         later = offset(2) - step0;
         odd = MN ? 0u : BK == 8 ? 64u : (fk & 2u) ? 112u : 144u;   // the next row, its chunk index with bit 0 flipped
+        single = fr < 4u ? 0u : odd - 8u * (BK * 8u);
     }
 };
 
@@ -115,37 +117,70 @@ __device__ __forceinline__ void load_frag(double (&f)[N], int i, uint32_t q, uin
     }
 }
 
-// load `n` fragments (n = 8 for A, 4 or 2 for B), all at once
-template <bool MN, int N, int BK>
-__device__ __forceinline__ void load_all(double (&f)[N], uint32_t q, uint32_t odd)
+// The last of an odd number of K-major fragments: eight rows of its own.
+template <int N, int BK>
+__device__ __forceinline__ void load_single(double (&f)[N], uint32_t q, uint32_t single)
 {
-#pragma unroll
-    for (int i = 0; i < N; ++i) load_frag<MN, N, BK>(f, i, q, odd);
+    f[N - 1] = ld_shared_f64(q + single + static_cast<uint32_t>(N >> 1) * FragOffsets<BK>::PITCH);
 }
 
-// One k4 step of a warp: 8 NF MMAs on the current fragments (NF = 4 or 2 column fragments); the fragment loads of the next
-// step are issued between them, where the FP64 tensor pipe leaves issue slots free.
-// acc[i][j][h]: row m = 16 (i / 2) + 4 (lane % 4) + 2 h + (i % 2), column n = 16 (j / 2) + 2 (lane / 4) + (j % 2).
-template <bool AMN, bool BMN, int NF, int BK>
-__device__ __forceinline__ void mma_step(double (&acc)[8][NF][2], const double (&ac)[8], const double (&bc)[NF], double (&an)[8],
-                                         double (&bn)[NF], uint32_t qa, uint32_t a_odd, uint32_t qb, uint32_t b_odd)
+// load N fragments (8 of A, 1 to 4 of B), all at once
+template <bool MN, int N, int BK>
+__device__ __forceinline__ void load_all(double (&f)[N], uint32_t q, const FragOffsets<BK>& o)
 {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if ((N & 1) && i == N - 1) load_single<N, BK>(f, q, o.single);
+        else load_frag<MN, N, BK>(f, i, q, o.odd);
+    }
+}
+
+// One k4 step of a warp: 8 NF MMAs on the current fragments (NF column fragments); the fragment loads of the next
+// step are issued between them, where the FP64 tensor pipe leaves issue slots free.
+// acc[i][j][h]: row m = 16 (i / 2) + 4 (lane % 4) + 2 h + (i % 2), column n = column_of(j).
+template <bool AMN, bool BMN, int NF, int BK, bool HALVES>
+__device__ __forceinline__ void mma_step(double (&acc)[8][NF][2], const double (&ac)[8], const double (&bc)[NF], double (&an)[8],
+                                         double (&bn)[NF], uint32_t qa, const FragOffsets<BK>& oa, uint32_t qb, const FragOffsets<BK>& ob, bool second)
+{
+    static_assert(!BMN || NF % 2 == 0, "fragments along the rows come in pairs");
+    if (HALVES && !second) {   // (one branch a step: with one at every MMA 373 248 x 24 x 72 gained nothing)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            dmma_m8n8k4(acc[i][0], bc[0], ac[i]);
+            load_frag<AMN, 8, BK>(an, i, qa, oa.odd);
+            if (i == 0) load_frag<false, NF, BK>(bn, 0, qb, ob.odd);
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
 #pragma unroll
         for (int j = 0; j < NF; ++j) dmma_m8n8k4(acc[i][j], bc[j], ac[i]);
-        load_frag<AMN, 8, BK>(an, i, qa, a_odd);
+        load_frag<AMN, 8, BK>(an, i, qa, oa.odd);
         if (BMN) {
-            if ((i == 1 || i == 3) && i < NF) load_frag<true, NF, BK>(bn, i - 1, qb, b_odd);
+            if ((i == 1 || i == 3) && i < NF) load_frag<true, NF, BK>(bn, i - 1, qb, ob.odd);
+        } else if ((NF & 1) && i == NF - 1) {
+            load_single<NF, BK>(bn, qb, ob.single);
         } else {
-            if (i < NF) load_frag<false, NF, BK>(bn, i, qb, b_odd);
+            if (i < NF) load_frag<false, NF, BK>(bn, i, qb, ob.odd);
         }
     }
+}
+// Column of a warp's fragment j that a lane's accumulators belong to (fr = lane / 4): pairs of fragments take 16 columns, a last
+// one by itself eight.
+template <int NF>
+__device__ __forceinline__ uint32_t column_of(int j, uint32_t fr)
+{
+    if ((NF & 1) && j == NF - 1) return 16u * (NF >> 1) + 2u * (fr & 3u) + (fr >> 2);
+    return 16u * static_cast<uint32_t>(j >> 1) + static_cast<uint32_t>(j & 1) + 2u * fr;
 }
 
 // SCALED: C = alpha A B + beta C in the epilogue (C read only when beta is not zero); a template parameter because the
 // overwriting kernel has no registers to spare for it.
-template <bool AMN, bool BMN, int NF, int BK, bool SCALED>
+// SLIM: one column of tiles, of at most 48 of its 64 columns or 24 of its 32 (B K-major).  Three column fragments a warp instead of
+// four; or (HALVES) two for the warps of one half and one for the others, the other way round in the second group, so that every
+// scheduler has three.  373 248 x 24 x 72 75.0 -> 68.2 us, 48 columns 143.6 -> 111.7, 200 000 x 48 x 200 163 -> 124.
+template <bool AMN, bool BMN, int NF, int BK, bool SCALED, bool SLIM>
 __global__ void __launch_bounds__(kThreads64, 1)
 dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                 const __grid_constant__ UmmaParams p)
@@ -163,7 +198,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     const uint32_t abort_flag = smem_u32(bar_empty + 8);
     uint64_t* tab_full = bar_empty + 10;   // [group][buffer]
     uint64_t* tab_empty = tab_full + 4;    // [group][buffer]
-    const uint32_t ragged = smem_u32(tab_empty + 4);   // [group][buffer]: 1 + number of the last tile with rows or columns beyond C
+    const uint32_t ragged = smem_u32(tab_empty + 4);   // [group][buffer]: 1 + number of the last tile with rows (not SLIM: or columns) beyond C
     const uint32_t tabs = smem_u32(aux + 256);  // [group][buffer]: long long [128] row offsets, [64] column offsets (-1 = beyond C)
 
     if (threadIdx.x == 0) {
@@ -280,7 +315,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     int d0 = 0;
                     const long long off = slab_c_offset(o, (is_row ? tm * SA : tn * SB) + sl, &d0, &ok);
                     ok = ok && (d0 * o.slab_w + in < o.slab_mode_ext);
-                    if (!ok) st_shared_u32(ragged + slot * 4u, i + 1u);
+                    if ((is_row || !SLIM) && !ok) st_shared_u32(ragged + slot * 4u, i + 1u);
                     st_shared_s64(tab + static_cast<uint32_t>(e) * 8u, ok ? off + slab_elem_offset(o, d0, in) : -1);
                 }
                 mbar_arrive(smem_u32(tab_full + slot));
@@ -311,14 +346,23 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
         FragOffsets<BK> fa, fb;
         fa.template set<AMN>(AMN ? static_cast<uint32_t>(wm * 4) * PITCH + (a8 ? (fr >> 2) * static_cast<uint32_t>(p.a.slab_bytes) : 0u)
                                  : (static_cast<uint32_t>(wm * 64) + 2u * fr) * (BK * 8u), fr, fk, a8);
+        const bool narrow = SLIM && NF == 2 && (wn ^ grp) != 0;
+        const uint32_t col0 = SLIM ? (NF == 2 ? (narrow ? 16u : 0u) : static_cast<uint32_t>(wn) * 24u) : static_cast<uint32_t>(wn * NF * 8);   // the warp's columns
         fb.template set<BMN>(a_tile_bytes + (BMN ? static_cast<uint32_t>(wn * (NF / 2)) * PITCH + (b8 ? (fr >> 2) * static_cast<uint32_t>(p.b.slab_bytes) : 0u)
-                                                 : (static_cast<uint32_t>(wn * NF * 8) + 2u * fr) * (BK * 8u)), fr, fk, b8);
+                                                 : (col0 + 2u * fr) * (BK * 8u)), fr, fk, b8);
 
-        double acc[8][NF][2];
+        if (narrow) {   // its one fragment is not one of a pair
+            fb.step0 += fb.single;
+            fb.step1 += fb.single;
+        }
+        const bool second = !narrow;
+        constexpr int W = SLIM && NF == 4 ? 3 : NF;   // column fragments of a warp (narrow: the first of them)
+        constexpr bool HALVES = SLIM && NF == 2;
+        double acc[8][W][2];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < NF; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+            for (int j = 0; j < W; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
         uint32_t stage = 0, phase = 0;
         const bool prof = p.prof != nullptr && (threadIdx.x & 127) == 0 && grp == 0;
@@ -336,7 +380,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             // first fragments of the next one, whose barrier is looked at a step earlier (behind the last stage of a tile the
             // fragments are fetched from that stage again and not used).  A wait that gave up leaves wrong fragments, and
             // tile_ok says so.
-            double fa0[8], fb0[NF], fa1[8], fb1[NF];
+            double fa0[8], fb0[W], fa1[8], fb1[W];
             uint32_t chunk = static_cast<uint32_t>(w.it0 ? w.it0 % p.k_digit_ext[0] : 0);   // chunk of the chunked mode
             {
                 const long long tw = prof ? clock64() : 0;
@@ -345,8 +389,8 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 if (prof) t_full += clock64() - tw;
             }
             uint32_t sb = smem_u32(smem) + (first + stage) * stage_bytes;
-            load_all<AMN, 8, BK>(fa0, sb + fa.step0, fa.odd);
-            load_all<BMN, NF, BK>(fb0, sb + fb.step0, fb.odd);
+            load_all<AMN, 8, BK>(fa0, sb + fa.step0, fa);
+            load_all<BMN, W, BK>(fb0, sb + fb.step0, fb);
             for (int left = w.n_it; left > 0; --left) {
                 if (i == 0 && my_tiles > 1 && left == w.n_it - w.n_it / 2) asm volatile("bar.arrive 1, 256;" ::: "memory");
                 const uint32_t bar_done = smem_u32(bar_empty + first + stage);
@@ -358,17 +402,17 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 // (the last chunk of a mode that is 1 to 8 past a multiple of 16 holds zeros in its second half: 5184^3 with
                 // contracted modes of 72 computed a tenth of its k for nothing, 9 520 us)
                 if (BK == 16 && chunk < static_cast<uint32_t>(p.full_chunks)) {
-                    mma_step<AMN, BMN, NF, BK>(acc, fa0, fb0, fa1, fb1, sb + fa.step1, fa.odd, sb + fb.step1, fb.odd);
+                    mma_step<AMN, BMN, W, BK, HALVES>(acc, fa0, fb0, fa1, fb1, sb + fa.step1, fa, sb + fb.step1, fb, second);
                     later_a = fa.later;
                     later_b = fb.later;
-                    mma_step<AMN, BMN, NF, BK>(acc, fa1, fb1, fa0, fb0, sb + fa.step0 + later_a, fa.odd, sb + fb.step0 + later_b, fb.odd);
+                    mma_step<AMN, BMN, W, BK, HALVES>(acc, fa1, fb1, fa0, fb0, sb + fa.step0 + later_a, fa, sb + fb.step0 + later_b, fb, second);
                 }
                 const uint32_t bar_next = smem_u32(bar_full + first + stage);
                 const bool more = left > 1, landed = !more || mbar_test_wait(bar_next, phase);
-                mma_step<AMN, BMN, NF, BK>(acc, fa0, fb0, fa1, fb1, sb + fa.step1 + later_a, fa.odd, sb + fb.step1 + later_b, fb.odd);
+                mma_step<AMN, BMN, W, BK, HALVES>(acc, fa0, fb0, fa1, fb1, sb + fa.step1 + later_a, fa, sb + fb.step1 + later_b, fb, second);
                 if (!__all_sync(0xffffffffu, landed)) tile_ok = __all_sync(0xffffffffu, mbar_wait(bar_next, phase, abort_flag)) && tile_ok;
                 if (more) sb = smem_u32(smem) + (first + stage) * stage_bytes;
-                mma_step<AMN, BMN, NF, BK>(acc, fa1, fb1, fa0, fb0, sb + fa.step0, fa.odd, sb + fb.step0, fb.odd);
+                mma_step<AMN, BMN, W, BK, HALVES>(acc, fa1, fb1, fa0, fb0, sb + fa.step0, fa, sb + fb.step0, fb, second);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_done);  // this warp is done reading the stage
                 if (++chunk == static_cast<uint32_t>(p.k_digit_ext[0])) chunk = 0;
@@ -381,14 +425,15 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             const uint32_t row_tab = tabs + slot * kTabBytes, col_tab = row_tab + kBM * 8u;
             if (prof) { const long long t1 = clock64(); t_tab += t1 - t0; t0 = t1; }
 
-            // Store.  Four elements of C a thread holds for each of 4 x NF (u, column fragment) lie next to each other:
+            // Store.  Four elements of C a thread holds for each of 4 x W (u, column fragment) lie next to each other:
             //   rows along C    : rows 16 u + 4 fk + q, element q in acc[2 u + (q & 1)][j][q >> 1]
             //   rows across slabs: the warp's 64 rows are four slabs of 16, slab q is index a0 + q of C's stride-1 mode; row
             //                      4 fk + u of the four slabs, element q in acc[2 q + (u & 1)][j][u >> 1]
-            long long cn[NF], cm[4];
+            long long cn[W], cm[4];
 #pragma unroll
-            for (int j = 0; j < NF; ++j)
-                cn[j] = ld_shared_s64(col_tab + (static_cast<uint32_t>(wn * NF * 8 + 16 * (j >> 1) + (j & 1)) + 2u * fr) * 8u);
+            for (int j = 0; j < W; ++j)
+                cn[j] = HALVES && narrow ? (j == 0 ? ld_shared_s64(col_tab + (col0 + column_of<1>(0, fr)) * 8u) : -1)
+                                         : ld_shared_s64(col_tab + (col0 + column_of<W>(j, fr)) * 8u);
             const uint32_t row_u = p.store_across_slabs ? 8u : 128u, row_q = p.store_across_slabs ? 128u : 8u;   // table bytes from u to u + 1, q to q + 1
             const uint32_t rows = row_tab + (static_cast<uint32_t>(wm * 64) + 4u * fk) * 8u;
 #pragma unroll
@@ -403,19 +448,20 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         if constexpr (SCALED) {   // the old values of all column fragments are asked for before the first is used
-                            double old[NF][4];
+                            double old[W][4];
 #pragma unroll
-                            for (int j = 0; j < NF; ++j) {
-                                if (p.beta != 0.0) ld_global_cs_v4f64(old[j], C + cm[u] + cn[j]);
+                            for (int j = 0; j < W; ++j) {
+                                if (p.beta != 0.0 && (!SLIM || cn[j] >= 0)) ld_global_cs_v4f64(old[j], C + cm[u] + cn[j]);
                                 else old[j][0] = old[j][1] = old[j][2] = old[j][3] = 0.0;
                             }
 #pragma unroll
-                            for (int j = 0; j < NF; ++j)
+                            for (int j = 0; j < W; ++j)
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) at(u, j, q) = p.alpha * at(u, j, q) + p.beta * old[j][q];
                         }
 #pragma unroll
-                        for (int j = 0; j < NF; ++j) st_global_cs_v4f64(C + cm[u] + cn[j], at(u, j, 0), at(u, j, 1), at(u, j, 2), at(u, j, 3));
+                        for (int j = 0; j < W; ++j)
+                            if (!SLIM || cn[j] >= 0) st_global_cs_v4f64(C + cm[u] + cn[j], at(u, j, 0), at(u, j, 1), at(u, j, 2), at(u, j, 3));
                     }
                 } else if (tile_ok) {
                     // ragged or odd-aligned pieces: 32 bytes where they can be, 16 where two elements are neighbours, else one by one
@@ -426,7 +472,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                         for (int q = 0; q < 4; ++q) r[q] = ld_shared_s64(rows + static_cast<uint32_t>(u) * row_u + static_cast<uint32_t>(q) * row_q);
                         const bool run4 = r[0] >= 0 && r[1] == r[0] + 1 && r[2] == r[0] + 2 && r[3] == r[0] + 3;
 #pragma unroll
-                        for (int j = 0; j < NF; ++j) {
+                        for (int j = 0; j < W; ++j) {
                             if (cn[j] < 0) continue;
                             double x[4];
 #pragma unroll
@@ -457,7 +503,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < NF; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+                for (int j = 0; j < W; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(tab_empty + slot));  // this warp is done with the tables
             if (prof) t_store += clock64() - t0;
@@ -476,23 +522,24 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     if (threadIdx.x == 0 && ld_shared_u32(abort_flag)) atomicMax(p.status, 1);
 }
 
-// The kernel's forms, one function per (majors, columns, k chunk, scaled); `use` is called with the one that matches.
-template <bool AMN, bool BMN, int NF, int BK, typename Use>
+// The kernel's forms, one function per (majors, columns, k chunk, slim, scaled); `use` is called with the one that matches.
+template <bool AMN, bool BMN, int NF, int BK, bool SLIM, typename Use>
 cudaError_t with_scaled(bool scaled, Use&& use)
 {
-    return scaled ? use(dmma_tma_kernel<AMN, BMN, NF, BK, true>) : use(dmma_tma_kernel<AMN, BMN, NF, BK, false>);
+    return scaled ? use(dmma_tma_kernel<AMN, BMN, NF, BK, true, SLIM>) : use(dmma_tma_kernel<AMN, BMN, NF, BK, false, SLIM>);
 }
 template <int NF, int BK, typename Use>
-cudaError_t with_majors(bool amn, bool bmn, bool scaled, Use&& use)
+cudaError_t with_majors(bool amn, bool bmn, bool slim, bool scaled, Use&& use)
 {
-    if (amn) return bmn ? with_scaled<true, true, NF, BK>(scaled, use) : with_scaled<true, false, NF, BK>(scaled, use);
-    return bmn ? with_scaled<false, true, NF, BK>(scaled, use) : with_scaled<false, false, NF, BK>(scaled, use);
+    if (slim) return bmn ? cudaErrorInvalidValue : amn ? with_scaled<true, false, NF, BK, true>(scaled, use) : with_scaled<false, false, NF, BK, true>(scaled, use);
+    if (amn) return bmn ? with_scaled<true, true, NF, BK, false>(scaled, use) : with_scaled<true, false, NF, BK, false>(scaled, use);
+    return bmn ? with_scaled<false, true, NF, BK, false>(scaled, use) : with_scaled<false, false, NF, BK, false>(scaled, use);
 }
 template <typename Use>
-cudaError_t with_kernel(int bn, int bk, bool amn, bool bmn, bool scaled, Use&& use)
+cudaError_t with_kernel(int bn, int bk, bool amn, bool bmn, bool slim, bool scaled, Use&& use)
 {
-    if (bk == 16) return bn == 64 ? with_majors<4, 16>(amn, bmn, scaled, use) : with_majors<2, 16>(amn, bmn, scaled, use);
-    return bn == 64 ? with_majors<4, 8>(amn, bmn, scaled, use) : with_majors<2, 8>(amn, bmn, scaled, use);
+    if (bk == 16) return bn == 64 ? with_majors<4, 16>(amn, bmn, slim, scaled, use) : with_majors<2, 16>(amn, bmn, slim, scaled, use);
+    return bn == 64 ? with_majors<4, 8>(amn, bmn, slim, scaled, use) : with_majors<2, 8>(amn, bmn, slim, scaled, use);
 }
 
 }  // namespace
@@ -501,8 +548,8 @@ cudaError_t with_kernel(int bn, int bk, bool amn, bool bmn, bool scaled, Use&& u
 cudaError_t dmma_tma_configure()
 {
     cudaError_t e = cudaSuccess;
-    for (int form = 0; form < 32 && e == cudaSuccess; ++form)
-        e = with_kernel(form & 1 ? 64 : 32, form & 2 ? 16 : 8, form & 4, form & 8, form & 16,
+    for (int form = 0; form < 48 && e == cudaSuccess; ++form)   // (the last 16: slim, B K-major)
+        e = with_kernel(form & 1 ? 64 : 32, form & 2 ? 16 : 8, form & 4, form < 32 && (form & 16), form >= 32, form & 8,
                         [](auto* kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes); });
     return e;
 }
@@ -513,7 +560,7 @@ cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* 
     if (total <= 0 || p.k_splits < 1 || p.stages < 2 || (p.stages & 1) || (p.BN != 64 && p.BN != 32) || (p.BK != 16 && p.BK != 8)) return cudaErrorInvalidValue;
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
     const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
-    return with_kernel(p.BN, p.BK, p.a.major != 0, p.b.major != 0, p.scaled != 0, [&](auto* kernel) {
+    return with_kernel(p.BN, p.BK, p.a.major != 0, p.b.major != 0, p.slim != 0, p.scaled != 0, [&](auto* kernel) {
         return launch_chained(kernel, dim3(grid), dim3(kThreads64), static_cast<size_t>(smem_bytes), stream, 1, ta, tb, p);
     });
 }

@@ -725,6 +725,7 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
         // (across slabs the first digit is C's stride-1 mode, in whole eights, and the elements of a slab lie along another mode)
         const bool rows = u->store_across_slabs ? fours(u->a, 1) && u->a.row_elem_cstride % 4 == 0
                                                 : fours(u->a, 0) && u->a.row_elem_cstride == 1 && u->a.split_inner % 4 == 0;
+        u->slim = u->tiles_n == 1 && u->b.major == 0 && u->b.total_slabs * u->b.slab_w <= u->BN / 4 * 3 && !std::getenv("TCONT_NO_SLIM");
         u->pieces32 = rows && fours(u->b, 0) && u->b.row_elem_cstride % 4 == 0;
     }
     u->eligible = true;
@@ -1511,7 +1512,7 @@ std::string describe_plan(const Plan& pl)
           << ",\"a_slab_w\":" << u.a.slab_w << ",\"b_slab_w\":" << u.b.slab_w << ",\"a_slabs_per_copy\":" << u.a.slabs_per_op << ",\"b_slabs_per_copy\":" << u.b.slabs_per_op << ",\"a_slabs\":" << u.a.slabs_per_tile
           << ",\"b_slabs\":" << u.b.slabs_per_tile << ",\"smem_bytes\":" << u.smem_bytes
           << ",\"coalesced_store\":" << (u.a.row_elem_cstride == 1 ? "true" : "false")
-          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"producers\":" << u.producers
+          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"slim\":" << (u.slim ? "true" : "false") << ",\"producers\":" << u.producers
           << ",\"a_fused\":" << u.a.split_inner << ",\"b_fused\":" << u.b.split_inner << ",\"column_ranges\":[";
         std::string why;
         for (int r = 2, n = 0; r <= 8; ++r)

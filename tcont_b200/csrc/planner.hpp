@@ -114,6 +114,9 @@ struct UmmaSpec {
     // FP64 kernel: the four elements of C a thread stores at a time are neighbours and, where C itself is, on a multiple of 32
     // bytes, unless some of them lie beyond C
     bool pieces32 = false;
+    // FP64 kernel: one column of tiles, of which at most three quarters are columns of C (B K-major): a warp computes three column
+    // fragments instead of four
+    bool slim = false;
     int smem_bytes = 0;
     int elt = 4;  // element bytes: 4 = tcgen05 TF32 kernel, 8 = TMA-fed FP64 tensor-path kernel
 };

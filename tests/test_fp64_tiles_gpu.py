@@ -49,6 +49,13 @@ STORES = {
     "fused_rows": ("acb", "abk", "kc", dict(a=12, b=60, c=128, k=24), 0),
     "fused_rows_odd": ("acb", "abk", "kc", dict(a=6, b=50, c=128, k=24), 0),
     "across_slabs": ("abcd", "dbea", "ec", dict(a=24, b=9, c=64, d=48, e=24), 0),
+    # one column of tiles that C fills to three quarters or less: fewer column fragments, the last one not one of a pair
+    "slim_24": ("ab", "ak", "kb", dict(a=1540, b=24, k=24), 0),
+    "slim_17": ("ab", "ka", "kb", dict(a=1540, b=17, k=40), 0),
+    "slim_48": ("ab", "ak", "kb", dict(a=1540, b=48, k=24), 0),
+    "slim_33": ("ab", "ka", "kb", dict(a=1538, b=33, k=40), 0),
+    "slim_across_slabs": ("abcd", "dbea", "ec", dict(a=24, b=9, c=24, d=48, e=24), 0),
+    "slim_across_slabs_48": ("abcd", "dbea", "ec", dict(a=24, b=9, c=42, d=40, e=40), 0),
     "across_slabs_ragged": ("abcd", "dbea", "ec", dict(a=24, b=9, c=60, d=54, e=40), 0),
 }
 
@@ -75,7 +82,8 @@ def test_stores(engine, oracle, monkeypatch, name, beta):
     run.set_scalars(1.0, beta)
     engine.launch(run)
     torch.cuda.synchronize()
-    assert plan.describe()["kernel"] == "dmma_f64_tma" and run.device_status() == 0
+    u = plan.describe()["umma"]
+    assert plan.describe()["kernel"] == "dmma_f64_tma" and u["slim"] == name.startswith("slim") and run.device_status() == 0
     outside = torch.cat([guarded[:shift], guarded[shift + n:]])
     assert bool((outside == 7.0).all())
     exact, scale = oracle.contract(c, A, B) + beta * C0, oracle.contract(c, np.abs(A), np.abs(B)) + abs(beta * C0)
