@@ -18,7 +18,7 @@
 //               narrow N) and takes every other tile of the block.  Group 1 starts half a main loop late, so one group's stores fall into the
 //               other's main loop instead of both storing with the FP64 pipe idle.
 // Fragment rows are permuted so that one 16-byte shared load of an MN-major operand feeds two
-// fragments (rows 2 r and 2 r + 1 of a 16-row slab) without bank conflicts, and the MMA is issued
+// fragments (rows 2 r and 2 r + 1 of a 16-row slab; with k in ascending order at two-way bank conflicts), and the MMA is issued
 // transposed (B fragment as the row operand): a thread then owns four consecutive elements of C's
 // stride-1 mode per fragment pair and a warp store instruction writes eight whole 128-byte lines.
 // The loads of the next k step are issued between the MMAs of the current one.
