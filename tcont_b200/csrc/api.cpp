@@ -543,7 +543,7 @@ tcontb_status finish_run(tcontb_run* run)
         run->umma.pair = u.pair ? 1 : 0;
         run->umma.producers = u.producers;
         run->umma.store_across_slabs = u.store_across_slabs ? 1 : 0;
-        run->umma.pieces32 = u.pieces32 ? 1 : 0;
+        run->umma.piece = u.piece;
         run->umma.slim = u.slim ? 1 : 0;
         run->umma.n_k_digits = u.n_k_digits;
         for (int i = 0; i < 3; ++i) run->umma.k_digit_ext[i] = static_cast<int>(u.k_digit_ext[i]);
@@ -637,7 +637,7 @@ tcontb_status finish_run(tcontb_run* run)
         }
         if (u.smem_bytes > kMaxDynamicSmemBytes) return fail(TCONTB_RUNTIME_ERROR, "plan asks for more shared memory than a block can have");
         if (pl.kernel == KERNEL_UMMA_TF32) TC_CUDA(umma_tf32_configure());
-        else TC_CUDA(dmma_tma_configure());
+        else TC_CUDA(dmma_tma_configure(run->umma));
         TC_CUDA(splitk_reduce_configure());
     } else {
         fill_gather(p, kA, kB, run->dC, pl.simt, pl.gather, &run->gather);

@@ -18,7 +18,8 @@
 //               narrow N) and takes every other tile of the block.  Group 1 starts half a main loop late, so one group's stores fall into the
 //               other's main loop instead of both storing with the FP64 pipe idle.
 // Fragment rows are permuted so that one 16-byte shared load of an MN-major operand feeds two
-// fragments (rows 2 r and 2 r + 1 of a 16-row slab; with k in ascending order at two-way bank conflicts), and the MMA is issued
+// fragments (rows 2 r and 2 r + 1 of a 16-row slab; two-way bank conflicts with k in ascending order, which cost nothing that could be timed:
+// 2048 x 8000 x 24 36.7 us, 36.6 with an order without them), and the MMA is issued
 // transposed (B fragment as the row operand): a thread then owns four consecutive elements of C's
 // stride-1 mode per fragment pair and a warp store instruction writes eight whole 128-byte lines.
 // The loads of the next k step are issued between the MMAs of the current one.
@@ -28,6 +29,8 @@
 // (backends/cogent/plan/generators/kernels/kernel_compute.py:127-850) and its cublasGemmEx FP64
 // call (backends/ttgt_cutt/src/ttgt_cutt.cpp:764-809).
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "chain.cuh"
 #include "kernels.hpp"
@@ -39,6 +42,7 @@ namespace {
 constexpr int kThreads64 = 384;
 constexpr int kBM = 128, kMaxBN = 64;
 constexpr uint32_t kTabBytes = (kBM + kMaxBN) * 8u;  // one tile's row and column offsets
+constexpr long long kBeyond = -(1ll << 61);          // entry of a row or column beyond C: a sum with any other entry is negative
 
 __device__ __forceinline__ double ld_shared_f64(uint32_t addr)
 {
@@ -61,6 +65,19 @@ __device__ __forceinline__ void dmma_m8n8k4(double (&c)[2], double a, double b)
 __device__ __forceinline__ void st_global_cs_v4f64(double* p, double a, double b, double c, double d)
 {
     asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+// The same at C + offset, by predicate: not where `offset` is negative.
+__device__ __forceinline__ void st_global_cs_v4f64_in(double* C, long long offset, double a, double b, double c, double d)
+{
+    asm volatile("{\n .reg .pred in;\n setp.ge.s64 in, %5, 0;\n @in st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};\n}" ::"l"(C + offset), "d"(a), "d"(b), "d"(c),
+                 "d"(d), "l"(offset)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_global_cs_v2f64_in(double* C, long long offset, double a, double b)
+{
+    asm volatile("{\n .reg .pred in;\n setp.ge.s64 in, %3, 0;\n @in st.global.cs.v2.f64 [%0], {%1, %2};\n}" ::"l"(C + offset), "d"(a), "d"(b), "l"(offset) : "memory");
 }
 
 __device__ __forceinline__ void ld_global_cs_v4f64(double (&o)[4], const double* p)
@@ -176,11 +193,12 @@ __device__ __forceinline__ uint32_t column_of(int j, uint32_t fr)
 }
 
 // SCALED: C = alpha A B + beta C in the epilogue (C read only when beta is not zero); a template parameter because the
-// overwriting kernel has no registers to spare for it.
+// overwriting kernel has no registers to spare for it.  PIECES: every store is 32 aligned bytes (UmmaSpec::piece); one kernel with both
+// epilogues is slower in either (9216 x 4096 x 24 102.5 us, 94.5 in a kernel of its own; 2050 x 8000 x 16 54.8 and 48.7).
 // SLIM: one column of tiles, of at most 48 of its 64 columns or 24 of its 32 (B K-major).  Three column fragments a warp instead of
 // four; or (HALVES) two for the warps of one half and one for the others, the other way round in the second group, so that every
-// scheduler has three.  373 248 x 24 x 72 75.0 -> 68.2 us, 48 columns 143.6 -> 111.7, 200 000 x 48 x 200 163 -> 124.
-template <bool AMN, bool BMN, int NF, int BK, bool SCALED, bool SLIM>
+// scheduler has three.  373 248 x 24 x 72 70.1 -> 65.0 us, 48 columns 128.5 -> 106.2, 200 000 x 24 x 200 83.8 -> 72.8.
+template <bool AMN, bool BMN, int NF, int BK, bool SCALED, bool SLIM, bool PIECES>
 __global__ void __launch_bounds__(kThreads64, 1)
 dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                 const __grid_constant__ UmmaParams p)
@@ -199,7 +217,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     uint64_t* tab_full = bar_empty + 10;   // [group][buffer]
     uint64_t* tab_empty = tab_full + 4;    // [group][buffer]
     const uint32_t ragged = smem_u32(tab_empty + 4);   // [group][buffer]: 1 + number of the last tile with rows (not SLIM: or columns) beyond C
-    const uint32_t tabs = smem_u32(aux + 256);  // [group][buffer]: long long [128] row offsets, [64] column offsets (-1 = beyond C)
+    const uint32_t tabs = smem_u32(aux + 256);  // [group][buffer]: long long [128] row offsets, [64] column offsets (kBeyond = beyond C)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
@@ -315,8 +333,8 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     int d0 = 0;
                     const long long off = slab_c_offset(o, (is_row ? tm * SA : tn * SB) + sl, &d0, &ok);
                     ok = ok && (d0 * o.slab_w + in < o.slab_mode_ext);
-                    if ((is_row || !SLIM) && !ok) st_shared_u32(ragged + slot * 4u, i + 1u);
-                    st_shared_s64(tab + static_cast<uint32_t>(e) * 8u, ok ? off + slab_elem_offset(o, d0, in) : -1);
+                    if (SCALED && PIECES && (is_row || !SLIM) && !ok) st_shared_u32(ragged + slot * 4u, i + 1u);
+                    st_shared_s64(tab + static_cast<uint32_t>(e) * 8u, ok ? off + slab_elem_offset(o, d0, in) : kBeyond);
                 }
                 mbar_arrive(smem_u32(tab_full + slot));
                 if (SCALED && p.beta != 0.0) {
@@ -429,69 +447,117 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             //   rows along C    : rows 16 u + 4 fk + q, element q in acc[2 u + (q & 1)][j][q >> 1]
             //   rows across slabs: the warp's 64 rows are four slabs of 16, slab q is index a0 + q of C's stride-1 mode; row
             //                      4 fk + u of the four slabs, element q in acc[2 q + (u & 1)][j][u >> 1]
-            long long cn[W], cm[4];
+            long long cn[W];
 #pragma unroll
             for (int j = 0; j < W; ++j)
-                cn[j] = HALVES && narrow ? (j == 0 ? ld_shared_s64(col_tab + (col0 + column_of<1>(0, fr)) * 8u) : -1)
+                cn[j] = HALVES && narrow ? (j == 0 ? ld_shared_s64(col_tab + (col0 + column_of<1>(0, fr)) * 8u) : kBeyond)
                                          : ld_shared_s64(col_tab + (col0 + column_of<W>(j, fr)) * 8u);
             const uint32_t row_u = p.store_across_slabs ? 8u : 128u, row_q = p.store_across_slabs ? 128u : 8u;   // table bytes from u to u + 1, q to q + 1
             const uint32_t rows = row_tab + (static_cast<uint32_t>(wm * 64) + 4u * fk) * 8u;
+            auto row_of = [&](int u, uint32_t q) { return ld_shared_s64(rows + static_cast<uint32_t>(u) * row_u + q * row_q); };   // C offset of element q of the four
+            const bool whole = SCALED && PIECES && ld_shared_u32(ragged + slot * 4u) != i + 1u;
+            // Straight-line: a warp alone on its scheduler takes 5 to 20 cycles for every instruction and branch between two stores (with
+            // alignment and bounds tested per store 4 200 cycles a tile, whatever the pieces' layout; 1 700 here).  Pieces beyond C are
+            // left out by predicate (tested per store, 300 000 x 40 x 24 took 50.1 us and accumulating 124, here 40.4 and 65.6); a whole
+            // tile's old values are not (9216 x 4096 x 24 accumulating: 176 us by predicate, 167 without).
+            auto store_pieces = [&](auto&& at, auto all) {
+                constexpr bool ALL = decltype(all)::value;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) cm[u] = ld_shared_s64(rows + static_cast<uint32_t>(u) * row_u);
-            const bool whole = p.pieces32 && tile_ok && (reinterpret_cast<uintptr_t>(C) & 31u) == 0 && ld_shared_u32(ragged + slot * 4u) != i + 1u;
-            auto store_tile = [&](auto&& at) {
-                if (whole) {
-                    // Straight-line: a warp alone on its scheduler takes 5 to 20 cycles for every instruction and branch between
-                    // two stores (with alignment and bounds tested per store 4 200 cycles a tile, whatever the pieces' layout;
-                    // tested per tile here 2 900, by the table builders 1 700).  9216 x 4096 x 24, C of 302 MB: accumulating 206 -> 168
-                    // us, with rows along C 223 -> 146; overwriting 110 -> 90.
+                for (int u = 0; u < 4; ++u) {
+                    const long long cm = row_of(u, 0);
+                    if constexpr (SCALED) {   // the old values of all column fragments are asked for before the first is used
+                        double old[W][4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if constexpr (SCALED) {   // the old values of all column fragments are asked for before the first is used
-                            double old[W][4];
-#pragma unroll
-                            for (int j = 0; j < W; ++j) {
-                                if (p.beta != 0.0 && (!SLIM || cn[j] >= 0)) ld_global_cs_v4f64(old[j], C + cm[u] + cn[j]);
-                                else old[j][0] = old[j][1] = old[j][2] = old[j][3] = 0.0;
-                            }
-#pragma unroll
-                            for (int j = 0; j < W; ++j)
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) at(u, j, q) = p.alpha * at(u, j, q) + p.beta * old[j][q];
+                        for (int j = 0; j < W; ++j) {
+                            if (p.beta != 0.0 && (ALL ? !SLIM || cn[j] >= 0 : cm + cn[j] >= 0)) ld_global_cs_v4f64(old[j], C + cm + cn[j]);
+                            else old[j][0] = old[j][1] = old[j][2] = old[j][3] = 0.0;
                         }
 #pragma unroll
                         for (int j = 0; j < W; ++j)
-                            if (!SLIM || cn[j] >= 0) st_global_cs_v4f64(C + cm[u] + cn[j], at(u, j, 0), at(u, j, 1), at(u, j, 2), at(u, j, 3));
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) at(u, j, q) = p.alpha * at(u, j, q) + p.beta * old[j][q];
+                    }
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        if (!ALL) st_global_cs_v4f64_in(C, cm + cn[j], at(u, j, 0), at(u, j, 1), at(u, j, 2), at(u, j, 3));
+                        else if (!SLIM || cn[j] >= 0) st_global_cs_v4f64(C + cm + cn[j], at(u, j, 0), at(u, j, 1), at(u, j, 2), at(u, j, 3));
+                    }
+                }
+            };
+            auto store_tile = [&](auto&& at) {
+                if constexpr (PIECES) {
+                    if (!tile_ok) return;
+                    if (SCALED && whole) store_pieces(at, std::bool_constant<SCALED>());
+                    else store_pieces(at, std::false_type());
+                } else if (tile_ok && p.piece == 2) {
+                    // halves of 16 bytes, straight-line as above
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const long long r[2] = {row_of(u, 0), row_of(u, 2)};
+                        if constexpr (SCALED) {
+                            double2 old[W][2];
+#pragma unroll
+                            for (int j = 0; j < W; ++j)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+                                    old[j][h] = p.beta != 0.0 && r[h] + cn[j] >= 0 ? __ldcs(reinterpret_cast<const double2*>(C + r[h] + cn[j])) : make_double2(0.0, 0.0);
+#pragma unroll
+                            for (int j = 0; j < W; ++j)
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) at(u, j, q) = p.alpha * at(u, j, q) + p.beta * (q & 1 ? old[j][q >> 1].y : old[j][q >> 1].x);
+                        }
+#pragma unroll
+                        for (int j = 0; j < W; ++j)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) st_global_cs_v2f64_in(C, r[h] + cn[j], at(u, j, 2 * h), at(u, j, 2 * h + 1));
                     }
                 } else if (tile_ok) {
-                    // ragged or odd-aligned pieces: 32 bytes where they can be, 16 where two elements are neighbours, else one by one
+                    // 32 bytes where they can be, 16 where two elements are neighbours, else one by one
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         long long r[4];
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) r[q] = ld_shared_s64(rows + static_cast<uint32_t>(u) * row_u + static_cast<uint32_t>(q) * row_q);
+                        for (int q = 0; q < 4; ++q) r[q] = row_of(u, static_cast<uint32_t>(q));
                         const bool run4 = r[0] >= 0 && r[1] == r[0] + 1 && r[2] == r[0] + 2 && r[3] == r[0] + 3;
+                        auto aligned32 = [&](int j) { return run4 && (reinterpret_cast<uintptr_t>(C + r[0] + cn[j]) & 31u) == 0; };
+                        if constexpr (SCALED) {   // (two fragments at a time: more spill)
+#pragma unroll
+                            for (int j0 = 0; j0 < W; j0 += 2) {
+                                double old[2][4];
+#pragma unroll
+                                for (int t = 0; t < 2 && j0 + t < W; ++t) {
+                                    const int j = j0 + t;
+                                    old[t][0] = old[t][1] = old[t][2] = old[t][3] = 0.0;
+                                    if (p.beta == 0.0 || cn[j] < 0) continue;
+                                    if (aligned32(j)) {
+                                        ld_global_cs_v4f64(old[t], C + r[0] + cn[j]);
+                                    } else {
+#pragma unroll
+                                        for (int q = 0; q < 4; ++q)
+                                            if (r[q] >= 0) old[t][q] = __ldcs(C + r[q] + cn[j]);
+                                    }
+                                }
+#pragma unroll
+                                for (int t = 0; t < 2 && j0 + t < W; ++t)
+#pragma unroll
+                                    for (int q = 0; q < 4; ++q) at(u, j0 + t, q) = p.alpha * at(u, j0 + t, q) + p.beta * old[t][q];
+                            }
+                        }
 #pragma unroll
                         for (int j = 0; j < W; ++j) {
                             if (cn[j] < 0) continue;
-                            double x[4];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                x[q] = at(u, j, q);
-                                if constexpr (SCALED) x[q] = p.alpha * x[q] + (p.beta != 0.0 && r[q] >= 0 ? p.beta * __ldcs(C + r[q] + cn[j]) : 0.0);
-                            }
-                            if (run4 && (reinterpret_cast<uintptr_t>(C + r[0] + cn[j]) & 31u) == 0) {
-                                st_global_cs_v4f64(C + r[0] + cn[j], x[0], x[1], x[2], x[3]);
+                            if (aligned32(j)) {
+                                st_global_cs_v4f64(C + r[0] + cn[j], at(u, j, 0), at(u, j, 1), at(u, j, 2), at(u, j, 3));
                                 continue;
                             }
 #pragma unroll
                             for (int q = 0; q < 4; q += 2) {
                                 double* d = C + r[q] + cn[j];
                                 if (r[q] >= 0 && r[q + 1] == r[q] + 1 && (reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
-                                    __stcs(reinterpret_cast<double2*>(d), make_double2(x[q], x[q + 1]));
+                                    __stcs(reinterpret_cast<double2*>(d), make_double2(at(u, j, q), at(u, j, q + 1)));
                                 } else {
-                                    if (r[q] >= 0) __stcs(d, x[q]);
-                                    if (r[q + 1] >= 0) __stcs(C + r[q + 1] + cn[j], x[q + 1]);
+                                    if (r[q] >= 0) __stcs(d, at(u, j, q));
+                                    if (r[q + 1] >= 0) __stcs(C + r[q + 1] + cn[j], at(u, j, q + 1));
                                 }
                             }
                         }
@@ -522,35 +588,42 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     if (threadIdx.x == 0 && ld_shared_u32(abort_flag)) atomicMax(p.status, 1);
 }
 
-// The kernel's forms, one function per (majors, columns, k chunk, slim, scaled); `use` is called with the one that matches.
+// The kernel's forms, one function per (majors, columns, k chunk, slim, scaled, pieces); `use` is called with the one that matches.
 template <bool AMN, bool BMN, int NF, int BK, bool SLIM, typename Use>
-cudaError_t with_scaled(bool scaled, Use&& use)
+cudaError_t with_epilogue(bool scaled, bool pieces, Use&& use)
 {
-    return scaled ? use(dmma_tma_kernel<AMN, BMN, NF, BK, true, SLIM>) : use(dmma_tma_kernel<AMN, BMN, NF, BK, false, SLIM>);
+    if (pieces) return scaled ? use(dmma_tma_kernel<AMN, BMN, NF, BK, true, SLIM, true>) : use(dmma_tma_kernel<AMN, BMN, NF, BK, false, SLIM, true>);
+    return scaled ? use(dmma_tma_kernel<AMN, BMN, NF, BK, true, SLIM, false>) : use(dmma_tma_kernel<AMN, BMN, NF, BK, false, SLIM, false>);
 }
 template <int NF, int BK, typename Use>
-cudaError_t with_majors(bool amn, bool bmn, bool slim, bool scaled, Use&& use)
+cudaError_t with_majors(bool amn, bool bmn, bool slim, bool scaled, bool pieces, Use&& use)
 {
-    if (slim) return bmn ? cudaErrorInvalidValue : amn ? with_scaled<true, false, NF, BK, true>(scaled, use) : with_scaled<false, false, NF, BK, true>(scaled, use);
-    if (amn) return bmn ? with_scaled<true, true, NF, BK, false>(scaled, use) : with_scaled<true, false, NF, BK, false>(scaled, use);
-    return bmn ? with_scaled<false, true, NF, BK, false>(scaled, use) : with_scaled<false, false, NF, BK, false>(scaled, use);
+    if (slim) return bmn ? cudaErrorInvalidValue : amn ? with_epilogue<true, false, NF, BK, true>(scaled, pieces, use) : with_epilogue<false, false, NF, BK, true>(scaled, pieces, use);
+    if (amn) return bmn ? with_epilogue<true, true, NF, BK, false>(scaled, pieces, use) : with_epilogue<true, false, NF, BK, false>(scaled, pieces, use);
+    return bmn ? with_epilogue<false, true, NF, BK, false>(scaled, pieces, use) : with_epilogue<false, false, NF, BK, false>(scaled, pieces, use);
 }
 template <typename Use>
-cudaError_t with_kernel(int bn, int bk, bool amn, bool bmn, bool slim, bool scaled, Use&& use)
+cudaError_t with_kernel(const UmmaParams& p, bool scaled, bool pieces, Use&& use)
 {
-    if (bk == 16) return bn == 64 ? with_majors<4, 16>(amn, bmn, slim, scaled, use) : with_majors<2, 16>(amn, bmn, slim, scaled, use);
-    return bn == 64 ? with_majors<4, 8>(amn, bmn, slim, scaled, use) : with_majors<2, 8>(amn, bmn, slim, scaled, use);
+    const bool amn = p.a.major != 0, bmn = p.b.major != 0, slim = p.slim != 0;
+    if (p.BK == 16) return p.BN == 64 ? with_majors<4, 16>(amn, bmn, slim, scaled, pieces, use) : with_majors<2, 16>(amn, bmn, slim, scaled, pieces, use);
+    return p.BN == 64 ? with_majors<4, 8>(amn, bmn, slim, scaled, pieces, use) : with_majors<2, 8>(amn, bmn, slim, scaled, pieces, use);
+}
+
+// Whether every piece of `of` elements starts on a multiple of its size.
+bool stores_pieces(const UmmaParams& p, int of)
+{
+    return p.piece >= of && reinterpret_cast<uintptr_t>(p.C64) % (8u * of) == 0 && (p.k_splits == 1 || p.split_stride % of == 0);
 }
 
 }  // namespace
 
-// The dynamic shared-memory cap is per function and device: every run sets the same opt-in maximum.
-cudaError_t dmma_tma_configure()
+// The dynamic shared-memory cap is per function and device: every run sets the same opt-in maximum, for the forms that it can launch.
+cudaError_t dmma_tma_configure(const UmmaParams& p)
 {
     cudaError_t e = cudaSuccess;
-    for (int form = 0; form < 48 && e == cudaSuccess; ++form)   // (the last 16: slim, B K-major)
-        e = with_kernel(form & 1 ? 64 : 32, form & 2 ? 16 : 8, form & 4, form < 32 && (form & 16), form >= 32, form & 8,
-                        [](auto* kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes); });
+    for (int form = 0; form < 4 && e == cudaSuccess; ++form)
+        e = with_kernel(p, form & 1, form & 2, [](auto* kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmemBytes); });
     return e;
 }
 
@@ -560,8 +633,14 @@ cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* 
     if (total <= 0 || p.k_splits < 1 || p.stages < 2 || (p.stages & 1) || (p.BN != 64 && p.BN != 32) || (p.BK != 16 && p.BK != 8)) return cudaErrorInvalidValue;
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
     const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
-    return with_kernel(p.BN, p.BK, p.a.major != 0, p.b.major != 0, p.slim != 0, p.scaled != 0, [&](auto* kernel) {
-        return launch_chained(kernel, dim3(grid), dim3(kThreads64), static_cast<size_t>(smem_bytes), stream, 1, ta, tb, p);
+    UmmaParams q = p;
+    // Strides of 2 modulo 4 elements: half of the columns could take 32 bytes at a time, but a test per store costs more than that spares
+    // where the epilogue is most of a tile (2050 x 8000, K 24 57.3 us tested, 49.9 in halves, K 48 74.9 and 67.2; accumulating 103 and 75).
+    // With more k iterations the stores fall into the other group's main loop (3002 x 3002, K 64 46.3 and 50.6, K 96 63.3 and 67.5), but
+    // for the old values (79.8 and 69.1).
+    q.piece = stores_pieces(p, 2) && (p.scaled || p.k_iters_per_split <= 3) ? 2 : 1;
+    return with_kernel(q, p.scaled != 0, stores_pieces(p, 4), [&](auto* kernel) {
+        return launch_chained(kernel, dim3(grid), dim3(kThreads64), static_cast<size_t>(smem_bytes), stream, 1, ta, tb, q);
     });
 }
 

@@ -178,7 +178,7 @@ struct UmmaParams {
     // owner_base[o][i].  owners = 0 or 1: everything goes to C.  `tn_rotate` shifts the order in which a GPU
     // visits the tile columns, so that the GPUs of a job write to different owners at any one time.
     int store_across_slabs;  // FP64 kernel: see UmmaSpec
-    int pieces32;            // FP64 kernel: see UmmaSpec
+    int piece;               // FP64 kernel: see UmmaSpec
     int slim;                // FP64 kernel: see UmmaSpec
     // tcgen05 kernel.  1: the next kernel's blocks may be scheduled when this one's copies are issued, 0: at once.  Late where
     // every block stores many tiles of few k iterations: 806400 x 112 x 48 behind its permutation, 43 tiles a block: let in at
@@ -226,7 +226,7 @@ cudaError_t launch_across_tf32(const AcrossParams& p, const void* tmapA, const v
 // ---- TMA-fed FP64 tensor-path contraction (dmma_tma_f64.cu), same parameter block ------------
 cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, int num_sms,
                             cudaStream_t stream);
-cudaError_t dmma_tma_configure();
+cudaError_t dmma_tma_configure(const UmmaParams& p);
 
 // ---- split-K: C[e] = sum over s of partial[s * stride + e], s ascending (splitk_reduce.cu) ----
 // With alpha != 1 or beta != 0: C[e] = alpha * sum + beta * C[e] (C is read only when beta != 0).

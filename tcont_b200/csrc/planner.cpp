@@ -717,16 +717,18 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
         }
     }
     if (f64) {
-        auto fours = [](const UmmaOperand& o, int from_digit) {
-            bool ok = o.split_inner == 0 || o.split_outer_cstride % 4 == 0;
-            for (int d = from_digit; d < o.n_row_digits; ++d) ok = ok && o.row_digit_cstride[d] % 4 == 0;
+        auto multiples = [&](const UmmaOperand& o, int from_digit, int64_t of) {
+            bool ok = o.split_inner == 0 || o.split_outer_cstride % of == 0;
+            for (int d = from_digit; d < o.n_row_digits; ++d) ok = ok && o.row_digit_cstride[d] % of == 0;
             return ok;
         };
-        // (across slabs the first digit is C's stride-1 mode, in whole eights, and the elements of a slab lie along another mode)
-        const bool rows = u->store_across_slabs ? fours(u->a, 1) && u->a.row_elem_cstride % 4 == 0
-                                                : fours(u->a, 0) && u->a.row_elem_cstride == 1 && u->a.split_inner % 4 == 0;
+        for (const int of : {4, 2}) {
+            // (across slabs the first digit is C's stride-1 mode, in whole eights, and the elements of a slab lie along another mode)
+            const bool rows = u->store_across_slabs ? multiples(u->a, 1, of) && u->a.row_elem_cstride % of == 0
+                                                    : multiples(u->a, 0, of) && u->a.row_elem_cstride == 1 && u->a.split_inner % of == 0 && u->a.slab_mode_ext % of == 0;
+            if (u->piece < of && rows && multiples(u->b, 0, of) && u->b.row_elem_cstride % of == 0) u->piece = of;
+        }
         u->slim = u->tiles_n == 1 && u->b.major == 0 && u->b.total_slabs * u->b.slab_w <= u->BN / 4 * 3 && !std::getenv("TCONT_NO_SLIM");
-        u->pieces32 = rows && fours(u->b, 0) && u->b.row_elem_cstride % 4 == 0;
     }
     u->eligible = true;
 }
@@ -1384,7 +1386,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         double us = transposes_us(i, cost, gathers || (i > 0 && i == padded_candidate)) + contraction_us(q, kernel, u, cost);
         // (stores come on top of the arithmetic where they are not all of 32 aligned bytes: 10469 x 9025 x 63, odd, 798 us with 360 of
         // arithmetic, 580 on the gather kernel; 82431 x 2205 x 7 818 and 546)
-        if (i > 0 && i == padded_candidate && kernel == KERNEL_DMMA_F64_TMA) us += double(q.sizeC) * double(u.k_splits) * (u.pieces32 ? 0.8e-6 : 4.6e-6);
+        if (i > 0 && i == padded_candidate && kernel == KERNEL_DMMA_F64_TMA) us += double(q.sizeC) * double(u.k_splits) * (u.piece == 4 ? 0.8e-6 : 4.6e-6);
         if (padded_forced && i > 0 && i == padded_candidate && kernel == KERNEL_DMMA_F64_TMA) us = 0;
         // Partial sums behind the FP64 kernel: a thread adds its partials up one after the other, 0.12 us each (96 x 64 x 2992
         // in 41 ranges: 20.8 us without that, 24.6 measured).  Where the operands lie the kernels' estimates are compared as they were fitted.
@@ -1512,7 +1514,7 @@ std::string describe_plan(const Plan& pl)
           << ",\"a_slab_w\":" << u.a.slab_w << ",\"b_slab_w\":" << u.b.slab_w << ",\"a_slabs_per_copy\":" << u.a.slabs_per_op << ",\"b_slabs_per_copy\":" << u.b.slabs_per_op << ",\"a_slabs\":" << u.a.slabs_per_tile
           << ",\"b_slabs\":" << u.b.slabs_per_tile << ",\"smem_bytes\":" << u.smem_bytes
           << ",\"coalesced_store\":" << (u.a.row_elem_cstride == 1 ? "true" : "false")
-          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"slim\":" << (u.slim ? "true" : "false") << ",\"producers\":" << u.producers
+          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"slim\":" << (u.slim ? "true" : "false") << ",\"piece\":" << u.piece << ",\"producers\":" << u.producers
           << ",\"a_fused\":" << u.a.split_inner << ",\"b_fused\":" << u.b.split_inner << ",\"column_ranges\":[";
         std::string why;
         for (int r = 2, n = 0; r <= 8; ++r)

@@ -111,9 +111,9 @@ struct UmmaSpec {
     // FP64 kernel: the slabs of an A tile are consecutive indices of C's stride-1 mode (which is not A's stride-1
     // mode); a thread stores the same row of four neighbouring slabs as one 32-byte piece
     bool store_across_slabs = false;
-    // FP64 kernel: the four elements of C a thread stores at a time are neighbours and, where C itself is, on a multiple of 32
-    // bytes, unless some of them lie beyond C
-    bool pieces32 = false;
+    // FP64 kernel: of the four elements of C a thread stores at a time so many (4, 2 or 1) are neighbours, lie together inside C or
+    // beyond it, and start on a multiple of so many elements from C's first
+    int piece = 1;
     // FP64 kernel: one column of tiles, of which at most three quarters are columns of C (B K-major): a warp computes three column
     // fragments instead of four
     bool slim = false;

@@ -9,6 +9,7 @@ import pytest
 from cases import to_equation
 from oracle_lib import F64, Contraction
 from test_contraction_gpu import run_contraction
+from test_scaled_epilogues_gpu import scaled_run
 
 pytestmark = pytest.mark.gpu
 
@@ -56,6 +57,14 @@ STORES = {
     "slim_33": ("ab", "ka", "kb", dict(a=1538, b=33, k=40), 0),
     "slim_across_slabs": ("abcd", "dbea", "ec", dict(a=24, b=9, c=24, d=48, e=24), 0),
     "slim_across_slabs_48": ("abcd", "dbea", "ec", dict(a=24, b=9, c=42, d=40, e=40), 0),
+    # a last column of tiles that is not filled, B along k and along its columns; pieces of two elements (C's strides 2 modulo 4),
+    # with few and many k chunks; of one (odd strides)
+    "columns_56": ("ab", "ak", "kb", dict(a=1540, b=56, k=24), 0),
+    "columns_40_mn": ("ab", "ak", "bk", dict(a=1540, b=40, k=24), 0),
+    "halves": ("ab", "ak", "bk", dict(a=1030, b=150, k=40), 0),
+    "halves_many_chunks": ("ab", "ka", "kb", dict(a=1030, b=150, k=136), 0),
+    "slim_halves": ("ab", "ak", "kb", dict(a=1538, b=22, k=40), 0),
+    "odd_strides": ("ab", "ka", "kb", dict(a=1029, b=149, k=40), 0),
     "across_slabs_ragged": ("abcd", "dbea", "ec", dict(a=24, b=9, c=60, d=54, e=40), 0),
 }
 
@@ -89,6 +98,29 @@ def test_stores(engine, oracle, monkeypatch, name, beta):
     exact, scale = oracle.contract(c, A, B) + beta * C0, oracle.contract(c, np.abs(A), np.abs(B)) + abs(beta * C0)
     k = ext.get("k", ext.get("e"))
     assert (np.abs(dC.cpu().numpy() - exact) <= (k + 4) * 2.0**-53 * scale).all()
+    stride = ext["a"]
+    assert u["piece"] == (4 if stride % 4 == 0 else 2 if stride % 2 == 0 else 1) or name.startswith("fused"), u
+
+
+@pytest.mark.parametrize("rows", [128, 130, 131])
+def test_rows_of_a_view(engine, oracle, monkeypatch, rows):
+    """C's columns lie on multiples of 32 bytes whatever their extent: pieces that C ends in are not stored whole."""
+    import torch
+    from tcont_b200 import api
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    c = Contraction("ab", "ka", "kb", dict(a=rows, b=70, k=40), F64)
+    A, B = oracle.inputs(c, 37, -1.0, 1.0)
+    big = torch.full((70, 136), 7.0, dtype=torch.float64, device="cuda")
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    plan = api.plan_views(to_equation(engine, c, 1), parent_c=[136, 70])
+    u = plan.describe()["umma"]
+    assert plan.describe()["kernel"] == "dmma_f64_tma" and u["piece"] == (4 if rows % 4 == 0 else 2 if rows % 2 == 0 else 1), u
+    run = api.prepare_on_device(plan, dA.data_ptr(), dB.data_ptr(), big.data_ptr(), keep=(dA, dB, big))
+    engine.launch(run)
+    torch.cuda.synchronize()
+    hold(oracle, c, A, B, big[:, :rows].contiguous().cpu().numpy().reshape(-1), 40)
+    big[:, :rows] = 7.0
+    assert bool((big == 7.0).all()) and run.device_status() == 0
 
 
 # odd strides: both operands copied to matrices whose strides are even, rows in one run or several, contracted modes in A's order,
@@ -117,3 +149,7 @@ def test_padded_copies(engine, oracle, monkeypatch, name):
     for m, e in ext.items():
         k *= 1 if m in C else e
     hold(oracle, c, A, B, out, k, desc["umma"]["k_splits"])
+    C0 = np.random.default_rng(13).uniform(-4.0, 4.0, c.size(C))
+    _, (scaled,) = scaled_run(engine, c, A, B, C0, [(0.3, -0.7)], 2)
+    want, scale = 0.3 * oracle.contract(c, A, B) - 0.7 * C0, 0.3 * oracle.contract(c, np.abs(A), np.abs(B)) + 0.7 * np.abs(C0)
+    assert (np.abs(scaled - want) <= (k + desc["umma"]["k_splits"] + 4) * 2.0**-53 * scale).all()
