@@ -1034,14 +1034,24 @@ AcrossSpec plan_across(const Problem& p, const CostTable& c)
     // two stages at least beside the staged pieces of C
     const int stage_bytes = 16 * 128 * s.BK + s.BN * s.BK * 4;
     s.stages = std::min(8, (227 * 1024 - 2 * 1024 - 64 * 1024) / stage_bytes);
-    // A CTA passes a stage no faster than an SM takes it in, and a piece of 8 columns no faster than it is staged and stored.
+    // A CTA passes a stage no faster than an SM takes it in: 110 GB/s, less where A's rows do not start on 128-byte lines (C of 55 MB, x = 24,
+    // K 72: 34 us, 24 behind copies), less than half where they start in the middle of a 32-byte sector (C of 138 MB, x = 20, K 48:
+    // 72 us, 42 behind copies), unless few SMs ask for them.  And a piece of 8 columns no faster than it is staged and stored, by
+    // one bulk store or, with x > 16, by two.
+    int64_t together = 32;
+    for (int d = 1; d < kMaxTmaRank; ++d)
+        while (s.a.ext[d] > 1 && s.a.stride[d] % together != 0) together /= 2;
+    const double stage_gbs = together == 32 || s.tiles_m * s.tiles_n < c.num_sms ? 110.0 : together >= 8 ? 65.0 : 50.0;
     const double pieces = std::ceil(std::min<double>(double(n_ext), s.BN) / 8.0);
-    const double tile_us = std::max(double(s.k_iters) * double(stage_bytes) / 110e3, c.across_piece_us * pieces) + c.across_tile_us;
+    const double tile_us = std::max(double(s.k_iters) * double(stage_bytes) / (stage_gbs * 1e3), c.across_piece_us * (s.x_ext > 16 ? 1.0 : 0.8) * pieces) + c.across_tile_us;
     // Rows of y that are no multiple of 32 bytes end inside a sector, which is then read first (C of 188 MB with y = 28: 91 us, y = 32
-    // 33); a C in L2 does not mind.
-    const double c_bytes = 4.0 * double(p.sizeC), torn = mode(y).extent % 8 != 0 && c_bytes > 64e6 ? 3.0 : 1.0;
-    const double bytes = 4.0 * (double(p.sizeA) + double(p.sizeB)) + torn * c_bytes;
-    s.est_us = c.launch_us + std::max(double(ceil_div(s.tiles_m * s.tiles_n, c.num_sms)) * tile_us, bytes / (c.across_gbs * 1e3));
+    // 33); a C that stays in L2 minds less (26 MB, y = 20: 18.3 us, where whole rows would take 14; 10 MB 8.5), and a small one does
+    // not.  Rows that end in half of a chunk leave in 64 and 32 bytes (C of 151 MB, y = 24: 44.3 us, 37 by its bytes; of 106 MB 30.7 and 28).
+    const double c_bytes = 4.0 * double(p.sizeC);
+    const bool torn = mode(y).extent % 8 != 0, half = mode(y).extent % 16 == 8, beyond_l2 = c_bytes > 64e6;
+    const double bytes = 4.0 * (double(p.sizeA) + double(p.sizeB)) + (beyond_l2 ? torn ? 3.0 : half ? 1.25 : 1.0 : 1.0) * c_bytes;
+    const double us = std::max(double(ceil_div(s.tiles_m * s.tiles_n, c.num_sms)) * tile_us, bytes / (c.across_gbs * 1e3));
+    s.est_us = c.launch_us + us * (torn && !beyond_l2 && c_bytes > 16e6 ? mode(y).extent < 32 ? 1.5 : 1.15 : 1.0);
     s.on = true;
     return s;
 }
@@ -1300,6 +1310,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     Problem ttgt;
     UmmaSpec ttgt_umma;
     int ttgt_kernel = KERNEL_SIMT;
+    double ttgt_by_tiles_us = 1e300;   // with the permutations' tiles counted
     TransposeSpec tA, tB;
     pl.est_ttgt_us = 1e300;
     auto padded = [&](size_t candidate, bool is_a) -> const std::vector<int64_t>& {
@@ -1393,6 +1404,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         if (kernel == KERNEL_DMMA_F64_TMA && u.k_splits > 1) us += 0.12 * u.k_splits;
         if (us < 0.97 * pl.est_ttgt_us) {   // (an alternative has to be clearly better than the first)
             pl.est_ttgt_us = us;
+            ttgt_by_tiles_us = us - transposes_us(i, cost, false) + transposes_us(i, cost, true);
             ttgt = q;
             ttgt_umma = u;
             ttgt_kernel = kernel;
@@ -1408,16 +1420,18 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     if (across && fuse_rows && tf32 && direct_kernel == KERNEL_UMMA_TF32 && backend_selection != 2 && !(x3 && x3[0] == '1') && !std::getenv("TCONT_NO_ROWS_ACROSS_SLABS")) {
         pl.across = plan_across(direct, cost);
         const char* force = std::getenv("TCONT_ACROSS");   // tuning switch: 1 wherever it can run
-        if (pl.across.on && (pl.across.est_us < 0.97 * pl.est_direct_us || (force && force[0] == '1'))) pl.est_direct_us = pl.across.est_us;
+        // Clearly better than either (C of 524 MB, estimated at 112 us and at 113 behind a copy of A of 3 MB, takes 104 and 94).  The copy of a
+        // large A by its tiles: with short modes on both sides it takes far longer than its bytes (A of 126 MB, 16 x 32: 227 us in all, not 97).
+        const bool clear = pl.across.est_us < 0.97 * pl.est_direct_us && (backend_selection == 1 || !(tA.needed || tB.needed) || pl.across.est_us < 0.97 * ttgt_by_tiles_us);
+        if (pl.across.on && (clear || (force && force[0] == '1'))) pl.est_direct_us = pl.across.est_us;
         else pl.across.on = false;
     }
     bool use_ttgt;
     if (backend_selection == 1) use_ttgt = false;
     else if (backend_selection == 2) use_ttgt = true;
-    else use_ttgt = (tA.needed || tB.needed) && pl.est_ttgt_us < pl.est_direct_us;
+    else use_ttgt = !pl.across.on && (tA.needed || tB.needed) && pl.est_ttgt_us < pl.est_direct_us;
 
     if (use_ttgt) {
-        pl.across.on = false;
         pl.backend = 1;
         pl.prob = ttgt;
         pl.prob.swapped = direct.swapped;  // roles still map to the caller's operands as in `direct`

@@ -195,10 +195,10 @@ struct CostTable {
     double umma_stage_us = 0.45;
     // What one SM's epilogue stores per second (GB/s): a 128 x 256 fp32 tile takes 3.7 us to leave (cfg4).
     double umma_store_gbs_per_sm = 35.5;
-    // Tiles across two stride-1 modes (across_tf32.cu): a piece of 512 rows x 8 columns leaves a CTA in this, a tile of 512 rows
-    // takes the other beside; tensors move at this rate.  Fitted to 90 drawn contractions: the choice is the faster one of the two
-    // forms for 79 of them, within 8 % for 4.
-    double across_piece_us = 0.29;
+    // Tiles across two stride-1 modes (across_tf32.cu): a piece of 512 rows x 8 columns leaves a CTA in this (four fifths of it with
+    // one bulk store), a tile of 512 rows takes the other beside; tensors move at this rate.  Fitted, with the rules of plan_across, to
+    // 176 drawn contractions of 0.2 to 1000 MB timed in both forms: the choice is the faster one or within 5 % of it for all but two (1.11, 1.21).
+    double across_piece_us = 0.34;
     double across_tile_us = 0.05;
     double across_gbs = 4900.0;
     // The line between IEEE single precision and TF32 (see make_plan): which Float32 contractions give up precision for time

@@ -320,3 +320,22 @@ def test_scattered_rows_are_not_fetched_twice(engine, modes, ext):
     """33 to 64 columns: not in 32-column tiles where every element of A comes in a sector of its own."""
     d = describe(engine, Contraction(*modes, ext, F64), 1)
     assert d["kernel"] in ("simt", "dmma_f64") and (d["gather"]["t0"] > 0 or d["gather"]["tile"] != 1)
+
+
+def test_float32_tiles_across_stride_1_modes_are_taken_where_they_are_faster(engine):
+    """Measured in both forms (microseconds across / behind a copy of A or where A lies)."""
+    def across(eq, extents):
+        C, A, B = eq.split()
+        return "across" in describe(engine, Contraction(C, A, B, dict(zip(sorted(set(C + A + B)), extents)), F32))
+    assert across("abcde efbad cf", (48, 32, 24, 32, 48, 32))             # 107 / 311
+    assert across("abcd dbea ec", (72, 72, 48, 72, 72))                   # 39.5 / 100
+    assert across("abcd deca be", (96, 64, 96, 96, 32))                   # 65.9 / 139
+    assert across("abcdef gfbc dega", (16, 16, 16, 24, 24, 16, 24))       # 27.2 / 37.5
+    assert across("abcde efba cfd", (32, 52, 36, 60, 32, 8))              # 87.0 / 91.5
+    assert across("abc bda dc", (212, 256, 216, 4))                       # 16.8 / 29.9
+    # rows that end in half of a chunk, that end inside a sector, A's rows off their lines or sectors, estimates that are level
+    assert not across("abcdef dfga gebc", (24, 16, 16, 24, 16, 16, 24))   # 44.3 / 39.2
+    assert not across("abcde efba cfd", (20, 20, 20, 40, 20, 8))          # 18.3 / 16.4
+    assert not across("abcde efba cfd", (40, 28, 32, 16, 24, 72))         # 33.5 / 23.9
+    assert not across("abcdef dfga gebc", (16, 20, 12, 20, 28, 16, 48))   # 71.7 / 41.9
+    assert not across("abcde efba cfd", (40, 40, 32, 40, 64, 8))          # 104 / 94.3
