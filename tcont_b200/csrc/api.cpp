@@ -175,6 +175,11 @@ struct tcontb_run {
     double alpha = 1.0, beta = 0.0;
     bool scale_pass = false;
     DeviceBuffer scaled_ws;
+    // Tiles across two stride-1 modes: another form of the same contraction, on the same tensors and the same stream, that launches
+    // with other scalars use while `scaled_elsewhere` is set.  Built beside this one, which plain launches (and graphs that hold
+    // them) go on using.
+    std::unique_ptr<tcontb_run> scaled_form;
+    bool scaled_elsewhere = false;
     // stage timing
     bool stage_timing = false;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -268,6 +273,8 @@ struct tcontb_run {
         if (pipe.s_in) cudaStreamDestroy(pipe.s_in);
         if (pipe.s_out) cudaStreamDestroy(pipe.s_out);
     }
+    bool scaled() const { return alpha != 1.0 || beta != 0.0; }
+    int64_t kernels() const { return scaled_elsewhere ? scaled_form->kernels() : kernels_per_launch + (scaled() && scale_pass ? 1 : 0); }
     const void* roleA_src() const { return plan.prob.swapped ? dR : dL; }
     const void* roleB_src() const { return plan.prob.swapped ? dL : dR; }
 };
@@ -388,7 +395,7 @@ tcontb_status finish_across(tcontb_run* run, const void* A, const void* B)
     if (st == TCONTB_OK) st = encode_across_map(s.b, const_cast<void*>(B), s.b_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, &run->tmB);
     if (st == TCONTB_OK) st = encode_across_map(s.c, run->dC, CU_TENSOR_MAP_SWIZZLE_64B, &run->tmC);
     if (st != TCONTB_OK) return st;
-    // alpha and beta: the kernel writes a workspace, a second pass applies them (C of 226 MB: 258 us, 413 with the copy of A)
+    // alpha and beta: the kernel writes a workspace, a second pass applies them, where no other form is faster (see choose_scaled_form)
     run->scale_pass = true;
     if (across_tf32_smem(s.stages, s.BN, s.BK) > kMaxDynamicSmemBytes) return fail(TCONTB_RUNTIME_ERROR, "plan asks for more shared memory than a block can have");
     TC_CUDA(across_tf32_configure());
@@ -660,11 +667,67 @@ tcontb_status set_up_again(tcontb_run* run, const Plan& plan)
         e = nullptr;
     }
     run->ev_valid = false;
+    run->scaled_elsewhere = false;
+    run->scaled_form.reset();
     run->plan = plan;
     run->half_built = true;
     const tcontb_status st = finish_run(run);
     if (st == TCONTB_OK) run->half_built = false;
     return st;
+}
+
+// The workspace of a second pass over C, allocated once, so that launches stay free of allocations.
+tcontb_status provide_workspace(tcontb_run* run)
+{
+    if (run->scaled_ws.ptr) return TCONTB_OK;
+    TC_CUDA(run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt));
+    if (!run->plan.across.on) return TCONTB_OK;
+    const tcontb_status st = encode_across_map(run->plan.across.c, run->scaled_ws.ptr, CU_TENSOR_MAP_SWIZZLE_64B, &run->tmWs);
+    if (st != TCONTB_OK) TC_CUDA(run->scaled_ws.release());
+    return st;
+}
+
+tcontb_status provide_scaled_form(tcontb_run* run, const Plan& plan)
+{
+    if (run->scaled_form) return TCONTB_OK;
+    std::unique_ptr<tcontb_run> form(new tcontb_run());
+    form->plan = plan;
+    form->elt = run->elt;
+    form->dL = run->dL;
+    form->dR = run->dR;
+    form->dC = run->dC;
+    form->stream = run->stream;
+    const tcontb_status st = finish_run(form.get());
+    if (st == TCONTB_OK) run->scaled_form = std::move(form);
+    return st;
+}
+
+// How a run with tiles across two stride-1 modes applies other scalars than (1, 0): by a second pass, or in the form that its plan has
+// without such tiles, whose epilogue applies them.  A C that is much larger than A is faster in that form (plain / accumulating us:
+// C of 460 MB 87 / 401 across, 92 / 259 in the other form; of 151 MB 27 / 109 and 38 / 97), one that is not is slower (226 MB, A of
+// 302: 107 / 265 and 311 / 413).  It has to look a tenth better, which is how far the estimates are off.  Where there is no room for
+// the one, the other is taken; without room for either the run stays as it was.
+tcontb_status choose_scaled_form(tcontb_run* run, double beta)
+{
+    int current = 0;
+    TC_CUDA(cudaGetDevice(&current));
+    DeviceGuard guard(current, current != run->device);
+    if (guard.active) TC_CUDA(cudaSetDevice(run->device));
+    Plan other;
+    const bool planned = plan_without_across(run->plan, &other);
+    const int reads = beta != 0.0 ? 1 : 0;
+    const char* force = std::getenv("TCONT_ACROSS");
+    const bool elsewhere = planned && !(force && force[0] == '1') && other.est_scaled_us[reads] > 0 && other.est_scaled_us[reads] < 0.9 * run->plan.est_scaled_us[reads];
+    for (const bool form : {elsewhere, !elsewhere}) {
+        if (form && !planned) continue;
+        const tcontb_status st = form ? provide_scaled_form(run, other) : provide_workspace(run);
+        if (st == TCONTB_OK) {
+            run->scaled_elsewhere = form;
+            return TCONTB_OK;
+        }
+        cudaGetLastError();
+    }
+    return TCONTB_RUNTIME_ERROR;
 }
 
 tcontb_status alloc_owned(tcontb_run* run)
@@ -837,7 +900,7 @@ tcontb_status make_shards(tcontb_run* run, int gpus)
     }
     TC_CUDA(cudaSetDevice(run->first_device));
     run->kernels_per_launch = 0;
-    for (auto& sh : run->shards) run->kernels_per_launch += sh->kernels_per_launch;
+    for (auto& sh : run->shards) run->kernels_per_launch += sh->kernels();
     return TCONTB_OK;
 }
 
@@ -1087,6 +1150,7 @@ tcontb_status tcontb_run_set_stream(tcontb_run* run, void* cuda_stream)
     if (!run) return fail(TCONTB_INVALID_ARGUMENT, "ExecutionRun is empty");
     TC_NOT_SHARDED(run, "a caller stream");
     run->stream = static_cast<cudaStream_t>(cuda_stream);
+    if (run->scaled_form) run->scaled_form->stream = run->stream;
     for (auto& part : run->pipe.parts) part->stream = run->stream;
     return TCONTB_OK;
 }
@@ -1110,28 +1174,14 @@ tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta)
     TC_NOT_SHARDED(run, "alpha and beta");
     const bool scaled = alpha != 1.0 || beta != 0.0;
     if (scaled && run->plan.prob.c_strided) return fail(TCONTB_UNSUPPORTED, "alpha and beta are not available when C is a sub-tensor view");
-    if (run->scale_pass) {
-        // allocated here, once, so that launches stay free of allocations
-        if (scaled && !run->scaled_ws.ptr) {
-            const cudaError_t e = run->scaled_ws.alloc(static_cast<size_t>(run->plan.sizeC) * run->elt);
-            if (e == cudaErrorMemoryAllocation && run->plan.across.on) {   // no room for it: the form whose epilogue applies them
-                cudaGetLastError();
-                Plan plain;
-                if (!plan_without_across(run->plan, &plain)) return fail(TCONTB_RUNTIME_ERROR, "no other plan for this contraction");
-                const tcontb_status st = set_up_again(run, plain);
-                return st == TCONTB_OK ? tcontb_run_set_scalars(run, alpha, beta) : st;
-            }
-            TC_CUDA(e);
-            if (run->plan.across.on) {
-                const tcontb_status st = encode_across_map(run->plan.across.c, run->scaled_ws.ptr, CU_TENSOR_MAP_SWIZZLE_64B, &run->tmWs);
-                if (st != TCONTB_OK) {
-                    TC_CUDA(run->scaled_ws.release());
-                    return st;
-                }
-            }
-        }
-        const bool was = run->alpha != 1.0 || run->beta != 0.0;
-        run->kernels_per_launch += (scaled ? 1 : 0) - (was ? 1 : 0);
+    if (scaled && run->scale_pass) {
+        const tcontb_status st = run->plan.across.on ? choose_scaled_form(run, beta) : provide_workspace(run);
+        if (st != TCONTB_OK) return st;
+    }
+    if (!scaled) run->scaled_elsewhere = false;
+    if (run->scaled_elsewhere) {
+        const tcontb_status st = tcontb_run_set_scalars(run->scaled_form.get(), alpha, beta);
+        if (st != TCONTB_OK) return st;
     }
     run->alpha = alpha;
     run->beta = beta;
@@ -1180,10 +1230,11 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         return TCONTB_OK;
     }
     if (run->half_built) return fail(TCONTB_RUNTIME_ERROR, "the run's set-up failed");
+    if (run->scaled_elsewhere) return tcontb_run_launch(run->scaled_form.get());
     const Plan& pl = run->plan;
     const bool t = run->stage_timing;
     // Other scalars than (1, 0): the contraction kernel's epilogue applies them, or the partial-sum pass of a split-K run
-    const bool scaled = run->alpha != 1.0 || run->beta != 0.0;
+    const bool scaled = run->scaled();
     UmmaParams umma = run->umma;
     const bool redirect = scaled && run->scale_pass;
     if (redirect) umma.C64 = static_cast<double*>(run->scaled_ws.ptr);
@@ -1289,6 +1340,7 @@ tcontb_status tcontb_run_stage_times(tcontb_run* run, float out[6])
     if (!run || !out) return fail(TCONTB_INVALID_ARGUMENT, "ExecutionRun is empty");
     for (int i = 0; i < 6; ++i) out[i] = 0.0f;
     if (!run->shards.empty()) return tcontb_run_stage_times(run->shards[0].get(), out);  // the first device's stages
+    if (run->scaled_elsewhere) return tcontb_run_stage_times(run->scaled_form.get(), out);
     if (!run->stage_timing || !run->ev_valid) return TCONTB_OK;
     TC_CUDA(cudaEventSynchronize(run->ev[3]));
     float ta = 0, tb = 0, tc = 0;
@@ -1370,7 +1422,7 @@ tcontb_status tcontb_run_time_launches(tcontb_run* run, int iterations, float* e
     cudaEventDestroy(e1);
     if (st != TCONTB_OK) return st;
     if (ce != cudaSuccess) return fail(TCONTB_RUNTIME_ERROR, std::string("CUDA error while timing launches: ") + cudaGetErrorString(ce));
-    if (kernel_launches) *kernel_launches = run->kernels_per_launch * iterations;
+    if (kernel_launches) *kernel_launches = run->kernels() * iterations;
     return TCONTB_OK;
 }
 
@@ -1457,6 +1509,12 @@ tcontb_status tcontb_run_device_status(tcontb_run* run, int* status)
     }
     TC_CUDA(cudaMemcpyAsync(status, run->status.ptr, sizeof(int), cudaMemcpyDeviceToHost, run->stream));
     TC_CUDA(cudaStreamSynchronize(run->stream));
+    if (run->scaled_form) {
+        int s1 = 0;
+        const tcontb_status st = tcontb_run_device_status(run->scaled_form.get(), &s1);
+        if (st != TCONTB_OK) return st;
+        if (s1 > *status) *status = s1;
+    }
     for (auto& part : run->pipe.parts) {
         int s1 = 0;
         const tcontb_status st = tcontb_run_device_status(part.get(), &s1);

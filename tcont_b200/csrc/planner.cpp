@@ -1056,6 +1056,18 @@ AcrossSpec plan_across(const Problem& p, const CostTable& c)
     return s;
 }
 
+// What alpha and beta add to a Float32 contraction on the tensor cores (microseconds), `reads` = beta is not zero.  Tiles across two
+// stride-1 modes go to a workspace that a second pass reads, with C, and writes C from: C three times or twice more.  The other
+// form's epilogue reads C as it stores it, slower than its plain stores in either case; rows stored element by element are read that
+// way, too.  Read off 176 contractions (C of 0.2 to 1000 MB) in both forms: C of 460 MB 314 us more across (226 without the old values),
+// 167 (72) in the other form, of 75 MB 37 (24) and 24 (11), of 25 MB 10 (9) and 12 (7), of 1.8 MB 2.8 and, element by element, 16.
+double scalars_us(bool across, double c_bytes, double scattered_us, bool reads)
+{
+    const double mb = c_bytes * 1e-6;
+    if (across) return 2.3 + (reads ? 3.0 : 2.0) * mb / (mb > 67.2 ? 4.85 : mb > 48.0 ? 6.4 : 8.0);
+    return (reads ? 1.5 + mb / 3.3 + 1.5 * scattered_us : 0.5 + 0.155 * mb + 0.6 * scattered_us) + (scattered_us > 0 ? 1.0 : 0.0);
+}
+
 // TF32 goes to the tcgen05 kernel whenever its tiles can be described to TMA.  FP64 takes the cheaper of the TMA-fed kernel
 // and the gather kernel, by the cost table; Float32 that TMA cannot describe goes to the gather kernel.  The gather kernel
 // is reported as KERNEL_DMMA_F64 where FP64 work fills the GPU with tiles, as KERNEL_SIMT otherwise.
@@ -1446,6 +1458,10 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         pl.umma = direct_umma;
     }
     const Problem& p = pl.prob;
+    if (pl.kernel == KERNEL_UMMA_TF32)
+        for (int reads = 0; reads < 2; ++reads)
+            pl.est_scaled_us[reads] = (use_ttgt ? ttgt_by_tiles_us : pl.est_direct_us) +
+                                      scalars_us(pl.across.on, double(p.sizeC) * elt, !pl.across.on && pl.umma.a.row_elem_cstride != 1 ? double(p.sizeC) * cost.scatter_store_f32_ps * 1e-6 : 0.0, reads != 0);
     auto first_is = [&](const std::vector<int>& t, const std::vector<int>& grp) {
         return !t.empty() && !grp.empty() && t[0] == grp[0];
     };

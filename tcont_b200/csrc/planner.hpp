@@ -227,6 +227,7 @@ struct Plan {
     UmmaSpec umma;
     AcrossSpec across;      // KERNEL_UMMA_TF32: this form of it runs when `on`
     double est_direct_us = 0, est_ttgt_us = 0;
+    double est_scaled_us[2] = {0, 0};   // Float32 on the tensor cores: with other alpha and beta than (1, 0), beta zero or not
     double flops = 0;
     int64_t sizeL = 1, sizeR = 1, sizeC = 1;  // caller's left, right, output element counts
 };

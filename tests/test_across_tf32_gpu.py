@@ -103,3 +103,66 @@ def test_error_compensated_keeps_its_form(engine, oracle, monkeypatch):
     engine.launch(run)
     diff, nonfinite = oracle.compare(oracle.contract(c, A, B, rounding=0), engine.copy_output_to_host(run), F32)
     assert diff == 0 and nonfinite == 0
+
+
+def big(engine, oracle, ext):
+    """A contraction the planner takes this form for by itself, a run of it on device tensors and 20 000 elements of its product."""
+    import torch
+    from tcont_b200 import api
+    c = Contraction("abcde", "efba", "cfd", ext, F32)
+    A, B = oracle.inputs(c, 47, -1.0, 1.0)
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    dC = torch.zeros(c.size("abcde"), device="cuda")
+    plan = engine.plan(to_equation(engine, c, 0))
+    assert "across" in plan.describe()
+    run = api.prepare_on_device(plan, dA.data_ptr(), dB.data_ptr(), dC.data_ptr(), keep=(dA, dB, dC))
+    at = np.sort(np.random.default_rng(5).integers(0, dC.numel(), 20000))
+    product, scale = (oracle.contract_sampled(c, a, b, at, rounding=1) for a, b in ((A, B), (np.abs(A), np.abs(B))))
+
+    def held(alpha, beta, old):
+        got = dC.cpu().numpy()[at]
+        want = alpha * product + beta * old
+        return bool((np.abs(got - want) <= 2e-5 * abs(alpha) * scale + 4 * 2.0**-24 * (np.abs(alpha * product) + np.abs(beta * old))).all())
+    return run, dC, held
+
+
+# a C 40 times the size of A is accumulated into by the form that applies scalars in its epilogue (copies of both operands in front of
+# it), one of A's size by a second pass over a workspace; kernels of a plain launch, of an accumulating one
+@pytest.mark.parametrize("ext,kernels", [(dict(a=32, b=24, c=40, d=32, e=40, f=16), 3), (dict(a=64, b=8, c=8, d=4, e=64, f=32), 2)])
+def test_form_of_accumulating_launches(engine, oracle, ext, kernels):
+    """Chosen when the scalars are set, beside the plain form: a graph that holds a plain launch stays what it is."""
+    import torch
+    run, dC, held = big(engine, oracle, ext)
+    stream = torch.cuda.Stream()
+    run.set_stream(stream.cuda_stream)
+    with torch.cuda.stream(stream):
+        engine.launch(run)
+        stream.synchronize()
+        assert held(1.0, 0.0, 0.0) and run.time_launches(1)[1] == 1
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            engine.launch(run)
+        for alpha, beta in ((0.3, -0.7), (-2.0, 0.0), (1.0, 1.0)):
+            dC.fill_(3.0)
+            run.set_scalars(alpha, beta)
+            engine.launch(run)
+            stream.synchronize()
+            assert held(alpha, beta, 3.0), (alpha, beta)
+        assert run.time_launches(1)[1] == kernels
+        dC.fill_(3.0)
+        graph.replay()
+        stream.synchronize()
+        assert held(1.0, 0.0, 0.0)
+        run.set_scalars(1.0, 0.0)
+        dC.fill_(3.0)
+        engine.launch(run)
+        stream.synchronize()
+        assert held(1.0, 0.0, 0.0) and run.time_launches(1)[1] == 1 and run.device_status() == 0
+    other = torch.cuda.Stream()
+    run.set_scalars(2.0, 1.0)
+    run.set_stream(other.cuda_stream)   # (the other form follows the run's stream)
+    with torch.cuda.stream(other):
+        dC.fill_(3.0)
+        engine.launch(run)
+        other.synchronize()
+    assert held(2.0, 1.0, 3.0) and run.device_status() == 0
