@@ -109,11 +109,14 @@ tcontb_status tcontb_run_upload_inputs(tcontb_run* run, const void* a_host, cons
 
 /* Beyond the reference, whose backends always overwrite (alpha = 1, beta = 0: cublasGemmEx scalars at
  * backends/ttgt_cutt/src/ttgt_cutt.cpp:742-743, generated kernels store a zeroed accumulator): later
- * launches compute C = alpha * (A*B) + beta * C.  The kernel that writes C applies the scalars, or
- * the partial-sum pass where k is split and for some FP64 runs with a C of up to 64 MB (whose
- * workspace of the size of C this call allocates); C is read only when beta is not zero.  Not
- * available on a
- * run that spans several GPUs. */
+ * launches compute C = alpha * (A*B) + beta * C; C is read only when beta is not zero.  The kernel that
+ * writes C applies the scalars, or the partial-sum pass where k is split.  For some FP64 runs (rows of C
+ * across A's, few k chunks) and for Float32 runs whose A and C have different stride-1 modes, the first
+ * call with other scalars than (1, 0) sets up what its launches need: a workspace of the size of C, or a
+ * second form of the contraction with its scratch copies of the operands, whichever is faster.  It is
+ * kept with the run; plain launches, and graphs that hold them, are not touched by it.  Such a call
+ * allocates and must not be made while a stream is captured.  An error leaves the run as it was.  Not
+ * available on a run that spans several GPUs or when C is a view. */
 tcontb_status tcontb_run_set_scalars(tcontb_run* run, double alpha, double beta);
 
 /* TconT::launch (src/tcont.cpp:102-108): one contraction, asynchronous. */

@@ -705,8 +705,9 @@ tcontb_status provide_scaled_form(tcontb_run* run, const Plan& plan)
 // How a run with tiles across two stride-1 modes applies other scalars than (1, 0): by a second pass, or in the form that its plan has
 // without such tiles, whose epilogue applies them.  A C that is much larger than A is faster in that form (plain / accumulating us:
 // C of 460 MB 87 / 401 across, 92 / 259 in the other form; of 151 MB 27 / 109 and 38 / 97), one that is not is slower (226 MB, A of
-// 302: 107 / 265 and 311 / 413).  It has to look a tenth better, which is how far the estimates are off.  Where there is no room for
-// the one, the other is taken; without room for either the run stays as it was.
+// 302: 107 / 265 and 311 / 413): copying A costs what the second pass does.  It has to look a tenth better, which is how far the
+// estimates are off: of 176 contractions two accumulate more than 7 % slower than in the better form (1.08, 1.18).  Where there is no
+// room for the one, the other is taken; without room for either the run stays as it was.
 tcontb_status choose_scaled_form(tcontb_run* run, double beta)
 {
     int current = 0;
@@ -717,7 +718,7 @@ tcontb_status choose_scaled_form(tcontb_run* run, double beta)
     const bool planned = plan_without_across(run->plan, &other);
     const int reads = beta != 0.0 ? 1 : 0;
     const char* force = std::getenv("TCONT_ACROSS");
-    const bool elsewhere = planned && !(force && force[0] == '1') && other.est_scaled_us[reads] > 0 && other.est_scaled_us[reads] < 0.9 * run->plan.est_scaled_us[reads];
+    const bool elsewhere = planned && !(force && force[0] == '1') && run->plan.sizeC > 2 * run->plan.prob.sizeA && other.est_scaled_us[reads] > 0 && other.est_scaled_us[reads] < 0.9 * run->plan.est_scaled_us[reads];
     for (const bool form : {elsewhere, !elsewhere}) {
         if (form && !planned) continue;
         const tcontb_status st = form ? provide_scaled_form(run, other) : provide_workspace(run);
