@@ -110,7 +110,13 @@ struct DeviceBuffer {
     {
         if (ptr) cudaFree(ptr);
     }
-    cudaError_t alloc(size_t bytes) { return cudaMalloc(&ptr, bytes ? bytes : 1); }
+    cudaError_t alloc(size_t bytes)
+    {
+        // Test hook: buffers of so many bytes or more find no room.
+        const char* no_room = std::getenv("TCONT_TEST_NO_ROOM");
+        if (no_room && bytes >= std::strtoull(no_room, nullptr, 10)) return cudaErrorMemoryAllocation;
+        return cudaMalloc(&ptr, bytes ? bytes : 1);
+    }
     cudaError_t release()
     {
         const cudaError_t e = ptr ? cudaFree(ptr) : cudaSuccess;
@@ -180,6 +186,7 @@ struct tcontb_run {
     // them) go on using.
     std::unique_ptr<tcontb_run> scaled_form;
     bool scaled_elsewhere = false;
+    bool keep_copies = false;  // set-up: no room for scratch copies of the operands is an error
     // stage timing
     bool stage_timing = false;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -470,14 +477,16 @@ bool plan_without_across(const Plan& d, Plan* out, int selection = -1)
 
 tcontb_status finish_run(tcontb_run* run);
 
-// The run without scratch copies of its operands.
+// The run without scratch copies of its operands.  Not where that would take Float32 from TF32 to IEEE single precision or back:
+// how much memory is free does not decide the precision.
 tcontb_status finish_where_they_lie(tcontb_run* run)
 {
     cudaGetLastError();
     TC_CUDA(run->tbufA.release());
     TC_CUDA(run->tbufB.release());
     Plan plain;
-    if (!plan_without_across(run->plan, &plain, 1)) return fail(TCONTB_RUNTIME_ERROR, "no other plan for this contraction");
+    if (!plan_without_across(run->plan, &plain, 1) || (plain.kernel == KERNEL_UMMA_TF32) != (run->plan.kernel == KERNEL_UMMA_TF32))
+        return fail(TCONTB_RUNTIME_ERROR, "no room for the scratch copies of the operands, and no other plan for this contraction");
     run->plan = plain;
     return finish_run(run);
 }
@@ -503,15 +512,15 @@ tcontb_status finish_run(tcontb_run* run)
     TC_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, run->device));
     if (major != 10) return fail(TCONTB_RUNTIME_ERROR, "this library holds sm_100a kernels only; the current device is not a B200-class GPU");
 
-    // Scratch copies: where there is no room for them and the caller left the route open, the operands are used where they lie.
+    // Scratch copies: where there is no room for them and the caller left the route open, the operands are used where they lie if they can be.
     if (pl.tA.needed && !run->borrowed_tA) {
         const cudaError_t e = run->tbufA.alloc(static_cast<size_t>(pl.tA.dst_elements) * run->elt);
-        if (e == cudaErrorMemoryAllocation && pl.backend_selection == 0) return finish_where_they_lie(run);
+        if (e == cudaErrorMemoryAllocation && pl.backend_selection == 0 && !run->keep_copies) return finish_where_they_lie(run);
         TC_CUDA(e);
     }
     if (pl.tB.needed && !run->borrowed_tB) {
         const cudaError_t e = run->tbufB.alloc(static_cast<size_t>(pl.tB.dst_elements) * run->elt);
-        if (e == cudaErrorMemoryAllocation && pl.backend_selection == 0) return finish_where_they_lie(run);
+        if (e == cudaErrorMemoryAllocation && pl.backend_selection == 0 && !run->keep_copies) return finish_where_they_lie(run);
         TC_CUDA(e);
     }
     const void* kA = run->roleA_src();
@@ -687,11 +696,12 @@ tcontb_status provide_workspace(tcontb_run* run)
     return st;
 }
 
-tcontb_status provide_scaled_form(tcontb_run* run, const Plan& plan)
+tcontb_status provide_scaled_form(tcontb_run* run, const Plan& plan, bool with_copies)
 {
     if (run->scaled_form) return TCONTB_OK;
     std::unique_ptr<tcontb_run> form(new tcontb_run());
     form->plan = plan;
+    form->keep_copies = with_copies;
     form->elt = run->elt;
     form->dL = run->dL;
     form->dR = run->dR;
@@ -707,7 +717,7 @@ tcontb_status provide_scaled_form(tcontb_run* run, const Plan& plan)
 // C of 460 MB 87 / 401 across, 92 / 259 in the other form; of 151 MB 27 / 109 and 38 / 97), one that is not is slower (226 MB, A of
 // 302: 107 / 265 and 311 / 413): copying A costs what the second pass does.  It has to look a tenth better, which is how far the
 // estimates are off: of 176 contractions two accumulate more than 7 % slower than in the better form (1.08, 1.18).  Where there is no
-// room for the one, the other is taken; without room for either the run stays as it was.
+// room for the one, the other is taken, then the form on the operands as they lie; without room for any the run stays as it was.
 tcontb_status choose_scaled_form(tcontb_run* run, double beta)
 {
     int current = 0;
@@ -719,11 +729,12 @@ tcontb_status choose_scaled_form(tcontb_run* run, double beta)
     const int reads = beta != 0.0 ? 1 : 0;
     const char* force = std::getenv("TCONT_ACROSS");
     const bool elsewhere = planned && !(force && force[0] == '1') && run->plan.sizeC > 2 * run->plan.prob.sizeA && other.est_scaled_us[reads] > 0 && other.est_scaled_us[reads] < 0.9 * run->plan.est_scaled_us[reads];
-    for (const bool form : {elsewhere, !elsewhere}) {
-        if (form && !planned) continue;
-        const tcontb_status st = form ? provide_scaled_form(run, other) : provide_workspace(run);
+    const bool attempts[3] = {elsewhere, !elsewhere, true};
+    for (int i = 0; i < 3; ++i) {
+        if (attempts[i] && !planned) continue;
+        const tcontb_status st = attempts[i] ? provide_scaled_form(run, other, i < 2) : provide_workspace(run);
         if (st == TCONTB_OK) {
-            run->scaled_elsewhere = form;
+            run->scaled_elsewhere = attempts[i];
             return TCONTB_OK;
         }
         cudaGetLastError();
