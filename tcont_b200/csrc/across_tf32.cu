@@ -18,7 +18,7 @@
 // here, 5.0 TB/s), for short contracted extents C leaving in pieces of 64 bytes (24 x 32 x 24 x 24 x 32 by 8, 57 MB: 22 -> 13.5 us),
 // for the smallest the way through one tile (16 x 8 x 8 x 8 x 16 by 8: 7.4 -> 4.5 us).  A first form without warp 6, its epilogue
 // working out every tile's coordinates, took 2.0 us a tile beside the pieces (109 and 29.7 us).
-// Every wait is bounded as in umma_tf32.cu.
+// Every wait is bounded as in umma_tf32.cu, with the same test hooks.
 //
 // Stands where the reference runs its generated TF32 WMMA kernels (backends/cogent/plan/generators/kernels/kernel_store.py:280-507).
 #include <cuda.h>
@@ -95,6 +95,7 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
     uint64_t* bar_free = bar_staged + kBuffers;             // [kBuffers]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_free + kBuffers);
     const uint32_t abort_flag = smem_u32(tmem_slot + 1);
+    const uint32_t bar_drain = smem_u32(tmem_slot + 2);
     const uint32_t tmem_cols = static_cast<uint32_t>(8 * p.BN);   // two sets of four accumulators: 256 or 512
 
     if (threadIdx.x == 0) {
@@ -110,6 +111,7 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
             mbar_init(smem_u32(bar_staged + b), 128);
             mbar_init(smem_u32(bar_free + b), 1);
         }
+        mbar_init(bar_drain, 1);
         st_shared_u32(abort_flag, 0u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -124,6 +126,7 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    auto wait = [&](uint32_t bar, uint32_t parity) { return mbar_wait(bar, parity, abort_flag, 0, p.wait_limit_ns); };
     // columns of a tile that lie inside C
     auto columns_of = [&](uint32_t unit) {
         uint32_t tn = fast_div(unit, p.inner);
@@ -138,15 +141,15 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
             asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmapA)) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmapB)) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmapC)) : "memory");
-            int stage = 0;
+            int stage = 0, cta_iter = 0;
             uint32_t phase = 0, issued_mask = 0, issued_parity = 0;
             const int b_copies = p.b_major ? p.BN / 32 : 1;
             TileIndex next = tile_index(blockIdx.x, p);
             for (uint32_t unit = blockIdx.x; unit < p.units; unit += gridDim.x) {
                 const TileIndex t = next;
                 int k0 = 0, k1 = 0, k2 = 0;
-                for (int it = 0; it < p.k_iters; ++it) {
-                    if (mbar_wait(smem_u32(bar_empty + stage), phase ^ 1u, abort_flag)) {
+                for (int it = 0; it < p.k_iters; ++it, ++cta_iter) {
+                    if (wait(smem_u32(bar_empty + stage), phase ^ 1u) && cta_iter != p.test_skip_iter) {
                         const uint32_t bar = smem_u32(bar_full + stage), dst = smem_u32(smem) + static_cast<uint32_t>(stage) * stage_bytes;
                         mbar_arrive_expect_tx(bar, stage_bytes);
                         tma_load_5d(dst, &tmapA, bar, t.x, k0, t.y, p.row_others > 0 ? t.o0 : k1, p.row_others > 1 ? t.o1 : p.row_others == 1 ? k1 : k2);
@@ -188,11 +191,11 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
             uint32_t phase = 0, tile = 0;
             for (uint32_t unit = blockIdx.x; unit < p.units; unit += gridDim.x, ++tile) {
                 const uint32_t acc = tile & 1u;
-                bool ok = mbar_wait(smem_u32(bar_tempty + acc), ((tile >> 1) & 1u) ^ 1u, abort_flag);
+                bool ok = wait(smem_u32(bar_tempty + acc), ((tile >> 1) & 1u) ^ 1u);
                 tcgen05_fence_after();
                 const uint32_t tmem_c = tmem_base + acc * 4u * static_cast<uint32_t>(p.BN);
                 for (int it = 0; it < p.k_iters; ++it) {
-                    ok = ok && mbar_wait(smem_u32(bar_full + stage), phase, abort_flag);
+                    ok = ok && wait(smem_u32(bar_full + stage), phase);
                     if (ok) {
                         tcgen05_fence_after();
                         const uint32_t a = smem_u32(smem) + static_cast<uint32_t>(stage) * stage_bytes, b = a + a_bytes;
@@ -212,6 +215,10 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
                 }
                 if (ok) umma_commit(smem_u32(bar_tfull + acc));
             }
+            if (ld_shared_u32(abort_flag)) {   // MMAs of stages that did arrive may be running: they end before tensor memory is given back
+                umma_commit(bar_drain);
+                drain_copies(bar_drain, 1, 1u, 0u);
+            }
         }
         __syncwarp();
     } else if (warp < 6) {
@@ -221,7 +228,7 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
         for (uint32_t unit = blockIdx.x; unit < p.units; unit += gridDim.x, ++tile) {
             const uint32_t acc = tile & 1u;
             const int columns = columns_of(unit);
-            bool ok = mbar_wait(smem_u32(bar_tfull + acc), (tile >> 1) & 1u, abort_flag);
+            bool ok = wait(smem_u32(bar_tfull + acc), (tile >> 1) & 1u);
             ok = __all_sync(0xffffffffu, ok);
             tcgen05_fence_after();
             const uint32_t taddr = tmem_base + (q << 21) + acc * 4u * static_cast<uint32_t>(p.BN);   // (lane 32 q in bits 16 and up)
@@ -229,7 +236,7 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
                 uint32_t v[4][8];
 #pragma unroll
                 for (uint32_t g = 0; g < 4; ++g) tmem_ld_32x8(taddr + g * static_cast<uint32_t>(p.BN) + static_cast<uint32_t>(j0), v[g]);
-                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar_free + buffer), (round & 1u) ^ 1u, abort_flag)) && ok;
+                ok = __all_sync(0xffffffffu, wait(smem_u32(bar_free + buffer), (round & 1u) ^ 1u)) && ok;
                 tmem_ld_wait();
                 if (j0 + 8 >= columns) {   // all of the tile is in registers
                     tcgen05_fence_before();
@@ -257,7 +264,7 @@ across_tf32_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_const
                 const int columns = columns_of(unit);
                 const int c3 = p.row_others > 0 ? t.o0 : t.p0, c4 = p.row_others > 1 ? t.o1 : p.row_others == 1 ? t.p0 : t.p1;
                 for (int j0 = 0; j0 < columns; j0 += 8) {
-                    if (mbar_wait(smem_u32(bar_staged + buffer), round & 1u, abort_flag)) {
+                    if (wait(smem_u32(bar_staged + buffer), round & 1u) && !ld_shared_u32(abort_flag)) {   // (a piece that was not staged is not stored)
                         const uint32_t from = buffers + buffer * kBufferBytes;
                         tma_store_5d(&tmapC, from, t.y, t.x, t.n + j0, c3, c4);
                         if (t.x + 16 < p.x_ext) tma_store_5d(&tmapC, from + kHalfBytes, t.y, t.x + 16, t.n + j0, c3, c4);

@@ -352,6 +352,15 @@ tcontb_status encode_map(const UmmaOperand& o, const void* base, int elt, CUtens
     return TCONTB_OK;
 }
 
+// Test hooks of the bounded-wait exit (tcgen05 kernels only; see UmmaParams).
+void set_test_hooks(unsigned long long* wait_limit_ns, int* skip_iter)
+{
+    const char* limit = std::getenv("TCONT_TEST_WAIT_LIMIT_NS");
+    const char* skip = std::getenv("TCONT_TEST_SKIP_STAGE");
+    *wait_limit_ns = limit ? std::strtoull(limit, nullptr, 10) : 0;
+    *skip_iter = skip ? std::atoi(skip) : -1;
+}
+
 // A tensor map of the across_tf32 kernel.
 tcontb_status encode_across_map(const AcrossSpec::Map& m, void* base, CUtensorMapSwizzle swizzle, CUtensorMap* out)
 {
@@ -398,6 +407,7 @@ tcontb_status finish_across(tcontb_run* run, const void* A, const void* B)
     p.x_ext = static_cast<int>(s.x_ext);
     p.release_late = p.units >= 16u * static_cast<uint32_t>(run->num_sms) && s.k_iters <= 4 ? 1 : 0;
     p.status = static_cast<int*>(run->status.ptr);
+    set_test_hooks(&p.wait_limit_ns, &p.test_skip_iter);
     tcontb_status st = encode_across_map(s.a, const_cast<void*>(A), CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, &run->tmA);
     if (st == TCONTB_OK) st = encode_across_map(s.b, const_cast<void*>(B), s.b_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, &run->tmB);
     if (st == TCONTB_OK) st = encode_across_map(s.c, run->dC, CU_TENSOR_MAP_SWIZZLE_64B, &run->tmC);
@@ -605,11 +615,7 @@ tcontb_status finish_run(tcontb_run* run)
         run->umma.C64 = static_cast<double*>(out);
         run->umma.status = static_cast<int*>(run->status.ptr);
         run->umma.prof = nullptr;
-        run->umma.wait_limit_ns = 0;
-        run->umma.test_skip_iter = -1;
-        // Test hooks of the bounded-wait exit (tcgen05 kernel only; see UmmaParams).
-        if (const char* e = std::getenv("TCONT_TEST_WAIT_LIMIT_NS")) run->umma.wait_limit_ns = std::strtoull(e, nullptr, 10);
-        if (const char* e = std::getenv("TCONT_TEST_SKIP_STAGE")) run->umma.test_skip_iter = std::atoi(e);
+        set_test_hooks(&run->umma.wait_limit_ns, &run->umma.test_skip_iter);
         if (const char* pe = std::getenv("TCONT_UMMA_PROF")) {
             if (pe[0] == '1') {
                 TC_CUDA(run->prof.alloc(static_cast<size_t>(run->num_sms) * 8 * sizeof(long long)));

@@ -217,6 +217,8 @@ struct AcrossParams {
     int b_major;            // 1: B's stride-1 mode is the column mode, 0: the chunked contracted mode
     int n_ext, x_ext;       // extents of the column mode and of A's stride-1 mode
     int release_late;       // see UmmaParams
+    unsigned long long wait_limit_ns;   // see UmmaParams
+    int test_skip_iter;
     int* status;
 };
 cudaError_t across_tf32_configure();  // once per device before the first launch

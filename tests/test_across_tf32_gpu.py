@@ -105,6 +105,39 @@ def test_error_compensated_keeps_its_form(engine, oracle, monkeypatch):
     assert diff == 0 and nonfinite == 0
 
 
+def test_bounded_wait_gives_up_cleanly(engine, oracle, monkeypatch):
+    """One stage of every CTA is neither announced nor filled: the waits behind it run out, the run's status says so, nothing outside
+    C is written, and the next run is right."""
+    import torch
+    from tcont_b200 import api
+    monkeypatch.setenv("TCONT_ACROSS", "1")
+    c = Contraction("abcd", "dbea", "ec", dict(a=64, b=24, c=20, d=160, e=36), F32)
+    A, B = oracle.inputs(c, 9, -1.0, 1.0)
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    n = c.size("abcd")
+    guarded = torch.full((n + 64,), 7.0, device="cuda")
+    plan = engine.plan(to_equation(engine, c, 1))
+    assert plan.describe()["across"]["k_iters"] == 2
+
+    def run():
+        return api.prepare_on_device(plan, dA.data_ptr(), dB.data_ptr(), guarded[32:].data_ptr(), keep=(dA, dB, guarded))
+    monkeypatch.setenv("TCONT_TEST_WAIT_LIMIT_NS", "2000000")
+    monkeypatch.setenv("TCONT_TEST_SKIP_STAGE", "3")   # the second tile's second k iteration
+    broken = run()
+    monkeypatch.delenv("TCONT_TEST_WAIT_LIMIT_NS")
+    monkeypatch.delenv("TCONT_TEST_SKIP_STAGE")
+    engine.launch(broken)
+    torch.cuda.synchronize()
+    assert broken.device_status() == 1
+    assert bool((torch.cat([guarded[:32], guarded[32 + n:]]) == 7.0).all())
+    del broken
+    good = run()
+    engine.launch(good)
+    torch.cuda.synchronize()
+    assert good.device_status() == 0
+    check(oracle, c, A, B, guarded[32:32 + n].cpu().numpy(), plan.describe())
+
+
 def big(engine, oracle, ext):
     """A contraction the planner takes this form for by itself, a run of it on device tensors and 20 000 elements of its product."""
     import torch
