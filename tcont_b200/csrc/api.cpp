@@ -509,10 +509,10 @@ tcontb_status finish_run(tcontb_run* run)
     TC_CUDA(cudaGetDevice(&run->device));
     TC_CUDA(cudaDeviceGetAttribute(&run->num_sms, cudaDevAttrMultiProcessorCount, run->device));
     if (pl.across.on) {
-        // What that kernel does not do: a C that bulk stores cannot address (the parts of a pass may start anywhere in one), and
-        // error compensation, when it is asked for after planning.
+        // That kernel has no error compensation, when it is asked for after planning.  (Bulk stores address C: every buffer, and every
+        // part of one that a pass writes, starts on a multiple of 16 bytes.)
         const char* x3 = std::getenv("TCONT_TF32X3");
-        if (reinterpret_cast<uintptr_t>(run->dC) % 16 || (x3 && x3[0] == '1')) {
+        if (x3 && x3[0] == '1') {
             Plan plain;
             if (!plan_without_across(pl, &plain)) return fail(TCONTB_RUNTIME_ERROR, "no other plan for this contraction");
             run->plan = plain;

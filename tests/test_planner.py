@@ -326,7 +326,9 @@ def test_float32_tiles_across_stride_1_modes_are_taken_where_they_are_faster(eng
     """Measured in both forms (microseconds across / behind a copy of A or where A lies)."""
     def across(eq, extents):
         C, A, B = eq.split()
-        return "across" in describe(engine, Contraction(C, A, B, dict(zip(sorted(set(C + A + B)), extents)), F32))
+        d = describe(engine, Contraction(C, A, B, dict(zip(sorted(set(C + A + B)), extents)), F32))
+        assert d["umma"]["in_use"] == ("across" not in d)
+        return "across" in d
     assert across("abcde efbad cf", (48, 32, 24, 32, 48, 32))             # 107 / 311
     assert across("abcd dbea ec", (72, 72, 48, 72, 72))                   # 39.5 / 100
     assert across("abcd deca be", (96, 64, 96, 96, 32))                   # 65.9 / 139
