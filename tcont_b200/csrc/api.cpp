@@ -604,10 +604,10 @@ tcontb_status finish_run(tcontb_run* run)
             run->kernels_per_launch += 4;  // two residual passes, two more contractions
         }
         // Tiles across slabs read the old values of C in pieces of 32 bytes: with a C of up to half of L2, or few k chunks, and k
-        // chunks of 16, the TMA-fed FP64 kernel writes a workspace instead, and a second pass applies alpha and beta (C of 72 MB,
-        // K 72: 107 us in two passes, 171 in one; 131 MB, K 48: 143 and 177; 755 MB, K 16: 699 and 738; 231 MB, K 312: 689 and 670;
-        // with chunks of 8, 302 MB, K 24: 242 and 168).  With rows along C one pass is faster (4.7 M elements, K 48: 24 us, 35 in
-        // two; 16.8 M, K 16: 66 and 96).  TCONT_SCALE_PASSES=1|2 overrides the rule.
+        // chunks of 16, the TMA-fed FP64 kernel writes a workspace instead, and a second pass applies alpha and beta (C of 31 MB,
+        // K 16: 29 us in two passes, 36 in one; 239 MB, K 48: 240 and 264; 106 MB, K 72: 133 and 142; the exceptions are large, 302 MB, K 48:
+        // 287 and 270; 746 MB, K 16: 600 and 519; with chunks of 8, 302 MB, K 24: 237 and 167).  With rows along C one pass is faster
+        // (4.7 M elements, K 48: 24 us, 34 in two; 16.8 M, K 16: 65 and 96).  TCONT_SCALE_PASSES=1|2 overrides the rule.
         const bool unsplit = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1;
         run->scale_pass = unsplit && u.store_across_slabs && u.BK == 16 && (pl.sizeC * static_cast<int64_t>(run->elt) <= kScalePassInL2 || u.k_iters <= 6);
         if (const char* sp = std::getenv("TCONT_SCALE_PASSES")) run->scale_pass = unsplit && sp[0] != '1';

@@ -910,6 +910,8 @@ double contraction_us(const Problem& p, int kernel, const UmmaSpec& u, const Cos
     double c_bytes = double(p.sizeC) * elt;
     double rate = 0;
     double extra_us = 0, scatter_us = 0, extra_floor_us = 0;
+    // (Whole tile columns, although `slim` computes fewer: charging what is computed here and for split-K changes 52 of 1434 drawn choices
+    // of kernel and ranges, 24 of them for the worse, up to 2.2 times; the other constants are fitted with whole columns.)
     // TMA-fed kernels: slabs and k chunks are whole, ragged extents are zero-filled and multiplied anyway
     // (extents of 72 in 32-wide slabs and chunks: abcd-aefb-fdce ran at 138 TFLOP/s direct, 415 after a
     // transpose that fuses the ragged modes away)
@@ -1323,6 +1325,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     UmmaSpec ttgt_umma;
     int ttgt_kernel = KERNEL_SIMT;
     double ttgt_by_tiles_us = 1e300;   // with the permutations' tiles counted
+    bool ttgt_padded = false;
     TransposeSpec tA, tB;
     pl.est_ttgt_us = 1e300;
     auto padded = [&](size_t candidate, bool is_a) -> const std::vector<int64_t>& {
@@ -1416,6 +1419,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         if (kernel == KERNEL_DMMA_F64_TMA && u.k_splits > 1) us += 0.12 * u.k_splits;
         if (us < 0.97 * pl.est_ttgt_us) {   // (an alternative has to be clearly better than the first)
             pl.est_ttgt_us = us;
+            ttgt_padded = i > 0 && i == padded_candidate;
             ttgt_by_tiles_us = us - transposes_us(i, cost, false) + transposes_us(i, cost, true);
             ttgt = q;
             ttgt_umma = u;
@@ -1441,7 +1445,8 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     bool use_ttgt;
     if (backend_selection == 1) use_ttgt = false;
     else if (backend_selection == 2) use_ttgt = true;
-    else use_ttgt = !pl.across.on && (tA.needed || tB.needed) && pl.est_ttgt_us < pl.est_direct_us;
+    // (padded copies take scratch for both operands and a millisecond to prepare: not for estimates that are level)
+    else use_ttgt = !pl.across.on && (tA.needed || tB.needed) && pl.est_ttgt_us < (ttgt_padded && !padded_forced ? 0.97 : 1.0) * pl.est_direct_us;
 
     if (use_ttgt) {
         pl.backend = 1;

@@ -169,7 +169,8 @@ struct CostTable {
     // where the fit has 28 to 32 and 4.0): a table it writes is close to this one, not equal, and gives other routes in ties.
     double hbm_gbs = 6178.9;                // copy through the permutation kernel, read + write
     double umma_tf32_tflops = 674.4;        // tcgen05 kernel, 8192 x 8192 x 4096, CTA pairs with a k chunk of 64
-    double dmma_f64_tflops = 33.5;          // TMA-fed tensor-path kernel
+    double dmma_f64_tflops = 33.5;          // TMA-fed tensor-path kernel (35.3 on whole tiles with its present main loop; the other FP64
+                                            // constants are fitted with this one: 35.3 sums 22 x 40 x 50 x 48 by 968 in 5 ranges, 230 us, not 4, 207)
     // Gather kernel, per tile shape (64 x 64, 128 x 32, 32 x 32, Float32 128 x 128): what a full GPU does in whole tiles,
     // and the least time one CTA needs per k tile of 16 when it has an SM to itself.
     double gather_f64_tflops[3] = {28.0, 18.0, 18.0};
