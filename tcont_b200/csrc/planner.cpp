@@ -1325,7 +1325,6 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     UmmaSpec ttgt_umma;
     int ttgt_kernel = KERNEL_SIMT;
     double ttgt_by_tiles_us = 1e300;   // with the permutations' tiles counted
-    bool ttgt_padded = false;
     TransposeSpec tA, tB;
     pl.est_ttgt_us = 1e300;
     auto padded = [&](size_t candidate, bool is_a) -> const std::vector<int64_t>& {
@@ -1419,7 +1418,6 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         if (kernel == KERNEL_DMMA_F64_TMA && u.k_splits > 1) us += 0.12 * u.k_splits;
         if (us < 0.97 * pl.est_ttgt_us) {   // (an alternative has to be clearly better than the first)
             pl.est_ttgt_us = us;
-            ttgt_padded = i > 0 && i == padded_candidate;
             ttgt_by_tiles_us = us - transposes_us(i, cost, false) + transposes_us(i, cost, true);
             ttgt = q;
             ttgt_umma = u;
@@ -1445,8 +1443,8 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     bool use_ttgt;
     if (backend_selection == 1) use_ttgt = false;
     else if (backend_selection == 2) use_ttgt = true;
-    // (padded copies take scratch for both operands and a millisecond to prepare: not for estimates that are level)
-    else use_ttgt = !pl.across.on && (tA.needed || tB.needed) && pl.est_ttgt_us < (ttgt_padded && !padded_forced ? 0.97 : 1.0) * pl.est_direct_us;
+    // (no margin for padded copies: 47 x 49 x 45 by 127 by 19, estimated level, takes 110 us on the gather kernel and 96 behind them)
+    else use_ttgt = !pl.across.on && (tA.needed || tB.needed) && pl.est_ttgt_us < pl.est_direct_us;
 
     if (use_ttgt) {
         pl.backend = 1;
