@@ -341,3 +341,15 @@ def test_float32_tiles_across_stride_1_modes_are_taken_where_they_are_faster(eng
     assert not across("abcde efba cfd", (40, 28, 32, 16, 24, 72))         # 33.5 / 23.9
     assert not across("abcdef dfga gebc", (16, 20, 12, 20, 28, 16, 48))   # 71.7 / 41.9
     assert not across("abcde efba cfd", (40, 40, 32, 40, 64, 8))          # 104 / 94.3
+
+
+@pytest.mark.parametrize("eq,extents,piece", [
+    ("ab ak kb", (1540, 56, 24), 4), ("ab ak bk", (1540, 40, 24), 4), ("ab ak bk", (1030, 150, 40), 2), ("ab ka kb", (1029, 149, 40), 1),
+    ("abcd dbea ec", (24, 9, 60, 54, 40), 4), ("acb abk kc", (12, 60, 128, 24), 4), ("acb abk kc", (6, 50, 128, 24), 2),
+])
+def test_fp64_pieces_follow_the_strides_of_c(engine, monkeypatch, eq, extents, piece):
+    """How many neighbouring elements of C the TMA-fed FP64 kernel may store at a time."""
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    C, A, B = eq.split()
+    d = describe(engine, Contraction(C, A, B, dict(zip(sorted(set(C + A + B)), extents)), F64), 1)
+    assert d["kernel"] == "dmma_f64_tma" and d["umma"]["piece"] == piece, d["umma"]
