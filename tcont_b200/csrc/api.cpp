@@ -187,6 +187,7 @@ struct tcontb_run {
     std::unique_ptr<tcontb_run> scaled_form;
     bool scaled_elsewhere = false;
     bool keep_copies = false;  // set-up: no room for scratch copies of the operands is an error
+    bool is_part = false;      // of a pipelined host-buffer pass
     // stage timing
     bool stage_timing = false;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -721,7 +722,8 @@ tcontb_status provide_scaled_form(tcontb_run* run, const Plan& plan, bool with_c
 // How a run with tiles across two stride-1 modes applies other scalars than (1, 0): by a second pass, or in the form that its plan has
 // without such tiles, whose epilogue applies them.  A C that is much larger than A is faster in that form (plain / accumulating us:
 // C of 460 MB 87 / 401 across, 92 / 259 in the other form; of 151 MB 27 / 109 and 38 / 97), one that is not is slower (226 MB, A of
-// 302: 107 / 265 and 311 / 413): copying A costs what the second pass does.  It has to look a tenth better, which is how far the
+// 302: 107 / 265 and 311 / 413): copying A costs what the second pass does.  (The parts of a
+// host-buffer pass, which the transfers bound, take the second pass: every one of them would hold copies of the shared operand.)  It has to look a tenth better, which is how far the
 // estimates are off: of 176 contractions two accumulate more than 7 % slower than in the better form (1.08, 1.18).  Where there is no
 // room for the one, the other is taken, then the form on the operands as they lie; without room for any the run stays as it was.
 tcontb_status choose_scaled_form(tcontb_run* run, double beta)
@@ -734,7 +736,7 @@ tcontb_status choose_scaled_form(tcontb_run* run, double beta)
     const bool planned = plan_without_across(run->plan, &other);
     const int reads = beta != 0.0 ? 1 : 0;
     const char* force = std::getenv("TCONT_ACROSS");
-    const bool elsewhere = planned && !(force && force[0] == '1') && run->plan.sizeC > 2 * run->plan.prob.sizeA && other.est_scaled_us[reads] > 0 && other.est_scaled_us[reads] < 0.9 * run->plan.est_scaled_us[reads];
+    const bool elsewhere = planned && !run->is_part && !(force && force[0] == '1') && run->plan.sizeC > 2 * run->plan.prob.sizeA && other.est_scaled_us[reads] > 0 && other.est_scaled_us[reads] < 0.9 * run->plan.est_scaled_us[reads];
     const bool attempts[3] = {elsewhere, !elsewhere, true};
     for (int i = 0; i < 3; ++i) {
         if (attempts[i] && !planned) continue;
@@ -988,6 +990,7 @@ tcontb_status build_host_pipeline(tcontb_run* run)
         part->dL = left ? static_cast<void*>(in) : run->dL;
         part->dR = left ? run->dR : static_cast<void*>(in);
         part->dC = static_cast<unsigned char*>(run->dC) + static_cast<size_t>(i) * pp.slice_out;
+        part->is_part = true;
         // the operand every part shares is transposed once, by the first part; the others read its copy
         if (!parts.empty()) {
             const bool carrier_is_role_a = part->plan.prob.swapped ? !left : left;

@@ -199,3 +199,22 @@ def test_form_of_accumulating_launches(engine, oracle, ext, kernels):
         engine.launch(run)
         other.synchronize()
     assert held(2.0, 1.0, 3.0) and run.device_status() == 0
+
+
+def test_accumulating_parts_of_a_host_pass(engine, oracle, monkeypatch):
+    """Each part applies the scalars to its range of C, whose old values are what the pass before left there."""
+    monkeypatch.setenv("TCONT_HOST_CHUNKS", "2")
+    c = Contraction("abcde", "efba", "cfd", dict(a=32, b=24, c=40, d=16, e=40, f=16), F32)
+    A, B = oracle.inputs(c, 59, -1.0, 1.0)
+    plan = engine.plan(to_equation(engine, c, 0))
+    assert "across" in plan.describe()
+    run = engine.prepare(plan, A, B)
+    first, second = np.empty(c.size("abcde"), np.float32), np.empty(c.size("abcde"), np.float32)
+    run.contract_host(A, B, first)
+    run.set_scalars(0.3, -0.7)
+    run.contract_host(A, B, second)
+    at = np.sort(np.random.default_rng(6).integers(0, first.size, 20000))
+    product, scale = (oracle.contract_sampled(c, a, b, at, rounding=1) for a, b in ((A, B), (np.abs(A), np.abs(B))))
+    assert (np.abs(first[at] - product) <= 2e-5 * scale).all()
+    want = 0.3 * product - 0.7 * first[at].astype(np.float64)
+    assert (np.abs(second[at] - want) <= 2e-5 * 0.3 * scale + 4 * 2.0**-24 * (np.abs(0.3 * product) + np.abs(0.7 * first[at]))).all()
