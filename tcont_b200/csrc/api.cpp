@@ -343,9 +343,9 @@ tcontb_status encode_map(const UmmaOperand& o, const void* base, int elt, CUtens
     }
     const CUresult r = fn(out, elt == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, kMaxTmaRank, const_cast<void*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          // an MN-major 32-bit operand must be swizzled in 32-byte units for tcgen05.mma;
+                          // an MN-major operand is swizzled in 32-byte units: tcgen05.mma wants it, and FP64 fragments are then loaded without conflicts;
                           // FP64 operands may have 64-byte rows (8 doubles of the k chunk or of the slab mode)
-                          (o.major && elt == 4) ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
+                          o.major && o.box[0] * elt == 128 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
                           : (o.box[0] * elt == 64) ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -561,7 +561,7 @@ tcontb_status finish_run(tcontb_run* run)
         const tcontb_status st = finish_across(run, kA, kB);
         if (st != TCONTB_OK) return st;
     } else if (pl.kernel == KERNEL_UMMA_TF32 || pl.kernel == KERNEL_DMMA_F64_TMA) {
-        const UmmaSpec& u = pl.umma;
+        const UmmaSpec& u = pl.narrow.eligible ? pl.narrow : pl.umma;
         fill_operand_dev(u.a, &run->umma.a);
         fill_operand_dev(u.b, &run->umma.b);
         run->umma.BN = u.BN;
@@ -604,13 +604,13 @@ tcontb_status finish_run(tcontb_run* run)
             TC_CUDA(run->loB.alloc(static_cast<size_t>(run->kernB_elements) * run->elt));
             run->kernels_per_launch += 4;  // two residual passes, two more contractions
         }
-        // Tiles across slabs read the old values of C in pieces of 32 bytes: with a C of up to half of L2, or few k chunks, and k
+        // 128 x 64 tiles across slabs read the old values of C in the epilogue: with a C of up to half of L2, or few k chunks, and k
         // chunks of 16, the TMA-fed FP64 kernel writes a workspace instead, and a second pass applies alpha and beta (C of 31 MB,
-        // K 16: 29 us in two passes, 36 in one; 239 MB, K 48: 240 and 264; 106 MB, K 72: 133 and 142; the exceptions are large, 302 MB, K 48:
-        // 287 and 270; 746 MB, K 16: 600 and 519; with chunks of 8, 302 MB, K 24: 237 and 167).  With rows along C one pass is faster
-        // (4.7 M elements, K 48: 24 us, 34 in two; 16.8 M, K 16: 65 and 96).  TCONT_SCALE_PASSES=1|2 overrides the rule.
+        // K 16: 29 us in two passes, 36 in one; 239 MB, K 48: 240 and 264; 106 MB, K 72: 133 and 142).  With rows along C one pass is faster
+        // (4.7 M elements, K 48: 24 us, 34 in two; 16.8 M, K 16: 65 and 96), and with 128 x 32 tiles (72 x 72 x 24 x 72 by 72: 72 us, 96 in
+        // two; 302 MB, K 48: 164 and 182).  TCONT_SCALE_PASSES=1|2 overrides the rule.
         const bool unsplit = pl.kernel == KERNEL_DMMA_F64_TMA && u.k_splits == 1;
-        run->scale_pass = unsplit && u.store_across_slabs && u.BK == 16 && (pl.sizeC * static_cast<int64_t>(run->elt) <= kScalePassInL2 || u.k_iters <= 6);
+        run->scale_pass = unsplit && u.store_across_slabs && u.BN == 64 && u.BK == 16 && (pl.sizeC * static_cast<int64_t>(run->elt) <= kScalePassInL2 || u.k_iters <= 6);
         if (const char* sp = std::getenv("TCONT_SCALE_PASSES")) run->scale_pass = unsplit && sp[0] != '1';
         run->umma.C = static_cast<float*>(out);
         run->umma.C64 = static_cast<double*>(out);
@@ -1299,7 +1299,7 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         TC_CUDA(launch_umma_tf32(umma, &run->tmA, &run->tmB, pl.umma.smem_bytes, run->num_sms, run->stream));
     }
     else if (pl.kernel == KERNEL_DMMA_F64_TMA)
-        TC_CUDA(launch_dmma_tma(umma, &run->tmA, &run->tmB, pl.umma.smem_bytes, run->num_sms, run->stream));
+        TC_CUDA(launch_dmma_tma(umma, &run->tmA, &run->tmB, (pl.narrow.eligible ? pl.narrow : pl.umma).smem_bytes, run->num_sms, run->stream));
     else {
         GatherParams g = run->gather;
         g.scaled = scaled ? 1 : 0;

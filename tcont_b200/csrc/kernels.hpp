@@ -180,6 +180,7 @@ struct UmmaParams {
     int store_across_slabs;  // FP64 kernel: see UmmaSpec
     int piece;               // FP64 kernel: see UmmaSpec
     int slim;                // FP64 kernel: see UmmaSpec
+    int old_staged;          // FP64 kernel, 128 x 32 tiles (set by the launcher): old values of C are copied to shared memory while a tile is computed
     // tcgen05 kernel.  1: the next kernel's blocks may be scheduled when this one's copies are issued, 0: at once.  Late where
     // every block stores many tiles of few k iterations: 806400 x 112 x 48 behind its permutation, 43 tiles a block: let in at
     // once 200 us, late 184, not chained 187.  Short kernels lose by it (4096 x 3072 x 32, 3 tiles: 16.9, late 17.3).  The FP64

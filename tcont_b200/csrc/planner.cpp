@@ -408,7 +408,7 @@ bool chunk_kmajor(UmmaOperand* o, int BK, int cta_slabs)
     return true;
 }
 
-void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int bk_request, bool fuse_rows)
+void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int bk_request, bool fuse_rows, bool narrow = false)
 {
     u->eligible = false;
     const bool f64 = p_in.scalar_type == 1;
@@ -572,6 +572,7 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
         finish_operand(p, p.B, p.N, 32, BK, kdigits, &probe);
         const int64_t padded = probe.total_slabs * probe.slab_w;
         bn = double(ceil_div(padded, 32) * 32) * 1.15 < double(ceil_div(padded, 64) * 64) ? 32 : 64;
+        if (narrow) bn = 32;
     } else {
         UmmaOperand probe = u->b;
         finish_operand(p, p.B, p.N, 32, BK, kdigits, &probe);
@@ -652,7 +653,11 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
     // both kernels own an SM; the FP64 one stops at eight 24 KB stages
     const int budget = f64 ? 200 * 1024 : 227 * 1024 - 8 * 1024;
     u->stages = std::max(2, std::min(8, budget / stage_bytes));
-    if (f64) u->stages &= ~1;  // one ring of stages per consumer group
+    if (f64) {   // one ring of stages per consumer group
+        const int groups = u->BN == 32 ? 3 : 2;
+        if (groups == 3) u->stages = std::max(3, std::min(12, (227 * 1024 - 7 * 1024) / stage_bytes));
+        u->stages -= u->stages % groups;
+    }
     // One CTA per tile (k chunks of up to 32: a stage is at most four MMAs, 512 cycles): two producer warps take
     // turns stage by stage, because one warp's wait-announce-copy round trip takes 700 to 900 cycles whatever the
     // stage holds (reference cases 13, 15, 21, 24 in TF32: 1.24 to 1.67 times faster; nothing to gain with one k
@@ -662,7 +667,7 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
     if (const char* e = std::getenv("TCONT_UMMA_PRODUCERS"))
         if (!f64) u->producers = std::atoi(e) == 2 && u->stages >= 4 ? 2 : 1;
     if (u->producers == 2) u->stages &= ~1;
-    u->smem_bytes = u->stages * stage_bytes + 8 * 1024 + 1024;
+    u->smem_bytes = u->stages * stage_bytes + (f64 ? u->BN == 32 ? 6 : 9 : 8) * 1024 + 1024;
     // Split-K: with few waves of tiles and a long contracted extent, cut the k iterations into ranges
     // computed as separate work units (partials summed by a second kernel).  Of the admissible counts
     // (ranges of at least 4 iterations, workspace of at most 512 MB) the one with the smallest estimate
@@ -704,6 +709,11 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
     }
     u->raster_group = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(u->tiles_m,
                       std::llround(std::sqrt(double(cost.num_sms) * u->BN / u->BM)))));
+    // Tiles across slabs store 64 bytes at a time.  Where the next mode of C is a row mode, neighbouring tile rows continue them, and C
+    // leaves the faster the more of those are in work together: all rows of a column of tiles one after the other, as long as their part
+    // of A stays in L2 (48 x 32 x 64 x 32 x 32 by 8: 6 rows 192 us, 24 175, 200 138, all 384 130; by 16, 48 in the place of the last 32: 347, 342, 297, 281).
+    if (u->store_across_slabs && p.C.size() > 1 && p.modes[static_cast<size_t>(p.C[1])].group == GROUP_M)
+        u->raster_group = static_cast<int>(std::min<int64_t>(u->tiles_m, std::max<int64_t>(u->raster_group, (int64_t(16) << 20) / (u->BM * elt * p.Ktot))));
     // Tuning switch: TCONT_UMMA_RASTER=<g> sets the number of tile rows (pair rows for CTA pairs) swept together.
     if (const char* e = std::getenv("TCONT_UMMA_RASTER"))
         u->raster_group = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(u->tiles_m, std::atoll(e))));
@@ -764,6 +774,25 @@ void plan_umma(const Problem& p, const CostTable& cost, UmmaSpec* u, bool fuse_r
     }
     *u = UmmaSpec();
     plan_umma_impl(p, cost, u, 32, true);
+}
+
+// FP64 with short contracted extents: 128 x 32 tiles, three of them in work on an SM, where a block of 128 x 64 tiles has two.  The
+// store of a tile then falls into two main loops of others, and old values of C are copied to shared memory while a tile is
+// computed, which 64 columns leave no room for.  Decided when route and kernel are (the estimates know 128 x 64 tiles).  Measured,
+// 9216 x 4096 by K, us, 64 and 32 columns: K 8 55 and 48, K 24 81 and 74, K 48 125 and 120, K 96 226 and 221, K 192 433 and 426;
+// 4096 x 4096 x 1024 976 and 997.  Accumulating: K 24 168 and 113, K 96 305 and 263, K 192 487 and 472; with rows along C K 24 124
+// and 121, K 72 229 and 217, K 96 261 and 267, K 128 325 and 337; in k chunks of 8 4096 x 4096 x 64 86 and 94.  Not with slabs of 8 rows of A: their 64-byte rows are loaded with bank
+// conflicts, which half as many columns a fragment do not hide (5184^3, 72 x 72 rows: 8 236 and 13 138).
+UmmaSpec narrow_tiles(const Problem& p, const CostTable& cost, const UmmaSpec& u)
+{
+    const char* want = std::getenv("TCONT_DMMA_BN");   // tuning switch: 32 or 64 columns
+    const bool short_k = u.k_computed <= (u.store_across_slabs ? 256 : u.BK == 8 ? 32 : 96) && !(u.a.major == 1 && u.a.slab_w == 8);
+    UmmaSpec v;
+    const bool whole = !u.slim && ceil_div(u.b.total_slabs * u.b.slab_w, 32) * 32 <= u.tiles_n * 64;   // as many columns computed
+    if (u.BN != 64 || u.k_splits != 1 || !whole || !(want ? std::atoi(want) == 32 : short_k)) return v;
+    plan_umma_impl(p, cost, &v, 32, true, true);
+    if (v.k_splits != 1) v.eligible = false;
+    return v;
 }
 
 std::string perm_modes(const Problem& p, const std::vector<int>& ids)
@@ -1461,6 +1490,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         pl.umma = direct_umma;
     }
     const Problem& p = pl.prob;
+    if (pl.kernel == KERNEL_DMMA_F64_TMA) pl.narrow = narrow_tiles(p, cost, pl.umma);
     if (pl.kernel == KERNEL_UMMA_TF32)
         for (int reads = 0; reads < 2; ++reads)
             pl.est_scaled_us[reads] = (use_ttgt ? ttgt_by_tiles_us : pl.est_direct_us) +
@@ -1538,11 +1568,14 @@ std::string describe_plan(const Plan& pl)
     if (pl.across.on)
         o << ",\"across\":{\"BN\":" << pl.across.BN << ",\"BK\":" << pl.across.BK << ",\"stages\":" << pl.across.stages << ",\"tiles_m\":" << pl.across.tiles_m
           << ",\"tiles_n\":" << pl.across.tiles_n << ",\"k_iters\":" << pl.across.k_iters << ",\"b_major\":\"" << (pl.across.b_major ? "MN" : "K") << "\"}";
+    if (pl.narrow.eligible)
+        o << ",\"narrow\":{\"BN\":" << pl.narrow.BN << ",\"BK\":" << pl.narrow.BK << ",\"stages\":" << pl.narrow.stages << ",\"slim\":" << (pl.narrow.slim ? "true" : "false") << ",\"tiles_m\":" << pl.narrow.tiles_m
+          << ",\"tiles_n\":" << pl.narrow.tiles_n << "}";
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";
     else {
-        // (not in use: the gather kernel was cheaper, or tiles across two stride-1 modes run)
-        o << ",\"in_use\":" << (!pl.across.on && (pl.kernel == KERNEL_UMMA_TF32 || pl.kernel == KERNEL_DMMA_F64_TMA) ? "true" : "false") << ",\"BM\":" << u.BM << ",\"BN\":" << u.BN << ",\"BK\":" << u.BK << ",\"stages\":" << u.stages
+        // (not in use: the gather kernel was cheaper, or tiles across two stride-1 modes or narrow ones run)
+        o << ",\"in_use\":" << (!pl.across.on && !pl.narrow.eligible && (pl.kernel == KERNEL_UMMA_TF32 || pl.kernel == KERNEL_DMMA_F64_TMA) ? "true" : "false") << ",\"BM\":" << u.BM << ",\"BN\":" << u.BN << ",\"BK\":" << u.BK << ",\"stages\":" << u.stages
           << ",\"pair\":" << (u.pair ? "true" : "false") << ",\"kc\":\"" << u.kc_names << "\",\"k_iters\":" << u.k_iters << ",\"k_splits\":" << u.k_splits << ",\"tiles_m\":" << u.tiles_m << ",\"tiles_n\":" << u.tiles_n
           << ",\"a_major\":\"" << (u.a.major ? "MN" : "K") << "\",\"b_major\":\"" << (u.b.major ? "MN" : "K") << "\""
           << ",\"a_slab_w\":" << u.a.slab_w << ",\"b_slab_w\":" << u.b.slab_w << ",\"a_slabs_per_copy\":" << u.a.slabs_per_op << ",\"b_slabs_per_copy\":" << u.b.slabs_per_op << ",\"a_slabs\":" << u.a.slabs_per_tile

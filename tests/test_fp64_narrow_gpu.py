@@ -1,0 +1,62 @@
+"""FP64 contractions on 128 x 32 and 128 x 64 tiles: the two fragment layouts, rows of a tile along C, along k and across slabs, the ends of
+tiles and slabs, contracted extents from one k chunk to more than fit the ring, old values of C staged and read in the epilogue.
+
+Every output is a chain of K fused multiply-adds and three roundings of the scalars, each off by at most 2^-53 of its partial sum.
+"""
+import numpy as np
+import pytest
+
+from oracle_lib import F64, Contraction
+from test_scaled_epilogues_gpu import SCALARS, scaled_run
+
+pytestmark = pytest.mark.gpu
+
+# name -> (descriptor, tiles across slabs)
+FORMS = {
+    "mn_k": ("ab", "ak", "kb", dict(a=272, b=97), False),
+    "mn_mn_odd_columns": ("abc", "ak", "bck", dict(a=146, b=34, c=3), False),
+    "mn_8_wide_slabs": ("abc", "akb", "ck", dict(a=24, b=11, c=60), False),
+    "k_mn_unaligned": ("ab", "ka", "bk", dict(a=131, b=62), False),
+    "k_k_unaligned": ("ab", "ka", "kb", dict(a=259, b=61), False),
+    "fused_rows": ("acb", "abk", "kc", dict(a=6, b=50, c=61), False),
+    "across": ("abcd", "dbka", "kc", dict(a=24, b=3, c=60, d=34), True),
+    "across_next_mode_a_row": ("abcd", "dkba", "ck", dict(a=8, b=9, c=62, d=48), True),
+}
+
+
+@pytest.mark.parametrize("name", list(FORMS))
+@pytest.mark.parametrize("columns", ["32", "64"])
+@pytest.mark.parametrize("k", [8, 24, 72, 136])
+def test_forms(engine, oracle, monkeypatch, name, columns, k):
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    monkeypatch.setenv("TCONT_SPLITK", "1")
+    monkeypatch.setenv("TCONT_SCALE_PASSES", "1")
+    monkeypatch.setenv("TCONT_DMMA_BN", columns)
+    C, A_, B_, ext, across = FORMS[name]
+    c = Contraction(C, A_, B_, dict(ext, k=k), F64)
+    A, B = oracle.inputs(c, 23, -1.0, 1.0)
+    C0 = np.random.default_rng(5).uniform(-4.0, 4.0, c.size(C))
+    desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
+    assert desc["kernel"] == "dmma_f64_tma" and desc["umma"]["store_across_slabs"] == across
+    assert desc["umma"]["BN"] == 64 and ("narrow" in desc) == (columns == "32") == (not desc["umma"]["in_use"])
+    product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
+    for (alpha, beta), out in zip(SCALARS, got):
+        bound = (k + 4) * 2.0**-53 * (abs(alpha) * scale + abs(beta * C0))
+        assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (alpha, beta)
+
+
+@pytest.mark.parametrize("columns", ["32", "64"])
+def test_several_tiles_a_group(engine, oracle, monkeypatch, columns):
+    """Rings, tables and staged values come round: 9 to 18 tiles a block, all slabs whole but the last."""
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    monkeypatch.setenv("TCONT_DMMA_BN", columns)
+    monkeypatch.setenv("TCONT_SCALE_PASSES", "1")
+    for C, A_, B_, ext in (("ab", "ak", "kb", dict(a=5130, b=2100, k=24)), ("abc", "cka", "kb", dict(a=24, b=2100, c=210, k=40))):
+        c = Contraction(C, A_, B_, ext, F64)
+        A, B = oracle.inputs(c, 29, -1.0, 1.0)
+        C0 = np.random.default_rng(6).uniform(-4.0, 4.0, c.size(C))
+        desc, got = scaled_run(engine, c, A, B, C0, [(1.0, 1.0), (1.0, 0.0)])
+        assert ("narrow" in desc) == (columns == "32")
+        product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
+        for beta, out in zip((1.0, 0.0), got):
+            assert (np.abs(out - (product + beta * C0)) <= (ext["k"] + 4) * 2.0**-53 * (scale + abs(beta * C0))).all()

@@ -353,3 +353,20 @@ def test_fp64_pieces_follow_the_strides_of_c(engine, monkeypatch, eq, extents, p
     C, A, B = eq.split()
     d = describe(engine, Contraction(C, A, B, dict(zip(sorted(set(C + A + B)), extents)), F64), 1)
     assert d["kernel"] == "dmma_f64_tma" and d["umma"]["piece"] == piece, d["umma"]
+
+
+def test_fp64_narrow_tiles(engine, monkeypatch):
+    """128 x 32 tiles for short contracted extents, unless they compute more columns, A comes in slabs of 8 rows, or k is cut."""
+    F64 = 1
+    narrow = lambda c: "narrow" in describe(engine, c, 1)
+    rows = lambda n, k: Contraction("ab", "ak", "kb", dict(a=9216, b=n, k=k), F64)
+    across = lambda k: Contraction("abcdef", "dega", "gfbc", dict(a=24, b=16, c=16, d=24, e=16, f=16, g=k), F64)
+    assert narrow(rows(4096, 16)) and narrow(rows(4096, 96)) and not narrow(rows(4096, 112))
+    assert narrow(rows(4096, 24)) and not narrow(rows(4096, 40))      # k chunks of 8
+    assert narrow(across(24)) and narrow(across(256)) and not narrow(across(272))
+    assert not narrow(rows(40, 64)) and not narrow(rows(24, 64))      # three column fragments a warp; 32 columns anyway
+    assert not narrow(Contraction("abc", "akb", "kc", dict(a=24, b=400, c=4096, k=64), F64))
+    d = describe(engine, rows(4096, 16), 1)
+    assert not d["umma"]["in_use"] and d["narrow"]["BN"] == 32 and d["narrow"]["stages"] % 3 == 0
+    monkeypatch.setenv("TCONT_DMMA_BN", "64")
+    assert not narrow(rows(4096, 16)) and describe(engine, rows(4096, 16), 1)["umma"]["in_use"]
