@@ -557,6 +557,17 @@ tcontb_status finish_run(tcontb_run* run)
     TC_CUDA(cudaMemset(run->status.ptr, 0, sizeof(int)));
 
     run->scale_pass = run->tf32x3 = false;
+    if (pl.narrow.eligible && pl.narrow.k_splits > 1) {
+        // Ranges of k need a workspace, which what they run in the place of may not: without room that runs.
+        const cudaError_t e = run->splitk.alloc(static_cast<size_t>(pl.narrow.k_splits) * static_cast<size_t>(pl.sizeC) * run->elt);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            run->plan.kernel = pl.kernel_without_narrow;
+            run->plan.narrow = UmmaSpec();
+        } else {
+            TC_CUDA(e);
+        }
+    }
     if (pl.across.on) {
         const tcontb_status st = finish_across(run, kA, kB);
         if (st != TCONTB_OK) return st;
@@ -587,8 +598,9 @@ tcontb_status finish_run(tcontb_run* run)
         const char* x3 = std::getenv("TCONT_TF32X3");
         run->tf32x3 = pl.kernel == KERNEL_UMMA_TF32 && x3 && x3[0] == '1' && !p.strided;
         if (u.k_splits > 1 || run->tf32x3) {
-            TC_CUDA(run->splitk.alloc(static_cast<size_t>(run->tf32x3 ? 3 : 1) * static_cast<size_t>(u.k_splits) *
-                                      static_cast<size_t>(pl.sizeC) * run->elt));
+            if (!run->splitk.ptr)
+                TC_CUDA(run->splitk.alloc(static_cast<size_t>(run->tf32x3 ? 3 : 1) * static_cast<size_t>(u.k_splits) *
+                                          static_cast<size_t>(pl.sizeC) * run->elt));
             out = run->splitk.ptr;
             run->kernels_per_launch++;
         }
@@ -1308,7 +1320,7 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         TC_CUDA(launch_gather_contract(g, pl.scalar_type, pl.gather.tile, run->num_sms, run->stream));
     }
     if (run->splitk.ptr)
-        TC_CUDA(launch_splitk_reduce(run->splitk.ptr, run->dC, pl.sizeC, pl.umma.k_splits * (run->tf32x3 ? 3 : 1), pl.sizeC,
+        TC_CUDA(launch_splitk_reduce(run->splitk.ptr, run->dC, pl.sizeC, (pl.narrow.eligible ? pl.narrow : pl.umma).k_splits * (run->tf32x3 ? 3 : 1), pl.sizeC,
                                      static_cast<int>(run->elt), run->stream, run->alpha, run->beta));
     else if (redirect)
         TC_CUDA(run->elt == 8 && pl.sizeC * static_cast<int64_t>(run->elt) > kScalePassInL2

@@ -795,6 +795,47 @@ UmmaSpec narrow_tiles(const Problem& p, const CostTable& cost, const UmmaSpec& u
     return v;
 }
 
+// Time of the TMA-fed FP64 kernel in `s` ranges of k, for up to a few rounds of work units.  A block's SM has `groups` units in work: all
+// of them together are bound by the FP64 pipe, each by itself by its chain of k iterations (no shorter than the copies of a stage
+// take) and its store.  Fitted to 663 (128 x 32) and 446 (128 x 64) launches of 113 contractions of 4 MFLOP to 3 GFLOP in 1 to 48
+// ranges: two thirds within 8 %, nine tenths within 15 %.
+double split_us(const Problem& p, const UmmaSpec& u, int64_t s, const CostTable& cost)
+{
+    const bool narrow = u.BN == 32;
+    const double setup = narrow ? 3.22 : 3.47, chain_it = narrow ? 0.362 : 0.966, store = narrow ? 1.52 : 2.1, pipe_it = narrow ? 0.614 : 1.2, copy0 = narrow ? 0.178 : -0.656,
+                 copy1 = narrow ? 0.035 : 0.067, sum0 = narrow ? 1.46 : 1.59, sum1 = narrow ? 0.188 : 0.192;
+    const int groups = narrow ? 3 : 2;
+    const double c_mb = double(p.sizeC) * 8e-6, chunk = u.BK / 16.0, copies = double(u.a.slabs_per_tile) / u.a.slabs_per_op + double(u.b.slabs_per_tile) / u.b.slabs_per_op;
+    const int64_t per = ceil_div(u.k_iters, s), units = ceil_div(u.tiles_m * u.tiles_n * ceil_div(u.k_iters, per), cost.num_sms);
+    const double pipe = double(units * per) * pipe_it * (u.slim ? 0.8 : 1.0) * chunk + store / groups;
+    const double chain = double(ceil_div(units, groups)) * (double(per) * std::max(chain_it * chunk, copy0 + copy1 * copies) + store);
+    const double us = setup + std::max(pipe, chain) + (s > 1 ? sum0 + (sum1 * c_mb + 0.12) * double(s) : 0.0);
+    return std::max(us, setup + (c_mb + (double(p.sizeA) + double(p.sizeB)) * 8e-6) / (narrow ? 4.93 : 4.54));
+}
+
+// FP64 with few tiles: 128 x 32 tiles in the number of ranges of k with the smallest estimate, `*us` (eligible = false: none).  More and
+// smaller units than the 128 x 64 tiles' even out better over the SMs: 16 x 16 outputs by 13 440 26.4 -> 20.9 us, 20 x 18 tiles by 384
+// in three ranges 46.8 -> 42.3, 144 x 1 by 312 33.2 -> 27.2.
+UmmaSpec narrow_ranges(const Problem& p, const CostTable& cost, const UmmaSpec& u, double* us)
+{
+    UmmaSpec v;
+    *us = 1e300;
+    if (!u.eligible || u.elt != 8 || std::getenv("TCONT_SPLITK") || std::getenv("TCONT_DMMA_BN")) return v;
+    if ((u.a.row_elem_cstride != 1 && !u.store_across_slabs) || u.a.slab_mode_ext < 8) return v;   // (stores of single elements)
+    if (u.BN == 32) v = u;
+    else plan_umma_impl(p, cost, &v, 32, true, true);
+    if (!v.eligible) return v;
+    int64_t best = 1;
+    for (int64_t s = 1; s <= (p.c_strided ? 1 : std::min<int64_t>(64, std::max<int64_t>(1, v.k_iters / 2))); ++s) {
+        if (double(s) * double(p.sizeC) * 8.0 > 512.0 * 1024 * 1024) break;   // workspace
+        const double t = split_us(p, v, s, cost);
+        if (t < 0.97 * *us) *us = t, best = s;
+    }
+    v.k_iters_per_split = ceil_div(v.k_iters, best);
+    v.k_splits = static_cast<int>(ceil_div(v.k_iters, v.k_iters_per_split));
+    return v;
+}
+
 std::string perm_modes(const Problem& p, const std::vector<int>& ids)
 {
     std::string s;
@@ -1490,7 +1531,27 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
         pl.umma = direct_umma;
     }
     const Problem& p = pl.prob;
-    if (pl.kernel == KERNEL_DMMA_F64_TMA) pl.narrow = narrow_tiles(p, cost, pl.umma);
+    pl.kernel_without_narrow = pl.kernel;
+    if (pl.kernel == KERNEL_DMMA_F64_TMA) {
+        pl.narrow = narrow_tiles(p, cost, pl.umma);
+        double us;
+        // (the smallest estimate has to be 5 % better than the one of what was planned: of 22 contractions in ranges 16 changed, 1.10 times as fast)
+        if (!pl.narrow.eligible && pl.umma.k_splits > 1) {
+            UmmaSpec v = narrow_ranges(p, cost, pl.umma, &us);
+            if (v.eligible && us < 0.95 * split_us(p, pl.umma, pl.umma.k_splits, cost)) pl.narrow = v;
+        }
+    } else if (p.scalar_type == 1 && p.Ktot <= 49152 && !std::getenv("TCONT_KERNEL")) {
+        // The gather kernel's estimate of the smallest contractions is off by up to a factor of two either way (10.9 us estimated: 5.8 to
+        // 12.9): only above 13.5 us does it say enough (17.9 estimated, 18.2 taken; 14.7 here).  Longer sums stay one chain (plan_gather).
+        const double gather_us = contraction_us(p, pl.kernel, pl.umma, cost);
+        double us = 1e300;
+        UmmaSpec v;
+        if (gather_us >= 13.5) v = narrow_ranges(p, cost, pl.umma, &us);
+        if (v.eligible && us < 0.9 * gather_us) {
+            pl.narrow = v;
+            pl.kernel = KERNEL_DMMA_F64_TMA;
+        }
+    }
     if (pl.kernel == KERNEL_UMMA_TF32)
         for (int reads = 0; reads < 2; ++reads)
             pl.est_scaled_us[reads] = (use_ttgt ? ttgt_by_tiles_us : pl.est_direct_us) +
@@ -1570,7 +1631,7 @@ std::string describe_plan(const Plan& pl)
           << ",\"tiles_n\":" << pl.across.tiles_n << ",\"k_iters\":" << pl.across.k_iters << ",\"b_major\":\"" << (pl.across.b_major ? "MN" : "K") << "\"}";
     if (pl.narrow.eligible)
         o << ",\"narrow\":{\"BN\":" << pl.narrow.BN << ",\"BK\":" << pl.narrow.BK << ",\"stages\":" << pl.narrow.stages << ",\"slim\":" << (pl.narrow.slim ? "true" : "false") << ",\"tiles_m\":" << pl.narrow.tiles_m
-          << ",\"tiles_n\":" << pl.narrow.tiles_n << "}";
+          << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << "}";
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";
     else {

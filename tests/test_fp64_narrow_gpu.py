@@ -60,3 +60,40 @@ def test_several_tiles_a_group(engine, oracle, monkeypatch, columns):
         product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
         for beta, out in zip((1.0, 0.0), got):
             assert (np.abs(out - (product + beta * C0)) <= (ext["k"] + 4) * 2.0**-53 * (scale + abs(beta * C0))).all()
+
+
+# what has few tiles -> (descriptor, kernel without narrow tiles)
+RANGES = {
+    "from_the_gather_kernel": ("abcd", "aebf", "fdec", dict(a=24, b=24, c=24, d=24, e=16, f=16), "simt"),
+    "more_ranges_of_less": ("abcd", "aedf", "fbec", dict(a=8, b=16, c=16, d=16, e=56, f=56), "dmma_f64_tma"),
+    "one_range": ("abcd", "deca", "be", dict(a=24, b=40, c=24, d=32, e=312), "dmma_f64_tma"),
+}
+
+
+@pytest.mark.parametrize("name", list(RANGES))
+def test_ranges(engine, oracle, monkeypatch, name):
+    C, A_, B_, ext, _ = RANGES[name]
+    c = Contraction(C, A_, B_, ext, F64)
+    A, B = oracle.inputs(c, 31, -1.0, 1.0)
+    C0 = np.random.default_rng(7).uniform(-4.0, 4.0, c.size(C))
+    desc, got = scaled_run(engine, c, A, B, C0, SCALARS, 0)
+    ranges = desc["narrow"]["k_splits"]
+    assert desc["kernel"] == "dmma_f64_tma" and (ranges == 1) == (name == "one_range")
+    product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
+    k = int(np.prod([ext[m] for m in ext if m not in C]))
+    for (alpha, beta), out in zip(SCALARS, got):   # (and a rounding for each partial sum)
+        bound = (k + ranges + 4) * 2.0**-53 * (abs(alpha) * scale + abs(beta * C0))
+        assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (alpha, beta)
+
+
+def test_no_room_for_ranges(engine, oracle, monkeypatch):
+    """The gather kernel runs where the partial sums find no room."""
+    C, A_, B_, ext, _ = RANGES["from_the_gather_kernel"]
+    c = Contraction(C, A_, B_, ext, F64)
+    A, B = oracle.inputs(c, 31, -1.0, 1.0)
+    monkeypatch.setenv("TCONT_TEST_NO_ROOM", "1000")
+    desc, got = scaled_run(engine, c, A, B, np.ones(c.size(C)), [(1.0, 1.0), (1.0, 0.0)], 0)
+    assert desc["narrow"]["k_splits"] > 1
+    product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
+    for beta, out in zip((1.0, 0.0), got):
+        assert (np.abs(out - (product + beta)) <= (256 + 8) * 2.0**-53 * (scale + beta)).all()

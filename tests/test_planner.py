@@ -370,3 +370,22 @@ def test_fp64_narrow_tiles(engine, monkeypatch):
     assert not d["umma"]["in_use"] and d["narrow"]["BN"] == 32 and d["narrow"]["stages"] % 3 == 0
     monkeypatch.setenv("TCONT_DMMA_BN", "64")
     assert not narrow(rows(4096, 16)) and describe(engine, rows(4096, 16), 1)["umma"]["in_use"]
+
+
+def test_fp64_ranges_on_narrow_tiles(engine, monkeypatch):
+    """Few tiles: ranges of k on narrow tiles in the place of ranges on wide ones, and of the gather kernel above 13.5 us."""
+    F64 = 1
+    small = Contraction("abcd", "aebf", "fdec", dict(a=24, b=24, c=24, d=24, e=16, f=16), F64)
+    d = describe(engine, small)
+    assert d["kernel"] == "dmma_f64_tma" and d["narrow"]["k_splits"] > 1 and not d["umma"]["in_use"]
+    monkeypatch.setenv("TCONT_KERNEL", "gather")
+    assert "narrow" not in describe(engine, small)
+    monkeypatch.delenv("TCONT_KERNEL")
+    smaller = Contraction("ab", "ak", "kb", dict(a=128, b=104, k=496), F64)
+    assert describe(engine, smaller)["kernel"] == "simt" and "narrow" not in describe(engine, smaller)
+    longer = Contraction("ab", "ak", "kb", dict(a=64, b=64, k=60000), F64)   # one chain of FMAs where nothing else was planned
+    assert describe(engine, longer)["kernel"] != "simt" or "narrow" not in describe(engine, longer)
+    many = describe(engine, Contraction("abcd", "aecf", "bfde", dict(a=32, b=32, c=32, d=40, e=16, f=24), F64))
+    assert many["umma"]["k_splits"] == 3 and many["narrow"]["k_splits"] == 2
+    monkeypatch.setenv("TCONT_SPLITK", "3")
+    assert "narrow" not in describe(engine, Contraction("abcd", "aecf", "bfde", dict(a=32, b=32, c=32, d=40, e=16, f=24), F64))
