@@ -12,8 +12,8 @@
 // of k, and the partial tiles are added through distributed shared memory in ascending rank order (one launch,
 // deterministic).
 //
-// What bounds it: large problems the FP64 pipe or the FP32 pipe (5 184^3: FP64 30.0 TFLOP/s, Float32 40, where the 64 x 64
-// kernel before it had 23.7; 3233 x 2773 x 851 FP64 1 055 -> 640 us), small ones the time a lone block needs per k tile (0.5 us
+// What bounds it: large problems the FP64 pipe or the FP32 pipe (5 184^3: FP64 30.0 TFLOP/s; 5 329^3 Float32 49.7, of the 66 that FMAs on
+// registers alone reach, 40 in warps of 128 x 16; 3233 x 2773 x 851 FP64 1 055 -> 640 us), small ones the time a lone block needs per k tile (0.5 us
 // in the 32 x 32 Float32 tile, 1.1 with a fourth of its warps; 0.7 / 1.5 us in the FP64 tiles of 32 / 64) and the way from
 // launch to launch (693 x 47 x 41 Float32 8.2 -> 4.0 us), short contracted extents the stores of C (48825 x 2627 x 7 Float32
 // 332 -> 208 us, 2.5 TB/s of odd-aligned runs).
@@ -116,7 +116,13 @@ struct GatherCfg {
     // Row pitches.  double: 4 past a multiple of 16, so that a fragment load (k = lane % 4, row = lane / 4) touches 16
     // different 8-byte banks per half warp.  float: A 2 past a multiple of 32 (K-major gathers without conflicts), B a
     // multiple of 4 (16-byte fragment loads).
-    static constexpr int LDA = F64 ? BM + 4 : BM + 2, LDB = BN + 4;
+    // WIDE: a Float32 warp tile of 64 x 64, lanes as 8 x 4, lane (m, n) holding rows 4 m .. 4 m + 3 (+ 32) and columns 4 n .. 4 n + 3
+    // (+ 16, 32, 48): all fragments are 16-byte loads, 6 of them to 64 packed FMAs instead of 8 to 32.  Two warps per scheduler, so the
+    // gathers of a later k tile are spread over the FMAs of this one (5329^3 40.5 -> 45.2 TFLOP/s without and 49.8 with that; without any
+    // gathers the FMAs reach 66), and the results leave through shared memory, 128 rows of a column at a time
+    // (sixteen columns' sums and old values asked for together: 3001 x 2001 x 601 in clusters of 2 277 -> 205 us).
+    static constexpr bool WIDE = !F64 && BN / WN == 64;
+    static constexpr int LDA = F64 || WIDE ? BM + 4 : BM + 2, LDB = BN + 4;
     static constexpr int A_ELEMS = BK * LDA, STAGE_ELEMS = (BK * (LDA + LDB) + 3) / 4 * 4;
     // Tiles whose row tables are live at once: the one being multiplied, up to STAGES behind it in the ring, one being built
     static constexpr int TABLES = FLAT ? STAGES + 2 : 1, TABLE_ENTRIES = 2 * (BM + BN);
@@ -127,7 +133,10 @@ struct GatherCfg {
     static_assert(!FLAT || KG == 1, "the ring is never free for partial tiles");
     static_assert((BK * LDA) % 4 == 0, "B tile alignment");
     static_assert(THREADS % BK == 0 && (THREADS % BM == 0) && (THREADS % BN == 0), "gather mapping");
-    static_assert(F64 || BN / WN == 16, "float warp tile is 16 columns wide");
+    static_assert(F64 || WIDE || BN / WN == 16, "float warp tile is 16 columns wide");
+    static_assert(!WIDE || (BM / WM == 64 && BM == BN && THREADS == BM && !FLAT && KG == 1), "wide warp tiles");
+    static constexpr int K_HALF = KTAB / BK / 2;   // WIDE: contracted ranges past KTAB have their k offsets in a ring of two halves
+    static_assert(!WIDE || (K_HALF * BK == THREADS && K_HALF >= STAGES), "one k offset per thread and half");
 };
 
 // Gathers a ROWS x BK operand tile into [k][row] shared memory.  along_k = false: a thread serves one row (`row_ptr`) for
@@ -163,6 +172,34 @@ __device__ __forceinline__ void gather_tile(uint32_t dst, const T* __restrict__ 
         }
     }
 }
+
+// Element i of the BK that a thread gathers of such a tile, by itself, for a block of as many threads as the tile has rows.
+template <typename T, int LD, int BK, int THREADS>
+struct TileGather {
+    const T* from;
+    uint32_t off, off_step;   // where in shared memory the offset of the next element is
+    uint32_t dst, dst_step;
+    int valid;
+    __device__ __forceinline__ void begin(uint32_t tile, const T* X, int row, const T* row_ptr, const long long* row_off, const long long* koff,
+                                          int k_left, bool along_k, int tid)
+    {
+        const int kl = tid % BK, r = tid / BK;
+        from = along_k ? X + koff[kl] : row_ptr;
+        off = smem_addr(along_k ? row_off + r : koff);
+        off_step = (along_k ? THREADS / BK : 1) * 8;
+        dst = tile + static_cast<uint32_t>(along_k ? kl * LD + r : row) * sizeof(T);
+        dst_step = (along_k ? THREADS / BK : LD) * sizeof(T);
+        valid = !along_k ? k_left : kl < k_left ? BK : 0;
+    }
+    __device__ __forceinline__ void element(int i)
+    {
+        long long at;
+        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(at) : "r"(off));
+        cp_async<sizeof(T)>(dst, from + at, i < valid);
+        off += off_step;
+        dst += dst_step;
+    }
+};
 
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kernel(const __grid_constant__ GatherParams p)
@@ -229,7 +266,29 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     const int b_r = tid % BN;
     const T *a_row = A, *b_row = B;
     const uint32_t ring_addr = smem_addr(ring);
+    // WIDE: starts the gathers of the next k tile.  Past the last one nothing is read, its slots are filled with zeros.
+    TileGather<T, LDA, BK, THREADS> next_a;
+    TileGather<T, LDB, BK, THREADS> next_b;
+    auto begin_issue = [&]() {
+        const long long left = k_end - k_begin - static_cast<long long>(is_kt) * BK;
+        const int k_left = left < 0 ? 0 : left < BK ? static_cast<int>(left) : BK, at = is_kt % (2 * Cfg::K_HALF) * BK;
+        const uint32_t st = ring_addr + static_cast<uint32_t>(is_slot * Cfg::STAGE_ELEMS) * sizeof(T);
+        next_a.begin(st, A, a_r, a_row, tables, k_a + at, k_left, a_k, tid);
+        next_b.begin(st + Cfg::A_ELEMS * sizeof(T), B, b_r, b_row, tables + BM, k_b + at, k_left, b_k, tid);
+        ++is_kt;
+        if (++is_slot == STAGES) is_slot = 0;
+    };
     auto issue = [&]() {
+        if constexpr (Cfg::WIDE) {
+            begin_issue();
+#pragma unroll
+            for (int i = 0; i < BK; ++i) {
+                next_a.element(i);
+                next_b.element(i);
+            }
+            cp_async_commit();
+            return;
+        }
         if (is_tile < my_tiles) {
             const long long* tab = tables + (is_tile % Cfg::TABLES) * Cfg::TABLE_ENTRIES;
             if (is_kt == 0) {
@@ -251,7 +310,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     };
 
     const int kg = warp / (Cfg::WM * Cfg::WN), wm = warp % Cfg::WM, wn = warp / Cfg::WM % Cfg::WN;
-    constexpr int FM = F64 ? TILE_M / 8 : TILE_M / 32, FN = F64 ? TILE_N / 8 : TILE_N / 2;
+    constexpr int FM = F64 || Cfg::WIDE ? TILE_M / 8 : TILE_M / 32, FN = F64 || Cfg::WIDE ? TILE_N / 8 : TILE_N / 2;
     using Acc = typename std::conditional<F64, double[2], unsigned long long[1]>::type;
     Acc acc[FM][FN];
 #pragma unroll
@@ -272,7 +331,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     } else {
         build(0);   // (also for the empty range of a cluster split, which only takes part in the sum below)
     }
-    if (k_whole) {
+    if (Cfg::WIDE) {
+        for (int t = tid / BK; t < 2 * Cfg::K_HALF; t += Cfg::K_HALF) fill_k(t, t * BK, tid % BK);
+    } else if (k_whole) {
         for (int i = tid; i < nk * BK; i += THREADS) fill_k(i / BK, i / BK * BK, i % BK);
     } else if (tid < STAGES * BK) {
         fill_k(tid / BK, tid / BK * BK, tid % BK);
@@ -281,6 +342,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     chain_wait();   // (everything above works on the parameters alone)
     __syncthreads();
 
+    if (Cfg::WIDE) {
+        a_row = A + tables[a_r];
+        b_row = B + tables[BM + b_r];
+    }
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) issue();
     const uint32_t steps = nk > 0 ? my_tiles * static_cast<uint32_t>(nk) : 0u;
@@ -289,10 +354,19 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     for (uint32_t q = 0; q < steps; ++q) {
         cp_async_wait<STAGES - 2>();
         __syncthreads();   // step q has landed for everyone; the slot refilled below was read at step q - 1
-        issue();
+        if constexpr (Cfg::WIDE) {
+            // the k offsets of the half ring after next, once those that lie there have all been used
+            if (is_kt % Cfg::K_HALF == 0) {
+                const int t = is_kt + Cfg::K_HALF + tid / BK;
+                fill_k(t, t % (2 * Cfg::K_HALF) * BK, tid % BK);
+            }
+            begin_issue();
+        } else {
+            issue();
+        }
         // what step q + STAGES needs, one barrier ahead of its issue
         if (Cfg::FLAT && is_kt == 0 && is_tile < my_tiles) build(is_tile);
-        if (!k_whole && tid < BK) fill_k(is_kt, slot * BK, tid);
+        if (!Cfg::WIDE && !k_whole && tid < BK) fill_k(is_kt, slot * BK, tid);
         if (add && kt == 0) {
             // the tile's old values into L2 while it is multiplied: the epilogue reads them a few at a time
             const long long* c_m = tables + (tile % Cfg::TABLES) * Cfg::TABLE_ENTRIES + BM + BN;
@@ -335,7 +409,27 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
 #pragma unroll
                     for (int j = 0; j < FN; ++j) ffma2(acc[i][j][0], a[i], b[j]);
             };
-            if (!Cfg::FLAT || left >= BK) {
+            if constexpr (Cfg::WIDE) {
+#pragma unroll
+                for (int k = 0; k < BK; ++k) {
+                    float4 a4[FM / 4];
+                    ulonglong2 b4[FN / 2];
+#pragma unroll
+                    for (int i = 0; i < FM / 4; ++i) a4[i] = *reinterpret_cast<const float4*>(As + k * LDA + wm * TILE_M + i * 32 + (lane & 7) * 4);
+#pragma unroll
+                    for (int j = 0; j < FN / 2; ++j) b4[j] = *reinterpret_cast<const ulonglong2*>(Bs + k * LDB + wn * TILE_N + j * 16 + (lane >> 3) * 4);
+                    next_a.element(k);
+                    next_b.element(k);
+#pragma unroll
+                    for (int i = 0; i < FM; ++i) {
+                        const float4 v = a4[i / 4];
+                        const unsigned long long a = dup2(i % 4 == 0 ? v.x : i % 4 == 1 ? v.y : i % 4 == 2 ? v.z : v.w);
+#pragma unroll
+                        for (int j = 0; j < FN; ++j) ffma2(acc[i][j][0], a, j & 1 ? b4[j / 2].y : b4[j / 2].x);
+                    }
+                }
+                cp_async_commit();
+            } else if (!Cfg::FLAT || left >= BK) {
 #pragma unroll
                 for (int k = 0; k < BK / Cfg::KG; ++k) step(k * Cfg::KG + kg);
             } else {
@@ -345,7 +439,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
         if (++slot == STAGES) slot = 0;
         if (++kt < nk) continue;
         kt = 0;
-        if (!Cfg::FLAT && (Cfg::KG > 1 || S > 1)) break;
+        if (Cfg::WIDE || (!Cfg::FLAT && (Cfg::KG > 1 || S > 1))) break;
         const long long* c_m = tables + (tile % Cfg::TABLES) * Cfg::TABLE_ENTRIES + BM + BN;
         const long long* c_n = c_m + BM;
         ++tile;
@@ -404,7 +498,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
         }
     }
     cp_async_wait<0>();
-    if (Cfg::FLAT || (Cfg::KG == 1 && S == 1)) return;
+    if (!Cfg::WIDE && (Cfg::FLAT || (Cfg::KG == 1 && S == 1))) return;
     if (p.release_late) chain_release();   // (not inside the loop: a test there costs the FP64 main loop 3 to 8 %)
 
     // k groups and cluster split: partial tiles into this CTA's shared memory as [group][n][m]; CTA r then adds up columns
@@ -419,6 +513,15 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
             for (int j = 0; j < FN; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) mine[(wn * TILE_N + j * 8 + 2 * fk + h) * BM + wm * TILE_M + i * 8 + fr] = acc[i][j][h];
+    } else if constexpr (Cfg::WIDE) {
+#pragma unroll
+        for (int i = 0; i < FM; i += 4)
+#pragma unroll
+            for (int j = 0; j < FN; ++j) {
+                float* to = mine + (wn * TILE_N + (j >> 1) * 16 + (lane >> 3) * 4 + (j & 1) * 2) * BM + wm * TILE_M + i * 8 + (lane & 7) * 4;
+                *reinterpret_cast<float4*>(to) = make_float4(lo2(acc[i][j][0]), lo2(acc[i + 1][j][0]), lo2(acc[i + 2][j][0]), lo2(acc[i + 3][j][0]));
+                *reinterpret_cast<float4*>(to + BM) = make_float4(hi2(acc[i][j][0]), hi2(acc[i + 1][j][0]), hi2(acc[i + 2][j][0]), hi2(acc[i + 3][j][0]));
+            }
     } else {
 #pragma unroll
         for (int i = 0; i < FM; ++i)
@@ -437,17 +540,44 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     constexpr int COLS_STEP = THREADS / BM;   // columns the block handles at a time (threads run along m)
     const int m = tid % BM;
     const long long cm = c_m[m];
-    for (uint32_t nl = rank + S * static_cast<uint32_t>(tid / BM); nl < static_cast<uint32_t>(BN); nl += S * COLS_STEP) {
-        const long long cn = c_n[nl];
-        if (cm < 0 || cn < 0) continue;
-        T v = 0;
-        for (uint32_t s = 0; s < S; ++s) {
-            const T* from = (S > 1 ? cluster.map_shared_rank(part, s) : part) + nl * BM + m;
+    if constexpr (Cfg::WIDE) {
+        // 16 columns at a time, their old values asked for before the first is used
+        constexpr int AT_ONCE = 16;
+        for (uint32_t n0 = rank; n0 < static_cast<uint32_t>(BN); n0 += S * AT_ONCE) {
+            long long cn[AT_ONCE];
+            T old[AT_ONCE], v[AT_ONCE];
 #pragma unroll
-            for (int g = 0; g < Cfg::KG; ++g) v += from[g * BM * BN];
+            for (int u = 0; u < AT_ONCE; ++u) {
+                const uint32_t nl = n0 + S * u;
+                cn[u] = nl < static_cast<uint32_t>(BN) && cm >= 0 ? c_n[nl] : -1;
+                old[u] = add && cn[u] >= 0 ? C[cm + cn[u]] : T(0);
+                v[u] = 0;
+            }
+            for (uint32_t s = 0; s < S; ++s) {
+                const T* from = S > 1 ? cluster.map_shared_rank(part, s) : part;
+#pragma unroll
+                for (int u = 0; u < AT_ONCE; ++u)
+                    if (cn[u] >= 0) v[u] += from[(n0 + S * u) * BM + m];
+            }
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) {
+                if (scaled) v[u] = alpha * v[u] + beta * old[u];
+                if (cn[u] >= 0) __stcs(C + cm + cn[u], v[u]);
+            }
         }
-        if (scaled) v = alpha * v + (add ? beta * C[cm + cn] : T(0));
-        __stcs(C + cm + cn, v);
+    } else {
+        for (uint32_t nl = rank + S * static_cast<uint32_t>(tid / BM); nl < static_cast<uint32_t>(BN); nl += S * COLS_STEP) {
+            const long long cn = c_n[nl];
+            if (cm < 0 || cn < 0) continue;
+            T v = 0;
+            for (uint32_t s = 0; s < S; ++s) {
+                const T* from = (S > 1 ? cluster.map_shared_rank(part, s) : part) + nl * BM + m;
+#pragma unroll
+                for (int g = 0; g < Cfg::KG; ++g) v += from[g * BM * BN];
+            }
+            if (scaled) v = alpha * v + (add ? beta * C[cm + cn] : T(0));
+            __stcs(C + cm + cn, v);
+        }
     }
     if (S > 1) cluster.sync();   // a CTA's shared memory stays until every other has read it
 }
@@ -485,12 +615,25 @@ using F64TallFlat = GatherCfg<double, 128, 32, 4, 1, 1, true, 3, 2>;
 using F64Small = GatherCfg<double, 32, 32, 1, 1, 4, false, 4, 4>;
 using F64SmallFlat = GatherCfg<double, 32, 32, 2, 2, 1, true, 4, 4>;
 using F32Big = GatherCfg<float, 128, 128, 1, 8, 1, false, 4, 2>;
+using F32Wide = GatherCfg<float, 128, 128, 2, 2, 1, false, 4, 2>;
 using F32BigFlat = GatherCfg<float, 128, 128, 1, 8, 1, true, 4, 2>;
 using F32Square = GatherCfg<float, 64, 64, 1, 4, 1, false, 4, 4>;
 using F32SquareFlat = GatherCfg<float, 64, 64, 1, 4, 1, true, 4, 4>;
 using F32Tall = GatherCfg<float, 128, 32, 2, 2, 1, false, 4, 4>;
 using F32TallFlat = GatherCfg<float, 128, 32, 2, 2, 1, true, 4, 3>;
 using F32Small = GatherCfg<float, 32, 32, 1, 2, 4, false, 4, 4>;
+
+// Whether the 128 x 128 Float32 tile runs in four wide warps instead of eight.  A wide block takes longer to begin and to end, with
+// half the threads, the more so in a large cluster, and has to make that good in its range of k.  Old / wide in us, by k per block:
+// one block to a tile, 5003 x 3001: 101 108 / 111, 201 194 / 183, 601 513 / 442; clusters of 2, 1401 x 1401: 100 52 / 39, 300 87 / 73;
+// of 4, 1801 x 1501: 75 77 / 80, 100 107 / 98; of 8, 701 x 701: 75 39 / 46, 400 170 / 142.  With no more blocks than SMs the one warp
+// on each scheduler has its latencies to itself (301 x 301 x 9201 in clusters of 16: 103 / 102), so the old kind stays there.
+bool wide(const GatherParams& p, int num_sms)
+{
+    const long long blocks = (p.M + F32Wide::BM - 1) / F32Wide::BM * ((p.N + F32Wide::BN - 1) / F32Wide::BN) * p.cluster;
+    const int least_k = p.cluster == 1 ? 160 : p.cluster <= 4 ? 96 : 192;
+    return blocks > num_sms && p.K / p.cluster >= least_k;
+}
 
 }  // namespace
 
@@ -508,6 +651,7 @@ cudaError_t gather_configure()
     set(gather_contract_kernel<F64Small>, F64Small::SMEM);
     set(gather_contract_kernel<F64SmallFlat>, F64SmallFlat::SMEM);
     set(gather_contract_kernel<F32Big>, F32Big::SMEM);
+    set(gather_contract_kernel<F32Wide>, F32Wide::SMEM);
     set(gather_contract_kernel<F32BigFlat>, F32BigFlat::SMEM);
     set(gather_contract_kernel<F32Square>, F32Square::SMEM);
     set(gather_contract_kernel<F32SquareFlat>, F32SquareFlat::SMEM);
@@ -525,6 +669,7 @@ cudaError_t launch_gather_contract(const GatherParams& p, int scalar_type, int t
         if (tile == GATHER_TALL) return p.flat ? launch<F64TallFlat>(p, num_sms, stream) : launch<F64Tall>(p, num_sms, stream);
         if (tile == GATHER_SMALL) return p.flat ? launch<F64SmallFlat>(p, num_sms, stream) : launch<F64Small>(p, num_sms, stream);
     } else {
+        if (tile == GATHER_BIG && !p.flat && wide(p, num_sms)) return launch<F32Wide>(p, num_sms, stream);
         if (tile == GATHER_BIG) return p.flat ? launch<F32BigFlat>(p, num_sms, stream) : launch<F32Big>(p, num_sms, stream);
         if (tile == GATHER_SQUARE) return p.flat ? launch<F32SquareFlat>(p, num_sms, stream) : launch<F32Square>(p, num_sms, stream);
         if (tile == GATHER_TALL) return p.flat ? launch<F32TallFlat>(p, num_sms, stream) : launch<F32Tall>(p, num_sms, stream);
