@@ -540,28 +540,33 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     constexpr int COLS_STEP = THREADS / BM;   // columns the block handles at a time (threads run along m)
     const int m = tid % BM;
     const long long cm = c_m[m];
-    if constexpr (Cfg::WIDE) {
-        // 16 columns at a time, their old values asked for before the first is used
-        constexpr int AT_ONCE = 16;
-        for (uint32_t n0 = rank; n0 < static_cast<uint32_t>(BN); n0 += S * AT_ONCE) {
+    if (Cfg::WIDE || (BM * BN > 1024 && S <= 4)) {
+        // Several columns at a time, so that neither C's old values nor other SMs' shared memory is waited for one by one.  Before / after
+        // in us, 64 x 64 tiles in clusters of 2 and 4: 1061 x 679 x 245 Float32 28.9 / 23.9, 34891 x 37 x 159 FP64 accumulating
+        // 63.7 / 50.1.  In larger clusters a thread has a column or two to add up: 295 x 189 x 955 FP64, clusters of 16, 17.5 / 22.1.
+        constexpr int AT_ONCE = Cfg::WIDE ? 16 : 4;
+        for (uint32_t n0 = rank + S * static_cast<uint32_t>(tid / BM); n0 < static_cast<uint32_t>(BN); n0 += S * COLS_STEP * AT_ONCE) {
             long long cn[AT_ONCE];
             T old[AT_ONCE], v[AT_ONCE];
 #pragma unroll
             for (int u = 0; u < AT_ONCE; ++u) {
-                const uint32_t nl = n0 + S * u;
+                const uint32_t nl = n0 + S * COLS_STEP * u;
                 cn[u] = nl < static_cast<uint32_t>(BN) && cm >= 0 ? c_n[nl] : -1;
                 old[u] = add && cn[u] >= 0 ? C[cm + cn[u]] : T(0);
                 v[u] = 0;
             }
             for (uint32_t s = 0; s < S; ++s) {
-                const T* from = S > 1 ? cluster.map_shared_rank(part, s) : part;
+                const T* from = (S > 1 ? cluster.map_shared_rank(part, s) : part) + n0 * BM + m;
 #pragma unroll
-                for (int u = 0; u < AT_ONCE; ++u)
-                    if (cn[u] >= 0) v[u] += from[(n0 + S * u) * BM + m];
+                for (int u = 0; u < AT_ONCE; ++u) {
+                    if (Cfg::WIDE ? n0 + S * COLS_STEP * u >= static_cast<uint32_t>(BN) : cn[u] < 0) continue;   // (wide: rows that are not stored take part)
+#pragma unroll
+                    for (int g = 0; g < Cfg::KG; ++g) v[u] += from[S * COLS_STEP * u * BM + g * BM * BN];
+                }
             }
 #pragma unroll
             for (int u = 0; u < AT_ONCE; ++u) {
-                if (scaled) v[u] = alpha * v[u] + beta * old[u];
+                if (scaled) v[u] = alpha * v[u] + (add ? beta * old[u] : T(0));
                 if (cn[u] >= 0) __stcs(C + cm + cn[u], v[u]);
             }
         }

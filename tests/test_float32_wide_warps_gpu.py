@@ -1,6 +1,6 @@
 """Float32 on the CUDA cores in 128 x 128 tiles of four wide warps: gathers along rows and along k on either side, a last k tile that is
-whole and one that is not, contracted ranges in one ring of offsets and past it, one range and clusters, rows
-that C and A hold in different orders.
+whole and one that is not, contracted ranges in one ring of offsets and past it, one range and clusters, rows that C and A hold in
+different orders; and the sums of small clusters of 64 x 64 tiles.
 
 Every output is a chain of K single-precision fused multiply-adds (the sums of a cluster's ranges a few more additions) and three roundings
 of the scalars, each off by at most 2^-24 of its partial sum.
@@ -8,7 +8,7 @@ of the scalars, each off by at most 2^-24 of its partial sum.
 import numpy as np
 import pytest
 
-from oracle_lib import F32, Contraction
+from oracle_lib import F32, F64, Contraction
 from test_scaled_epilogues_gpu import SCALARS, scaled_run
 
 pytestmark = pytest.mark.gpu
@@ -35,9 +35,26 @@ def test_forms(engine, oracle, monkeypatch, name):
     desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
     assert desc["kernel"] == "simt" and desc["gather"]["tile"] == 3 and not desc["gather"]["flat"], desc["gather"]
     assert desc["gather"]["cluster"] == cluster, desc["gather"]
-    c64 = Contraction(C, A_, B_, ext, 1)
+    c64 = Contraction(C, A_, B_, ext, F64)
     product, scale = oracle.contract(c64, A.astype(np.float64), B.astype(np.float64)), oracle.contract(c64, np.abs(A).astype(np.float64), np.abs(B).astype(np.float64))
     k = int(np.prod([ext[m] for m in A_ if m not in C]))
     for (alpha, beta), out in zip(SCALARS, got):
         bound = (k + 20) * 2.0**-24 * (abs(alpha) * scale + abs(beta * C0))
         assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (name, alpha, beta)
+
+
+@pytest.mark.parametrize("scalar_type,a,b,k,cluster", [(F32, 3001, 131, 131, 2), (F32, 331, 679, 245, 4), (F64, 1061, 679, 131, 2), (F64, 331, 679, 245, 4)])
+def test_small_clusters_of_64_by_64_tiles(engine, oracle, monkeypatch, scalar_type, a, b, k, cluster):
+    """Sums over 2 and 4 blocks four columns at a time, the last tile of a row with a few columns of its own."""
+    monkeypatch.setenv("TCONT_KERNEL", "simt")
+    c = Contraction("ab", "ka", "bk", dict(a=a, b=b, k=k), scalar_type)
+    A, B = oracle.inputs(c, 37, -1.0, 1.0)
+    C0 = np.random.default_rng(8).uniform(-4.0, 4.0, c.size("ab")).astype(A.dtype)
+    desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
+    assert desc["gather"]["tile"] == 0 and desc["gather"]["cluster"] == cluster, desc["gather"]
+    c64 = Contraction("ab", "ka", "bk", dict(a=a, b=b, k=k), F64)
+    product, scale = oracle.contract(c64, A.astype(np.float64), B.astype(np.float64)), oracle.contract(c64, np.abs(A).astype(np.float64), np.abs(B).astype(np.float64))
+    unit = 2.0**-24 if scalar_type == F32 else 2.0**-53
+    for (alpha, beta), out in zip(SCALARS, got):
+        bound = (k + 20) * unit * (abs(alpha) * scale + abs(beta * C0))
+        assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (alpha, beta)
