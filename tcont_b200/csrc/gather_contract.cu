@@ -116,13 +116,16 @@ struct GatherCfg {
     // Row pitches.  double: 4 past a multiple of 16, so that a fragment load (k = lane % 4, row = lane / 4) touches 16
     // different 8-byte banks per half warp.  float: A 2 past a multiple of 32 (K-major gathers without conflicts), B a
     // multiple of 4 (16-byte fragment loads).
-    // WIDE: a Float32 warp tile of 64 x 64, lanes as 8 x 4, lane (m, n) holding rows 4 m .. 4 m + 3 (+ 32) and columns 4 n .. 4 n + 3
-    // (+ 16, 32, 48): all fragments are 16-byte loads, 6 of them to 64 packed FMAs instead of 8 to 32.  Two warps per scheduler, so the
-    // gathers of a later k tile are spread over the FMAs of this one (5329^3 40.5 -> 45.2 TFLOP/s without and 49.8 with that; without any
-    // gathers the FMAs reach 66), and the results leave through shared memory, 128 rows of a column at a time
-    // (sixteen columns' sums and old values asked for together: 3001 x 2001 x 601 in clusters of 2 277 -> 205 us).
-    static constexpr bool WIDE = !F64 && BN / WN == 64;
-    static constexpr int LDA = F64 || WIDE ? BM + 4 : BM + 2, LDB = BN + 4;
+    // GRID: a Float32 warp tile of 32 x 32 or 64 x 64, lanes as 8 x 4, lane (m, n) holding rows 4 m .. 4 m + 3 (+ 32) and columns
+    // 4 n .. 4 n + 3 (+ 16, 32, 48): all fragments are 16-byte loads, 3 of them to 16 packed FMAs instead of 6, or 6 to 64 instead of 8 to
+    // 32, and the results leave through shared memory, whole columns of the tile.  45 drawn contractions on 64 x 64 tiles are 1.11 times
+    // as fast (675 x 825 x 990 94 -> 75 us); on 128 x 32 tiles, whose columns are often few, as many are slower as faster (9177 x 18 x
+    // 301 27 -> 35, 3060 x 23 x 313 12.5 -> 15.4, others 10 % faster), so those keep lines of rows.
+    // WIDE: 64 x 64.  Two warps per scheduler, so the gathers of a later k tile are spread over the FMAs of this one (5329^3 40.5 -> 45.2
+    // TFLOP/s without and 49.8 with that; without any gathers the FMAs reach 66), and sixteen columns leave at a time (3001 x 2001 x 601 in
+    // clusters of 2 277 -> 205 us).
+    static constexpr bool WIDE = !F64 && BN / WN == 64, GRID = !F64 && BN / WN >= 32;
+    static constexpr int LDA = F64 || GRID ? BM + 4 : BM + 2, LDB = BN + 4;
     static constexpr int A_ELEMS = BK * LDA, STAGE_ELEMS = (BK * (LDA + LDB) + 3) / 4 * 4;
     // Tiles whose row tables are live at once: the one being multiplied, up to STAGES behind it in the ring, one being built
     static constexpr int TABLES = FLAT ? STAGES + 2 : 1, TABLE_ENTRIES = 2 * (BM + BN);
@@ -133,7 +136,8 @@ struct GatherCfg {
     static_assert(!FLAT || KG == 1, "the ring is never free for partial tiles");
     static_assert((BK * LDA) % 4 == 0, "B tile alignment");
     static_assert(THREADS % BK == 0 && (THREADS % BM == 0) && (THREADS % BN == 0), "gather mapping");
-    static_assert(F64 || WIDE || BN / WN == 16, "float warp tile is 16 columns wide");
+    static_assert(F64 || GRID || BN / WN == 16, "float warp tile is 16 columns wide");
+    static_assert(!GRID || (BM / WM % 32 == 0 && !FLAT && KG == 1), "float warp tile of lanes 8 x 4");
     static_assert(!WIDE || (BM / WM == 64 && BM == BN && THREADS == BM && !FLAT && KG == 1), "wide warp tiles");
     static constexpr int K_HALF = KTAB / BK / 2;   // WIDE: contracted ranges past KTAB have their k offsets in a ring of two halves
     static_assert(!WIDE || (K_HALF * BK == THREADS && K_HALF >= STAGES), "one k offset per thread and half");
@@ -310,7 +314,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
     };
 
     const int kg = warp / (Cfg::WM * Cfg::WN), wm = warp % Cfg::WM, wn = warp / Cfg::WM % Cfg::WN;
-    constexpr int FM = F64 || Cfg::WIDE ? TILE_M / 8 : TILE_M / 32, FN = F64 || Cfg::WIDE ? TILE_N / 8 : TILE_N / 2;
+    constexpr int FM = F64 || Cfg::GRID ? TILE_M / 8 : TILE_M / 32, FN = F64 || Cfg::GRID ? TILE_N / 8 : TILE_N / 2;
     using Acc = typename std::conditional<F64, double[2], unsigned long long[1]>::type;
     Acc acc[FM][FN];
 #pragma unroll
@@ -409,7 +413,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
 #pragma unroll
                     for (int j = 0; j < FN; ++j) ffma2(acc[i][j][0], a[i], b[j]);
             };
-            if constexpr (Cfg::WIDE) {
+            if constexpr (Cfg::GRID) {
 #pragma unroll
                 for (int k = 0; k < BK; ++k) {
                     float4 a4[FM / 4];
@@ -418,8 +422,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
                     for (int i = 0; i < FM / 4; ++i) a4[i] = *reinterpret_cast<const float4*>(As + k * LDA + wm * TILE_M + i * 32 + (lane & 7) * 4);
 #pragma unroll
                     for (int j = 0; j < FN / 2; ++j) b4[j] = *reinterpret_cast<const ulonglong2*>(Bs + k * LDB + wn * TILE_N + j * 16 + (lane >> 3) * 4);
-                    next_a.element(k);
-                    next_b.element(k);
+                    if constexpr (Cfg::WIDE) {
+                        next_a.element(k);
+                        next_b.element(k);
+                    }
 #pragma unroll
                     for (int i = 0; i < FM; ++i) {
                         const float4 v = a4[i / 4];
@@ -428,7 +434,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
                         for (int j = 0; j < FN; ++j) ffma2(acc[i][j][0], a, j & 1 ? b4[j / 2].y : b4[j / 2].x);
                     }
                 }
-                cp_async_commit();
+                if constexpr (Cfg::WIDE) cp_async_commit();
             } else if (!Cfg::FLAT || left >= BK) {
 #pragma unroll
                 for (int k = 0; k < BK / Cfg::KG; ++k) step(k * Cfg::KG + kg);
@@ -439,7 +445,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
         if (++slot == STAGES) slot = 0;
         if (++kt < nk) continue;
         kt = 0;
-        if (Cfg::WIDE || (!Cfg::FLAT && (Cfg::KG > 1 || S > 1))) break;
+        if (Cfg::GRID || (!Cfg::FLAT && (Cfg::KG > 1 || S > 1))) break;
         const long long* c_m = tables + (tile % Cfg::TABLES) * Cfg::TABLE_ENTRIES + BM + BN;
         const long long* c_n = c_m + BM;
         ++tile;
@@ -498,7 +504,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
         }
     }
     cp_async_wait<0>();
-    if (!Cfg::WIDE && (Cfg::FLAT || (Cfg::KG == 1 && S == 1))) return;
+    if (!Cfg::GRID && (Cfg::FLAT || (Cfg::KG == 1 && S == 1))) return;
     if (p.release_late) chain_release();   // (not inside the loop: a test there costs the FP64 main loop 3 to 8 %)
 
     // k groups and cluster split: partial tiles into this CTA's shared memory as [group][n][m]; CTA r then adds up columns
@@ -513,7 +519,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) gather_contract_kerne
             for (int j = 0; j < FN; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) mine[(wn * TILE_N + j * 8 + 2 * fk + h) * BM + wm * TILE_M + i * 8 + fr] = acc[i][j][h];
-    } else if constexpr (Cfg::WIDE) {
+    } else if constexpr (Cfg::GRID) {
 #pragma unroll
         for (int i = 0; i < FM; i += 4)
 #pragma unroll
@@ -622,7 +628,8 @@ using F64SmallFlat = GatherCfg<double, 32, 32, 2, 2, 1, true, 4, 4>;
 using F32Big = GatherCfg<float, 128, 128, 1, 8, 1, false, 4, 2>;
 using F32Wide = GatherCfg<float, 128, 128, 2, 2, 1, false, 4, 2>;
 using F32BigFlat = GatherCfg<float, 128, 128, 1, 8, 1, true, 4, 2>;
-using F32Square = GatherCfg<float, 64, 64, 1, 4, 1, false, 4, 4>;
+using F32Square = GatherCfg<float, 64, 64, 2, 2, 1, false, 4, 4>;
+using F32SquareShort = GatherCfg<float, 64, 64, 1, 4, 1, false, 4, 4>;
 using F32SquareFlat = GatherCfg<float, 64, 64, 1, 4, 1, true, 4, 4>;
 using F32Tall = GatherCfg<float, 128, 32, 2, 2, 1, false, 4, 4>;
 using F32TallFlat = GatherCfg<float, 128, 32, 2, 2, 1, true, 4, 3>;
@@ -659,6 +666,7 @@ cudaError_t gather_configure()
     set(gather_contract_kernel<F32Wide>, F32Wide::SMEM);
     set(gather_contract_kernel<F32BigFlat>, F32BigFlat::SMEM);
     set(gather_contract_kernel<F32Square>, F32Square::SMEM);
+    set(gather_contract_kernel<F32SquareShort>, F32SquareShort::SMEM);
     set(gather_contract_kernel<F32SquareFlat>, F32SquareFlat::SMEM);
     set(gather_contract_kernel<F32Tall>, F32Tall::SMEM);
     set(gather_contract_kernel<F32TallFlat>, F32TallFlat::SMEM);
@@ -676,6 +684,8 @@ cudaError_t launch_gather_contract(const GatherParams& p, int scalar_type, int t
     } else {
         if (tile == GATHER_BIG && !p.flat && wide(p, num_sms)) return launch<F32Wide>(p, num_sms, stream);
         if (tile == GATHER_BIG) return p.flat ? launch<F32BigFlat>(p, num_sms, stream) : launch<F32Big>(p, num_sms, stream);
+        // One block to a tile and few k: direct stores of whole lines (126 x 145 x 95 by 27 10.6 us, 11.3 by way of shared memory).
+        if (tile == GATHER_SQUARE && !p.flat && p.cluster == 1 && p.K < 48) return launch<F32SquareShort>(p, num_sms, stream);
         if (tile == GATHER_SQUARE) return p.flat ? launch<F32SquareFlat>(p, num_sms, stream) : launch<F32Square>(p, num_sms, stream);
         if (tile == GATHER_TALL) return p.flat ? launch<F32TallFlat>(p, num_sms, stream) : launch<F32Tall>(p, num_sms, stream);
         if (tile == GATHER_SMALL && !p.flat) return launch<F32Small>(p, num_sms, stream);

@@ -58,3 +58,23 @@ def test_small_clusters_of_64_by_64_tiles(engine, oracle, monkeypatch, scalar_ty
     for (alpha, beta), out in zip(SCALARS, got):
         bound = (k + 20) * unit * (abs(alpha) * scale + abs(beta * C0))
         assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (alpha, beta)
+
+
+@pytest.mark.parametrize("cluster,A_,B_,k", [(1, "ka", "bk", 47), (1, "ka", "bk", 49), (1, "ak", "kb", 48), (2, "ak", "kb", 131), (2, "ka", "bk", 49)])
+def test_64_by_64_tiles(engine, oracle, monkeypatch, cluster, A_, B_, k):
+    """Warps of 32 x 32 with lanes 8 x 4, and one block's short range of k in warps of full lines."""
+    monkeypatch.setenv("TCONT_KERNEL", "simt")
+    monkeypatch.setenv("TCONT_GATHER_TILE", "0")
+    monkeypatch.setenv("TCONT_GATHER_CLUSTER", str(cluster))
+    monkeypatch.setenv("TCONT_GATHER_FLAT", "0")
+    ext = dict(a=323, b=103, k=k)
+    c, c64 = Contraction("ab", A_, B_, ext, F32), Contraction("ab", A_, B_, ext, F64)
+    A, B = oracle.inputs(c, 41, -1.0, 1.0)
+    C0 = np.random.default_rng(9).uniform(-4.0, 4.0, c.size("ab")).astype(np.float32)
+    desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
+    g = desc["gather"]
+    assert g["tile"] == 0 and g["cluster"] == cluster and not g["flat"], g
+    product, scale = oracle.contract(c64, A.astype(np.float64), B.astype(np.float64)), oracle.contract(c64, np.abs(A).astype(np.float64), np.abs(B).astype(np.float64))
+    for (alpha, beta), out in zip(SCALARS, got):
+        bound = (k + 20) * 2.0**-24 * (abs(alpha) * scale + abs(beta * C0))
+        assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (alpha, beta)
