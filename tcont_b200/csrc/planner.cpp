@@ -961,7 +961,12 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors 
             if (us < best.est_us) {
                 best = g;
                 best.cluster = s;
-                best.flat = flat;
+                // One column of Float32 tiles: blocks of one tile each, of which more fit an SM at different stages, read a long A in
+                // step better than a few persistent ones.  Persistent / one tile a block in us, 64 x 64: 2689715 x 37 x 19 1491 / 873,
+                // 4604655 x 55 x 33 5106 / 3044, 100233 x 49 x 25 23.8 / 22.8, but 423948 x 59 x 50 127 / 131; 128 x 128: 462231 x 69 x 43
+                // 311 / 247, 769356 x 71 x 57 470 / 429, but 1026189 x 95 x 23 308 / 325.  FP64 is up to twice as slow that way.
+                const bool few_k_tiles = (t == GATHER_SQUARE && iters >= 2 && iters <= 3) || (t == GATHER_BIG && iters >= 3);
+                best.flat = flat && (f64 || tiles_n > 1 || !few_k_tiles);
                 if (force_flat) best.flat = s == 1 && force_flat[0] == '1' && (f64 || t != GATHER_SMALL);   // (the small Float32 tile has no such form)
                 best.est_us = us;
                 sector_us = double(scattered_a * g.rows * tiles_n + scattered_b * p.Ntot * tiles_m) * double(p.Ktot) * 32.0 / (c.gather_sector_gbs * 1e3);
