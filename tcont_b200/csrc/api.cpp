@@ -353,7 +353,7 @@ tcontb_status encode_map(const UmmaOperand& o, const void* base, int elt, CUtens
     return TCONTB_OK;
 }
 
-// Test hooks of the bounded-wait exit (tcgen05 kernels only; see UmmaParams).
+// Test hooks of the bounded-wait exit (see UmmaParams).
 void set_test_hooks(unsigned long long* wait_limit_ns, int* skip_iter)
 {
     const char* limit = std::getenv("TCONT_TEST_WAIT_LIMIT_NS");

@@ -24,7 +24,8 @@
 // 64 bytes that four lanes have together: with 32-byte pieces of one lane each 9216 x 4096 x 24 took 94 us, with these 76).
 // The loads of the next k step are issued between the MMAs of the current one, which go column fragment by column fragment
 // (5184^3 8 225 us, row by row 8 266).
-// Every wait is bounded and raises the run's status word instead of hanging.
+// Every wait is bounded and raises the run's status word instead of hanging.  Behind one that gave up a group stores nothing, and the
+// block ends when the copies that were issued have landed.
 //
 // Stands where the reference runs its generated FP64 WMMA kernels
 // (backends/cogent/plan/generators/kernels/kernel_compute.py:127-850) and its cublasGemmEx FP64
@@ -305,6 +306,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     const uint32_t total_tiles = tiles_m * tiles_n * static_cast<uint32_t>(p.k_splits);  // work units (tile, k range)
     const uint32_t my_tiles = blockIdx.x < total_tiles ? (total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const uint32_t ring = static_cast<uint32_t>(p.stages) / G;  // stages per group
+    auto block_done = [] { asm volatile("bar.sync 0;" ::: "memory"); };   // the role's last act, but for what is in flight
 
     if (warp < 4) {
         if (G == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -327,9 +329,8 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             KSteps ks;
             k_steps(o, ks);
             uint32_t stage = 0, phase = 0;
-            uint32_t issued_mask = 0, issued_parity = 0;
             bool ok = true;
-            for (uint32_t i = static_cast<uint32_t>(warp); i < my_tiles; i += G) {
+            for (uint32_t i = static_cast<uint32_t>(warp); ok && i < my_tiles; i += G) {
                 const WorkUnit w = decode_unit(blockIdx.x + i * gridDim.x, p, tiles_m, tiles_n);
                 const uint32_t tm = w.tm, tn = w.tn;
                 int base[kMaxTmaRank];
@@ -342,8 +343,13 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 }
                 for (int it = 0; it < w.n_it; ++it) {
                     const uint32_t ps = first + stage;
-                    ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(bar_empty + ps), phase ^ 1u, abort_flag, 200u));
-                    if (ok) {
+                    ok = __all_sync(0xffffffffu, mbar_wait_for(smem_u32(bar_empty + ps), phase ^ 1u, abort_flag, 200u, p.wait_limit_ns));
+                    // (a stage given back behind a wait that gave up may never have been filled, or is still on its way: not filled again.  Asked
+                    // here, one producer warp reads one word a stage; 9216 x 4096 x 24 accumulating into a 6-D C 120.8 us, 121.9 with it, 123.1
+                    // where the warps that gave up keep their stages)
+                    ok = ok && ld_shared_u32(abort_flag) == 0u;
+                    if (!ok) break;
+                    if (static_cast<int>(i) * p.k_iters_per_split + it != p.test_skip_iter) {
                         if (lane == 0) mbar_arrive_expect_tx(smem_u32(bar_full + ps), stage_bytes);
                         __syncwarp();
                         if (active) {
@@ -352,8 +358,6 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                             tma_load_5d(smem_u32(smem + static_cast<size_t>(ps) * stage_bytes + my_off), tmap,
                                         smem_u32(bar_full + ps), c[0], c[1], c[2], c[3], c[4]);
                         }
-                        issued_mask |= 1u << ps;
-                        issued_parity = (issued_parity & ~(1u << ps)) | (phase << ps);
                     }
                     if (++kd0 == p.k_digit_ext[0]) {
                         kd0 = 0;
@@ -368,15 +372,11 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     }
                 }
             }
-            if (ld_shared_u32(abort_flag) && lane == 0) {
-                // Give the bulk copies issued into these barriers a bounded time to land before the block ends.
-                for (int s = 0; s < p.stages; ++s) {
-                    if (!(issued_mask & (1u << s))) continue;
-                    const unsigned long long t0 = global_timer();
-                    while (!mbar_try_wait(smem_u32(bar_full + s), (issued_parity >> s) & 1u))
-                        if (global_timer() - t0 > 100000000ull) break;
-                }
-            }
+            // Here, and not when the last copy is issued: a group may give up, or pass over stages that are still on their way, later on.
+            // (stages before `stage` were filled in this phase, the others in the last one, or never, which a barrier takes for the last one)
+            block_done();
+            if (ld_shared_u32(abort_flag) && lane == 0)
+                drain_copies(smem_u32(bar_full + first), static_cast<int>(ring), 0xffffffffu, phase ? (1u << stage) - 1u : ~((1u << stage) - 1u));
         } else {
             // ---------------- table builders: one warp a tile, lane s works out its slab s (at most 32) ----------------
             const bool of_a = lane < SA;
@@ -401,7 +401,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             for (uint32_t i = static_cast<uint32_t>(warp) - G; i < my_tiles; i += kBuilders) {
                 const WorkUnit w = decode_unit(blockIdx.x + i * gridDim.x, p, tiles_m, tiles_n);
                 const uint32_t round = i / G, slot = (i - round * G) * 2u + (round & 1u);   // group, buffer
-                if (!mbar_wait(smem_u32(tab_empty + slot), (round >> 1 & 1u) ^ 1u, abort_flag, 100u)) break;
+                if (!mbar_wait_for(smem_u32(tab_empty + slot), (round >> 1 & 1u) ^ 1u, abort_flag, 100u, p.wait_limit_ns)) break;
                 const uint32_t tab = tabs + slot * kTabBytes<FM>;
                 SlabEntry entry;
                 int d0 = 0;
@@ -430,6 +430,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 last_tab = tab;
             }
             if (SCALED && !kOldInSmem<FM> && p.beta != 0.0 && last_tab != 0) prefetch(last_tab);
+            block_done();
         }
     } else {
         if (G == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
@@ -517,7 +518,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             int copied = SCALED && staged && p.beta != 0.0 ? 0 : kCopySteps;
             long long cc[W];
             if (SCALED && staged && p.beta != 0.0) {
-                tile_ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag)) && tile_ok;
+                tile_ok = __all_sync(0xffffffffu, mbar_wait_for(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag, 0, p.wait_limit_ns)) && tile_ok;
                 if (!tile_ok) copied = kCopySteps;
                 tile_cols(slot, cc);
             }
@@ -544,7 +545,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             double fa0[FM], fb0[W], fa1[FM], fb1[W];
             uint32_t chunk = static_cast<uint32_t>(w.it0 ? w.it0 % p.k_digit_ext[0] : 0);   // chunk of the chunked mode
             {
-                const bool landed = mbar_wait(smem_u32(bar_full + first + stage), phase, abort_flag);
+                const bool landed = mbar_wait_for(smem_u32(bar_full + first + stage), phase, abort_flag, 0, p.wait_limit_ns);
                 tile_ok = __all_sync(0xffffffffu, landed) && tile_ok;
                 mark(1);
             }
@@ -581,7 +582,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 const uint32_t bar_next = smem_u32(bar_full + first + stage);
                 const bool more = left > 1, landed = !more || mbar_test_wait(bar_next, phase);
                 mma_step<L, BMN, FM, W, BK>(acc, fa0, fb0, fa1, fb1, sb + fa.step1 + later_a, fa, sb + fb.step1 + later_b, fb);
-                if (!__all_sync(0xffffffffu, landed)) tile_ok = __all_sync(0xffffffffu, mbar_wait(bar_next, phase, abort_flag)) && tile_ok;
+                if (!__all_sync(0xffffffffu, landed)) tile_ok = __all_sync(0xffffffffu, mbar_wait_for(bar_next, phase, abort_flag, 0, p.wait_limit_ns)) && tile_ok;
                 if (more) sb = smem_u32(smem) + (first + stage) * stage_bytes;
                 mma_step<L, BMN, FM, W, BK>(acc, fa1, fb1, fa0, fb0, sb + fa.step0, fa, sb + fb.step0, fb);
                 __syncwarp();
@@ -591,7 +592,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             mark(2);
 
             // the tile's offset tables were built while it was being computed
-            tile_ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag)) && tile_ok;
+            tile_ok = __all_sync(0xffffffffu, mbar_wait_for(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag, 0, p.wait_limit_ns)) && tile_ok;
             if (SCALED && staged) {
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 __syncwarp();   // (a thread's old values were copied by the four lanes of its rows)
@@ -756,8 +757,8 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             for (uint32_t c = 1; c < 5; ++c) q[0] += q[c] = ld_shared_s64(profile + c * 8u);
             q[5] = 0;
         }
+        block_done();
     }
-    __syncthreads();
     if (threadIdx.x == 0 && ld_shared_u32(abort_flag)) atomicMax(p.status, 1);
 }
 
@@ -815,6 +816,7 @@ cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* 
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
     const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
     UmmaParams q = p;
+    if (q.wait_limit_ns == 0) q.wait_limit_ns = kWaitLimitNs;
     int smem = smem_bytes;
     // Room for the old values leaves two or three stages a group, where the tile's main loop is long enough to hide them behind anyway:
     // 172032 x 72 x 112, rows along C, 149 us staged, 137 read in the epilogue; K 48 168 and 174; across slabs K 72 73 and 86, K 128 342 and 344.

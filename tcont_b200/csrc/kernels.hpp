@@ -167,9 +167,9 @@ struct UmmaParams {
     double alpha, beta;
     int* status;  // device status word: set non-zero when a bounded wait gives up
     long long* prof;  // optional per-CTA cycle counters [grid][8] (TCONT_UMMA_PROF=1), else null
-    // Test hooks of the bounded-wait exit (tcgen05 kernel): a shorter wait limit (0 = the default 2 s), and
-    // the index of one k iteration per CTA whose stage the producer leaves unfilled and unannounced
-    // (-1 = none), so that the MMA warp's wait on it runs out with nothing in flight for that stage.
+    // Test hooks of the bounded-wait exit: a shorter wait limit (0 = the default 2 s), and the index of one k iteration
+    // per CTA whose stage the producer leaves unfilled and unannounced (-1 = none), so
+    // that the wait on it runs out with nothing in flight for that stage.
     unsigned long long wait_limit_ns;
     int test_skip_iter;
     // Contracted-mode split over several GPUs (tcgen05 kernel): this GPU's partial C is cut into `owners`

@@ -62,17 +62,5 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-
-// Give the bulk copies issued into these barriers a bounded time to land before the CTA ends (after a wait gave up).
-__device__ __forceinline__ void drain_copies(uint32_t bar_full, int stages, uint32_t issued_mask, uint32_t issued_parity)
-{
-    for (int s = 0; s < stages; ++s) {
-        if (!(issued_mask & (1u << s))) continue;
-        const unsigned long long t0 = global_timer();
-        while (!mbar_try_wait(bar_full + 8u * static_cast<uint32_t>(s), (issued_parity >> s) & 1u))
-            if (global_timer() - t0 > 100000000ull) break;
-    }
-}
-
 }  // namespace
 }  // namespace tcontb

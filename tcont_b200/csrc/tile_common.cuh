@@ -90,11 +90,8 @@ __device__ __forceinline__ long long ld_shared_s64(uint32_t addr)
 // flag, when the limit passes; returns false at once when another thread already gave up.
 // `sleep_ns` > 0: the thread sleeps that long after a failed poll, for warps whose polling would
 // otherwise take issue slots from the warps doing the arithmetic on the same scheduler.
-// `limit_ns` = 0 means the default limit.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t sleep_ns = 0,
-                                          unsigned long long limit_ns = 0)
+__device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t sleep_ns, unsigned long long limit_ns)
 {
-    const unsigned long long limit = limit_ns ? limit_ns : kWaitLimitNs;
     unsigned long long t0 = 0;
     for (uint32_t spin = 0;; ++spin) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -104,11 +101,28 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
             if (spin == 0) continue;
             const unsigned long long now = global_timer();
             if (t0 == 0) t0 = now;
-            else if (now - t0 > limit) {
+            else if (now - t0 > limit_ns) {
                 st_shared_u32(abort_addr, 1u);
                 return false;
             }
         }
+    }
+}
+// The same; `limit_ns` = 0 means the default limit.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t sleep_ns = 0,
+                                          unsigned long long limit_ns = 0)
+{
+    return mbar_wait_for(bar, parity, abort_addr, sleep_ns, limit_ns ? limit_ns : kWaitLimitNs);
+}
+
+// Give the bulk copies issued into these barriers a bounded time to land before the CTA ends (after a wait gave up).
+__device__ __forceinline__ void drain_copies(uint32_t bar_full, int stages, uint32_t issued_mask, uint32_t issued_parity)
+{
+    for (int s = 0; s < stages; ++s) {
+        if (!(issued_mask & (1u << s))) continue;
+        const unsigned long long t0 = global_timer();
+        while (!mbar_try_wait(bar_full + 8u * static_cast<uint32_t>(s), (issued_parity >> s) & 1u))
+            if (global_timer() - t0 > 100000000ull) break;
     }
 }
 

@@ -6,6 +6,7 @@ Every output is a chain of K fused multiply-adds and three roundings of the scal
 import numpy as np
 import pytest
 
+from cases import to_equation
 from oracle_lib import F64, Contraction
 from test_scaled_epilogues_gpu import SCALARS, scaled_run
 
@@ -97,3 +98,45 @@ def test_no_room_for_ranges(engine, oracle, monkeypatch):
     product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
     for beta, out in zip((1.0, 0.0), got):
         assert (np.abs(out - (product + beta)) <= (256 + 8) * 2.0**-53 * (scale + beta)).all()
+
+
+@pytest.mark.parametrize("columns", ["32", "64"])
+@pytest.mark.parametrize("beta", [0.0, 1.0])
+@pytest.mark.parametrize("skip", [2, 8])
+def test_bounded_wait_gives_up_cleanly(engine, oracle, monkeypatch, columns, beta, skip):
+    """One stage of every block, of its first or of its second tile, is neither announced nor filled: the waits behind it run out, the
+    run's status says so, what is stored of C is right, nothing outside it is written, and the next run is right."""
+    import torch
+    from tcont_b200 import api
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    monkeypatch.setenv("TCONT_DMMA_BN", columns)
+    k = 72
+    c = Contraction("ab", "ak", "kb", dict(a=5130, b=700, k=k), F64)
+    A, B = oracle.inputs(c, 43, -1.0, 1.0)
+    C0 = np.random.default_rng(10).uniform(-4.0, 4.0, c.size("ab"))
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    guarded = torch.full((C0.size + 64,), 7.0, dtype=torch.float64, device="cuda")
+    plan = engine.plan(to_equation(engine, c, 1))
+    desc = plan.describe()
+    assert desc["kernel"] == "dmma_f64_tma" and ("narrow" in desc) == (columns == "32") and desc["umma"]["k_iters"] == 5
+    want = oracle.contract(c, A, B) + beta * C0
+    bound = (k + 4) * 2.0**-53 * (oracle.contract(c, np.abs(A), np.abs(B)) + abs(beta * C0))
+
+    def launched(**hooks):
+        for name, value in hooks.items():
+            monkeypatch.setenv(name, value)
+        run = api.prepare_on_device(plan, dA.data_ptr(), dB.data_ptr(), guarded[32:].data_ptr(), keep=(dA, dB, guarded))
+        for name in hooks:
+            monkeypatch.delenv(name)
+        run.set_scalars(1.0, beta)
+        guarded[32:32 + C0.size].copy_(torch.from_numpy(C0))
+        engine.launch(run)
+        torch.cuda.synchronize()
+        got = guarded.cpu().numpy()
+        assert (got[:32] == 7.0).all() and (got[32 + C0.size:] == 7.0).all()
+        return run.device_status(), got[32:32 + C0.size]
+    status, got = launched(TCONT_TEST_WAIT_LIMIT_NS="2000000", TCONT_TEST_SKIP_STAGE=str(skip))
+    right = np.abs(got - want) <= bound
+    assert status == 1 and not right.all() and (right | (got == C0)).all()
+    status, got = launched()
+    assert status == 0 and (np.abs(got - want) <= bound).all()
