@@ -330,7 +330,8 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             k_steps(o, ks);
             uint32_t stage = 0, phase = 0;
             bool ok = true;
-            for (uint32_t i = static_cast<uint32_t>(warp); ok && i < my_tiles; i += G) {
+            const uint32_t filled = my_tiles < static_cast<uint32_t>(p.test_skip_iter) ? my_tiles : static_cast<uint32_t>(p.test_skip_iter);   // (test hook)
+            for (uint32_t i = static_cast<uint32_t>(warp); ok && i < filled; i += G) {
                 const WorkUnit w = decode_unit(blockIdx.x + i * gridDim.x, p, tiles_m, tiles_n);
                 const uint32_t tm = w.tm, tn = w.tn;
                 int base[kMaxTmaRank];
@@ -343,21 +344,20 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 }
                 for (int it = 0; it < w.n_it; ++it) {
                     const uint32_t ps = first + stage;
-                    ok = __all_sync(0xffffffffu, mbar_wait_for(smem_u32(bar_empty + ps), phase ^ 1u, abort_flag, 200u, p.wait_limit_ns));
-                    // (a stage given back behind a wait that gave up may never have been filled, or is still on its way: not filled again.  Asked
-                    // here, one producer warp reads one word a stage; 9216 x 4096 x 24 accumulating into a 6-D C 120.8 us, 121.9 with it, 123.1
-                    // where the warps that gave up keep their stages)
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar_empty + ps), phase ^ 1u, abort_flag, 200u));
+                    // A stage given back behind a wait that gave up may never have been filled, or is still on its way: not filled again.  (One
+                    // read for the warp, converged behind the vote, so its lanes go the same way; the word inside the vote costs 3 % where a
+                    // stage is 20 copies, and 9216 x 4096 x 24 accumulating into a 6-D C 123 us instead of 121 where the warps that gave up
+                    // keep their stages.)
                     ok = ok && ld_shared_u32(abort_flag) == 0u;
                     if (!ok) break;
-                    if (static_cast<int>(i) * p.k_iters_per_split + it != p.test_skip_iter) {
-                        if (lane == 0) mbar_arrive_expect_tx(smem_u32(bar_full + ps), stage_bytes);
-                        __syncwarp();
-                        if (active) {
-                            int c[kMaxTmaRank];
-                            k_coords(base, ks, kd0, kd1, kd2, c);
-                            tma_load_5d(smem_u32(smem + static_cast<size_t>(ps) * stage_bytes + my_off), tmap,
-                                        smem_u32(bar_full + ps), c[0], c[1], c[2], c[3], c[4]);
-                        }
+                    if (lane == 0) mbar_arrive_expect_tx(smem_u32(bar_full + ps), stage_bytes);
+                    __syncwarp();
+                    if (active) {
+                        int c[kMaxTmaRank];
+                        k_coords(base, ks, kd0, kd1, kd2, c);
+                        tma_load_5d(smem_u32(smem + static_cast<size_t>(ps) * stage_bytes + my_off), tmap,
+                                    smem_u32(bar_full + ps), c[0], c[1], c[2], c[3], c[4]);
                     }
                     if (++kd0 == p.k_digit_ext[0]) {
                         kd0 = 0;
@@ -371,6 +371,11 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                         phase ^= 1u;
                     }
                 }
+            }
+            if (filled < my_tiles) {   // (test hook: the group's waits end as if one of the block had run out)
+                const unsigned long long t0 = global_timer();
+                while (global_timer() - t0 < p.wait_limit_ns) __nanosleep(1000);
+                st_shared_u32(abort_flag, 1u);
             }
             // Here, and not when the last copy is issued: a group may give up, or pass over stages that are still on their way, later on.
             // (stages before `stage` were filled in this phase, the others in the last one, or never, which a barrier takes for the last one)
@@ -401,7 +406,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             for (uint32_t i = static_cast<uint32_t>(warp) - G; i < my_tiles; i += kBuilders) {
                 const WorkUnit w = decode_unit(blockIdx.x + i * gridDim.x, p, tiles_m, tiles_n);
                 const uint32_t round = i / G, slot = (i - round * G) * 2u + (round & 1u);   // group, buffer
-                if (!mbar_wait_for(smem_u32(tab_empty + slot), (round >> 1 & 1u) ^ 1u, abort_flag, 100u, p.wait_limit_ns)) break;
+                if (!mbar_wait(smem_u32(tab_empty + slot), (round >> 1 & 1u) ^ 1u, abort_flag, 100u)) break;
                 const uint32_t tab = tabs + slot * kTabBytes<FM>;
                 SlabEntry entry;
                 int d0 = 0;
@@ -518,7 +523,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             int copied = SCALED && staged && p.beta != 0.0 ? 0 : kCopySteps;
             long long cc[W];
             if (SCALED && staged && p.beta != 0.0) {
-                tile_ok = __all_sync(0xffffffffu, mbar_wait_for(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag, 0, p.wait_limit_ns)) && tile_ok;
+                tile_ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag)) && tile_ok;
                 if (!tile_ok) copied = kCopySteps;
                 tile_cols(slot, cc);
             }
@@ -545,7 +550,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             double fa0[FM], fb0[W], fa1[FM], fb1[W];
             uint32_t chunk = static_cast<uint32_t>(w.it0 ? w.it0 % p.k_digit_ext[0] : 0);   // chunk of the chunked mode
             {
-                const bool landed = mbar_wait_for(smem_u32(bar_full + first + stage), phase, abort_flag, 0, p.wait_limit_ns);
+                const bool landed = mbar_wait(smem_u32(bar_full + first + stage), phase, abort_flag);
                 tile_ok = __all_sync(0xffffffffu, landed) && tile_ok;
                 mark(1);
             }
@@ -582,7 +587,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                 const uint32_t bar_next = smem_u32(bar_full + first + stage);
                 const bool more = left > 1, landed = !more || mbar_test_wait(bar_next, phase);
                 mma_step<L, BMN, FM, W, BK>(acc, fa0, fb0, fa1, fb1, sb + fa.step1 + later_a, fa, sb + fb.step1 + later_b, fb);
-                if (!__all_sync(0xffffffffu, landed)) tile_ok = __all_sync(0xffffffffu, mbar_wait_for(bar_next, phase, abort_flag, 0, p.wait_limit_ns)) && tile_ok;
+                if (!__all_sync(0xffffffffu, landed)) tile_ok = __all_sync(0xffffffffu, mbar_wait(bar_next, phase, abort_flag)) && tile_ok;
                 if (more) sb = smem_u32(smem) + (first + stage) * stage_bytes;
                 mma_step<L, BMN, FM, W, BK>(acc, fa1, fb1, fa0, fb0, sb + fa.step0, fa, sb + fb.step0, fb);
                 __syncwarp();
@@ -592,7 +597,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             mark(2);
 
             // the tile's offset tables were built while it was being computed
-            tile_ok = __all_sync(0xffffffffu, mbar_wait_for(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag, 0, p.wait_limit_ns)) && tile_ok;
+            tile_ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag)) && tile_ok;
             if (SCALED && staged) {
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 __syncwarp();   // (a thread's old values were copied by the four lanes of its rows)
@@ -816,6 +821,10 @@ cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* 
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
     const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
     UmmaParams q = p;
+    // test hooks: tiles of a block below this one are filled, the rest given up after the limit (in the waits themselves a limit that is
+    // not a constant cost 32 x 512 x 3824 by 16 95 -> 101 us by way of other registers; a test per stage in the producer 3 % where it
+    // issues 20 copies)
+    q.test_skip_iter = p.test_skip_iter < 0 ? -1 : p.test_skip_iter / p.k_iters_per_split;
     if (q.wait_limit_ns == 0) q.wait_limit_ns = kWaitLimitNs;
     int smem = smem_bytes;
     // Room for the old values leaves two or three stages a group, where the tile's main loop is long enough to hide them behind anyway:

@@ -168,8 +168,9 @@ struct UmmaParams {
     int* status;  // device status word: set non-zero when a bounded wait gives up
     long long* prof;  // optional per-CTA cycle counters [grid][8] (TCONT_UMMA_PROF=1), else null
     // Test hooks of the bounded-wait exit: a shorter wait limit (0 = the default 2 s), and the index of one k iteration
-    // per CTA whose stage the producer leaves unfilled and unannounced (-1 = none), so
-    // that the wait on it runs out with nothing in flight for that stage.
+    // per CTA whose stage the producer leaves unfilled and unannounced (-1 = none), so that the wait on it runs out with
+    // nothing in flight for that stage.  FP64 kernel: the tile of a block with this iteration and those behind it are not
+    // filled, and the producers raise the block's abort flag after the limit, which ends its waits as one that ran out does.
     unsigned long long wait_limit_ns;
     int test_skip_iter;
     // Contracted-mode split over several GPUs (tcgen05 kernel): this GPU's partial C is cut into `owners`

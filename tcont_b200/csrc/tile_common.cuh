@@ -90,8 +90,11 @@ __device__ __forceinline__ long long ld_shared_s64(uint32_t addr)
 // flag, when the limit passes; returns false at once when another thread already gave up.
 // `sleep_ns` > 0: the thread sleeps that long after a failed poll, for warps whose polling would
 // otherwise take issue slots from the warps doing the arithmetic on the same scheduler.
-__device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t sleep_ns, unsigned long long limit_ns)
+// `limit_ns` = 0 means the default limit.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t sleep_ns = 0,
+                                          unsigned long long limit_ns = 0)
 {
+    const unsigned long long limit = limit_ns ? limit_ns : kWaitLimitNs;
     unsigned long long t0 = 0;
     for (uint32_t spin = 0;; ++spin) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -101,18 +104,12 @@ __device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, uin
             if (spin == 0) continue;
             const unsigned long long now = global_timer();
             if (t0 == 0) t0 = now;
-            else if (now - t0 > limit_ns) {
+            else if (now - t0 > limit) {
                 st_shared_u32(abort_addr, 1u);
                 return false;
             }
         }
     }
-}
-// The same; `limit_ns` = 0 means the default limit.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t sleep_ns = 0,
-                                          unsigned long long limit_ns = 0)
-{
-    return mbar_wait_for(bar, parity, abort_addr, sleep_ns, limit_ns ? limit_ns : kWaitLimitNs);
 }
 
 // Give the bulk copies issued into these barriers a bounded time to land before the CTA ends (after a wait gave up).

@@ -102,10 +102,10 @@ def test_no_room_for_ranges(engine, oracle, monkeypatch):
 
 @pytest.mark.parametrize("columns", ["32", "64"])
 @pytest.mark.parametrize("beta", [0.0, 1.0])
-@pytest.mark.parametrize("skip", [2, 8])
+@pytest.mark.parametrize("skip", [2, 8, 17])
 def test_bounded_wait_gives_up_cleanly(engine, oracle, monkeypatch, columns, beta, skip):
-    """One stage of every block, of its first or of its second tile, is neither announced nor filled: the waits behind it run out, the
-    run's status says so, what is stored of C is right, nothing outside it is written, and the next run is right."""
+    """The first, second or fourth tile of every block and those behind it are never filled, and the waits for them are given up after 2 ms:
+    the run's status says so, what is stored of C is right, nothing outside it is written, and the next run is right."""
     import torch
     from tcont_b200 import api
     monkeypatch.setenv("TCONT_KERNEL", "tma")
