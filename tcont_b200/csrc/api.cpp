@@ -672,7 +672,11 @@ tcontb_status finish_run(tcontb_run* run)
         }
         if (u.smem_bytes > kMaxDynamicSmemBytes) return fail(TCONTB_RUNTIME_ERROR, "plan asks for more shared memory than a block can have");
         if (pl.kernel == KERNEL_UMMA_TF32) TC_CUDA(umma_tf32_configure());
-        else TC_CUDA(dmma_tma_configure(run->umma));
+        else
+            for (int reads = 0; reads < (u.groups[0] == u.groups[1] ? 1 : 2); ++reads) {
+                run->umma.groups = u.groups[reads];
+                TC_CUDA(dmma_tma_configure(run->umma));
+            }
         TC_CUDA(splitk_reduce_configure());
     } else {
         fill_gather(p, kA, kB, run->dC, pl.simt, pl.gather, &run->gather);
@@ -1310,8 +1314,10 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         if (umma.pace) TC_CUDA(cudaMemsetAsync(umma.pace, 0, run->pace_bytes, run->stream));
         TC_CUDA(launch_umma_tf32(umma, &run->tmA, &run->tmB, pl.umma.smem_bytes, run->num_sms, run->stream));
     }
-    else if (pl.kernel == KERNEL_DMMA_F64_TMA)
-        TC_CUDA(launch_dmma_tma(umma, &run->tmA, &run->tmB, (pl.narrow.eligible ? pl.narrow : pl.umma).smem_bytes, run->num_sms, run->stream));
+    else if (pl.kernel == KERNEL_DMMA_F64_TMA) {
+        umma.groups = (pl.narrow.eligible ? pl.narrow : pl.umma).groups[umma.scaled && umma.beta != 0.0 ? 1 : 0];
+        TC_CUDA(launch_dmma_tma(umma, &run->tmA, &run->tmB, run->num_sms, run->stream));
+    }
     else {
         GatherParams g = run->gather;
         g.scaled = scaled ? 1 : 0;

@@ -5,10 +5,11 @@
 // engine: the planner's slab machinery, the same as for the tcgen05 kernel but with 16 doubles per
 // 128-byte row, describes every operand tile as a few multi-mode TMA boxes.
 //
-// One block per SM.  128 x 64 tiles: three warpgroups, two of them consumer groups of 2 x 2 warps with a 64 x 32 warp tile; 128 x 32
-// tiles (narrow N, and short contracted extents: narrow_tiles in planner.cpp): four warpgroups, three of them consumer groups of 4 x 1
-// warps with a 32 x 32 warp tile.  G consumer groups take every G-th tile of the block; setmaxnreg moves registers from the first
-// warpgroup to them (72 and 216 a thread, or 56 and 152).
+// One block per SM.  128 x 64 tiles: three warpgroups, two of them consumer groups of 2 x 2 warps with a 64 x 32 warp tile.  128 x 32
+// tiles (narrow N, and short contracted extents: narrow_tiles in planner.cpp): the same with a 64 x 16 warp tile, or four warpgroups,
+// three of them consumer groups of 4 x 1 warps with a 32 x 32 warp tile (dmma_groups in planner.cpp has the choice and its figures).
+// G consumer groups take every G-th tile of the block; setmaxnreg moves registers from the first warpgroup to them (72 and 216 a
+// thread with two of them, 56 and 152 with three).
 //   warps 0 .. G-1    producers, one per consumer group: lane i issues copy i of a stage (5-D tensor
 //                     maps, no multicast) into the group's own ring of stages,
 //                     full/empty mbarriers per stage, the ring runs across tile boundaries
@@ -32,6 +33,7 @@
 // call (backends/ttgt_cutt/src/ttgt_cutt.cpp:764-809).
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "chain.cuh"
@@ -42,9 +44,9 @@ namespace tcontb {
 namespace {
 
 constexpr int kMaxGroups = 3, kMaxStages64 = 12;
-template <int FM>   // row fragments of a warp: 8 with 128 x 64 tiles, 4 with 128 x 32
+template <int FM>   // row fragments of a warp: 8 with two groups, 4 with three
 constexpr int kGroups = FM == 8 ? 2 : 3;
-// Narrow tiles: every thread copies the old values of C that it will need to shared memory of its own when a tile begins.
+// Three groups: every thread copies the old values of C that it will need to shared memory of its own when a tile begins.
 template <int FM>
 constexpr bool kOldInSmem = FM == 4;
 constexpr int kOldBytes = 128 * 32 * 8;   // of one group
@@ -53,8 +55,8 @@ constexpr int kThreads64 = 128 * (1 + kGroups<FM>);
 constexpr int kBM = 128, kMaxBN = 64;
 constexpr int kAuxBytes = 512;   // barriers, abort flag, ragged tiles
 static_assert(8 * (2 * kMaxStages64 + 4 * kMaxGroups) + 4 + 8 * kMaxGroups + 48 <= kAuxBytes);
-// Where a tile lies in C: an entry for each of its slabs, A's first, the offset of each column and, with 128 x 64 tiles, of each row
-// (which a thread of 128 x 32 tiles works out from its slab: one warp has not the time to write them).
+// Where a tile lies in C: an entry for each of its slabs, A's first, the offset of each column and, with two groups, of each row
+// (which a thread of three groups works out from its slab: one warp has not the time to write them).
 constexpr uint32_t kColumnTab = 32 * 16u, kRowTab = kColumnTab + kMaxBN * 8u;
 template <int FM>
 constexpr uint32_t kTabBytes = FM == 8 ? kRowTab + kBM * 8u : kColumnTab + 32 * 8u;
@@ -260,12 +262,13 @@ __device__ __forceinline__ uint32_t column_of(int j, uint32_t fr)
 // overwriting kernel has no registers to spare for it.  PIECES: every store is 32 aligned bytes (UmmaSpec::piece); one kernel with both
 // epilogues is slower in either (9216 x 4096 x 24 102.5 us, 94.5 in a kernel of its own; 2050 x 8000 x 16 54.8 and 48.7).
 // SLIM: one column of tiles, of at most three quarters of its columns (B K-major): three column fragments a warp instead of four.
-template <RowLayout L, bool BMN, int FM, int BK, bool SCALED, bool SLIM, bool PIECES>
+template <RowLayout L, bool BMN, int FM, int BN, int BK, bool SCALED, bool SLIM, bool PIECES>
 __global__ void __launch_bounds__(kThreads64<FM>, 1)
 dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                 const __grid_constant__ UmmaParams p)
 {
-    constexpr int G = kGroups<FM>, BN = FM * 8, W = SLIM ? 3 : 4;   // W: column fragments of a warp
+    constexpr int G = kGroups<FM>, W = SLIM ? 3 : FM == 8 ? BN / 16 : 4;   // W: column fragments of a warp
+    static_assert(FM == 8 ? BN == 64 || !SLIM : BN == 32);
     constexpr uint32_t kBuilders = 4 - G;   // warps of the first warpgroup that build tables
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // 1024-byte aligned
@@ -440,7 +443,7 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     } else {
         if (G == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         else asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
-        // ---------------- consumers: groups of 2 x 2 warps (64 x 32 warp tiles) or 4 x 1 (32 x 32) ----------------
+        // ---------------- consumers: groups of 2 x 2 warps (64 x 32 or 64 x 16 warp tiles) or 4 x 1 (32 x 32) ----------------
         constexpr int WM = 16 / FM;   // warps along the rows
         const int cw = warp & 3, grp = (warp >> 2) - 1, wm = cw % WM, wn = cw / WM;
         const uint32_t fr = static_cast<uint32_t>(lane >> 2), fk = static_cast<uint32_t>(lane & 3);
@@ -767,32 +770,36 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     if (threadIdx.x == 0 && ld_shared_u32(abort_flag)) atomicMax(p.status, 1);
 }
 
-// The kernel's forms, one function per (layouts, row fragments, k chunk, slim, scaled, pieces); `use` is called with the one that matches.
-template <RowLayout L, bool BMN, int FM, int BK, bool SLIM, typename Use>
+// The kernel's forms, one function per (layouts, row fragments, columns, k chunk, slim, scaled, pieces); `use` is called with the one that matches.
+template <RowLayout L, bool BMN, int FM, int BN, int BK, bool SLIM, typename Use>
 cudaError_t with_epilogue(bool scaled, bool pieces, Use&& use)
 {
-    if (pieces) return scaled ? use(dmma_tma_kernel<L, BMN, FM, BK, true, SLIM, true>) : use(dmma_tma_kernel<L, BMN, FM, BK, false, SLIM, true>);
-    return scaled ? use(dmma_tma_kernel<L, BMN, FM, BK, true, SLIM, false>) : use(dmma_tma_kernel<L, BMN, FM, BK, false, SLIM, false>);
+    if (pieces) return scaled ? use(dmma_tma_kernel<L, BMN, FM, BN, BK, true, SLIM, true>) : use(dmma_tma_kernel<L, BMN, FM, BN, BK, false, SLIM, true>);
+    return scaled ? use(dmma_tma_kernel<L, BMN, FM, BN, BK, true, SLIM, false>) : use(dmma_tma_kernel<L, BMN, FM, BN, BK, false, SLIM, false>);
 }
-template <RowLayout L, int FM, int BK, typename Use>
+template <RowLayout L, int FM, int BN, int BK, typename Use>
 cudaError_t with_columns(bool bmn, bool slim, bool scaled, bool pieces, Use&& use)
 {
-    if (slim) return bmn ? cudaErrorInvalidValue : with_epilogue<L, false, FM, BK, true>(scaled, pieces, use);
-    return bmn ? with_epilogue<L, true, FM, BK, false>(scaled, pieces, use) : with_epilogue<L, false, FM, BK, false>(scaled, pieces, use);
+    if (slim) {
+        if constexpr (FM == 8 && BN == 32) return cudaErrorInvalidValue;
+        else return bmn ? cudaErrorInvalidValue : with_epilogue<L, false, FM, BN, BK, true>(scaled, pieces, use);
+    }
+    return bmn ? with_epilogue<L, true, FM, BN, BK, false>(scaled, pieces, use) : with_epilogue<L, false, FM, BN, BK, false>(scaled, pieces, use);
 }
-template <int FM, int BK, typename Use>
+template <int FM, int BN, int BK, typename Use>
 cudaError_t with_rows(const UmmaParams& p, bool scaled, bool pieces, Use&& use)
 {
     const bool bmn = p.b.major != 0, slim = p.slim != 0;
-    if (p.a.major == 0) return with_columns<ROWS_K_MAJOR, FM, BK>(bmn, slim, scaled, pieces, use);
-    if (!p.store_across_slabs) return with_columns<ROWS_MN, FM, BK>(bmn, slim, scaled, pieces, use);
-    return with_columns<ROWS_ACROSS, FM, BK>(bmn, slim, scaled, pieces, use);
+    if (p.a.major == 0) return with_columns<ROWS_K_MAJOR, FM, BN, BK>(bmn, slim, scaled, pieces, use);
+    if (!p.store_across_slabs) return with_columns<ROWS_MN, FM, BN, BK>(bmn, slim, scaled, pieces, use);
+    return with_columns<ROWS_ACROSS, FM, BN, BK>(bmn, slim, scaled, pieces, use);
 }
 template <typename Use>
 cudaError_t with_kernel(const UmmaParams& p, bool scaled, bool pieces, Use&& use)
 {
-    if (p.BN == 64) return p.BK == 16 ? with_rows<8, 16>(p, scaled, pieces, use) : with_rows<8, 8>(p, scaled, pieces, use);
-    return p.BK == 16 ? with_rows<4, 16>(p, scaled, pieces, use) : with_rows<4, 8>(p, scaled, pieces, use);
+    if (p.BN == 64) return p.BK == 16 ? with_rows<8, 64, 16>(p, scaled, pieces, use) : with_rows<8, 64, 8>(p, scaled, pieces, use);
+    if (p.groups == 2) return p.BK == 16 ? with_rows<8, 32, 16>(p, scaled, pieces, use) : with_rows<8, 32, 8>(p, scaled, pieces, use);
+    return p.BK == 16 ? with_rows<4, 32, 16>(p, scaled, pieces, use) : with_rows<4, 32, 8>(p, scaled, pieces, use);
 }
 
 // Whether every piece of `of` elements starts on a multiple of its size.
@@ -812,12 +819,13 @@ cudaError_t dmma_tma_configure(const UmmaParams& p)
     return e;
 }
 
-cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, int num_sms, cudaStream_t stream)
+cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int num_sms, cudaStream_t stream)
 {
     const long long total = p.tiles_m * p.tiles_n * p.k_splits;
     if (total <= 0 || p.k_splits < 1 || (p.BN != 64 && p.BN != 32) || (p.BK != 16 && p.BK != 8)) return cudaErrorInvalidValue;
-    const int groups = p.BN == 64 ? kGroups<8> : kGroups<4>;
-    if (p.stages < 2 * groups || p.stages > kMaxStages64 || p.stages % groups) return cudaErrorInvalidValue;
+    const int groups = p.groups;
+    if (groups != kGroups<8> && (groups != kGroups<4> || p.BN != 32)) return cudaErrorInvalidValue;
+    if (p.stages < 2 * groups || p.stages > kMaxStages64) return cudaErrorInvalidValue;
     const unsigned grid = static_cast<unsigned>(total < num_sms ? total : num_sms);
     const CUtensorMap &ta = *static_cast<const CUtensorMap*>(tmapA), &tb = *static_cast<const CUtensorMap*>(tmapB);
     UmmaParams q = p;
@@ -826,17 +834,17 @@ cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* 
     // issues 20 copies)
     q.test_skip_iter = p.test_skip_iter < 0 ? -1 : p.test_skip_iter / p.k_iters_per_split;
     if (q.wait_limit_ns == 0) q.wait_limit_ns = kWaitLimitNs;
-    int smem = smem_bytes;
+    const int stage_bytes = p.a.slabs_per_tile * p.a.slab_bytes + p.b.slabs_per_tile * p.b.slab_bytes;
+    // a ring of as many of the planned stages as the groups can share and `bytes` of other things leave room for
+    auto share_stages = [&](int bytes) { q.stages = std::min(p.stages, (kMaxDynamicSmemBytes - bytes) / stage_bytes) / groups * groups; };
+    int fixed = 1024 + kAuxBytes + 2 * groups * static_cast<int>(groups == 2 ? kTabBytes<8> : kTabBytes<4>);
+    share_stages(fixed);
     // Room for the old values leaves two or three stages a group, where the tile's main loop is long enough to hide them behind anyway:
     // 172032 x 72 x 112, rows along C, 149 us staged, 137 read in the epilogue; K 48 168 and 174; across slabs K 72 73 and 86, K 128 342 and 344.
-    q.old_staged = p.BN == 32 && p.scaled && p.beta != 0.0 && p.k_iters * p.BK <= (p.store_across_slabs ? 128 : 64) ? 1 : 0;
-    if (q.old_staged) {
-        const int stage_bytes = p.a.slabs_per_tile * p.a.slab_bytes + p.b.slabs_per_tile * p.b.slab_bytes;
-        const int fixed = 1024 + kAuxBytes + 2 * groups * static_cast<int>(kTabBytes<4>) + groups * kOldBytes, most = (kMaxDynamicSmemBytes - fixed) / stage_bytes;
-        if (q.stages > most) q.stages = most / groups * groups;
-        if (q.stages < 2 * groups) return cudaErrorInvalidValue;
-        smem = fixed + q.stages * stage_bytes;
-    }
+    q.old_staged = groups == 3 && p.scaled && p.beta != 0.0 && p.k_iters * p.BK <= (p.store_across_slabs ? 128 : 64) ? 1 : 0;
+    if (q.old_staged) share_stages(fixed += groups * kOldBytes);
+    if (q.stages < 2 * groups) return cudaErrorInvalidValue;
+    const int smem = fixed + q.stages * stage_bytes;
     // Strides of 2 modulo 4 elements: half of the columns could take 32 bytes at a time, but a test per store costs more than that spares
     // where the epilogue is most of a tile (2050 x 8000, K 24 57.3 us tested, 49.9 in halves, K 48 74.9 and 67.2; accumulating 103 and 75).
     // With more k iterations the stores fall into the other group's main loop (3002 x 3002, K 64 46.3 and 50.6, K 96 63.3 and 67.5), but

@@ -181,7 +181,8 @@ struct UmmaParams {
     int store_across_slabs;  // FP64 kernel: see UmmaSpec
     int piece;               // FP64 kernel: see UmmaSpec
     int slim;                // FP64 kernel: see UmmaSpec
-    int old_staged;          // FP64 kernel, 128 x 32 tiles (set by the launcher): old values of C are copied to shared memory while a tile is computed
+    int groups;              // FP64 kernel: consumer groups of a block, see UmmaSpec
+    int old_staged;          // FP64 kernel, three groups (set by the launcher): old values of C are copied to shared memory while a tile is computed
     // tcgen05 kernel.  1: the next kernel's blocks may be scheduled when this one's copies are issued, 0: at once.  Late where
     // every block stores many tiles of few k iterations: 806400 x 112 x 48 behind its permutation, 43 tiles a block: let in at
     // once 200 us, late 184, not chained 187.  Short kernels lose by it (4096 x 3072 x 32, 3 tiles: 16.9, late 17.3).  The FP64
@@ -228,8 +229,7 @@ int across_tf32_smem(int stages, int BN, int BK);
 cudaError_t launch_across_tf32(const AcrossParams& p, const void* tmapA, const void* tmapB, const void* tmapC, int num_sms, cudaStream_t stream);
 
 // ---- TMA-fed FP64 tensor-path contraction (dmma_tma_f64.cu), same parameter block ------------
-cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int smem_bytes, int num_sms,
-                            cudaStream_t stream);
+cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* tmapB, int num_sms, cudaStream_t stream);
 cudaError_t dmma_tma_configure(const UmmaParams& p);
 
 // ---- split-K: C[e] = sum over s of partial[s * stride + e], s ascending (splitk_reduce.cu) ----

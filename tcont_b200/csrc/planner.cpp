@@ -795,6 +795,35 @@ UmmaSpec narrow_tiles(const Problem& p, const CostTable& cost, const UmmaSpec& u
     return v;
 }
 
+// Consumer groups of a block of 128 x 32 tiles, as time with three / time with two (the best of five bursts with pauses between them):
+//   as many rounds of tiles either way (1, 2 or 4 tiles a block): two of them copy ahead further and finish a tile sooner.  40 x 4 x 96 x 24
+//     by 1000 47.0 / 43.8 us, 3560 x 96 by 120 accumulating 11.5 / 10.3, 32 x 6 x 88 x 32 by 300 accumulating 21.6 / 18.4, 59976 x 8 by 48
+//     12.7 / 11.9.  Not in short ranges of k, which end in stores of whole partial tensors (fewer than 12 k iterations: 56 x 8 x 8 x 8
+//     by 1792 in 32 17.5 / 17.9, 24 x 8 x 32 x 8 by 2560 in 18 21.8 / 22.1, but 56 x 8 x 16 x 8 by 3584 in 16 27.8 / 26.8)
+//   stores in pieces of 8 or 16 bytes: 29 x 19 x 31 x 22 x 23 x 15 by 18 604 / 521, 51 x 30 x 29 x 30 x 49 by 7 217 / 188; reading the old
+//     values, in pieces of 8 bytes 402 / 300 and 819 / 707, in pieces of 16 555 / 769 (23 x 23 x 24 .. by 32, 25 x 16 .. by 17, 26 x 12 .. by 14)
+//   rows along C, one or two k chunks of 16: 127776 x 88 by 16 23.3 / 21.4, 105984 x 512 by 16 90.0 / 84.1, 78080 x 128 by 32 28.9 / 27.0
+//     (but 306904 x 16 by 16 16.5 / 17.4); more of them 67584 x 128 by 48 31.6 / 33.0
+// Elsewhere three: 24 x 42 x 1024 x 32 by 16 across slabs 52.7 / 62.4, 259056 x 32 by 24 accumulating 33.6 / 44.9, 64 x 236 x 1024 by 24
+// 33.5 / 37.4, and always where A's slabs and k chunks of 8 meet, whose loads the narrower warp tile repeats twice as often with
+// conflicts (72 x 48 x 16 x 16 by 960 70.8 / 105).
+void set_dmma_groups(UmmaSpec* u, const CostTable& cost)
+{
+    const char* want = std::getenv("TCONT_DMMA_GROUPS");   // tuning switch: 2 or 3
+    const bool slabs8 = u->a.major == 1 && u->a.slab_w == 8;
+    const int64_t rounds = ceil_div(u->tiles_m * u->tiles_n * u->k_splits, cost.num_sms);
+    for (int reads = 0; reads < 2; ++reads) {
+        bool two = u->BN == 64;
+        if (!two && !u->slim && !(slabs8 && u->BK == 8)) {
+            if (u->k_splits > 1 ? u->k_iters_per_split >= 12 : true) two = rounds <= 2 || rounds == 4;
+            if (!u->store_across_slabs && u->piece < (reads ? 2 : 4)) two = true;
+            if (!u->store_across_slabs && !reads && u->k_splits == 1 && u->BK == 16 && u->k_iters <= 2) two = true;
+        }
+        if (want && u->BN == 32 && !u->slim) two = std::atoi(want) == 2;
+        u->groups[reads] = two ? 2 : 3;
+    }
+}
+
 // Time of the TMA-fed FP64 kernel in `s` ranges of k, for up to a few rounds of work units.  A block's SM has `groups` units in work: all
 // of them together are bound by the FP64 pipe, each by itself by its chain of k iterations (no shorter than the copies of a stage
 // take) and its store.  Fitted to 663 (128 x 32) and 446 (128 x 64) launches of 113 contractions of 4 MFLOP to 3 GFLOP in 1 to 48
@@ -1557,6 +1586,8 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
             pl.kernel = KERNEL_DMMA_F64_TMA;
         }
     }
+    for (UmmaSpec* u : {&pl.umma, &pl.narrow})
+        if (u->eligible && u->elt == 8) set_dmma_groups(u, cost);
     if (pl.kernel == KERNEL_UMMA_TF32)
         for (int reads = 0; reads < 2; ++reads)
             pl.est_scaled_us[reads] = (use_ttgt ? ttgt_by_tiles_us : pl.est_direct_us) +
@@ -1636,7 +1667,7 @@ std::string describe_plan(const Plan& pl)
           << ",\"tiles_n\":" << pl.across.tiles_n << ",\"k_iters\":" << pl.across.k_iters << ",\"b_major\":\"" << (pl.across.b_major ? "MN" : "K") << "\"}";
     if (pl.narrow.eligible)
         o << ",\"narrow\":{\"BN\":" << pl.narrow.BN << ",\"BK\":" << pl.narrow.BK << ",\"stages\":" << pl.narrow.stages << ",\"slim\":" << (pl.narrow.slim ? "true" : "false") << ",\"tiles_m\":" << pl.narrow.tiles_m
-          << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << "}";
+          << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << ",\"groups\":[" << pl.narrow.groups[0] << "," << pl.narrow.groups[1] << "]}";
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";
     else {
@@ -1647,7 +1678,7 @@ std::string describe_plan(const Plan& pl)
           << ",\"a_slab_w\":" << u.a.slab_w << ",\"b_slab_w\":" << u.b.slab_w << ",\"a_slabs_per_copy\":" << u.a.slabs_per_op << ",\"b_slabs_per_copy\":" << u.b.slabs_per_op << ",\"a_slabs\":" << u.a.slabs_per_tile
           << ",\"b_slabs\":" << u.b.slabs_per_tile << ",\"smem_bytes\":" << u.smem_bytes
           << ",\"coalesced_store\":" << (u.a.row_elem_cstride == 1 ? "true" : "false")
-          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"slim\":" << (u.slim ? "true" : "false") << ",\"piece\":" << u.piece << ",\"producers\":" << u.producers
+          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"slim\":" << (u.slim ? "true" : "false") << ",\"piece\":" << u.piece << ",\"groups\":[" << u.groups[0] << "," << u.groups[1] << "],\"producers\":" << u.producers
           << ",\"a_fused\":" << u.a.split_inner << ",\"b_fused\":" << u.b.split_inner << ",\"column_ranges\":[";
         std::string why;
         for (int r = 2, n = 0; r <= 8; ++r)

@@ -117,6 +117,8 @@ struct UmmaSpec {
     // FP64 kernel: one column of tiles, of which at most three quarters are columns of C (B K-major): a warp computes three column
     // fragments instead of four
     bool slim = false;
+    // FP64 kernel: consumer groups of a block where the old values of C are not read, and where they are
+    int groups[2] = {2, 2};
     int smem_bytes = 0;
     int elt = 4;  // element bytes: 4 = tcgen05 TF32 kernel, 8 = TMA-fed FP64 tensor-path kernel
 };

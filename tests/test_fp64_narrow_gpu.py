@@ -46,6 +46,29 @@ def test_forms(engine, oracle, monkeypatch, name, columns, k):
         assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (alpha, beta)
 
 
+@pytest.mark.parametrize("name", list(FORMS) + ["several_tiles", "several_tiles_across"])
+@pytest.mark.parametrize("groups", ["2", "3"])
+@pytest.mark.parametrize("k", [8, 40, 104])
+def test_two_and_three_groups(engine, oracle, monkeypatch, name, groups, k):
+    """128 x 32 tiles in either number of consumer groups, whichever the planner would take."""
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    monkeypatch.setenv("TCONT_SPLITK", "1")
+    monkeypatch.setenv("TCONT_SCALE_PASSES", "1")
+    monkeypatch.setenv("TCONT_DMMA_BN", "32")
+    monkeypatch.setenv("TCONT_DMMA_GROUPS", groups)
+    several = {"several_tiles": ("ab", "ak", "kb", dict(a=1930, b=2100), False), "several_tiles_across": ("abc", "cka", "kb", dict(a=24, b=1100, c=210), True)}
+    C, A_, B_, ext, across = (FORMS | several)[name]
+    c = Contraction(C, A_, B_, dict(ext, k=k), F64)
+    A, B = oracle.inputs(c, 47, -1.0, 1.0)
+    C0 = np.random.default_rng(11).uniform(-4.0, 4.0, c.size(C))
+    desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
+    assert desc["narrow"]["groups"] == [int(groups)] * 2 and desc["umma"]["store_across_slabs"] == across
+    product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
+    for (alpha, beta), out in zip(SCALARS, got):
+        bound = (k + 4) * 2.0**-53 * (abs(alpha) * scale + abs(beta * C0))
+        assert (np.abs(out - (alpha * product + beta * C0)) <= bound).all(), (alpha, beta)
+
+
 @pytest.mark.parametrize("columns", ["32", "64"])
 def test_several_tiles_a_group(engine, oracle, monkeypatch, columns):
     """Rings, tables and staged values come round: 9 to 18 tiles a block, all slabs whole but the last."""

@@ -372,6 +372,32 @@ def test_fp64_narrow_tiles(engine, monkeypatch):
     assert not narrow(rows(4096, 16)) and describe(engine, rows(4096, 16), 1)["umma"]["in_use"]
 
 
+def test_fp64_consumer_groups(engine, monkeypatch):
+    """Two consumer groups on 128 x 32 tiles: where three would not spare a round of them, for pieces of 8 or 16 bytes, and for one or two
+    k chunks of 16 along C; three where old values are read in wider pieces, across slabs, and where A's slabs and k chunks of 8 meet."""
+    F64 = 1
+
+    def groups(C, A, B, **ext):
+        d = describe(engine, Contraction(C, A, B, ext, F64), 1)
+        u = d.get("narrow", d["umma"])
+        assert d["kernel"] == "dmma_f64_tma" and d["umma"]["in_use"] == ("narrow" not in d)
+        return u["BN"], *u["groups"]
+    monkeypatch.setenv("TCONT_KERNEL", "tma")
+    for tiles, rounds in ((1, 2), (2, 2), (3, 3), (4, 2), (5, 3)):
+        assert groups("ab", "ak", "kb", a=128 * 148 * tiles, b=32, k=96) == (32, rounds, rounds), tiles
+    assert groups("ab", "ak", "kb", a=9216, b=4096, k=32) == (32, 2, 3)
+    assert groups("ab", "ak", "kb", a=9216, b=4096, k=48) == (32, 3, 3)
+    assert groups("ab", "ak", "kb", a=9216, b=4096, k=24) == (32, 3, 3)            # k chunks of 8
+    assert groups("ab", "ka", "kb", a=9217, b=4096, k=24) == (32, 2, 2)            # columns on odd multiples of 8 bytes
+    assert groups("ab", "ka", "kb", a=9218, b=4096, k=24) == (32, 2, 3)            # of 16 bytes
+    assert groups("abcd", "dbka", "kc", a=24, b=42, c=1024, d=32, k=16) == (32, 3, 3)
+    assert groups("abc", "akb", "kc", a=24, b=740, c=32, k=24) == (32, 3, 3) and groups("abc", "akb", "kc", a=24, b=740, c=32, k=48) == (32, 2, 2)
+    assert groups("ab", "ak", "kb", a=9216, b=24, k=96) == (32, 3, 3)              # three column fragments a warp
+    assert groups("ab", "ak", "kb", a=9216, b=4096, k=200) == (64, 2, 2)
+    monkeypatch.setenv("TCONT_DMMA_GROUPS", "3")
+    assert groups("ab", "ak", "kb", a=9216, b=4096, k=32) == (32, 3, 3)
+
+
 def test_fp64_ranges_on_narrow_tiles(engine, monkeypatch):
     """Few tiles: ranges of k on narrow tiles in the place of ranges on wide ones, and of the gather kernel above 13.5 us."""
     F64 = 1
