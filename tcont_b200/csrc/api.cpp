@@ -161,6 +161,9 @@ struct tcontb_run {
     // UMMA
     UmmaParams umma{};
     CUtensorMap tmA{}, tmB{};
+    // FP64 kernel: the 128 x 64 tiles of launches that read the old values of C (Plan::wide_reads)
+    UmmaParams umma_wide{};
+    CUtensorMap tmAWide{}, tmBWide{};
     // tiles across two stride-1 modes: C, and the workspace that alpha and beta are applied from
     AcrossParams across{};
     CUtensorMap tmC{}, tmWs{};
@@ -326,6 +329,32 @@ void fill_raster_divs(const UmmaSpec& u, UmmaParams* p)
     p->div_rows = make_fast_div(u.raster_group);
     p->div_last_rows = make_fast_div(last ? last : u.raster_group);
     p->div_splits = make_fast_div(u.k_splits);
+}
+
+// The tiles of a plan as the TMA-fed kernels take them.
+void fill_tiles(const UmmaSpec& u, int64_t size_c, UmmaParams* out)
+{
+    fill_operand_dev(u.a, &out->a);
+    fill_operand_dev(u.b, &out->b);
+    out->BN = u.BN;
+    out->BK = u.BK;
+    out->stages = u.stages;
+    out->pair = u.pair ? 1 : 0;
+    out->producers = u.producers;
+    out->store_across_slabs = u.store_across_slabs ? 1 : 0;
+    out->piece = u.piece;
+    out->slim = u.slim ? 1 : 0;
+    out->n_k_digits = u.n_k_digits;
+    for (int i = 0; i < 3; ++i) out->k_digit_ext[i] = static_cast<int>(u.k_digit_ext[i]);
+    out->k_iters = static_cast<int>(u.k_iters);
+    out->tiles_m = u.tiles_m;
+    out->tiles_n = u.tiles_n;
+    out->raster_group = u.raster_group;
+    out->k_splits = u.k_splits;
+    out->k_iters_per_split = static_cast<int>(u.k_iters_per_split);
+    out->full_chunks = static_cast<int>(u.full_chunks);
+    out->split_stride = size_c;
+    fill_raster_divs(u, out);
 }
 
 tcontb_status encode_map(const UmmaOperand& o, const void* base, int elt, CUtensorMap* out)
@@ -573,27 +602,7 @@ tcontb_status finish_run(tcontb_run* run)
         if (st != TCONTB_OK) return st;
     } else if (pl.kernel == KERNEL_UMMA_TF32 || pl.kernel == KERNEL_DMMA_F64_TMA) {
         const UmmaSpec& u = pl.narrow.eligible ? pl.narrow : pl.umma;
-        fill_operand_dev(u.a, &run->umma.a);
-        fill_operand_dev(u.b, &run->umma.b);
-        run->umma.BN = u.BN;
-        run->umma.BK = u.BK;
-        run->umma.stages = u.stages;
-        run->umma.pair = u.pair ? 1 : 0;
-        run->umma.producers = u.producers;
-        run->umma.store_across_slabs = u.store_across_slabs ? 1 : 0;
-        run->umma.piece = u.piece;
-        run->umma.slim = u.slim ? 1 : 0;
-        run->umma.n_k_digits = u.n_k_digits;
-        for (int i = 0; i < 3; ++i) run->umma.k_digit_ext[i] = static_cast<int>(u.k_digit_ext[i]);
-        run->umma.k_iters = static_cast<int>(u.k_iters);
-        run->umma.tiles_m = u.tiles_m;
-        run->umma.tiles_n = u.tiles_n;
-        run->umma.raster_group = u.raster_group;
-        run->umma.k_splits = u.k_splits;
-        run->umma.k_iters_per_split = static_cast<int>(u.k_iters_per_split);
-        run->umma.full_chunks = static_cast<int>(u.full_chunks);
-        run->umma.split_stride = pl.sizeC;
-        fill_raster_divs(u, &run->umma);
+        fill_tiles(u, pl.sizeC, &run->umma);
         void* out = run->dC;
         const char* x3 = std::getenv("TCONT_TF32X3");
         run->tf32x3 = pl.kernel == KERNEL_UMMA_TF32 && x3 && x3[0] == '1' && !p.strided;
@@ -677,6 +686,15 @@ tcontb_status finish_run(tcontb_run* run)
                 run->umma.groups = u.groups[reads];
                 TC_CUDA(dmma_tma_configure(run->umma));
             }
+        if (pl.kernel == KERNEL_DMMA_F64_TMA && pl.wide_reads) {
+            run->umma_wide = run->umma;
+            fill_tiles(pl.umma, pl.sizeC, &run->umma_wide);
+            run->umma_wide.groups = pl.umma.groups[1];
+            st = encode_map(pl.umma.a, kA, pl.umma.elt, &run->tmAWide);
+            if (st == TCONTB_OK) st = encode_map(pl.umma.b, kB, pl.umma.elt, &run->tmBWide);
+            if (st != TCONTB_OK) return st;
+            TC_CUDA(dmma_tma_configure(run->umma_wide));
+        }
         TC_CUDA(splitk_reduce_configure());
     } else {
         fill_gather(p, kA, kB, run->dC, pl.simt, pl.gather, &run->gather);
@@ -1315,8 +1333,17 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
         TC_CUDA(launch_umma_tf32(umma, &run->tmA, &run->tmB, pl.umma.smem_bytes, run->num_sms, run->stream));
     }
     else if (pl.kernel == KERNEL_DMMA_F64_TMA) {
-        umma.groups = (pl.narrow.eligible ? pl.narrow : pl.umma).groups[umma.scaled && umma.beta != 0.0 ? 1 : 0];
-        TC_CUDA(launch_dmma_tma(umma, &run->tmA, &run->tmB, run->num_sms, run->stream));
+        const bool reads = umma.scaled && umma.beta != 0.0, wide = reads && pl.wide_reads;
+        if (wide) {
+            UmmaParams q = run->umma_wide;
+            q.scaled = umma.scaled;
+            q.alpha = umma.alpha;
+            q.beta = umma.beta;
+            umma = q;
+        } else {
+            umma.groups = (pl.narrow.eligible ? pl.narrow : pl.umma).groups[reads ? 1 : 0];
+        }
+        TC_CUDA(launch_dmma_tma(umma, wide ? &run->tmAWide : &run->tmA, wide ? &run->tmBWide : &run->tmB, run->num_sms, run->stream));
     }
     else {
         GatherParams g = run->gather;

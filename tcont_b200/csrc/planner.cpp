@@ -824,6 +824,17 @@ void set_dmma_groups(UmmaSpec* u, const CostTable& cost)
     }
 }
 
+// Whether launches that read the old values of C take the 128 x 64 tiles although plain ones are faster on narrow ones: rows along C, a C
+// a fifth larger than L2 or more.  128 x 64 reads the values a tile ahead from L2, narrow tiles copy them while they compute (K up to 64) or
+// ask for them at the end.  32 and 64 columns in us, C of 318 to 480 MB: 19456 x 2048 by 56 193 / 176, 39040 x 1024 by 56 196 / 189,
+// 39472 x 1520 by 80 380 / 348, 16096 x 2816 by 80 281 / 269, 31912 x 1880 by 96 439 / 406, and of 165 MB 89008 x 232 by 72 139 / 133; but
+// 624896 x 64 by 48 178 / 185, 156160 x 256 by 32 134 / 145, with a C of 135 MB 15424 x 1100 by 64 94.3 / 96.1 and of 80 MB 9728 x 1024 by 80
+// 66.5 / 74.3, by 96 74.7 / 78.3.
+bool wide_reads(const Problem& p, const UmmaSpec& wide, const UmmaSpec& narrow)
+{
+    return narrow.eligible && wide.BN == 64 && wide.k_splits == 1 && narrow.k_splits == 1 && !wide.store_across_slabs && wide.k_computed > 48 && double(p.sizeC) * 8.0 > 150e6;
+}
+
 // Time of the TMA-fed FP64 kernel in `s` ranges of k, for up to a few rounds of work units.  A block's SM has `groups` units in work: all
 // of them together are bound by the FP64 pipe, each by itself by its chain of k iterations (no shorter than the copies of a stage
 // take) and its store.  Fitted to 663 (128 x 32) and 446 (128 x 64) launches of 113 contractions of 4 MFLOP to 3 GFLOP in 1 to 48
@@ -1586,6 +1597,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
             pl.kernel = KERNEL_DMMA_F64_TMA;
         }
     }
+    pl.wide_reads = pl.kernel_without_narrow == KERNEL_DMMA_F64_TMA && wide_reads(p, pl.umma, pl.narrow) && !std::getenv("TCONT_DMMA_BN");
     for (UmmaSpec* u : {&pl.umma, &pl.narrow})
         if (u->eligible && u->elt == 8) set_dmma_groups(u, cost);
     if (pl.kernel == KERNEL_UMMA_TF32)
@@ -1667,7 +1679,7 @@ std::string describe_plan(const Plan& pl)
           << ",\"tiles_n\":" << pl.across.tiles_n << ",\"k_iters\":" << pl.across.k_iters << ",\"b_major\":\"" << (pl.across.b_major ? "MN" : "K") << "\"}";
     if (pl.narrow.eligible)
         o << ",\"narrow\":{\"BN\":" << pl.narrow.BN << ",\"BK\":" << pl.narrow.BK << ",\"stages\":" << pl.narrow.stages << ",\"slim\":" << (pl.narrow.slim ? "true" : "false") << ",\"tiles_m\":" << pl.narrow.tiles_m
-          << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << ",\"groups\":[" << pl.narrow.groups[0] << "," << pl.narrow.groups[1] << "]}";
+          << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << ",\"groups\":[" << pl.narrow.groups[0] << "," << pl.narrow.groups[1] << "],\"wide_reads\":" << (pl.wide_reads ? "true" : "false") << "}";
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";
     else {

@@ -230,6 +230,7 @@ struct Plan {
     UmmaSpec umma;
     UmmaSpec narrow;        // KERNEL_DMMA_F64_TMA: the 128 x 32 tiles that run in the place of `umma`'s where eligible
     int kernel_without_narrow = KERNEL_SIMT;   // which kernel that would be otherwise
+    bool wide_reads = false;                   // launches that read the old values of C run `umma`'s tiles all the same
     AcrossSpec across;      // KERNEL_UMMA_TF32: this form of it runs when `on`
     double est_direct_us = 0, est_ttgt_us = 0;
     double est_scaled_us[2] = {0, 0};   // Float32 on the tensor cores: with other alpha and beta than (1, 0), beta zero or not

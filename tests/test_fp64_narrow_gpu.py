@@ -163,3 +163,20 @@ def test_bounded_wait_gives_up_cleanly(engine, oracle, monkeypatch, columns, bet
     assert status == 1 and not right.all() and (right | (got == C0)).all()
     status, got = launched()
     assert status == 0 and (np.abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("A_,B_", [("ak", "kb"), ("ka", "bk")])
+def test_wide_tiles_where_old_values_are_read(engine, oracle, A_, B_):
+    """A C of 152 MB, rows along C: one run takes narrow tiles for plain launches and 128 x 64 for accumulating ones, in any order."""
+    c = Contraction("ab", A_, B_, dict(a=16400, b=1160, k=72), F64)
+    A, B = oracle.inputs(c, 53, -1.0, 1.0)
+    C0 = np.random.default_rng(12).uniform(-4.0, 4.0, c.size("ab"))
+    scalars = [(1.0, 1.0), (1.0, 0.0), (0.3, -0.7), (-0.75, 0.0), (1.0, 1.0)]
+    desc, got = scaled_run(engine, c, A, B, C0, scalars)
+    assert desc["kernel"] == "dmma_f64_tma" and desc["narrow"]["wide_reads"]
+    at = np.sort(np.random.default_rng(13).integers(0, C0.size, 20000))
+    product, scale = oracle.contract_sampled(c, A, B, at), oracle.contract_sampled(c, np.abs(A), np.abs(B), at)
+    for (alpha, beta), out in zip(scalars, got):
+        bound = (72 + 4) * 2.0**-53 * (abs(alpha) * scale + abs(beta * C0[at]))
+        assert (np.abs(out[at] - (alpha * product + beta * C0[at])) <= bound).all(), (alpha, beta)
+    assert (got[0] == got[4]).all()

@@ -398,6 +398,21 @@ def test_fp64_consumer_groups(engine, monkeypatch):
     assert groups("ab", "ak", "kb", a=9216, b=4096, k=32) == (32, 3, 3)
 
 
+def test_fp64_wide_tiles_where_old_values_are_read(engine, monkeypatch):
+    """Rows along C, a C of more than 150 MB and more than 48 k: accumulating launches on 128 x 64 tiles, plain ones on narrow ones."""
+    F64 = 1
+
+    def wide(C, A, B, **ext):
+        d = describe(engine, Contraction(C, A, B, ext, F64), 1)
+        assert "narrow" in d and d["kernel"] == "dmma_f64_tma"
+        return d["narrow"]["wide_reads"]
+    assert wide("ab", "ak", "kb", a=18432, b=1024, k=64) and not wide("ab", "ak", "kb", a=18304, b=1024, k=64)
+    assert wide("ab", "ka", "bk", a=39040, b=1024, k=56) and not wide("ab", "ka", "bk", a=39040, b=1024, k=48)
+    assert not wide("abcd", "dbka", "kc", a=24, b=64, c=512, d=32, k=96)
+    monkeypatch.setenv("TCONT_DMMA_BN", "32")
+    assert not wide("ab", "ak", "kb", a=18432, b=1024, k=64)
+
+
 def test_fp64_ranges_on_narrow_tiles(engine, monkeypatch):
     """Few tiles: ranges of k on narrow tiles in the place of ranges on wide ones, and of the gather kernel above 13.5 us."""
     F64 = 1
