@@ -862,6 +862,11 @@ UmmaSpec narrow_ranges(const Problem& p, const CostTable& cost, const UmmaSpec& 
     *us = 1e300;
     if (!u.eligible || u.elt != 8 || std::getenv("TCONT_SPLITK") || std::getenv("TCONT_DMMA_BN")) return v;
     if ((u.a.row_elem_cstride != 1 && !u.store_across_slabs) || u.a.slab_mode_ext < 8) return v;   // (stores of single elements)
+    // Where A's slabs and k chunks of 8 meet, a stage is 16 to 20 copies of 512 bytes, which three producers wait for each other with, more
+    // than the estimate knows, and 64 columns halve: of 20 contractions half were faster on narrow tiles, 40 x 8 x 8 x 8 by 1536 18.6 us of
+    // 21.2, half slower, 24 x 56 x 40 x 24 by 384 58.3 of 49.6.  With k chunks of 16 they gain: 72 x 16 x 72 x 64 by 2560 (27 GFLOP, one range
+    // instead of three) 788 us of 847, and all but 5 of 48 others, which gain in two consumer groups.
+    if (u.BK == 8 && u.a.major == 1 && u.a.slab_w == 8) return v;
     if (u.BN == 32) v = u;
     else plan_umma_impl(p, cost, &v, 32, true, true);
     if (!v.eligible) return v;

@@ -372,6 +372,16 @@ def test_fp64_narrow_tiles(engine, monkeypatch):
     assert not narrow(rows(4096, 16)) and describe(engine, rows(4096, 16), 1)["umma"]["in_use"]
 
 
+def test_fp64_ranges_where_slabs_and_k_chunks_of_8_meet(engine):
+    """These stay on the tiles and ranges planned without narrow ones, whatever their size; with k chunks of 16 large ones go narrow too."""
+    F64 = 1
+    plan = lambda C, A, B, *extents: describe(engine, Contraction(C, A, B, dict(zip("abcdef", extents)), F64))
+    for d in (plan("abcd", "aecf", "fbed", 24, 56, 40, 24, 16, 24), plan("abcd", "aebf", "fdec", 24, 32, 40, 40, 32, 40), plan("abcd", "aebf", "dfce", 40, 8, 8, 8, 64, 24)):
+        assert d["kernel"] == "dmma_f64_tma" and "narrow" not in d and (d["umma"]["BK"], d["umma"]["a_slab_w"]) == (8, 8) and d["umma"]["k_splits"] > 1
+    d = plan("abcd", "aebf", "dfce", 72, 16, 72, 64, 40, 64)
+    assert (d["umma"]["BK"], d["umma"]["a_slab_w"], d["umma"]["k_splits"]) == (16, 8, 3) and d["narrow"]["k_splits"] == 1
+
+
 def test_fp64_consumer_groups(engine, monkeypatch):
     """Two consumer groups on 128 x 32 tiles: where three would not spare a round of them, for pieces of 8 or 16 bytes, and for one or two
     k chunks of 16 along C; three where old values are read in wider pieces, across slabs, and where A's slabs and k chunks of 8 meet."""
