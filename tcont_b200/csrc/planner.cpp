@@ -1006,11 +1006,16 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors 
             if (us < best.est_us) {
                 best = g;
                 best.cluster = s;
-                // One column of Float32 tiles: blocks of one tile each, of which more fit an SM at different stages, read a long A in
-                // step better than a few persistent ones.  Persistent / one tile a block in us, 64 x 64: 2689715 x 37 x 19 1491 / 873,
-                // 4604655 x 55 x 33 5106 / 3044, 100233 x 49 x 25 23.8 / 22.8, but 423948 x 59 x 50 127 / 131; 128 x 128: 462231 x 69 x 43
-                // 311 / 247, 769356 x 71 x 57 470 / 429, but 1026189 x 95 x 23 308 / 325.  FP64 is up to twice as slow that way.
-                const bool few_k_tiles = (t == GATHER_SQUARE && iters >= 2 && iters <= 3) || (t == GATHER_BIG && iters >= 3);
+                // One column of Float32 tiles in two or three (64 x 64) and three or four (128 x 128) k tiles: blocks of one tile each, of which
+                // more fit an SM at different stages, instead of a few persistent ones.  They read an A whose stride-1 mode is another row
+                // mode than C's, a sector an element, in step.  Persistent / one tile a block in us: 2689715 x 35 x 19 1510 / 872, 4604655 x 45
+                // x 33 5177 / 2979, 462231 x 113 x 43 315 / 250.  Elsewhere they multiply a last k tile whole, which the persistent ones cut
+                // off: 64 x 64 by the k in it 2 149 / 172, 3 44 / 51, 8 70 / 74, 11 23.0 / 25.0 to 84 / 80, 12 295 / 281, 14 30.1 / 26.3; 128 x
+                // 128 4 89 / 99, 7 350 / 362, 8 147 / 147, 9 190 / 177, 10 34.7 / 30.1, 14 196 / 176.  FP64 is up to twice as slow that way.
+                const bool scattered_rows = g.t0 == 0 && p.A[0] != p.M[0] && p.modes[static_cast<size_t>(p.A[0])].group == GROUP_M;
+                const int64_t last_k = (p.Ktot - 1) % 16 + 1;
+                const bool few_k_tiles = (t == GATHER_SQUARE && iters >= 2 && iters <= 3 && (scattered_rows || last_k >= 12)) ||
+                                         (t == GATHER_BIG && iters >= 3 && (scattered_rows || last_k >= 9));
                 best.flat = flat && (f64 || tiles_n > 1 || !few_k_tiles);
                 if (force_flat) best.flat = s == 1 && force_flat[0] == '1' && (f64 || t != GATHER_SMALL);   // (the small Float32 tile has no such form)
                 best.est_us = us;

@@ -442,11 +442,15 @@ def test_fp64_ranges_on_narrow_tiles(engine, monkeypatch):
     assert "narrow" not in describe(engine, Contraction("abcd", "aecf", "bfde", dict(a=32, b=32, c=32, d=40, e=16, f=24), F64))
 
 
-@pytest.mark.parametrize("b,k,tile,flat", [(57, 16, 0, True), (57, 17, 0, False), (57, 48, 0, False), (57, 49, 0, True), (77, 32, 3, True), (77, 33, 3, False), (77, 64, 3, False),
-                                           (131, 33, None, True)])
+@pytest.mark.parametrize("b,k,tile,flat", [(57, 16, 0, True), (57, 17, 0, True), (57, 27, 0, True), (57, 28, 0, False), (57, 48, 0, False), (57, 49, 0, True),
+                                           (77, 32, 3, True), (77, 33, 3, True), (77, 40, 3, True), (77, 41, 3, False), (77, 64, 3, False), (131, 33, None, True)])
 def test_one_column_of_float32_tiles(engine, monkeypatch, b, k, tile, flat):
-    """Many rows and one column of tiles: one tile a block where a tile has a few k tiles, persistent blocks otherwise."""
+    """Many rows and one column of tiles: one tile a block where a tile has a few k tiles, the last of them well filled, persistent blocks
+    otherwise; whatever the last one holds where A's rows lie scattered."""
     monkeypatch.setenv("TCONT_KERNEL", "simt")
     monkeypatch.setenv("TCONT_GATHER_TILE", str(3 if tile is None else tile))
     g = describe(engine, Contraction("ab", "ka", "bk", dict(a=400003, b=b, k=k), F32), 1)["gather"]
     assert g["cluster"] == 1 and g["flat"] == flat, g
+    if tile is not None:
+        g = describe(engine, Contraction("abcd", "dbea", "ec", dict(a=57, b=81, c=b, d=83, e=k), F32), 1)["gather"]
+        assert g["cluster"] == 1 and g["flat"] == (k <= 16 or (tile == 0 and k > 48) or (tile == 3 and k <= 32)), g
