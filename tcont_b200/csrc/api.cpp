@@ -501,6 +501,7 @@ void fill_gather(const Problem& p, const void* A, const void* B, void* C, const 
     g.b_along_k = simt.b_load_along_k;
     g.cluster = spec.cluster;
     g.flat = spec.flat ? 1 : 0;
+    g.form = spec.form;
     g.alpha = 1.0;
     *out = g;
 }

@@ -635,18 +635,6 @@ using F32Tall = GatherCfg<float, 128, 32, 2, 2, 1, false, 4, 4>;
 using F32TallFlat = GatherCfg<float, 128, 32, 2, 2, 1, true, 4, 3>;
 using F32Small = GatherCfg<float, 32, 32, 1, 2, 4, false, 4, 4>;
 
-// Whether the 128 x 128 Float32 tile runs in four wide warps instead of eight.  A wide block takes longer to begin and to end, with
-// half the threads, the more so in a large cluster, and has to make that good in its range of k.  Old / wide in us, by k per block:
-// one block to a tile, 5003 x 3001: 101 108 / 111, 201 194 / 183, 601 513 / 442; clusters of 2, 1401 x 1401: 100 52 / 39, 300 87 / 73;
-// of 4, 1801 x 1501: 75 77 / 80, 100 107 / 98; of 8, 701 x 701: 75 39 / 46, 400 170 / 142.  With no more blocks than SMs the one warp
-// on each scheduler has its latencies to itself (301 x 301 x 9201 in clusters of 16: 103 / 102), so the old kind stays there.
-bool wide(const GatherParams& p, int num_sms)
-{
-    const long long blocks = (p.M + F32Wide::BM - 1) / F32Wide::BM * ((p.N + F32Wide::BN - 1) / F32Wide::BN) * p.cluster;
-    const int least_k = p.cluster == 1 ? 160 : p.cluster <= 4 ? 96 : 192;
-    return blocks > num_sms && p.K / p.cluster >= least_k;
-}
-
 }  // namespace
 
 cudaError_t gather_configure()
@@ -682,10 +670,9 @@ cudaError_t launch_gather_contract(const GatherParams& p, int scalar_type, int t
         if (tile == GATHER_TALL) return p.flat ? launch<F64TallFlat>(p, num_sms, stream) : launch<F64Tall>(p, num_sms, stream);
         if (tile == GATHER_SMALL) return p.flat ? launch<F64SmallFlat>(p, num_sms, stream) : launch<F64Small>(p, num_sms, stream);
     } else {
-        if (tile == GATHER_BIG && !p.flat && wide(p, num_sms)) return launch<F32Wide>(p, num_sms, stream);
+        if (tile == GATHER_BIG && p.form == GATHER_FORM_WIDE) return launch<F32Wide>(p, num_sms, stream);
         if (tile == GATHER_BIG) return p.flat ? launch<F32BigFlat>(p, num_sms, stream) : launch<F32Big>(p, num_sms, stream);
-        // One block to a tile and few k: direct stores of whole lines (126 x 145 x 95 by 27 10.6 us, 11.3 by way of shared memory).
-        if (tile == GATHER_SQUARE && !p.flat && p.cluster == 1 && p.K < 48) return launch<F32SquareShort>(p, num_sms, stream);
+        if (tile == GATHER_SQUARE && p.form == GATHER_FORM_SHORT) return launch<F32SquareShort>(p, num_sms, stream);
         if (tile == GATHER_SQUARE) return p.flat ? launch<F32SquareFlat>(p, num_sms, stream) : launch<F32Square>(p, num_sms, stream);
         if (tile == GATHER_TALL) return p.flat ? launch<F32TallFlat>(p, num_sms, stream) : launch<F32Tall>(p, num_sms, stream);
         if (tile == GATHER_SMALL && !p.flat) return launch<F32Small>(p, num_sms, stream);

@@ -99,6 +99,7 @@ struct GatherParams {
     int a_along_k, b_along_k;  // 0: neighbouring threads gather neighbouring rows, 1: neighbouring k
     int cluster;               // CTAs that share a tile, each a range of k (1: no split)
     int flat;                  // 1: persistent blocks, one ring of stages across their tiles (cluster 1 only)
+    int form;                  // GATHER_FORM_*
     int scaled;                // 0: C = A B; 1: C = alpha A B + beta C (C read only when beta is not zero)
     double alpha, beta;
     int release_late;          // the rest is filled in by the launcher: when the next kernel's blocks may be scheduled

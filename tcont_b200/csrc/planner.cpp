@@ -919,6 +919,19 @@ double wave_efficiency(int64_t tiles, int sms)
 // (throughput), but none faster than one alone (latency), which is what bounds small problems and what a split of k
 // shortens.  Measured on 60 contractions of 2 MFLOP to 280 GFLOP with every tile, cluster and form: the choice is within
 // 11 % of the best one on average.
+// The 128 x 128 Float32 tile in four wide warps instead of eight.  A wide block takes longer to begin and to end, with
+// half the threads, the more so in a large cluster, and has to make that good in its range of k.  Old / wide in us, by k per block:
+// one block to a tile, 5003 x 3001: 101 108 / 111, 201 194 / 183, 601 513 / 442; clusters of 2, 1401 x 1401: 100 52 / 39, 300 87 / 73;
+// of 4, 1801 x 1501: 75 77 / 80, 100 107 / 98; of 8, 701 x 701: 75 39 / 46, 400 170 / 142.  With no more blocks than SMs the one warp
+// on each scheduler has its latencies to itself (301 x 301 x 9201 in clusters of 16: 103 / 102), so the old kind stays there.
+// 64 x 64 tiles, one block to a tile and few k: direct stores of whole lines (126 x 145 x 95 by 27 10.6 us, 11.3 by way of shared memory).
+int float32_form(const GatherSpec& g, const Problem& p, const CostTable& c)
+{
+    if (g.tile == GATHER_SQUARE && g.cluster == 1 && p.Ktot < 48) return GATHER_FORM_SHORT;
+    const int64_t blocks = ceil_div(g.rows, 128) * ceil_div(p.Ntot, 128) * g.cluster, least_k = g.cluster == 1 ? 160 : g.cluster <= 4 ? 96 : 192;
+    return g.tile == GATHER_BIG && blocks > c.num_sms && p.Ktot / g.cluster >= least_k ? GATHER_FORM_WIDE : GATHER_FORM_PLAIN;
+}
+
 GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors = true)
 {
     const bool f64 = p.scalar_type == 1;
@@ -1023,6 +1036,7 @@ GatherSpec plan_gather(const Problem& p, const CostTable& c, bool count_sectors 
             }
         }
     }
+    best.form = f64 || best.flat ? GATHER_FORM_PLAIN : float32_form(best, p, c);
     best.est_us += sector_us;   // (the choice of a tile is as good without it: its rates have it in part)
     return best;
 }
@@ -1654,6 +1668,11 @@ bool cuts_into_ranges(const Plan& pl, int ranges, std::string* why)
     return u.b.total_slabs % ranges == 0 && (u.b.total_slabs / ranges) % tile_slabs == 0;
 }
 
+static const char* kernel_name(int kernel)
+{
+    return kernel == KERNEL_UMMA_TF32 ? "umma_tf32" : kernel == KERNEL_DMMA_F64 ? "dmma_f64" : kernel == KERNEL_DMMA_F64_TMA ? "dmma_f64_tma" : "simt";
+}
+
 std::string describe_plan(const Plan& pl)
 {
     std::ostringstream o;
@@ -1672,8 +1691,7 @@ std::string describe_plan(const Plan& pl)
         return s + "]";
     };
     o << "{\"backend\":\"" << (pl.backend == 0 ? "direct" : "ttgt") << "\",\"kernel\":\""
-      << (pl.kernel == KERNEL_UMMA_TF32 ? "umma_tf32" : pl.kernel == KERNEL_DMMA_F64 ? "dmma_f64"
-          : pl.kernel == KERNEL_DMMA_F64_TMA ? "dmma_f64_tma" : "simt") << "\""
+      << kernel_name(pl.kernel) << "\""
       << ",\"scalar\":\"" << (pl.scalar_type == 1 ? "f64" : "f32") << "\",\"swapped\":" << (p.swapped ? "true" : "false")
       << ",\"views\":" << (p.strided ? "true" : "false")
       << ",\"A\":" << list(p.A) << ",\"B\":" << list(p.B) << ",\"C\":" << list(p.C) << ",\"M\":" << list(p.M)
@@ -1682,14 +1700,15 @@ std::string describe_plan(const Plan& pl)
       << ",\"transpose_b\":" << (pl.tB.needed ? perm(pl.tB) : "null") << ",\"est_direct_us\":" << pl.est_direct_us
       << ",\"est_ttgt_us\":" << pl.est_ttgt_us << ",\"simt\":{\"a_along_k\":" << pl.simt.a_load_along_k
       << ",\"b_along_k\":" << pl.simt.b_load_along_k << "},\"gather\":{\"tile\":" << pl.gather.tile
-      << ",\"cluster\":" << pl.gather.cluster << ",\"flat\":" << (pl.gather.flat ? "true" : "false") << ",\"t0\":" << pl.gather.t0 << ",\"t1\":" << pl.gather.t1 << ",\"rows\":" << pl.gather.rows << ",\"est_us\":" << pl.gather.est_us << "}";
+      << ",\"cluster\":" << pl.gather.cluster << ",\"flat\":" << (pl.gather.flat ? "true" : "false")
+      << ",\"form\":\"" << (pl.gather.form == GATHER_FORM_WIDE ? "wide" : pl.gather.form == GATHER_FORM_SHORT ? "short" : "plain") << "\",\"t0\":" << pl.gather.t0 << ",\"t1\":" << pl.gather.t1 << ",\"rows\":" << pl.gather.rows << ",\"est_us\":" << pl.gather.est_us << "}";
     const UmmaSpec& u = pl.umma;
     if (pl.across.on)
         o << ",\"across\":{\"BN\":" << pl.across.BN << ",\"BK\":" << pl.across.BK << ",\"stages\":" << pl.across.stages << ",\"tiles_m\":" << pl.across.tiles_m
           << ",\"tiles_n\":" << pl.across.tiles_n << ",\"k_iters\":" << pl.across.k_iters << ",\"b_major\":\"" << (pl.across.b_major ? "MN" : "K") << "\"}";
     if (pl.narrow.eligible)
         o << ",\"narrow\":{\"BN\":" << pl.narrow.BN << ",\"BK\":" << pl.narrow.BK << ",\"stages\":" << pl.narrow.stages << ",\"slim\":" << (pl.narrow.slim ? "true" : "false") << ",\"tiles_m\":" << pl.narrow.tiles_m
-          << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << ",\"groups\":[" << pl.narrow.groups[0] << "," << pl.narrow.groups[1] << "],\"wide_reads\":" << (pl.wide_reads ? "true" : "false") << "}";
+          << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << ",\"groups\":[" << pl.narrow.groups[0] << "," << pl.narrow.groups[1] << "],\"wide_reads\":" << (pl.wide_reads ? "true" : "false") << ",\"instead_of\":\"" << kernel_name(pl.kernel_without_narrow) << "\"}";
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";
     else {

@@ -151,11 +151,13 @@ struct SimtSpec {
 
 // Tiles of the gather kernel (gather_contract.cu).
 enum GatherTile { GATHER_SQUARE = 0, GATHER_TALL = 1, GATHER_SMALL = 2, GATHER_BIG = 3 };
+enum GatherForm { GATHER_FORM_PLAIN = 0, GATHER_FORM_SHORT = 1, GATHER_FORM_WIDE = 2 };   // Float32 blocks of one tile, see float32_form
 constexpr int kMaxGatherCluster = 16;
 struct GatherSpec {
     int tile = GATHER_SQUARE;
     int cluster = 1;     // CTAs that share an output tile, each contracting a range of k
     bool flat = false;   // persistent blocks (see GatherParams)
+    int form = GATHER_FORM_PLAIN;
     // Rows cut in two modes: a tile is t0 indices of C's stride-1 mode times t1 of A's (0: rows in C's order)
     int t0 = 0, t1 = 0;
     int64_t rows = 1;    // rows of the GEMM view, cut modes rounded up

@@ -34,7 +34,7 @@ def test_forms(engine, oracle, monkeypatch, name):
     C0 = np.random.default_rng(7).uniform(-4.0, 4.0, c.size(C)).astype(np.float32)
     desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
     assert desc["kernel"] == "simt" and desc["gather"]["tile"] == 3 and not desc["gather"]["flat"], desc["gather"]
-    assert desc["gather"]["cluster"] == cluster, desc["gather"]
+    assert desc["gather"]["cluster"] == cluster and desc["gather"]["form"] == "wide", desc["gather"]
     c64 = Contraction(C, A_, B_, ext, F64)
     product, scale = oracle.contract(c64, A.astype(np.float64), B.astype(np.float64)), oracle.contract(c64, np.abs(A).astype(np.float64), np.abs(B).astype(np.float64))
     k = int(np.prod([ext[m] for m in A_ if m not in C]))
@@ -51,7 +51,7 @@ def test_small_clusters_of_64_by_64_tiles(engine, oracle, monkeypatch, scalar_ty
     A, B = oracle.inputs(c, 37, -1.0, 1.0)
     C0 = np.random.default_rng(8).uniform(-4.0, 4.0, c.size("ab")).astype(A.dtype)
     desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
-    assert desc["gather"]["tile"] == 0 and desc["gather"]["cluster"] == cluster, desc["gather"]
+    assert desc["gather"]["tile"] == 0 and desc["gather"]["cluster"] == cluster and desc["gather"]["form"] == "plain", desc["gather"]
     c64 = Contraction("ab", "ka", "bk", dict(a=a, b=b, k=k), F64)
     product, scale = oracle.contract(c64, A.astype(np.float64), B.astype(np.float64)), oracle.contract(c64, np.abs(A).astype(np.float64), np.abs(B).astype(np.float64))
     unit = 2.0**-24 if scalar_type == F32 else 2.0**-53
@@ -73,7 +73,7 @@ def test_64_by_64_tiles(engine, oracle, monkeypatch, cluster, A_, B_, k):
     C0 = np.random.default_rng(9).uniform(-4.0, 4.0, c.size("ab")).astype(np.float32)
     desc, got = scaled_run(engine, c, A, B, C0, SCALARS)
     g = desc["gather"]
-    assert g["tile"] == 0 and g["cluster"] == cluster and not g["flat"], g
+    assert g["tile"] == 0 and g["cluster"] == cluster and not g["flat"] and g["form"] == ("short" if cluster == 1 and k < 48 else "plain"), g
     product, scale = oracle.contract(c64, A.astype(np.float64), B.astype(np.float64)), oracle.contract(c64, np.abs(A).astype(np.float64), np.abs(B).astype(np.float64))
     for (alpha, beta), out in zip(SCALARS, got):
         bound = (k + 20) * 2.0**-24 * (abs(alpha) * scale + abs(beta * C0))

@@ -96,13 +96,14 @@ RANGES = {
 
 @pytest.mark.parametrize("name", list(RANGES))
 def test_ranges(engine, oracle, monkeypatch, name):
-    C, A_, B_, ext, _ = RANGES[name]
+    C, A_, B_, ext, instead_of = RANGES[name]
     c = Contraction(C, A_, B_, ext, F64)
     A, B = oracle.inputs(c, 31, -1.0, 1.0)
     C0 = np.random.default_rng(7).uniform(-4.0, 4.0, c.size(C))
     desc, got = scaled_run(engine, c, A, B, C0, SCALARS, 0)
     ranges = desc["narrow"]["k_splits"]
-    assert desc["kernel"] == "dmma_f64_tma" and (ranges == 1) == (name == "one_range")
+    assert desc["kernel"] == "dmma_f64_tma" and (ranges == 1) == (name == "one_range") and desc["narrow"]["instead_of"] == instead_of
+    assert desc["umma"]["k_splits"] != ranges
     product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
     k = int(np.prod([ext[m] for m in ext if m not in C]))
     for (alpha, beta), out in zip(SCALARS, got):   # (and a rounding for each partial sum)
@@ -111,13 +112,23 @@ def test_ranges(engine, oracle, monkeypatch, name):
 
 
 def test_no_room_for_ranges(engine, oracle, monkeypatch):
-    """The gather kernel runs where the partial sums find no room."""
+    """The gather kernel runs where the partial sums find no room: one kernel a launch, no sum behind it."""
+    import torch
     C, A_, B_, ext, _ = RANGES["from_the_gather_kernel"]
     c = Contraction(C, A_, B_, ext, F64)
     A, B = oracle.inputs(c, 31, -1.0, 1.0)
+    from tcont_b200 import api
+    plan = engine.plan(to_equation(engine, c, 0))
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    dC = torch.zeros(c.size(C), dtype=dA.dtype, device="cuda")
+
+    def kernels():
+        return api.prepare_on_device(plan, dA.data_ptr(), dB.data_ptr(), dC.data_ptr(), keep=(dA, dB, dC)).time_launches(1)[1]
+    assert kernels() == 2   # the ranges and their sum
     monkeypatch.setenv("TCONT_TEST_NO_ROOM", "1000")
+    assert kernels() == 1
     desc, got = scaled_run(engine, c, A, B, np.ones(c.size(C)), [(1.0, 1.0), (1.0, 0.0)], 0)
-    assert desc["narrow"]["k_splits"] > 1
+    assert desc["narrow"]["k_splits"] > 1 and desc["narrow"]["instead_of"] == RANGES["from_the_gather_kernel"][4]
     product, scale = oracle.contract(c, A, B), oracle.contract(c, np.abs(A), np.abs(B))
     for beta, out in zip((1.0, 0.0), got):
         assert (np.abs(out - (product + beta)) <= (256 + 8) * 2.0**-53 * (scale + beta)).all()

@@ -434,12 +434,28 @@ def test_fp64_ranges_on_narrow_tiles(engine, monkeypatch):
     monkeypatch.delenv("TCONT_KERNEL")
     smaller = Contraction("ab", "ak", "kb", dict(a=128, b=104, k=496), F64)
     assert describe(engine, smaller)["kernel"] == "simt" and "narrow" not in describe(engine, smaller)
-    longer = Contraction("ab", "ak", "kb", dict(a=64, b=64, k=60000), F64)   # one chain of FMAs where nothing else was planned
-    assert describe(engine, longer)["kernel"] != "simt" or "narrow" not in describe(engine, longer)
+    # more than 49 152 k on the gather kernel, operands that TMA could stage: one chain of FMAs
+    longer = describe(engine, Contraction("abcdef", "degb", "gfac", dict(a=4, b=16, c=12, d=24, e=16, f=12, g=62714), F64), 1)
+    assert longer["kernel"] != "dmma_f64_tma" and longer["umma"]["eligible"] and "narrow" not in longer and longer["gather"]["cluster"] == 1
+    long_on_tma = describe(engine, Contraction("ab", "ak", "kb", dict(a=64, b=64, k=60000), F64))
+    assert long_on_tma["kernel"] == "dmma_f64_tma" and long_on_tma["narrow"]["k_splits"] > 1 and long_on_tma["narrow"]["instead_of"] == "dmma_f64_tma"
     many = describe(engine, Contraction("abcd", "aecf", "bfde", dict(a=32, b=32, c=32, d=40, e=16, f=24), F64))
     assert many["umma"]["k_splits"] == 3 and many["narrow"]["k_splits"] == 2
     monkeypatch.setenv("TCONT_SPLITK", "3")
     assert "narrow" not in describe(engine, Contraction("abcd", "aecf", "bfde", dict(a=32, b=32, c=32, d=40, e=16, f=24), F64))
+
+
+@pytest.mark.parametrize("tile,cluster,a,k,form", [(3, 1, 3201, 159, "plain"), (3, 1, 3201, 160, "wide"), (3, 2, 1401, 191, "plain"), (3, 2, 1401, 192, "wide"),
+                                                   (3, 4, 1801, 383, "plain"), (3, 4, 1801, 384, "wide"), (3, 8, 701, 1535, "plain"), (3, 8, 701, 1536, "wide"),
+                                                   (3, 4, 700, 384, "plain"), (0, 1, 323, 47, "short"), (0, 1, 323, 48, "plain"), (0, 2, 323, 49, "plain")])
+def test_forms_of_float32_tiles(engine, monkeypatch, tile, cluster, a, k, form):
+    """Four wide warps from a number of k per block on and with more blocks than SMs; full lines for short ranges of k."""
+    monkeypatch.setenv("TCONT_KERNEL", "simt")
+    monkeypatch.setenv("TCONT_GATHER_TILE", str(tile))
+    monkeypatch.setenv("TCONT_GATHER_CLUSTER", str(cluster))
+    monkeypatch.setenv("TCONT_GATHER_FLAT", "0")
+    g = describe(engine, Contraction("ab", "ka", "bk", dict(a=a, b=a - 1, k=k), F32), 1)["gather"]
+    assert (g["tile"], g["cluster"], g["form"]) == (tile, cluster, form), g
 
 
 @pytest.mark.parametrize("b,k,tile,flat", [(57, 16, 0, True), (57, 17, 0, True), (57, 27, 0, True), (57, 28, 0, False), (57, 48, 0, False), (57, 49, 0, True),
