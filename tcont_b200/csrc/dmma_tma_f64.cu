@@ -523,9 +523,9 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
             // Old values of C: a step copies what the four lanes of a quad need of one piece of their rows (two elements a lane, W columns),
             // neighbouring lanes neighbouring bytes at both ends (with the bytes a lane needs lying together instead, each 16 were a request
             // of their own: 9216 x 4096 x 24, rows along C, 163 us).
-            int copied = SCALED && staged && p.beta != 0.0 ? 0 : kCopySteps;
+            int copied = SCALED && staged ? 0 : kCopySteps;   // (staged: beta is not zero)
             long long cc[W];
-            if (SCALED && staged && p.beta != 0.0) {
+            if (SCALED && staged) {
                 tile_ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(tab_full + slot), (round >> 1) & 1u, abort_flag)) && tile_ok;
                 if (!tile_ok) copied = kCopySteps;
                 tile_cols(slot, cc);
@@ -610,9 +610,8 @@ dmma_tma_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
                     for (int q = 0; q < PIECE; q += 2)
 #pragma unroll
                         for (int j = 0; j < W; ++j) {
-                            double x = 0.0, y = 0.0;
-                            if (p.beta == 0.0) {
-                            } else if (PIECES || p.piece >= 2) {
+                            double x, y;
+                            if (PIECES || p.piece >= 2) {
                                 ld_shared_v2f64(old_from + static_cast<uint32_t>(u * PIECE / 2 * W + j) * 2048u + static_cast<uint32_t>(q) * 8u, x, y);
                             } else {
                                 const uint32_t at_u = old_from + static_cast<uint32_t>(u * PIECE * W + j) * 1024u;
@@ -839,7 +838,7 @@ cudaError_t launch_dmma_tma(const UmmaParams& p, const void* tmapA, const void* 
     auto share_stages = [&](int bytes) { q.stages = std::min(p.stages, (kMaxDynamicSmemBytes - bytes) / stage_bytes) / groups * groups; };
     int fixed = 1024 + kAuxBytes + 2 * groups * static_cast<int>(groups == 2 ? kTabBytes<8> : kTabBytes<4>);
     share_stages(fixed);
-    // Room for the old values leaves two or three stages a group, where the tile's main loop is long enough to hide them behind anyway:
+    // Room for the old values leaves two or three stages a group (four with k chunks of 8), where the tile's main loop is long enough to hide them behind anyway:
     // 172032 x 72 x 112, rows along C, 149 us staged, 137 read in the epilogue; K 48 168 and 174; across slabs K 72 73 and 86, K 128 342 and 344.
     q.old_staged = groups == 3 && p.scaled && p.beta != 0.0 && p.k_iters * p.BK <= (p.store_across_slabs ? 128 : 64) ? 1 : 0;
     if (q.old_staged) share_stages(fixed += groups * kOldBytes);
