@@ -544,8 +544,8 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
     // 4, 6-8: C[a,...] from A[d,...,a]).  Rows that run along A's stride-1 mode alone would be stored element by
     // element, and moving a 200-300 MB A through a transpose first costs more than the contraction.  Instead a
     // tile is 8 slabs of 16 rows: 16 consecutive elements of A's stride-1 mode (one 128-byte TMA row) times 8
-    // consecutive indices of C's stride-1 mode, fetched by ONE box that spans both modes, and a thread stores
-    // the same row of four neighbouring slabs as one 32-byte piece of C.  Needs C's stride-1 mode behind the
+    // consecutive indices of C's stride-1 mode, fetched by ONE box that spans both modes, and four
+    // lanes store the same row of the eight slabs, 64 bytes of C, two slabs each.  Needs C's stride-1 mode behind the
     // chunked contracted mode in A's memory order (the box then lands slab by slab) and an extent that is a
     // multiple of 8 (a tile never wraps to the next chunk).
     int lead_a = -1;

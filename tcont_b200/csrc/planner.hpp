@@ -109,7 +109,7 @@ struct UmmaSpec {
     bool pair = false;  // two-CTA clusters working on 256-row tiles (tcgen05 cta_group::2)
     int producers = 1;  // tcgen05 kernel: producer warps taking turns stage by stage (2 needs an even number of stages)
     // FP64 kernel: the slabs of an A tile are consecutive indices of C's stride-1 mode (which is not A's stride-1
-    // mode); a thread stores the same row of four neighbouring slabs as one 32-byte piece
+    // mode); a thread stores the same row of two neighbouring slabs, 16 of the 64 bytes that four lanes have together
     bool store_across_slabs = false;
     // FP64 kernel: of the four elements of C a thread stores at a time so many (4, 2 or 1) are neighbours, lie together inside C or
     // beyond it, and start on a multiple of so many elements from C's first
