@@ -343,7 +343,7 @@ void fill_tiles(const UmmaSpec& u, int64_t size_c, UmmaParams* out)
     out->producers = u.producers;
     out->store_across_slabs = u.store_across_slabs ? 1 : 0;
     out->piece = u.piece;
-    out->slim = u.slim ? 1 : 0;
+    out->slim = u.slim[0] ? 1 : 0;
     out->n_k_digits = u.n_k_digits;
     for (int i = 0; i < 3; ++i) out->k_digit_ext[i] = static_cast<int>(u.k_digit_ext[i]);
     out->k_iters = static_cast<int>(u.k_iters);
@@ -683,8 +683,9 @@ tcontb_status finish_run(tcontb_run* run)
         if (u.smem_bytes > kMaxDynamicSmemBytes) return fail(TCONTB_RUNTIME_ERROR, "plan asks for more shared memory than a block can have");
         if (pl.kernel == KERNEL_UMMA_TF32) TC_CUDA(umma_tf32_configure());
         else
-            for (int reads = 0; reads < (u.groups[0] == u.groups[1] ? 1 : 2); ++reads) {
+            for (int reads = 0; reads < (u.groups[0] == u.groups[1] && u.slim[0] == u.slim[1] ? 1 : 2); ++reads) {
                 run->umma.groups = u.groups[reads];
+                run->umma.slim = u.slim[reads] ? 1 : 0;
                 TC_CUDA(dmma_tma_configure(run->umma));
             }
         if (pl.kernel == KERNEL_DMMA_F64_TMA && pl.wide_reads) {
@@ -1342,7 +1343,9 @@ tcontb_status tcontb_run_launch(tcontb_run* run)
             q.beta = umma.beta;
             umma = q;
         } else {
-            umma.groups = (pl.narrow.eligible ? pl.narrow : pl.umma).groups[reads ? 1 : 0];
+            const UmmaSpec& u = pl.narrow.eligible ? pl.narrow : pl.umma;
+            umma.groups = u.groups[reads ? 1 : 0];
+            umma.slim = u.slim[reads ? 1 : 0] ? 1 : 0;
         }
         TC_CUDA(launch_dmma_tma(umma, wide ? &run->tmAWide : &run->tmA, wide ? &run->tmBWide : &run->tmB, run->num_sms, run->stream));
     }

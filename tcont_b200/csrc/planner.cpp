@@ -738,7 +738,19 @@ void plan_umma_impl(const Problem& p_in, const CostTable& cost, UmmaSpec* u, int
                                                     : multiples(u->a, 0, of) && u->a.row_elem_cstride == 1 && u->a.split_inner % of == 0 && u->a.slab_mode_ext % of == 0;
             if (u->piece < of && rows && multiples(u->b, 0, of) && u->b.row_elem_cstride % of == 0) u->piece = of;
         }
-        u->slim = u->tiles_n == 1 && u->b.major == 0 && u->b.total_slabs * u->b.slab_w <= u->BN / 4 * 3 && !std::getenv("TCONT_NO_SLIM");
+        // (not where a C larger than L2 is stored in pieces of 64 bytes after a short main loop: there the stores bound the time, and they
+        //  go faster the slower they come, or with narrow tiles in place of 64 slim columns.  Slim and not, us: k chunks of 16,
+        //  16 x 48 x 24 x 24 x 48 by 48 101 / 94.4, 48 x 400 x 24 x 128 by 48 297 / 246, 24 x 400 x 24 x 128 by 32 117 / 99.4 (two groups), 16 x 64 x
+        //  32 x 48 x 72 by 16 392 / 298, 72 x 96 x 48 x 128 by 16 118 / 103.  Slim is better with a C of 126 MB, 48 x 32 x 16 x 20 x 32 by 48
+        //  73.7 / 83.3; on 24 columns by 16 168 / 170 (454 MB) and by 64 220 / 233 (340 MB); on 48 columns by 32 108 / 118 (315 MB); in k chunks of 8,
+        //  24 columns by 40 179 / 173 (340 MB) but 20 by 24 146 / 150 (283 MB); and where a fourth of the rows are padding, as with 24 rows in
+        //  slabs of 16, 48 x 32 x 72 x 20 x 24 by 48 275 / 343.  Reading the old values slim is better with three chunks of k, 48 x 400 x 24 x 128 by 48
+        //  318 / 346, but not with two, 48 x 32 x 32 x 24 x 48 by 32 309 / 286.)
+        const bool stores_bound = u->store_across_slabs && u->BK == 16 && double(p.sizeC) * 8.0 > 150e6 && u->a.total_slabs * u->a.slab_w * 3 < p.Mtot * 4 &&
+                                  (u->BN == 64 ? u->k_iters == 1 : u->k_iters == 2 || u->k_iters == 3);
+        const bool slim = u->tiles_n == 1 && u->b.major == 0 && u->b.total_slabs * u->b.slab_w <= u->BN / 4 * 3 && !std::getenv("TCONT_NO_SLIM");
+        u->slim[0] = slim && !stores_bound;
+        u->slim[1] = slim && !(stores_bound && (u->BN == 64 || u->k_iters != 3));
     }
     u->eligible = true;
 }
@@ -788,7 +800,7 @@ UmmaSpec narrow_tiles(const Problem& p, const CostTable& cost, const UmmaSpec& u
     const char* want = std::getenv("TCONT_DMMA_BN");   // tuning switch: 32 or 64 columns
     const bool short_k = u.k_computed <= (u.store_across_slabs ? 256 : u.BK == 8 ? 32 : 96) && !(u.a.major == 1 && u.a.slab_w == 8);
     UmmaSpec v;
-    const bool whole = !u.slim && ceil_div(u.b.total_slabs * u.b.slab_w, 32) * 32 <= u.tiles_n * 64;   // as many columns computed
+    const bool whole = !u.slim[0] && ceil_div(u.b.total_slabs * u.b.slab_w, 32) * 32 <= u.tiles_n * 64;   // as many columns computed
     if (u.BN != 64 || u.k_splits != 1 || !whole || !(want ? std::atoi(want) == 32 : short_k)) return v;
     plan_umma_impl(p, cost, &v, 32, true, true);
     if (v.k_splits != 1) v.eligible = false;
@@ -804,22 +816,25 @@ UmmaSpec narrow_tiles(const Problem& p, const CostTable& cost, const UmmaSpec& u
 //     values, in pieces of 8 bytes 402 / 300 and 819 / 707, in pieces of 16 555 / 769 (23 x 23 x 24 .. by 32, 25 x 16 .. by 17, 26 x 12 .. by 14)
 //   rows along C, one or two k chunks of 16: 127776 x 88 by 16 23.3 / 21.4, 105984 x 512 by 16 90.0 / 84.1, 78080 x 128 by 32 28.9 / 27.0
 //     (but 306904 x 16 by 16 16.5 / 17.4); more of them 67584 x 128 by 48 31.6 / 33.0
+//   across slabs the same in one column of tiles, with a C of twice L2 and more: 48 x 32 x 24 x 32 x 48 by 32 211 / 181 (453 MB); with a C of
+//     201 MB three are 9 % faster, with 637 MB on 20 columns by 16 3 %, on 48 columns (906 MB, by 32) 12 %
 // Elsewhere three: 24 x 42 x 1024 x 32 by 16 across slabs 52.7 / 62.4, 259056 x 32 by 24 accumulating 33.6 / 44.9, 64 x 236 x 1024 by 24
 // 33.5 / 37.4, and always where A's slabs and k chunks of 8 meet, whose loads the narrower warp tile repeats twice as often with
 // conflicts (72 x 48 x 16 x 16 by 960 70.8 / 105).
-void set_dmma_groups(UmmaSpec* u, const CostTable& cost)
+void set_dmma_groups(const Problem& p, UmmaSpec* u, const CostTable& cost)
 {
     const char* want = std::getenv("TCONT_DMMA_GROUPS");   // tuning switch: 2 or 3
     const bool slabs8 = u->a.major == 1 && u->a.slab_w == 8;
     const int64_t rounds = ceil_div(u->tiles_m * u->tiles_n * u->k_splits, cost.num_sms);
     for (int reads = 0; reads < 2; ++reads) {
         bool two = u->BN == 64;
-        if (!two && !u->slim && !(slabs8 && u->BK == 8)) {
+        if (!two && !u->slim[reads] && !(slabs8 && u->BK == 8)) {
             if (u->k_splits > 1 ? u->k_iters_per_split >= 12 : true) two = rounds <= 2 || rounds == 4;
             if (!u->store_across_slabs && u->piece < (reads ? 2 : 4)) two = true;
-            if (!u->store_across_slabs && !reads && u->k_splits == 1 && u->BK == 16 && u->k_iters <= 2) two = true;
+            if (!reads && u->k_splits == 1 && u->BK == 16 && u->k_iters <= 2)
+                two = two || !u->store_across_slabs || (u->tiles_n == 1 && double(p.sizeC) * 8.0 > 250e6);
         }
-        if (want && u->BN == 32 && !u->slim) two = std::atoi(want) == 2;
+        if (want && u->BN == 32 && !u->slim[reads]) two = std::atoi(want) == 2;
         u->groups[reads] = two ? 2 : 3;
     }
 }
@@ -847,7 +862,7 @@ double split_us(const Problem& p, const UmmaSpec& u, int64_t s, const CostTable&
     const int groups = narrow ? 3 : 2;
     const double c_mb = double(p.sizeC) * 8e-6, chunk = u.BK / 16.0, copies = double(u.a.slabs_per_tile) / u.a.slabs_per_op + double(u.b.slabs_per_tile) / u.b.slabs_per_op;
     const int64_t per = ceil_div(u.k_iters, s), units = ceil_div(u.tiles_m * u.tiles_n * ceil_div(u.k_iters, per), cost.num_sms);
-    const double pipe = double(units * per) * pipe_it * (u.slim ? 0.8 : 1.0) * chunk + store / groups;
+    const double pipe = double(units * per) * pipe_it * (u.slim[0] ? 0.8 : 1.0) * chunk + store / groups;
     const double chain = double(ceil_div(units, groups)) * (double(per) * std::max(chain_it * chunk, copy0 + copy1 * copies) + store);
     const double us = setup + std::max(pipe, chain) + (s > 1 ? sum0 + (sum1 * c_mb + 0.12) * double(s) : 0.0);
     return std::max(us, setup + (c_mb + (double(p.sizeA) + double(p.sizeB)) * 8e-6) / (narrow ? 4.93 : 4.54));
@@ -1623,7 +1638,7 @@ int make_plan(const char* modeC, int nC, const char* modeA, int nA, const char* 
     }
     pl.wide_reads = pl.kernel_without_narrow == KERNEL_DMMA_F64_TMA && wide_reads(p, pl.umma, pl.narrow) && !std::getenv("TCONT_DMMA_BN");
     for (UmmaSpec* u : {&pl.umma, &pl.narrow})
-        if (u->eligible && u->elt == 8) set_dmma_groups(u, cost);
+        if (u->eligible && u->elt == 8) set_dmma_groups(p, u, cost);
     if (pl.kernel == KERNEL_UMMA_TF32)
         for (int reads = 0; reads < 2; ++reads)
             pl.est_scaled_us[reads] = (use_ttgt ? ttgt_by_tiles_us : pl.est_direct_us) +
@@ -1707,7 +1722,7 @@ std::string describe_plan(const Plan& pl)
         o << ",\"across\":{\"BN\":" << pl.across.BN << ",\"BK\":" << pl.across.BK << ",\"stages\":" << pl.across.stages << ",\"tiles_m\":" << pl.across.tiles_m
           << ",\"tiles_n\":" << pl.across.tiles_n << ",\"k_iters\":" << pl.across.k_iters << ",\"b_major\":\"" << (pl.across.b_major ? "MN" : "K") << "\"}";
     if (pl.narrow.eligible)
-        o << ",\"narrow\":{\"BN\":" << pl.narrow.BN << ",\"BK\":" << pl.narrow.BK << ",\"stages\":" << pl.narrow.stages << ",\"slim\":" << (pl.narrow.slim ? "true" : "false") << ",\"tiles_m\":" << pl.narrow.tiles_m
+        o << ",\"narrow\":{\"BN\":" << pl.narrow.BN << ",\"BK\":" << pl.narrow.BK << ",\"stages\":" << pl.narrow.stages << ",\"slim\":" << (pl.narrow.slim[0] ? "true" : "false") << ",\"tiles_m\":" << pl.narrow.tiles_m
           << ",\"tiles_n\":" << pl.narrow.tiles_n << ",\"k_splits\":" << pl.narrow.k_splits << ",\"groups\":[" << pl.narrow.groups[0] << "," << pl.narrow.groups[1] << "],\"wide_reads\":" << (pl.wide_reads ? "true" : "false") << ",\"instead_of\":\"" << kernel_name(pl.kernel_without_narrow) << "\"}";
     o << ",\"umma\":{\"eligible\":" << (u.eligible ? "true" : "false");
     if (!u.eligible) o << ",\"why_not\":\"" << u.why_not << "\"";
@@ -1719,7 +1734,7 @@ std::string describe_plan(const Plan& pl)
           << ",\"a_slab_w\":" << u.a.slab_w << ",\"b_slab_w\":" << u.b.slab_w << ",\"a_slabs_per_copy\":" << u.a.slabs_per_op << ",\"b_slabs_per_copy\":" << u.b.slabs_per_op << ",\"a_slabs\":" << u.a.slabs_per_tile
           << ",\"b_slabs\":" << u.b.slabs_per_tile << ",\"smem_bytes\":" << u.smem_bytes
           << ",\"coalesced_store\":" << (u.a.row_elem_cstride == 1 ? "true" : "false")
-          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"slim\":" << (u.slim ? "true" : "false") << ",\"piece\":" << u.piece << ",\"groups\":[" << u.groups[0] << "," << u.groups[1] << "],\"producers\":" << u.producers
+          << ",\"store_across_slabs\":" << (u.store_across_slabs ? "true" : "false") << ",\"slim\":" << (u.slim[0] ? "true" : "false") << ",\"slim_reads\":" << (u.slim[1] ? "true" : "false") << ",\"piece\":" << u.piece << ",\"groups\":[" << u.groups[0] << "," << u.groups[1] << "],\"producers\":" << u.producers
           << ",\"a_fused\":" << u.a.split_inner << ",\"b_fused\":" << u.b.split_inner << ",\"column_ranges\":[";
         std::string why;
         for (int r = 2, n = 0; r <= 8; ++r)

@@ -115,8 +115,8 @@ struct UmmaSpec {
     // beyond it, and start on a multiple of so many elements from C's first
     int piece = 1;
     // FP64 kernel: one column of tiles, of which at most three quarters are columns of C (B K-major): a warp computes three column
-    // fragments instead of four
-    bool slim = false;
+    // fragments instead of four.  Where the old values of C are not read, and where they are
+    bool slim[2] = {false, false};
     // FP64 kernel: consumer groups of a block where the old values of C are not read, and where they are
     int groups[2] = {2, 2};
     int smem_bytes = 0;

@@ -191,3 +191,22 @@ def test_wide_tiles_where_old_values_are_read(engine, oracle, A_, B_):
         bound = (72 + 4) * 2.0**-53 * (abs(alpha) * scale + abs(beta * C0[at]))
         assert (np.abs(out[at] - (alpha * product + beta * C0[at])) <= bound).all(), (alpha, beta)
     assert (got[0] == got[4]).all()
+
+
+@pytest.mark.parametrize("extents,k,forms", [(dict(a=48, b=96, c=24, d=192), 48, (False, True)), (dict(a=40, b=132, c=22, d=288), 32, (False, False))])
+def test_slim_where_old_values_are_read(engine, oracle, extents, k, forms):
+    """Across slabs, C of 170 and 268 MB: three column fragments a warp in accumulating launches only, and two consumer groups in plain ones only."""
+    c = Contraction("abcd", "dbka", "kc", dict(extents, k=k), F64)
+    A, B = oracle.inputs(c, 59, -1.0, 1.0)
+    C0 = np.random.default_rng(14).uniform(-4.0, 4.0, c.size("abcd"))
+    scalars = [(1.0, 1.0), (1.0, 0.0), (0.3, -0.7), (-0.75, 0.0), (1.0, 1.0)]
+    desc, got = scaled_run(engine, c, A, B, C0, scalars)
+    u = desc["umma"]
+    assert desc["kernel"] == "dmma_f64_tma" and u["in_use"] and (u["slim"], u["slim_reads"]) == forms
+    assert u["groups"] == ([3, 3] if k == 48 else [2, 3])
+    at = np.sort(np.random.default_rng(15).integers(0, C0.size, 20000))
+    product, scale = oracle.contract_sampled(c, A, B, at), oracle.contract_sampled(c, np.abs(A), np.abs(B), at)
+    for (alpha, beta), out in zip(scalars, got):
+        bound = (k + 4) * 2.0**-53 * (abs(alpha) * scale + abs(beta * C0[at]))
+        assert (np.abs(out[at] - (alpha * product + beta * C0[at])) <= bound).all(), (alpha, beta)
+    assert (got[0] == got[4]).all()

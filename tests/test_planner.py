@@ -384,7 +384,7 @@ def test_fp64_ranges_where_slabs_and_k_chunks_of_8_meet(engine):
 
 def test_fp64_consumer_groups(engine, monkeypatch):
     """Two consumer groups on 128 x 32 tiles: where three would not spare a round of them, for pieces of 8 or 16 bytes, and for one or two
-    k chunks of 16 along C; three where old values are read in wider pieces, across slabs, and where A's slabs and k chunks of 8 meet."""
+    k chunks of 16 along C, or across slabs into one column of a C of more than 250 MB; three where old values are read in wider pieces, across slabs, and where A's slabs and k chunks of 8 meet."""
     F64 = 1
 
     def groups(C, A, B, **ext):
@@ -404,8 +404,33 @@ def test_fp64_consumer_groups(engine, monkeypatch):
     assert groups("abc", "akb", "kc", a=24, b=740, c=32, k=24) == (32, 3, 3) and groups("abc", "akb", "kc", a=24, b=740, c=32, k=48) == (32, 2, 2)
     assert groups("ab", "ak", "kb", a=9216, b=24, k=96) == (32, 3, 3)              # three column fragments a warp
     assert groups("ab", "ak", "kb", a=9216, b=4096, k=200) == (64, 2, 2)
+    long = dict(a=48, b=32, c=24, d=32, e=48)                                      # across slabs, C of 453 MB
+    for k, plain in ((16, 2), (32, 2), (24, 3), (48, 3)):
+        assert groups("abcde", "ekbad", "ck", k=k, **dict(long, c=28, a=40)) == (32, plain, 3), k
+    assert groups("abcde", "ekbad", "ck", k=32, **dict(long, b=16)) == (32, 3, 3)  # of 226 MB
+    assert groups("abcde", "ekbad", "ck", k=32, **dict(long, c=48)) == (32, 3, 3)  # two columns of tiles
     monkeypatch.setenv("TCONT_DMMA_GROUPS", "3")
     assert groups("ab", "ak", "kb", a=9216, b=4096, k=32) == (32, 3, 3)
+
+
+def test_fp64_slim_across_slabs(engine):
+    """Three column fragments a warp: not across slabs where a C of more than 150 MB is stored after one, two or three k chunks of 16."""
+    F64 = 1
+
+    def slim(**ext):
+        d = describe(engine, Contraction("abcd", "dbka", "kc", dict(dict(a=48, b=96, c=24, d=192), **ext), F64), 1)
+        u = d.get("narrow", d["umma"])
+        assert d["kernel"] == "dmma_f64_tma" and d["umma"]["store_across_slabs"] and d["umma"]["in_use"] == ("narrow" not in d)
+        if "narrow" not in d:
+            assert u["slim_reads"] == (u["slim"] or ext["k"] == 48)                # accumulating launches keep it with three k chunks
+        return u["BN"], u["slim"], u["groups"][0]
+    for k in (16, 24, 32, 40, 48, 64):
+        assert slim(k=k) == (32, k not in (32, 48), 3), k                          # 170 MB
+        assert slim(k=k, b=64) == (32, True, 3), k                                 # 113 MB
+    assert slim(k=32, b=192) == (32, False, 2) and slim(k=48, b=192) == (32, False, 3)
+    assert slim(k=48, d=24, b=800) == (32, True, 3)                                # a fourth of the rows of its tiles is padding
+    assert slim(k=16, c=48) == (32, False, 3) and slim(k=16, c=48, b=32) == (64, True, 2)
+    assert slim(k=24, c=48) == (64, True, 2) and slim(k=32, c=48) == (64, True, 2)
 
 
 def test_fp64_wide_tiles_where_old_values_are_read(engine, monkeypatch):
