@@ -7,7 +7,7 @@
 //
 // One block per SM.  128 x 64 tiles: three warpgroups, two of them consumer groups of 2 x 2 warps with a 64 x 32 warp tile.  128 x 32
 // tiles (narrow N, and short contracted extents: narrow_tiles in planner.cpp): the same with a 64 x 16 warp tile, or four warpgroups,
-// three of them consumer groups of 4 x 1 warps with a 32 x 32 warp tile (dmma_groups in planner.cpp has the choice and its figures).
+// three of them consumer groups of 4 x 1 warps with a 32 x 32 warp tile (set_dmma_groups in planner.cpp has the choice and its figures).
 // G consumer groups take every G-th tile of the block; setmaxnreg moves registers from the first warpgroup to them (72 and 216 a
 // thread with two of them, 56 and 152 with three).
 //   warps 0 .. G-1    producers, one per consumer group: lane i issues copy i of a stage (5-D tensor
